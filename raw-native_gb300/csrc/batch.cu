@@ -56,8 +56,8 @@ __global__ void __launch_bounds__(256, kMinBlocks) trace_batch_kernel(const Batc
     for (int v = threadIdx.x; v < nviews; v += blockDim.x) { sp[v] = views[v].tp; begins[v] = views[v].tile_begin; }
     __syncthreads();
     const unsigned lane = threadIdx.x & 31u;
-    __shared__ trace_dev::FrontierEntry frontier[8][trace_dev::kFrontier];
-    trace_dev::FrontierEntry* F = frontier[threadIdx.x >> 5];
+    __shared__ Node4 frontier[8][trace_dev::kFrontierNodes];
+    Node4* F = frontier[threadIdx.x >> 5];
     Counts cn;
     while (true) {
         uint32_t tile = 0;

@@ -963,7 +963,7 @@ __device__ __forceinline__ void collapse_tasks(const Task* in, uint32_t m, uint3
         for (int k = 0; k < 4; ++k) {
             nd.lox[k] = nd.loy[k] = nd.loz[k] = 1e30f;
             nd.hix[k] = nd.hiy[k] = nd.hiz[k] = -1e30f;
-            nd.child[k] = 0;
+            nd.child[k] = kNoChild;
             nd.meta[k] = 0;
         }
         nd.meta[0] = nc;

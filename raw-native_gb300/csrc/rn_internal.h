@@ -156,6 +156,8 @@ struct alignas(16) Node4 {
     int32_t meta[4];   // meta[0] = number of valid children
 };
 static_assert(sizeof(Node4) == 128, "Node4 layout");
+// The child word of an unused slot, whose box is inverted: no leaf has it (first < 2^28 - 1).
+constexpr int32_t kNoChild = INT32_MIN;
 constexpr int kLeafCap = 8;   // triangles a leaf may hold (the child word's 3-bit count)
 
 // A leaf triangle: vertices a, b, c as float4 (w of a = input triangle index).

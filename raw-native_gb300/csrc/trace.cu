@@ -31,15 +31,15 @@ using namespace trace_dev;
 // fetches to counts[0..3] (hemisphere rays, nodes, tris, sky continuations); the outputs of
 // the other tiles are left unwritten. "Sky continuations" are the open hemisphere rays whose
 // walk went on past the radius: the same walk serves both queries.
-template <bool kCount, int kMinBlocks, int kStackN, bool kLeafPass = false>
+template <bool kCount, int kMinBlocks, int kStackN, bool kLeafPass>
 __global__ void __launch_bounds__(256, kMinBlocks) trace_kernel(const __grid_constant__ TraceParams p, uint32_t* tile_ctr,
                                                                 unsigned long long* counts, uint32_t stride) {
     const int pl = p.packet_log2, tw = 1 << pl, th = 32 >> pl;
     const int tiles_x = (p.w + tw - 1) >> pl, tiles_y = (p.h + th - 1) / th;
     const uint32_t ntiles = (uint32_t)tiles_x * tiles_y;
     const unsigned lane = threadIdx.x & 31u;
-    __shared__ FrontierEntry frontier[8][kFrontier];
-    FrontierEntry* F = frontier[threadIdx.x >> 5];
+    __shared__ Node4 frontier[8][kFrontierNodes];
+    Node4* F = frontier[threadIdx.x >> 5];
     Counts cn;
     // lighting model 2's sun direction, normalized on the device as computeRTVisibility does
     const v3 toLight = normalize(mk(p.lx, p.ly, p.lz));
@@ -86,14 +86,14 @@ __global__ void __launch_bounds__(256, kMinBlocks) trace_ao_pool_kernel(const __
     const uint32_t ntiles = (uint32_t)tiles_x * tiles_y;
     const unsigned lane = threadIdx.x & 31u;
     const unsigned below = (1u << lane) - 1u;
-    __shared__ FrontierEntry frontier[8][kFrontier];
+    __shared__ Node4 frontier[8][kFrontierNodes];
     __shared__ int open_sh[8][32];
     __shared__ uint8_t lane_sh[8][32];
     __shared__ uint16_t perm_sh[8][32 * kSortSpp];
     __shared__ uint32_t oct_sh[8][8];
     uint16_t* perm = perm_sh[threadIdx.x >> 5];
     uint32_t* octs = oct_sh[threadIdx.x >> 5];
-    FrontierEntry* F = frontier[threadIdx.x >> 5];
+    Node4* F = frontier[threadIdx.x >> 5];
     int* opens = open_sh[threadIdx.x >> 5];
     uint8_t* lane_of = lane_sh[threadIdx.x >> 5];   // the covered lanes in lane order
     const size_t np = (size_t)p.w * p.h;
@@ -223,10 +223,9 @@ __global__ void __launch_bounds__(256, kMinBlocks) trace_ao_pool_kernel(const __
                         bool hit = false;
                         for (int e = 0; e < fn && !hit; ++e) {
                             float tn;
-                            if (!slab(F[e].lo[0], F[e].hi[0], F[e].lo[1], F[e].hi[1], F[e].lo[2], F[e].hi[2], o, iv,
-                                      tmax, tn))
-                                continue;
-                            const int32_t c = F[e].word;
+                            const FrontierBox fb = frontier_get(F, e);
+                            if (!slab(fb.lo[0], fb.hi[0], fb.lo[1], fb.hi[1], fb.lo[2], fb.hi[2], iv, tmax, tn)) continue;
+                            const int32_t c = fb.word;
                             if (c < 0) {
                                 if (!wr_ready) { wr = make_wray(o, d); wr_ready = true; }
                                 const uint32_t w = (uint32_t)~c;
@@ -274,7 +273,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) trace_ao_pool_kernel(const __
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 float tn;
-                if (hit || k >= cnt || !slab(LX[k], HX[k], LY[k], HY[k], LZ[k], HZ[k], o, iv, tmax, tn)) continue;
+                if (hit || k >= cnt || !slab(LX[k], HX[k], LY[k], HY[k], LZ[k], HZ[k], iv, tmax, tn)) continue;
                 const int32_t c = CH[k];
                 if (c < 0) {
                     if (!wr_ready) { wr = make_wray(o, d); wr_ready = true; }
@@ -382,13 +381,13 @@ void launch_variant(const TraceParams& p, int sm_count, cudaStream_t s, uint32_t
     const int blocks = sm_count * kMB;
     const int pool = ctx().tune.trace_pool;
     if (counts)
-        trace_kernel<true, kMB, kStack><<<blocks, 256, 0, s>>>(p, tile_ctr, counts, stride < 1 ? 1 : stride);
+        trace_kernel<true, kMB, kStack, false><<<blocks, 256, 0, s>>>(p, tile_ctr, counts, stride < 1 ? 1 : stride);
     else if (pool > 0 && !p.want_sky)
         trace_ao_pool_kernel<kMB, kStackN><<<blocks, 256, 0, s>>>(p, tile_ctr, pool, ctx().tune.trace_pool_sort);
     else if (ctx().tune.trace_leaf_pass)
         trace_kernel<false, kMB, kStackN, true><<<blocks, 256, 0, s>>>(p, tile_ctr, nullptr, 1);
     else
-        trace_kernel<false, kMB, kStackN><<<blocks, 256, 0, s>>>(p, tile_ctr, nullptr, 1);
+        trace_kernel<false, kMB, kStackN, false><<<blocks, 256, 0, s>>>(p, tile_ctr, nullptr, 1);
 }
 
 template <int kStackN>

@@ -13,55 +13,98 @@ constexpr int kStack = 96;
 constexpr uint32_t kGuard = 1u << 24;       // node visits per ray before giving up
 constexpr int kTileW = 8, kTileH = 4;
 
-__device__ __forceinline__ float min_nan(float a, float b) {
-    float r;
-    asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ float max_nan(float a, float b) {
-    float r;
-    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
-    return r;
-}
-// inverse(d) of src/renderer/bvh.cpp:29-33: 1/x, or a signed infinity for a zero component.
+// inverse(d) of src/renderer/bvh.cpp:29-33: 1/x, a signed infinity for a zero component.
 // The slab tests only prune, so 1/x need not be correctly rounded: the hardware reciprocal
-// (rcp.approx, at most 1 ulp off) scales each axis's plane distances by at most 1 +- 2^-23,
-// and a box the ray truly enters then still passes t0 <= t1 x (1 + 2^-22 or so), inside the
-// test's exit widening of 1.0000008 (about 1 + 2^-20.2).
-__device__ __forceinline__ float rcp_fast(float x) {
+// (rcp.approx, at most 1 ulp off; a signed zero gives its signed infinity) scales each axis's
+// plane distances by at most 1 +- 2^-23, and a box the ray truly enters then still passes
+// t0 <= t1 x (1 + 2^-22 or so), inside the test's exit widening of 1.0000008 (about
+// 1 + 2^-20.2). A component below 1e-28 that is not zero gives NaN, so that its axis
+// constrains nothing: with its reciprocal one of plane * inv and o * inv could overflow alone
+// and cull a box that the ray enters.
+__device__ __forceinline__ float safe_inv(float x) {
     float r;
     asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return r;
+    return fabsf(x) < 1e-28f && x != 0.0f ? __int_as_float(0x7fffffff) : r;
 }
-__device__ __forceinline__ float safe_inv(float x) { return x != 0.0f ? rcp_fast(x) : copysignf(__int_as_float(0x7f800000), x); }
 
-// The ray's inverse direction and origin x inverse direction, formed once per walk.
-struct Inv { float x, y, z, ox, oy, oz; };
+// The ray's inverse direction, origin x inverse direction, and the byte offset of each axis's
+// near plane in a node (nx, ny, nz: the lo plane for a direction that is not negative, else
+// the hi plane 16 bytes further; the far plane sits at the other of the two), formed once
+// per walk.
+struct Inv { float x, y, z, ox, oy, oz; uint32_t nx, ny, nz; };
 __device__ __forceinline__ Inv make_inv(const v3& o, const v3& d) {
     Inv r;
     r.x = safe_inv(d.x); r.y = safe_inv(d.y); r.z = safe_inv(d.z);
     r.ox = o.x * r.x; r.oy = o.y * r.y; r.oz = o.z * r.z;
+    r.nx = (__float_as_uint(r.x) >> 31) * 16u;
+    r.ny = 32u + (__float_as_uint(r.y) >> 31) * 16u;
+    r.nz = 64u + (__float_as_uint(r.z) >> 31) * 16u;
     return r;
 }
 
-// Slab entry of one child box, each plane distance as one fused multiply-add,
-// lo * inv - o * inv. The BVH only prunes, so the test has to be conservative, not exact:
-// against (lo - o) * inv the fused form is off by at most about 2^-24 |o| in position, far
-// inside the child boxes' outward padding (2^-19 of the coordinate plus 1e-6 of the
-// extent), so no box a triangle hit lies in is culled. An axis whose distances are NaN
-// (origin on the plane, zero or vanishing direction component) constrains nothing, as in
-// the reference's entry(); that only keeps more boxes.
-__device__ __forceinline__ bool slab(float lox, float hix, float loy, float hiy, float loz, float hiz,
-                                     const v3& o, const Inv& iv, float tmax, float& tnear) {
-    (void)o;
-    const float ax = __fmaf_rn(lox, iv.x, -iv.ox), bx = __fmaf_rn(hix, iv.x, -iv.ox);
-    const float ay = __fmaf_rn(loy, iv.y, -iv.oy), by = __fmaf_rn(hiy, iv.y, -iv.oy);
-    const float az = __fmaf_rn(loz, iv.z, -iv.oz), bz = __fmaf_rn(hiz, iv.z, -iv.oz);
-    const float t0 = fmaxf(fmaxf(fmaxf(0.0f, min_nan(ax, bx)), min_nan(ay, by)), min_nan(az, bz));
-    const float t1 = fminf(fminf(fminf(tmax, max_nan(ax, bx)), max_nan(ay, by)), max_nan(az, bz));
+// Three-input maximum and minimum (one instruction each on sm_100 and later); a NaN operand
+// is left out, as fmaxf and fminf leave it out.
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+__device__ __forceinline__ float min3(float a, float b, float c) {
+    float r;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+
+// Slab test of one box from its near and far planes along the ray (near = lo where the
+// direction is positive, hi where it is negative), each plane distance as one fused
+// multiply-add, plane * inv - o * inv. The BVH only prunes, so the test has to be
+// conservative, not exact: against (plane - o) * inv the fused form is off by at most about
+// 2^-24 |o| in position, far inside the child boxes' outward padding (2^-19 of the coordinate
+// plus 1e-6 of the extent), so no box a triangle hit lies in is culled. A rounded product is
+// monotonic in the plane, so picking the planes by the direction's sign gives the values that
+// the smaller and larger of the two distances had. A plane whose distance is NaN (origin on
+// the plane, zero or vanishing direction component) constrains nothing; its partner along the
+// same zero direction is NaN too, or an infinity of the sign that says on which side of the
+// slab the whole ray lies.
+__device__ __forceinline__ bool slab_nf(float nx, float fx, float ny, float fy, float nz, float fz, const Inv& iv,
+                                        float tmax, float& tnear) {
+    const float ax = __fmaf_rn(nx, iv.x, -iv.ox), bx = __fmaf_rn(fx, iv.x, -iv.ox);
+    const float ay = __fmaf_rn(ny, iv.y, -iv.oy), by = __fmaf_rn(fy, iv.y, -iv.oy);
+    const float az = __fmaf_rn(nz, iv.z, -iv.oz), bz = __fmaf_rn(fz, iv.z, -iv.oz);
+    const float t0 = max3(ax, ay, fmaxf(az, 0.0f)), t1 = min3(bx, by, fminf(bz, tmax));
     tnear = t0;
     return t0 <= t1 * 1.0000008f;
 }
+__device__ __forceinline__ bool slab(float lox, float hix, float loy, float hiy, float loz, float hiz, const Inv& iv,
+                                     float tmax, float& tnear) {
+    return slab_nf(iv.nx & 16u ? hix : lox, iv.nx & 16u ? lox : hix, iv.ny & 16u ? hiy : loy, iv.ny & 16u ? loy : hiy,
+                   iv.nz & 16u ? hiz : loz, iv.nz & 16u ? loz : hiz, iv, tmax, tnear);
+}
+
+// The four slab tests of a node: its planes are read near and far by address (no select, no
+// minimum or maximum of a plane pair), so a child costs six multiply-adds, four three-input
+// minima and maxima, one multiply and one compare. hit[k] also says that child k exists: an
+// unused slot holds an inverted box, which only a ray without a finite direction component
+// can pass, and the child word kNoChild.
+template <typename L>
+__device__ __forceinline__ void node_test(const char* node, L ld, const Inv& iv, float tmax, int32_t (&CH)[4],
+                                          float (&tn)[4], bool (&hit)[4]) {
+    const float4 nx = ld(node + iv.nx), fx = ld(node + (iv.nx ^ 16u));
+    const float4 ny = ld(node + iv.ny), fy = ld(node + (iv.ny ^ 16u));
+    const float4 nz = ld(node + iv.nz), fz = ld(node + (iv.nz ^ 16u));
+    const float4 ch = ld(node + 96);
+    hit[0] = slab_nf(nx.x, fx.x, ny.x, fy.x, nz.x, fz.x, iv, tmax, tn[0]);
+    hit[1] = slab_nf(nx.y, fx.y, ny.y, fy.y, nz.y, fz.y, iv, tmax, tn[1]);
+    hit[2] = slab_nf(nx.z, fx.z, ny.z, fy.z, nz.z, fz.z, iv, tmax, tn[2]);
+    hit[3] = slab_nf(nx.w, fx.w, ny.w, fy.w, nz.w, fz.w, iv, tmax, tn[3]);
+    CH[0] = __float_as_int(ch.x); CH[1] = __float_as_int(ch.y); CH[2] = __float_as_int(ch.z); CH[3] = __float_as_int(ch.w);
+}
+struct LdGlobal {
+    __device__ __forceinline__ float4 operator()(const char* p) const { return __ldg(reinterpret_cast<const float4*>(p)); }
+};
+struct LdShared {
+    __device__ __forceinline__ float4 operator()(const char* p) const { return *reinterpret_cast<const float4*>(p); }
+};
 
 // Per-thread traversal counters (the measurement build; compiled out otherwise).
 struct Counts { unsigned long long rays = 0, nodes = 0, tris = 0, sky = 0; };
@@ -74,12 +117,25 @@ enum : int { HIT_NEAR = 1, HIT_FAR = 2 };
 // the tile's origins grown by the radius; the frontier is the set of Q-overlapping nodes
 // reached by expanding Q-overlapping nodes from the root, level by level, while at most
 // kFrontier entries result. AO walks start from it instead of re-descending from the root.
-constexpr int kFrontier = 16;
-struct FrontierEntry {
-    float lo[3], hi[3];
-    int32_t word;
-    int32_t pad;
-};
+// The entries are kept in the node layout, four to a group: a walk tests a group exactly as
+// it tests a node.
+constexpr int kFrontier = 16, kFrontierNodes = kFrontier / 4;
+struct FrontierBox { float lo[3], hi[3]; int32_t word; };
+__device__ __forceinline__ void frontier_put(Node4* F, int e, const FrontierBox& b) {
+    Node4& n = F[e >> 2];
+    const int k = e & 3;
+    n.lox[k] = b.lo[0]; n.loy[k] = b.lo[1]; n.loz[k] = b.lo[2];
+    n.hix[k] = b.hi[0]; n.hiy[k] = b.hi[1]; n.hiz[k] = b.hi[2];
+    n.child[k] = b.word;
+}
+__device__ __forceinline__ FrontierBox frontier_get(const Node4* F, int e) {
+    const Node4& n = F[e >> 2];
+    const int k = e & 3;
+    return FrontierBox{{n.lox[k], n.loy[k], n.loz[k]}, {n.hix[k], n.hiy[k], n.hiz[k]}, n.child[k]};
+}
+__device__ __forceinline__ FrontierBox frontier_child(const Node4* N, int k) {
+    return FrontierBox{{N->lox[k], N->loy[k], N->loz[k]}, {N->hix[k], N->hiy[k], N->hiz[k]}, N->child[k]};
+}
 
 __device__ __forceinline__ bool box_overlaps(float lx, float ly, float lz, float hx, float hy, float hz,
                                              const float* qlo, const float* qhi) {
@@ -94,7 +150,7 @@ __device__ __forceinline__ bool box_overlaps(float lx, float ly, float lz, float
 // so the build takes about the tree's depth in fetch latencies. Up to `tail` greedy steps
 // follow, each replacing the largest interior entry by its children while the frontier fits.
 __device__ inline int build_frontier(const Node4* __restrict__ nodes, const float* qlo, const float* qhi,
-                                     FrontierEntry* F, int tail) {
+                                     Node4* F, int tail) {
     const int lane = (int)(threadIdx.x & 31u);
     int32_t word = 0;                       // lane 0 starts with the root node
     float lo[3] = {0.0f, 0.0f, 0.0f}, hi[3] = {0.0f, 0.0f, 0.0f};
@@ -120,27 +176,15 @@ __device__ inline int build_frontier(const Node4* __restrict__ nodes, const floa
         int pos = incl - c;
         if (inner) {
             for (int k = 0; k < 4; ++k)
-                if (hit & (1u << k)) {
-                    FrontierEntry e;
-                    e.lo[0] = N->lox[k]; e.lo[1] = N->loy[k]; e.lo[2] = N->loz[k];
-                    e.hi[0] = N->hix[k]; e.hi[1] = N->hiy[k]; e.hi[2] = N->hiz[k];
-                    e.word = N->child[k];
-                    e.pad = 0;
-                    F[pos++] = e;
-                }
+                if (hit & (1u << k)) frontier_put(F, pos++, frontier_child(N, k));
         } else if (mine) {
-            FrontierEntry e;
-            e.lo[0] = lo[0]; e.lo[1] = lo[1]; e.lo[2] = lo[2];
-            e.hi[0] = hi[0]; e.hi[1] = hi[1]; e.hi[2] = hi[2];
-            e.word = word;
-            e.pad = 0;
-            F[pos] = e;
+            frontier_put(F, pos, FrontierBox{{lo[0], lo[1], lo[2]}, {hi[0], hi[1], hi[2]}, word});
         }
         __syncwarp();
         n = total;
         built = 1;
         if (lane < n) {
-            const FrontierEntry& e = F[lane];
+            const FrontierBox e = frontier_get(F, lane);
             lo[0] = e.lo[0]; lo[1] = e.lo[1]; lo[2] = e.lo[2];
             hi[0] = e.hi[0]; hi[1] = e.hi[1]; hi[2] = e.hi[2];
             word = e.word;
@@ -170,27 +214,25 @@ __device__ inline int build_frontier(const Node4* __restrict__ nodes, const floa
             // the children replace entry bl and append after the last entry; none: the last
             // entry moves into slot bl
             int pos = bl;
-            if (c == 0 && bl != n - 1) F[bl] = F[n - 1];
+            if (c == 0 && bl != n - 1) frontier_put(F, bl, frontier_get(F, n - 1));
             for (int k = 0; k < 4; ++k)
                 if (hit & (1u << k)) {
-                    FrontierEntry e;
-                    e.lo[0] = N->lox[k]; e.lo[1] = N->loy[k]; e.lo[2] = N->loz[k];
-                    e.hi[0] = N->hix[k]; e.hi[1] = N->hiy[k]; e.hi[2] = N->hiz[k];
-                    e.word = N->child[k];
-                    e.pad = 0;
-                    F[pos] = e;
+                    frontier_put(F, pos, frontier_child(N, k));
                     pos = pos == bl ? n : pos + 1;
                 }
         }
         __syncwarp();
         n = n - 1 + c;
         if (lane < n) {
-            const FrontierEntry& e = F[lane];
+            const FrontierBox e = frontier_get(F, lane);
             lo[0] = e.lo[0]; lo[1] = e.lo[1]; lo[2] = e.lo[2];
             hi[0] = e.hi[0]; hi[1] = e.hi[1]; hi[2] = e.hi[2];
             word = e.word;
         }
     }
+    // the last group's unused slots: boxes no ray passes
+    if (built && lane >= n && lane < ((n + 3) & ~3))
+        frontier_put(F, lane, FrontierBox{{1e30f, 1e30f, 1e30f}, {-1e30f, -1e30f, -1e30f}, kNoChild});
     return built ? n : 0;
 }
 
@@ -203,10 +245,9 @@ __device__ inline int build_frontier(const Node4* __restrict__ nodes, const floa
 // together, and the triangle test exists once in the code instead of once per position).
 // Either order finds the same answers: boxes are only culled against tmax >= tnear, and a
 // far hit only lowers tmax to tnear.
-template <bool kCount, int kStackN = kStack, bool kLeafPass = false>
+template <bool kCount, int kStackN = kStack, bool kLeafPass = true>
 __device__ int walk(const Node4* __restrict__ nodes, const LeafTri* __restrict__ tris, const v3& o, const v3& d,
-                    float tnear, float tfar, uint32_t* err, Counts& cn, const FrontierEntry* F = nullptr,
-                    int fn = 0) {
+                    float tnear, float tfar, uint32_t* err, Counts& cn, const Node4* F = nullptr, int fn = 0) {
     const Inv iv = make_inv(o, d);
     WRay wr;                             // the watertight set-up: formed at the first leaf
     bool wr_ready = false;
@@ -215,33 +256,63 @@ __device__ int walk(const Node4* __restrict__ nodes, const LeafTri* __restrict__
     int32_t stack[kStackN];
     int sp = 0;
     int32_t cur = 0;                     // the root is always node 0
+    // the triangles of leaf word c: true when one is hit nearer than tnear (the walk ends)
+    auto leaf = [&](int32_t c) -> bool {
+        if (c == kNoChild) return false;
+        if (!wr_ready) { wr = make_wray(o, d); wr_ready = true; }
+        const uint32_t w = (uint32_t)~c;
+        const uint32_t first = w >> 3, count = (w & 7u) + 1u;
+        for (uint32_t i = 0; i < count; ++i) {
+            if (kCount) ++cn.tris;
+            const float4* tq = reinterpret_cast<const float4*>(tris + first + i);
+            const float4 A = __ldg(tq), B = __ldg(tq + 1), C = __ldg(tq + 2);
+            float t;
+            if (!hit_tri(wr, mk(A.x, A.y, A.z), mk(B.x, B.y, B.z), mk(C.x, C.y, C.z), t)) continue;
+            if (t < tnear) return true;
+            if (t < tmax) { far_hit = HIT_FAR; tmax = tnear; }
+        }
+        return false;
+    };
+    // The children that passed node_test: leaves are tested (true: one is hit nearer than tnear,
+    // the walk ends), the nearest interior child so far stays in `nearest`, the others are
+    // stacked. Written without branches up to the leaves, so a warp's lanes stay together
+    // whatever mix of children each of them hit.
+    int32_t nearest;
+    float tbest;
+    auto visit = [&](const int32_t (&CH)[4], const float (&tn)[4], const bool (&hit)[4]) -> bool {
+        unsigned leaves = 0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int32_t c = CH[k];
+            const bool in = hit[k] && c >= 0;
+            if (hit[k] && c < 0) {
+                if (kLeafPass) leaves |= 1u << k;
+                else if (leaf(c)) return true;
+            }
+            const bool closer = in && tn[k] < tbest;
+            const int32_t push = closer ? nearest : c;
+            if (in && nearest >= 0) stack[sp++] = push;
+            nearest = closer ? c : nearest;
+            tbest = closer ? tn[k] : tbest;
+        }
+        if (kLeafPass)
+            while (leaves) {
+                const int k = __ffs(leaves) - 1;
+                leaves &= leaves - 1u;
+                if (leaf(k == 0 ? CH[0] : k == 1 ? CH[1] : k == 2 ? CH[2] : CH[3])) return true;
+            }
+        return false;
+    };
     if (fn > 0) {
         // start from the frontier: its entries are the root's stand-ins
-        int32_t nearest = -1;
-        float tbest = 3.0e38f;
-        for (int e = 0; e < fn; ++e) {
-            float tn;
-            if (!slab(F[e].lo[0], F[e].hi[0], F[e].lo[1], F[e].hi[1], F[e].lo[2], F[e].hi[2], o, iv, tmax, tn)) continue;
-            const int32_t c = F[e].word;
-            if (c < 0) {
-                if (!wr_ready) { wr = make_wray(o, d); wr_ready = true; }
-                const uint32_t w = (uint32_t)~c;
-                const uint32_t first = w >> 3, count = (w & 7u) + 1u;
-                for (uint32_t i = 0; i < count; ++i) {
-                    if (kCount) ++cn.tris;
-                    const float4* tq = reinterpret_cast<const float4*>(tris + first + i);
-                    const float4 A = __ldg(tq), B = __ldg(tq + 1), C = __ldg(tq + 2);
-                    float t;
-                    if (!hit_tri(wr, mk(A.x, A.y, A.z), mk(B.x, B.y, B.z), mk(C.x, C.y, C.z), t)) continue;
-                    if (t < tnear) return HIT_NEAR | HIT_FAR;
-                    if (t < tmax) { far_hit = HIT_FAR; tmax = tnear; }
-                }
-                continue;
-            }
-            if (nearest < 0) { nearest = c; tbest = tn; continue; }
-            int32_t push = c;
-            if (tn < tbest) { push = nearest; nearest = c; tbest = tn; }
-            stack[sp++] = push;                  // fn <= kFrontier < kStackN
+        nearest = -1;
+        tbest = 3.0e38f;
+        for (int g = 0; 4 * g < fn; ++g) {            // at most kFrontier - 1 < kStackN entries stacked
+            float tn[4];
+            bool hit[4];
+            int32_t CH[4];
+            node_test(reinterpret_cast<const char*>(F + g), LdShared(), iv, tmax, CH, tn, hit);
+            if (visit(CH, tn, hit)) return HIT_NEAR | HIT_FAR;
         }
         if (nearest >= 0) cur = nearest;
         else if (sp > 0) cur = stack[--sp];
@@ -249,65 +320,16 @@ __device__ int walk(const Node4* __restrict__ nodes, const LeafTri* __restrict__
     }
     for (uint32_t guard = 0; guard < kGuard; ++guard) {
         if (kCount) ++cn.nodes;
-        const float4* q = reinterpret_cast<const float4*>(nodes + cur);
-        const float4 lx = __ldg(q + 0), hx = __ldg(q + 1), ly = __ldg(q + 2), hy = __ldg(q + 3);
-        const float4 lz = __ldg(q + 4), hz = __ldg(q + 5);
-        const int4 ch = __ldg(reinterpret_cast<const int4*>(q + 6));
-        const int cnt = __ldg(reinterpret_cast<const int*>(q + 7));
-        const float LX[4] = {lx.x, lx.y, lx.z, lx.w}, HX[4] = {hx.x, hx.y, hx.z, hx.w};
-        const float LY[4] = {ly.x, ly.y, ly.z, ly.w}, HY[4] = {hy.x, hy.y, hy.z, hy.w};
-        const float LZ[4] = {lz.x, lz.y, lz.z, lz.w}, HZ[4] = {hz.x, hz.y, hz.z, hz.w};
-        const int32_t CH[4] = {ch.x, ch.y, ch.z, ch.w};
-        int32_t nearest = -1;
-        float tbest = 3.0e38f;
-        unsigned leaves = 0;                  // kLeafPass: child positions of leaves to test
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            float tn;
-            if (k >= cnt || !slab(LX[k], HX[k], LY[k], HY[k], LZ[k], HZ[k], o, iv, tmax, tn)) continue;
-            const int32_t c = CH[k];
-            if (kLeafPass && c < 0) { leaves |= 1u << k; continue; }
-            if (c < 0) {
-                // a leaf: test its triangles now (a near hit ends the walk)
-                if (!wr_ready) { wr = make_wray(o, d); wr_ready = true; }
-                const uint32_t w = (uint32_t)~c;
-                const uint32_t first = w >> 3, count = (w & 7u) + 1u;
-                for (uint32_t i = 0; i < count; ++i) {
-                    if (kCount) ++cn.tris;
-                    const float4* tq = reinterpret_cast<const float4*>(tris + first + i);
-                    const float4 A = __ldg(tq), B = __ldg(tq + 1), C = __ldg(tq + 2);
-                    float t;
-                    if (!hit_tri(wr, mk(A.x, A.y, A.z), mk(B.x, B.y, B.z), mk(C.x, C.y, C.z), t)) continue;
-                    if (t < tnear) return HIT_NEAR | HIT_FAR;
-                    if (t < tmax) { far_hit = HIT_FAR; tmax = tnear; }
-                }
-                continue;
-            }
-            if (nearest < 0) { nearest = c; tbest = tn; continue; }
-            // keep the nearer child to descend into, stack the other
-            int32_t push = c;
-            if (tn < tbest) { push = nearest; nearest = c; tbest = tn; }
-            if (sp >= kStackN) { atomicOr(err, DEV_STACK_OVERFLOW); return far_hit; }
-            stack[sp++] = push;
-        }
-        if (kLeafPass)
-            while (leaves) {
-                const int k = __ffs(leaves) - 1;
-                leaves &= leaves - 1u;
-                const int32_t c = k == 0 ? ch.x : k == 1 ? ch.y : k == 2 ? ch.z : ch.w;
-                if (!wr_ready) { wr = make_wray(o, d); wr_ready = true; }
-                const uint32_t w = (uint32_t)~c;
-                const uint32_t first = w >> 3, count = (w & 7u) + 1u;
-                for (uint32_t i = 0; i < count; ++i) {
-                    if (kCount) ++cn.tris;
-                    const float4* tq = reinterpret_cast<const float4*>(tris + first + i);
-                    const float4 A = __ldg(tq), B = __ldg(tq + 1), C = __ldg(tq + 2);
-                    float t;
-                    if (!hit_tri(wr, mk(A.x, A.y, A.z), mk(B.x, B.y, B.z), mk(C.x, C.y, C.z), t)) continue;
-                    if (t < tnear) return HIT_NEAR | HIT_FAR;
-                    if (t < tmax) { far_hit = HIT_FAR; tmax = tnear; }
-                }
-            }
+        float tn[4];
+        bool hit[4];
+        int32_t CH[4];
+        node_test(reinterpret_cast<const char*>(nodes + cur), LdGlobal(), iv, tmax, CH, tn, hit);
+        // a node stacks at most three of its children (the build refuses trees whose depth
+        // could need more than the stack holds)
+        if (sp + 3 > kStackN) { atomicOr(err, DEV_STACK_OVERFLOW); return far_hit; }
+        nearest = -1;
+        tbest = 3.0e38f;
+        if (visit(CH, tn, hit)) return HIT_NEAR | HIT_FAR;
         if (nearest >= 0) { cur = nearest; continue; }
         if (sp == 0) return far_hit;
         cur = stack[--sp];
@@ -330,51 +352,53 @@ __device__ inline int walk_closest(const Node4* __restrict__ nodes, const LeafTr
     int sp = 0;
     int32_t cur = 0;
     for (uint32_t guard = 0; guard < kGuard; ++guard) {
-        const float4* q = reinterpret_cast<const float4*>(nodes + cur);
-        const float4 lx = __ldg(q + 0), hx = __ldg(q + 1), ly = __ldg(q + 2), hy = __ldg(q + 3);
-        const float4 lz = __ldg(q + 4), hz = __ldg(q + 5);
-        const int4 ch = __ldg(reinterpret_cast<const int4*>(q + 6));
-        const int cnt = __ldg(reinterpret_cast<const int*>(q + 7));
-        const float LX[4] = {lx.x, lx.y, lx.z, lx.w}, HX[4] = {hx.x, hx.y, hx.z, hx.w};
-        const float LY[4] = {ly.x, ly.y, ly.z, ly.w}, HY[4] = {hy.x, hy.y, hy.z, hy.w};
-        const float LZ[4] = {lz.x, lz.y, lz.z, lz.w}, HZ[4] = {hz.x, hz.y, hz.z, hz.w};
-        const int32_t CH[4] = {ch.x, ch.y, ch.z, ch.w};
-        // interior children that the ray enters before `best`, nearest first
-        int32_t kid[4];
-        float kt[4];
-        int nk = 0;
+        float tn[4];
+        bool hit[4];
+        int32_t CH[4];
+        node_test(reinterpret_cast<const char*>(nodes + cur), LdGlobal(), iv, best, CH, tn, hit);
+        // the leaves among them, tested in one loop
+        unsigned leaves = 0;
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            float tn;
-            if (k >= cnt || !slab(LX[k], HX[k], LY[k], HY[k], LZ[k], HZ[k], o, iv, best, tn)) continue;
-            const int32_t c = CH[k];
-            if (c < 0) {
-                const uint32_t u = (uint32_t)~c;
-                const uint32_t first = u >> 3, count = (u & 7u) + 1u;
-                for (uint32_t i = 0; i < count; ++i) {
-                    const float4* tq = reinterpret_cast<const float4*>(tris + first + i);
-                    const float4 A = __ldg(tq), B = __ldg(tq + 1), C = __ldg(tq + 2);
-                    float t;
-                    if (!hit_tri(wr, mk(A.x, A.y, A.z), mk(B.x, B.y, B.z), mk(C.x, C.y, C.z), t)) continue;
-                    const int id = __float_as_int(A.w);
-                    if (t < best || (best_tri >= 0 && t == best && id < best_tri)) {
-                        best = t;
-                        best_tri = id;
-                    }
+        for (int k = 0; k < 4; ++k)
+            if (hit[k] && CH[k] < 0) leaves |= 1u << k;
+        while (leaves) {
+            const int k = __ffs(leaves) - 1;
+            leaves &= leaves - 1u;
+            const int32_t c = k == 0 ? CH[0] : k == 1 ? CH[1] : k == 2 ? CH[2] : CH[3];
+            if (c == kNoChild) continue;
+            const uint32_t u = (uint32_t)~c;
+            const uint32_t first = u >> 3, count = (u & 7u) + 1u;
+            for (uint32_t i = 0; i < count; ++i) {
+                const float4* tq = reinterpret_cast<const float4*>(tris + first + i);
+                const float4 A = __ldg(tq), B = __ldg(tq + 1), C = __ldg(tq + 2);
+                float t;
+                if (!hit_tri(wr, mk(A.x, A.y, A.z), mk(B.x, B.y, B.z), mk(C.x, C.y, C.z), t)) continue;
+                const int id = __float_as_int(A.w);
+                if (t < best || (best_tri >= 0 && t == best && id < best_tri)) {
+                    best = t;
+                    best_tri = id;
                 }
-                continue;
             }
-            int j = nk++;
-            while (j > 0 && kt[j - 1] < tn) { kt[j] = kt[j - 1]; kid[j] = kid[j - 1]; --j; }
-            kt[j] = tn;
-            kid[j] = c;
         }
+        // the interior children that the ray still enters before `best`, sorted in registers
+        // farthest first by five compare-exchanges (the others sort to the front as -1)
+        const float lim = best * 1.0000008f;
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (!(hit[k] && CH[k] >= 0 && tn[k] <= lim)) { CH[k] = -1; tn[k] = 3.0e38f; }
+        auto cx = [&](int a, int b) {
+            const bool s = tn[a] < tn[b];
+            const float ta = s ? tn[b] : tn[a], tb = s ? tn[a] : tn[b];
+            const int32_t ca = s ? CH[b] : CH[a], cb = s ? CH[a] : CH[b];
+            tn[a] = ta; tn[b] = tb; CH[a] = ca; CH[b] = cb;
+        };
+        cx(0, 1); cx(2, 3); cx(0, 2); cx(1, 3); cx(1, 2);
         // push the farther children, descend into the nearest
-        for (int j = 0; j + 1 < nk; ++j) {
-            if (sp >= kStack) { atomicOr(err, DEV_STACK_OVERFLOW); t_hit = best; return best_tri; }
-            stack[sp++] = kid[j];
-        }
-        if (nk > 0) { cur = kid[nk - 1]; continue; }
+        if (sp + 3 > kStack) { atomicOr(err, DEV_STACK_OVERFLOW); t_hit = best; return best_tri; }
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+            if (CH[k] >= 0) stack[sp++] = CH[k];
+        if (CH[3] >= 0) { cur = CH[3]; continue; }
         // pop the next pushed node: its children meet the best hit found since
         if (sp == 0) { t_hit = best; return best_tri; }
         cur = stack[--sp];
@@ -386,7 +410,7 @@ __device__ inline int walk_closest(const Node4* __restrict__ nodes, const LeafTr
 
 // The frontier of the warp's tile for AO walks of `radius` (all 32 lanes call it and build
 // it together). Returns its size, 0 when the tile has no covered pixel.
-__device__ __forceinline__ int tile_frontier(const TraceParams& p, int x, int y, bool valid, FrontierEntry* F) {
+__device__ __forceinline__ int tile_frontier(const TraceParams& p, int x, int y, bool valid, Node4* F) {
     float lo[3] = {3.0e38f, 3.0e38f, 3.0e38f}, hi[3] = {-3.0e38f, -3.0e38f, -3.0e38f}, mag = 0.0f;
     if (valid) {
         const size_t i = (size_t)y * p.w + x;
@@ -429,9 +453,9 @@ __device__ __forceinline__ v3 sample_direction(const v3& t, const v3& b, const v
 }
 
 // One pixel: its spp cosine-weighted rays (AO and, when asked, the sky), then the sun ray.
-template <bool kCount, int kStackN = kStack, bool kLeafPass = false>
+template <bool kCount, int kStackN = kStack, bool kLeafPass = true>
 __device__ __forceinline__ void trace_pixel(const TraceParams& p, int x, int y, const v3& toLight, Counts& cn,
-                                            const FrontierEntry* F = nullptr, int fn = 0) {
+                                            const Node4* F = nullptr, int fn = 0) {
     const float kFar = 1e30f;
     const size_t i = (size_t)y * p.w + x;
     const uint8_t m = p.mask[i];

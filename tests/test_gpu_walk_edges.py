@@ -1,0 +1,64 @@
+"""The node test of the traversal (near and far planes picked by the direction's sign) where it
+can go wrong: directions with zero, negative-zero and vanishing components, origins on box
+planes, rays without a direction, and trees whose last nodes have unused child slots. The BVH
+only prunes, so closest and any-hit answers must equal the oracle's scans bit for bit."""
+import os
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+THREADS = os.cpu_count() or 1
+
+
+def _edge_rays(tris, n, seed):
+    rng = np.random.default_rng(seed)
+    v = tris.reshape(-1, 3)
+    o = v[rng.integers(0, len(v), n)].astype(np.float64)
+    o[rng.random((n, 3)) < 0.5] += 0.75                      # the others stay on a vertex's (and a box's) plane
+    o += rng.choice([0.0, -3.0, 3.0], (n, 3))
+    d = rng.normal(0, 1, (n, 3))
+    kind = rng.integers(0, 5, n)
+    for k in range(n):
+        if kind[k] == 0:                                     # one axis only, the others +0 or -0
+            a = rng.integers(0, 3)
+            d[k] = rng.choice([0.0, -0.0], 3)
+            d[k, a] = rng.choice([-1.0, 1.0])
+        elif kind[k] == 1:                                   # one zero component
+            d[k, rng.integers(0, 3)] = rng.choice([0.0, -0.0])
+        elif kind[k] == 2:                                   # one vanishing component, denormals among them
+            d[k, rng.integers(0, 3)] = rng.choice([1e-30, -1e-38, 1e-42])
+        elif kind[k] == 3 and k % 8 == 0:                    # no direction at all
+            d[k] = 0.0
+    return np.concatenate([o, d], 1).astype(np.float32)
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 5, 6, 9, 17, 400])
+def test_axis_parallel_and_degenerate_rays(rn, oracle, n):
+    rng = np.random.default_rng(100 + n)
+    # vertices on a coarse grid: many boxes share planes, many triangles are flat in one axis
+    tris = rng.integers(-4, 5, (n, 9)).astype(np.float32)
+    rays = _edge_rays(tris, 6000, n)
+    tmax = np.where(rng.random(len(rays)) < 0.3, rng.uniform(0.5, 6.0, len(rays)), 1e30).astype(np.float32)
+    acc = rn.LinearAccel(tris)
+    tri, t = rn.closest(acc, rays, tmax)
+    rtri, rt = oracle.closest_scan(tris, rays, tmax, threads=THREADS)
+    assert np.array_equal(tri, rtri), int((tri != rtri).sum())
+    assert np.array_equal(t, rt)
+    assert np.array_equal(rn.occluded(acc, rays, tmax) != 0, tri >= 0)
+
+
+@pytest.mark.parametrize("spp", [1, 16, 40])
+def test_frontier_groups_against_the_scan(rn, oracle, spp):
+    """AO-only walks start from the warp's frontier, tested in groups of four with the last one
+    padded: against the oracle's trace on a scene dense enough to fill it."""
+    import scene as scenes
+    sc = scenes.build_synthetic_scene(3, 60, 10, grid=20, half=8.0, subdiv=2)
+    cam = (6.0, 4.0, 5.0, 0.0, 0.5, 0.0, 0.0, 1.0, 0.0, 0.9)
+    _, pos, nrm, mask = oracle.rasterize(sc.tris, sc.normals, cam, 75, 53)
+    acc = rn.LinearAccel(sc.tris)
+    for radius in (0.05, 1.0):
+        ao = rn.compute_rtao(rn.GBuffer(pos, nrm, mask), acc, spp, radius)
+        ref = oracle.trace(pos, nrm, mask, sc.tris, spp, radius, threads=THREADS)
+        ref = ref[0] if isinstance(ref, tuple) else ref
+        assert np.array_equal(ao, ref), int((ao != ref).sum())
