@@ -59,6 +59,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) trace_batch_kernel(const Batc
     __shared__ Node4 frontier[8][trace_dev::kFrontierNodes];
     Node4* F = frontier[threadIdx.x >> 5];
     Counts cn;
+    int skip = 0;                               // packets to walk without the sieve (trace_packet)
     while (true) {
         uint32_t tile = 0;
         if (lane == 0) tile = atomicAdd(tile_ctr, 1u);
@@ -73,7 +74,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) trace_batch_kernel(const Batc
         const v3 toLight = normalize(mk(p.lx, p.ly, p.lz));
         const int fn = (!p.want_sky && p.has_geometry && p.frontier)
                             ? trace_dev::tile_frontier(p, x, y, x < p.w && y < p.h, F) : 0;
-        if (x < p.w && y < p.h) trace_dev::trace_pixel<false>(p, x, y, toLight, cn, F, fn);
+        trace_dev::trace_packet<false>(p, x, y, x < p.w && y < p.h, toLight, cn, skip, F, fn);
         __syncwarp();
     }
 }

@@ -41,6 +41,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) trace_kernel(const __grid_con
     __shared__ Node4 frontier[8][kFrontierNodes];
     Node4* F = frontier[threadIdx.x >> 5];
     Counts cn;
+    int skip = 0;                                  // packets to walk without the sieve (trace_packet)
     // lighting model 2's sun direction, normalized on the device as computeRTVisibility does
     const v3 toLight = normalize(mk(p.lx, p.ly, p.lz));
     while (true) {
@@ -53,7 +54,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) trace_kernel(const __grid_con
         // no lane leaves the loop body early: the next tile fetch is a full-warp shuffle
         if (kCount && tile % stride != 0) continue;
         const int fn = (!p.want_sky && p.has_geometry && p.frontier) ? tile_frontier(p, x, y, x < p.w && y < p.h, F) : 0;
-        if (x < p.w && y < p.h) trace_pixel<kCount, kStackN, kLeafPass>(p, x, y, toLight, cn, F, fn);
+        trace_packet<kCount, kStackN, kLeafPass>(p, x, y, x < p.w && y < p.h, toLight, cn, skip, F, fn);
         __syncwarp();                              // the frontier is rebuilt for the next tile
     }
     if (kCount) {
@@ -70,7 +71,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) trace_kernel(const __grid_con
 // still walking, the idle lanes take the next walks of the queue, whichever pixel they
 // belong to. A lane is therefore not held by the slowest walk of its own pixel's sample
 // round, as in trace_kernel's one-pixel-per-lane loop; only the queue's last walks leave
-// lanes idle. A walk's rays, box tests and hit test are trace_pixel's (sample_direction,
+// lanes idle. A walk's rays, box tests and hit test are trace_packet's (sample_direction,
 // slab, hit_tri, the frontier start), and a pixel's AO is its count of open walks over spp:
 // an integer count, so the order the walks finish in changes no bit.
 // With `sort` (at most kSortSpp samples a pixel) the queue is ordered by the walks' direction
@@ -327,7 +328,7 @@ __global__ void occluded_kernel(const Node4* __restrict__ nodes, const LeafTri* 
 }
 
 // AO of listed pixels with one thread per (pixel, sample): the same rays and hit rule as
-// trace_pixel (AO only), for pixel sets too small or too uneven to keep packets of pixels
+// trace_packet (AO only), for pixel sets too small or too uneven to keep packets of pixels
 // busy (the surrogate's fallback tiles). open[list[i]] receives pixel list[i]'s open rays,
 // added by one atomic per warp and pixel.
 __global__ void __launch_bounds__(256) ao_samples_kernel(const __grid_constant__ TraceParams p,

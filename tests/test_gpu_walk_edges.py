@@ -62,3 +62,18 @@ def test_frontier_groups_against_the_scan(rn, oracle, spp):
         ref = oracle.trace(pos, nrm, mask, sc.tris, spp, radius, threads=THREADS)
         ref = ref[0] if isinstance(ref, tuple) else ref
         assert np.array_equal(ao, ref), int((ao != ref).sum())
+
+
+@pytest.mark.parametrize("spp", [1, 63, 64, 65, 130])
+def test_sieve_chunks_against_the_scan(rn, oracle, spp):
+    """Sample counts around the sieve's 64-sample chunks (the sun's slot falls into the last one
+    or opens another), in a frame whose packets are ragged at the right and lower edge."""
+    import scene as scenes
+    sc = scenes.build_test_scene()
+    _, pos, nrm, mask = oracle.rasterize(sc.tris, sc.normals, sc.camera, 61, 43)
+    acc = rn.LinearAccel(sc.tris)
+    g = rn.GBuffer(pos, nrm, mask)
+    ao, sky, sun = rn.compute_rt_visibility(g, acc, spp, 2.0, to_light=sc.to_light)
+    rao, rsky, rsun = oracle.trace(pos, nrm, mask, sc.tris, spp, 2.0, to_light=sc.to_light, threads=THREADS)
+    assert np.array_equal(ao, rao) and np.array_equal(sky, rsky) and np.array_equal(sun, rsun)
+    assert np.array_equal(rn.compute_rtao(g, acc, spp, 2.0), rao)
