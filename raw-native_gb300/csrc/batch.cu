@@ -72,9 +72,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) trace_batch_kernel(const Batc
         const int x = (int)(local % tiles_x) * kTileW + (int)(lane % kTileW);
         const int y = (int)(local / tiles_x) * kTileH + (int)(lane / kTileW);
         const v3 toLight = normalize(mk(p.lx, p.ly, p.lz));
-        const int fn = (!p.want_sky && p.has_geometry && p.frontier)
-                            ? trace_dev::tile_frontier(p, x, y, x < p.w && y < p.h, F) : 0;
-        trace_dev::trace_packet<false>(p, x, y, x < p.w && y < p.h, toLight, cn, skip, F, fn);
+        trace_dev::trace_packet<false>(p, x, y, x < p.w && y < p.h, toLight, cn, skip, F);
         __syncwarp();
     }
 }

@@ -53,8 +53,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) trace_kernel(const __grid_con
         const int y = (int)(tile / tiles_x) * th + (int)(lane >> pl);
         // no lane leaves the loop body early: the next tile fetch is a full-warp shuffle
         if (kCount && tile % stride != 0) continue;
-        const int fn = (!p.want_sky && p.has_geometry && p.frontier) ? tile_frontier(p, x, y, x < p.w && y < p.h, F) : 0;
-        trace_packet<kCount, kStackN, kLeafPass>(p, x, y, x < p.w && y < p.h, toLight, cn, skip, F, fn);
+        trace_packet<kCount, kStackN, kLeafPass>(p, x, y, x < p.w && y < p.h, toLight, cn, skip, F);
         __syncwarp();                              // the frontier is rebuilt for the next tile
     }
     if (kCount) {
@@ -133,7 +132,9 @@ __global__ void __launch_bounds__(256, kMinBlocks) trace_ao_pool_kernel(const __
             B = cross(n, T);
             O = add(P, scale(n, 1e-3f));
         }
-        const int fn = (p.has_geometry && p.frontier) ? tile_frontier(p, x, y, valid, F) : 0;
+        // no plane: an empty frontier is left to the walk's own test
+        const int fn = (p.has_geometry && p.frontier)
+                           ? max(0, tile_frontier(p, O, covered, TilePlane{0.0f, 0.0f, 0.0f, 0.0f, 0.0f}, F)) : 0;
         const unsigned cov = __ballot_sync(0xffffffffu, covered);
         const int nc = __popc(cov);
         opens[lane] = 0;

@@ -142,15 +142,46 @@ __device__ __forceinline__ bool box_overlaps(float lx, float ly, float lz, float
     return lx <= qhi[0] && hx >= qlo[0] && ly <= qhi[1] && hy >= qlo[1] && lz <= qhi[2] && hz >= qlo[2];
 }
 
+// The tangent plane of a warp's packet where its covered pixels share one normal (flat
+// surfaces): every hemisphere ray leaves its origin o with direction . n > 0 (the sampler's lz
+// is sqrt(1 - u) >= 2.4e-4, far above the rounding of the frame and the direction), so a box
+// that lies wholly below the lowest origin's plane holds no triangle that a ray of the packet
+// can reach. `below` asks for 2e-6 of the coordinates more than that (16 units in the last
+// place: the rounding of the support point's product, and of the triangle test, which may be
+// off by a few ulps of the coordinates). Off (n all zero) when the normals differ or are far
+// from unit length: nothing is then below.
+struct TilePlane { float nx, ny, nz, low, mag; };
+__device__ __forceinline__ TilePlane tile_plane(const v3& n, const v3& o, bool covered, unsigned any) {
+    const int first = __ffs(any) - 1;
+    const v3 f = mk(__shfl_sync(0xffffffffu, n.x, first), __shfl_sync(0xffffffffu, n.y, first),
+                    __shfl_sync(0xffffffffu, n.z, first));
+    const float d2 = f.x * f.x + f.y * f.y + f.z * f.z;
+    const bool alike = !covered || (fabsf(n.x - f.x) <= 1e-5f && fabsf(n.y - f.y) <= 1e-5f && fabsf(n.z - f.z) <= 1e-5f);
+    if (!(__all_sync(0xffffffffu, alike) && d2 > 0.9f && d2 < 1.1f)) return TilePlane{0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+    float low = covered ? f.x * o.x + f.y * o.y + f.z * o.z : 3.0e38f;
+    float mag = covered ? fabsf(o.x) + fabsf(o.y) + fabsf(o.z) : 0.0f;
+    for (int off = 16; off > 0; off >>= 1) {
+        low = fminf(low, __shfl_xor_sync(0xffffffffu, low, off));
+        mag = fmaxf(mag, __shfl_xor_sync(0xffffffffu, mag, off));
+    }
+    return TilePlane{f.x, f.y, f.z, low, mag};
+}
+__device__ __forceinline__ bool below(const TilePlane& t, float lx, float ly, float lz, float hx, float hy, float hz) {
+    const float cx = t.nx > 0.0f ? hx : lx, cy = t.ny > 0.0f ? hy : ly, cz = t.nz > 0.0f ? hz : lz;
+    const float m = 2e-6f * (fabsf(cx) + fabsf(cy) + fabsf(cz) + t.mag);
+    return (t.nx != 0.0f || t.ny != 0.0f || t.nz != 0.0f) && t.nx * cx + t.ny * cy + t.nz * cz < t.low - m;
+}
+
 // The warp builds the frontier of box [qlo, qhi] into F (all 32 lanes call it); returns its
-// size (0: start at the root). Breadth first: each round every entry that is an interior
-// node is replaced by its Q-overlapping children, the lanes expanding their entries in
+// size (0: start at the root; -1: nothing within reach). Breadth first: each round every entry
+// that is an interior node is replaced by its children that overlap Q and are not below the
+// packet's plane, the lanes expanding their entries in
 // parallel (one node fetch per lane, a prefix sum over the lanes for the output slots),
 // while the result stays within kFrontier entries. A round costs one dependent node fetch,
 // so the build takes about the tree's depth in fetch latencies. Up to `tail` greedy steps
 // follow, each replacing the largest interior entry by its children while the frontier fits.
 __device__ inline int build_frontier(const Node4* __restrict__ nodes, const float* qlo, const float* qhi,
-                                     Node4* F, int tail) {
+                                     const TilePlane& pl, Node4* F, int tail) {
     const int lane = (int)(threadIdx.x & 31u);
     int32_t word = 0;                       // lane 0 starts with the root node
     float lo[3] = {0.0f, 0.0f, 0.0f}, hi[3] = {0.0f, 0.0f, 0.0f};
@@ -162,7 +193,8 @@ __device__ inline int build_frontier(const Node4* __restrict__ nodes, const floa
         unsigned hit = 0;
         if (inner)
             for (int k = 0; k < N->meta[0]; ++k)
-                if (box_overlaps(N->lox[k], N->loy[k], N->loz[k], N->hix[k], N->hiy[k], N->hiz[k], qlo, qhi))
+                if (box_overlaps(N->lox[k], N->loy[k], N->loz[k], N->hix[k], N->hiy[k], N->hiz[k], qlo, qhi) &&
+                    !below(pl, N->lox[k], N->loy[k], N->loz[k], N->hix[k], N->hiy[k], N->hiz[k]))
                     hit |= 1u << k;
         const int c = inner ? __popc(hit) : (mine ? 1 : 0);
         int incl = c;
@@ -205,7 +237,8 @@ __device__ inline int build_frontier(const Node4* __restrict__ nodes, const floa
         const Node4* N = nodes + (lane == bl ? word : 0);
         if (lane == bl)
             for (int k = 0; k < N->meta[0]; ++k)
-                if (box_overlaps(N->lox[k], N->loy[k], N->loz[k], N->hix[k], N->hiy[k], N->hiz[k], qlo, qhi))
+                if (box_overlaps(N->lox[k], N->loy[k], N->loz[k], N->hix[k], N->hiy[k], N->hiz[k], qlo, qhi) &&
+                    !below(pl, N->lox[k], N->loy[k], N->loz[k], N->hix[k], N->hiy[k], N->hiz[k]))
                     hit |= 1u << k;
         const int c = __popc(__shfl_sync(0xffffffffu, hit, bl));
         if (n - 1 + c > kFrontier) break;
@@ -233,7 +266,7 @@ __device__ inline int build_frontier(const Node4* __restrict__ nodes, const floa
     // the last group's unused slots: boxes no ray passes
     if (built && lane >= n && lane < ((n + 3) & ~3))
         frontier_put(F, lane, FrontierBox{{1e30f, 1e30f, 1e30f}, {-1e30f, -1e30f, -1e30f}, kNoChild});
-    return built ? n : 0;
+    return built ? (n > 0 ? n : -1) : 0;
 }
 
 // One walk, two limits (tnear <= tfar): HIT_NEAR | HIT_FAR when some triangle is hit at
@@ -408,18 +441,15 @@ __device__ inline int walk_closest(const Node4* __restrict__ nodes, const LeafTr
     return best_tri;
 }
 
-// The frontier of the warp's tile for AO walks of `radius` (all 32 lanes call it and build
-// it together). Returns its size, 0 when the tile has no covered pixel.
-__device__ __forceinline__ int tile_frontier(const TraceParams& p, int x, int y, bool valid, Node4* F) {
+// The frontier of the warp's packet for AO walks of `radius` (all 32 lanes call it and build
+// it together; o: the lane's ray origin, where `covered`). Returns its size, 0: the walks start
+// at the root, -1: no triangle is within reach.
+__device__ __forceinline__ int tile_frontier(const TraceParams& p, const v3& o, bool covered, const TilePlane& pl,
+                                             Node4* F) {
     float lo[3] = {3.0e38f, 3.0e38f, 3.0e38f}, hi[3] = {-3.0e38f, -3.0e38f, -3.0e38f}, mag = 0.0f;
-    if (valid) {
-        const size_t i = (size_t)y * p.w + x;
-        if (p.mask[i]) {
-            const v3 P = load3(p.pos + 3 * i), n = load3(p.nrm + 3 * i);
-            const v3 o = add(P, scale(n, 1e-3f));
-            lo[0] = hi[0] = o.x; lo[1] = hi[1] = o.y; lo[2] = hi[2] = o.z;
-            mag = fmaxf(fmaxf(fabsf(o.x), fabsf(o.y)), fabsf(o.z));
-        }
+    if (covered) {
+        lo[0] = hi[0] = o.x; lo[1] = hi[1] = o.y; lo[2] = hi[2] = o.z;
+        mag = fmaxf(fmaxf(fabsf(o.x), fabsf(o.y)), fabsf(o.z));
     }
     for (int off = 16; off > 0; off >>= 1)
         for (int a = 0; a < 3; ++a) {
@@ -431,9 +461,25 @@ __device__ __forceinline__ int tile_frontier(const TraceParams& p, int x, int y,
     // grow by the radius with margin for the rounding of t, |d| and the hit point
     const float g = p.radius * 1.0001f + 1e-5f * (mag + 1.0f);
     for (int a = 0; a < 3; ++a) { lo[a] -= g; hi[a] += g; }
-    const int n = build_frontier(p.nodes, lo, hi, F, p.frontier_tail);
+    const int n = build_frontier(p.nodes, lo, hi, pl, F, p.frontier_tail);
     __syncwarp();
     return n;
+}
+// For walks that start at the root: its children that are not below the packet's plane, put
+// into F as frontier entries (all 32 lanes call it). Returns their number, -1: none.
+__device__ __forceinline__ int root_frontier(const Node4* __restrict__ nodes, const TilePlane& pl, Node4* F) {
+    const int lane = (int)(threadIdx.x & 31u);
+    bool live = false;
+    if (lane < nodes->meta[0])
+        live = !below(pl, nodes->lox[lane], nodes->loy[lane], nodes->loz[lane], nodes->hix[lane], nodes->hiy[lane],
+                      nodes->hiz[lane]);
+    const unsigned m = __ballot_sync(0xffffffffu, live);
+    const int n = __popc(m);
+    if (live) frontier_put(F, __popc(m & ((1u << lane) - 1u)), frontier_child(nodes, lane));
+    if (lane >= n && lane < 4)
+        frontier_put(F, lane, FrontierBox{{1e30f, 1e30f, 1e30f}, {-1e30f, -1e30f, -1e30f}, kNoChild});
+    __syncwarp();
+    return n > 0 ? n : -1;
 }
 
 // Hemisphere direction of sample s of pixel (ux, uy) with frame (t, b, n): the arithmetic of
@@ -452,23 +498,19 @@ __device__ __forceinline__ v3 sample_direction(const v3& t, const v3& b, const v
     return normalize(add(add(scale(t, lx), scale(b, ly)), scale(n, lz)));
 }
 
-// Whether a walk of this ray has anything to descend into: any entry of the frontier (fn > 0),
-// else any child of the root, is entered before tmax.
-__device__ __forceinline__ bool walk_starts(const Node4* __restrict__ nodes, const v3& o, const v3& d, float tmax,
-                                            const Node4* F, int fn) {
+// Whether a walk of this ray has anything to descend into: any of the fn entries of F is
+// entered before tmax.
+__device__ __forceinline__ bool walk_starts(const v3& o, const v3& d, float tmax, const Node4* F, int fn) {
     const Inv iv = make_inv(o, d);
-    float tn[4];
-    bool hit[4];
-    int32_t CH[4];
-    if (fn == 0) {
-        node_test(reinterpret_cast<const char*>(nodes), LdGlobal(), iv, tmax, CH, tn, hit);
-        return hit[0] || hit[1] || hit[2] || hit[3];
-    }
-    bool any = false;
-    for (int g = 0; 4 * g < fn && !any; ++g) {
+    bool any;
+    int g = 0;
+    do {
+        float tn[4];
+        bool hit[4];
+        int32_t CH[4];
         node_test(reinterpret_cast<const char*>(F + g), LdShared(), iv, tmax, CH, tn, hit);
         any = hit[0] || hit[1] || hit[2] || hit[3];
-    }
+    } while (4 * ++g < fn && !any);
     return any;
 }
 
@@ -488,7 +530,7 @@ __device__ __forceinline__ bool walk_starts(const Node4* __restrict__ nodes, con
 constexpr int kChunk = 64, kSieveNum = 7, kSieveDen = 8, kSieveSkip = 15;
 template <bool kCount, int kStackN = kStack, bool kLeafPass = true>
 __device__ __forceinline__ void trace_packet(const TraceParams& p, int x, int y, bool valid, const v3& toLight,
-                                             Counts& cn, int& skip, const Node4* F = nullptr, int fn = 0) {
+                                             Counts& cn, int& skip, Node4* F) {
     const float kFar = 1e30f;
     const size_t i = valid ? (size_t)y * p.w + x : 0;
     const uint8_t m = valid ? p.mask[i] : 0;
@@ -514,6 +556,14 @@ __device__ __forceinline__ void trace_packet(const TraceParams& p, int x, int y,
     const uint32_t ux = (uint32_t)x, uy = (uint32_t)y;
     const float tfar_h = p.want_sky ? kFar : p.radius;
     const int slots = p.spp + ((p.want_sky && !p.sun_forced) ? 1 : 0);
+    // what the packet's rays can reach: AO-only walks start from the entries within the radius,
+    // the sky's at the root, whose live children serve the sieve (the frontier is rebuilt for
+    // every packet)
+    int fn = 0;
+    if (p.has_geometry && (p.want_sky || p.frontier)) {
+        const TilePlane pl = tile_plane(n, origin, m != 0, covered);
+        fn = p.want_sky ? root_frontier(p.nodes, pl, F) : tile_frontier(p, origin, m != 0, pl, F);
+    }
     int open = 0, freec = 0;
     bool lit = true;
     // sample s's direction from its angle's index k2 and correction byte (both fetched ahead)
@@ -533,10 +583,16 @@ __device__ __forceinline__ void trace_packet(const TraceParams& p, int x, int y,
         k2n = hash24(ux, uy, (uint32_t)(2 * s + 1));
         cbn = p.corr ? __ldg(p.corr + k2n) : 0;
     };
-    const bool geometry = p.has_geometry;
-    bool sieve = !kCount && geometry && skip == 0;
-    if (!kCount && skip > 0) --skip;
-    for (int s0 = 0; s0 < slots; s0 += kChunk) {
+    // nothing within reach: every hemisphere ray is open and free, only the sun ray is left
+    const bool walks = p.has_geometry && fn >= 0;
+    const int first = walks ? 0 : p.spp;
+    if (!walks) {
+        open = freec = p.spp;
+        if (kCount && m) { cn.rays += p.spp; if (p.want_sky) cn.sky += p.spp; }
+    }
+    bool sieve = !kCount && fn > 0 && skip == 0;
+    if (!kCount && fn > 0 && skip > 0) --skip;
+    for (int s0 = first; s0 < slots; s0 += kChunk) {
         const int nslot = min(kChunk, slots - s0), nsamp = min(kChunk, p.spp - s0);
         uint64_t todo = m ? (nslot == 64 ? ~0ull : (1ull << nslot) - 1ull) : 0ull;
         if (sieve && nsamp > 0) {
@@ -547,7 +603,7 @@ __device__ __forceinline__ void trace_packet(const TraceParams& p, int x, int y,
                     const uint32_t k2 = k2n;
                     const int cb = cbn;
                     if (k + 1 < nsamp) fetch(s0 + k + 1);
-                    if (!walk_starts(p.nodes, origin, direction(s0 + k, k2, cb), tfar_h, F, fn)) {
+                    if (!walk_starts(origin, direction(s0 + k, k2, cb), tfar_h, F, fn)) {
                         keep &= ~(1ull << k);
                         ++open;
                         ++freec;
@@ -580,9 +636,10 @@ __device__ __forceinline__ void trace_packet(const TraceParams& p, int x, int y,
             }
             // AO-only walks may start from the warp's frontier; the sky and the sun need the root
             const bool local = s < p.spp && tf == p.radius;
-            const int h = geometry ? walk<kCount, kStackN, kLeafPass>(p.nodes, p.tris, origin, dir, tn, tf, p.err_word,
-                                                                     cn, local ? F : nullptr, local ? fn : 0)
-                                   : 0;
+            const int h = p.has_geometry
+                              ? walk<kCount, kStackN, kLeafPass>(p.nodes, p.tris, origin, dir, tn, tf, p.err_word, cn,
+                                                                 local ? F : nullptr, local ? fn : 0)
+                              : 0;
             if (s < p.spp) {
                 if (kCount) { ++cn.rays; if (p.want_sky && !(h & HIT_NEAR)) ++cn.sky; }
                 if (!(h & HIT_NEAR)) {
