@@ -986,9 +986,9 @@ __device__ __forceinline__ void collapse_tasks(const Task* in, uint32_t m, uint3
                     if (tri[x] >= 0) {
                         const float* v = tris + (size_t)tri[x] * 9;
                         LeafTri lt;
-                        lt.ax = v[0]; lt.ay = v[1]; lt.az = v[2]; lt.id = __int_as_float(tri[x]);
-                        lt.bx = v[3]; lt.by = v[4]; lt.bz = v[5]; lt.pad0 = 0.0f;
-                        lt.cx = v[6]; lt.cy = v[7]; lt.cz = v[8]; lt.pad1 = 0.0f;
+                        lt.ax = v[0]; lt.bx = v[3]; lt.cx = v[6]; lt.id = __int_as_float(tri[x]);
+                        lt.ay = v[1]; lt.by = v[4]; lt.cy = v[7]; lt.pad0 = 0.0f;
+                        lt.az = v[2]; lt.bz = v[5]; lt.cz = v[8]; lt.pad1 = 0.0f;
                         leaf[first + w++] = lt;
                     } else if (sp + 2 <= 2 * kLeafCap) {
                         stack[sp++] = right[x];

@@ -128,31 +128,66 @@ __device__ __forceinline__ WRay make_wray(v3 o, v3 d) {
     return r;
 }
 
-// The reference's hit rule (raw/math/primitives.hpp:31-64): the watertight sign test
-// decides; t comes from Moeller-Trumbore unless its determinant is within 1e-7 of zero,
-// then from the sheared sums. Returns true with t when the test accepts and t > 1e-4.
-// u and v are not formed: no caller of the AO path reads them.
-__device__ __forceinline__ bool hit_tri(const WRay& r, v3 a, v3 b, v3 c, float& t) {
-    const v3 A = wframe(sub(a, r.o), r.kz, r.sw), B = wframe(sub(b, r.o), r.kz, r.sw),
-             C = wframe(sub(c, r.o), r.kz, r.sw);
-    const float Ax = fsub(A.x, fmul(r.sx, A.z)), Ay = fsub(A.y, fmul(r.sy, A.z));
-    const float Bx = fsub(B.x, fmul(r.sx, B.z)), By = fsub(B.y, fmul(r.sy, B.z));
-    const float Cx = fsub(C.x, fmul(r.sx, C.z)), Cy = fsub(C.y, fmul(r.sy, C.z));
+// Per-ray constants of the test of a leaf triangle: the byte offsets of its planes in the ray's
+// permuted axis order (16 x axis), the origin in that order, and the shear. wframe's permutation
+// and swap happen by address, once per ray, instead of by selects, once per vertex.
+struct LeafRay {
+    uint32_t fx, fy, fz;
+    float ox, oy, oz, sx, sy;
+};
+__device__ __forceinline__ LeafRay make_leaf_ray(const v3& o, const v3& d) {
+    const float ax = fabsf(d.x), ay = fabsf(d.y), az = fabsf(d.z);
+    const int kz = ax > ay ? (ax > az ? 0 : 2) : (ay > az ? 1 : 2);
+    const v3 q = wframe(d, kz, false), po = wframe(o, kz, false);
+    const bool sw = q.z < 0.0f;
+    const uint32_t k1 = kz == 2 ? 0u : 16u * (uint32_t)(kz + 1), k2 = kz == 0 ? 32u : 16u * (uint32_t)(kz - 1);
+    LeafRay r;
+    r.fx = sw ? k2 : k1;
+    r.fy = sw ? k1 : k2;
+    r.fz = 16u * (uint32_t)kz;
+    r.ox = sw ? po.y : po.x;
+    r.oy = sw ? po.x : po.y;
+    r.oz = po.z;
+    r.sx = fdiv(sw ? q.y : q.x, q.z);
+    r.sy = fdiv(sw ? q.x : q.y, q.z);
+    return r;
+}
+
+// The reference's hit rule (raw/math/primitives.hpp:31-64) for one leaf triangle: the
+// watertight sign test decides; t comes from Moeller-Trumbore unless its determinant is within
+// 1e-7 of zero, then from the sheared sums. Returns true with t when the test accepts and
+// t > 1e-4. u and v are not formed: no caller of the walks reads them. `id` receives the
+// triangle's input index (its bits as a float). The vertices in axis order are read again only
+// where the sign test accepts.
+__device__ __forceinline__ bool hit_leaf(const LeafRay& r, const v3& o, const v3& d, const LeafTri* tri, float& t,
+                                         float& id) {
+    const char* q = reinterpret_cast<const char*>(tri);
+    auto plane = [&](uint32_t off) { return __ldg(reinterpret_cast<const float4*>(q + off)); };
+    const float4 X = plane(r.fx), Y = plane(r.fy), Z = plane(r.fz);
+    const float Az = fsub(Z.x, r.oz), Bz = fsub(Z.y, r.oz), Cz = fsub(Z.z, r.oz);
+    const float Ax = fsub(fsub(X.x, r.ox), fmul(r.sx, Az)), Ay = fsub(fsub(Y.x, r.oy), fmul(r.sy, Az));
+    const float Bx = fsub(fsub(X.y, r.ox), fmul(r.sx, Bz)), By = fsub(fsub(Y.y, r.oy), fmul(r.sy, Bz));
+    const float Cx = fsub(fsub(X.z, r.ox), fmul(r.sx, Cz)), Cy = fsub(fsub(Y.z, r.oy), fmul(r.sy, Cz));
     const float U = fsub(fmul(Cx, By), fmul(Cy, Bx));
     const float V = fsub(fmul(Ax, Cy), fmul(Ay, Cx));
     const float W = fsub(fmul(Bx, Ay), fmul(By, Ax));
-    if ((U < 0.0f || V < 0.0f || W < 0.0f) && (U > 0.0f || V > 0.0f || W > 0.0f)) return false;
+    // a NaN is neither below nor above zero, and fminf / fmaxf leave it out
+    if (fminf(fminf(U, V), W) < 0.0f && fmaxf(fmaxf(U, V), W) > 0.0f) return false;
     const float det = fadd(fadd(U, V), W);
     if (det == 0.0f) return false;
-    const v3 e1 = sub(b, a), e2 = sub(c, a), p = cross(r.d, e2);
+    const float4 PX = plane(0), PY = plane(16), PZ = plane(32);
+    id = PX.w;
+    const v3 a = mk(PX.x, PY.x, PZ.x), b = mk(PX.y, PY.y, PZ.y), c = mk(PX.z, PY.z, PZ.z);
+    const v3 e1 = sub(b, a), e2 = sub(c, a), p = cross(d, e2);
     const float dm = dot(e1, p);
     if (dm > -1e-7f && dm < 1e-7f) {
-        const float T = fadd(fadd(fmul(U, fmul(r.sz, A.z)), fmul(V, fmul(r.sz, B.z))), fmul(W, fmul(r.sz, C.z)));
+        const float dz = r.fz == 0u ? d.x : r.fz == 16u ? d.y : d.z, sz = frcp(dz);
+        const float T = fadd(fadd(fmul(U, fmul(sz, Az)), fmul(V, fmul(sz, Bz))), fmul(W, fmul(sz, Cz)));
         t = fmul(T, frcp(det));
     } else {
         const float inv = frcp(dm);
-        const v3 q = cross(sub(r.o, a), e1);
-        t = fmul(dot(e2, q), inv);
+        const v3 s = cross(sub(o, a), e1);
+        t = fmul(dot(e2, s), inv);
     }
     return t > 1e-4f;
 }

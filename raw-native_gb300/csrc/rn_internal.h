@@ -160,12 +160,15 @@ static_assert(sizeof(Node4) == 128, "Node4 layout");
 constexpr int32_t kNoChild = INT32_MIN;
 constexpr int kLeafCap = 8;   // triangles a leaf may hold (the child word's 3-bit count)
 
-// A leaf triangle: vertices a, b, c as float4 (w of a = input triangle index).
+// A leaf triangle, one float4 per axis: that coordinate of a, b and c (w of the x plane = input
+// triangle index). The watertight test permutes the axes by the ray's largest component: it
+// reads the planes in that order by address.
 struct alignas(16) LeafTri {
-    float ax, ay, az, id;
-    float bx, by, bz, pad0;
-    float cx, cy, cz, pad1;
+    float ax, bx, cx, id;
+    float ay, by, cy, pad0;
+    float az, bz, cz, pad1;
 };
+static_assert(sizeof(LeafTri) == 48, "LeafTri layout");
 
 }  // namespace rn
 

@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) trace_kernel(const __grid_con
 // belong to. A lane is therefore not held by the slowest walk of its own pixel's sample
 // round, as in trace_kernel's one-pixel-per-lane loop; only the queue's last walks leave
 // lanes idle. A walk's rays, box tests and hit test are trace_packet's (sample_direction,
-// slab, hit_tri, the frontier start), and a pixel's AO is its count of open walks over spp:
+// slab, hit_leaf, the frontier start), and a pixel's AO is its count of open walks over spp:
 // an integer count, so the order the walks finish in changes no bit.
 // With `sort` (at most kSortSpp samples a pixel) the queue is ordered by the walks' direction
 // octant first (a counting sort of the packet's walks in shared memory), so the lanes that
@@ -183,7 +183,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) trace_ao_pool_kernel(const __
         int q = 0;                    // the lane whose pixel the current walk belongs to
         v3 o = O, d = O;
         Inv iv;
-        WRay wr;
+        LeafRay wr;
         bool wr_ready = false;
         int32_t cur = 0;
         int sp = 0;
@@ -229,16 +229,12 @@ __global__ void __launch_bounds__(256, kMinBlocks) trace_ao_pool_kernel(const __
                             if (!slab(fb.lo[0], fb.hi[0], fb.lo[1], fb.hi[1], fb.lo[2], fb.hi[2], iv, tmax, tn)) continue;
                             const int32_t c = fb.word;
                             if (c < 0) {
-                                if (!wr_ready) { wr = make_wray(o, d); wr_ready = true; }
+                                if (!wr_ready) { wr = make_leaf_ray(o, d); wr_ready = true; }
                                 const uint32_t w = (uint32_t)~c;
                                 const uint32_t first = w >> 3, count = (w & 7u) + 1u;
                                 for (uint32_t k = 0; k < count && !hit; ++k) {
-                                    const float4* tq = reinterpret_cast<const float4*>(p.tris + first + k);
-                                    const float4 A = __ldg(tq), Bq = __ldg(tq + 1), C = __ldg(tq + 2);
-                                    float t;
-                                    if (hit_tri(wr, mk(A.x, A.y, A.z), mk(Bq.x, Bq.y, Bq.z), mk(C.x, C.y, C.z), t) &&
-                                        t < tmax)
-                                        hit = true;
+                                    float t, id;
+                                    if (hit_leaf(wr, o, d, p.tris + first + k, t, id) && t < tmax) hit = true;
                                 }
                                 continue;
                             }
@@ -278,14 +274,12 @@ __global__ void __launch_bounds__(256, kMinBlocks) trace_ao_pool_kernel(const __
                 if (hit || k >= cnt || !slab(LX[k], HX[k], LY[k], HY[k], LZ[k], HZ[k], iv, tmax, tn)) continue;
                 const int32_t c = CH[k];
                 if (c < 0) {
-                    if (!wr_ready) { wr = make_wray(o, d); wr_ready = true; }
+                    if (!wr_ready) { wr = make_leaf_ray(o, d); wr_ready = true; }
                     const uint32_t w = (uint32_t)~c;
                     const uint32_t first = w >> 3, count = (w & 7u) + 1u;
                     for (uint32_t j = 0; j < count; ++j) {
-                        const float4* tq = reinterpret_cast<const float4*>(p.tris + first + j);
-                        const float4 A = __ldg(tq), Bq = __ldg(tq + 1), C = __ldg(tq + 2);
-                        float t;
-                        if (hit_tri(wr, mk(A.x, A.y, A.z), mk(Bq.x, Bq.y, Bq.z), mk(C.x, C.y, C.z), t) && t < tmax) {
+                        float t, id;
+                        if (hit_leaf(wr, o, d, p.tris + first + j, t, id) && t < tmax) {
                             hit = true;
                             break;
                         }

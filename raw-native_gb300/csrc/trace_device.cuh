@@ -282,7 +282,7 @@ template <bool kCount, int kStackN = kStack, bool kLeafPass = true>
 __device__ int walk(const Node4* __restrict__ nodes, const LeafTri* __restrict__ tris, const v3& o, const v3& d,
                     float tnear, float tfar, uint32_t* err, Counts& cn, const Node4* F = nullptr, int fn = 0) {
     const Inv iv = make_inv(o, d);
-    WRay wr;                             // the watertight set-up: formed at the first leaf
+    LeafRay wr;                          // the watertight set-up: formed at the first leaf
     bool wr_ready = false;
     float tmax = tfar;
     int far_hit = 0;
@@ -292,15 +292,13 @@ __device__ int walk(const Node4* __restrict__ nodes, const LeafTri* __restrict__
     // the triangles of leaf word c: true when one is hit nearer than tnear (the walk ends)
     auto leaf = [&](int32_t c) -> bool {
         if (c == kNoChild) return false;
-        if (!wr_ready) { wr = make_wray(o, d); wr_ready = true; }
+        if (!wr_ready) { wr = make_leaf_ray(o, d); wr_ready = true; }
         const uint32_t w = (uint32_t)~c;
         const uint32_t first = w >> 3, count = (w & 7u) + 1u;
         for (uint32_t i = 0; i < count; ++i) {
             if (kCount) ++cn.tris;
-            const float4* tq = reinterpret_cast<const float4*>(tris + first + i);
-            const float4 A = __ldg(tq), B = __ldg(tq + 1), C = __ldg(tq + 2);
-            float t;
-            if (!hit_tri(wr, mk(A.x, A.y, A.z), mk(B.x, B.y, B.z), mk(C.x, C.y, C.z), t)) continue;
+            float t, id;
+            if (!hit_leaf(wr, o, d, tris + first + i, t, id)) continue;
             if (t < tnear) return true;
             if (t < tmax) { far_hit = HIT_FAR; tmax = tnear; }
         }
@@ -378,7 +376,7 @@ __device__ int walk(const Node4* __restrict__ nodes, const LeafTri* __restrict__
 __device__ inline int walk_closest(const Node4* __restrict__ nodes, const LeafTri* __restrict__ tris, const v3& o,
                             const v3& d, float tmax, float& t_hit, uint32_t* err) {
     const Inv iv = make_inv(o, d);
-    const WRay wr = make_wray(o, d);
+    const LeafRay wr = make_leaf_ray(o, d);
     float best = tmax;
     int best_tri = -1;
     int32_t stack[kStack];
@@ -402,11 +400,9 @@ __device__ inline int walk_closest(const Node4* __restrict__ nodes, const LeafTr
             const uint32_t u = (uint32_t)~c;
             const uint32_t first = u >> 3, count = (u & 7u) + 1u;
             for (uint32_t i = 0; i < count; ++i) {
-                const float4* tq = reinterpret_cast<const float4*>(tris + first + i);
-                const float4 A = __ldg(tq), B = __ldg(tq + 1), C = __ldg(tq + 2);
-                float t;
-                if (!hit_tri(wr, mk(A.x, A.y, A.z), mk(B.x, B.y, B.z), mk(C.x, C.y, C.z), t)) continue;
-                const int id = __float_as_int(A.w);
+                float t, fid;
+                if (!hit_leaf(wr, o, d, tris + first + i, t, fid)) continue;
+                const int id = __float_as_int(fid);
                 if (t < best || (best_tri >= 0 && t == best && id < best_tri)) {
                     best = t;
                     best_tri = id;
