@@ -473,6 +473,17 @@ __global__ void __launch_bounds__(kConvThreads, 1) tc_conv_kernel(const __grid_c
 #pragma unroll
                     for (int j = 0; j < 16; ++j) hz += __bfloat162float(__float2bfloat16_rn(f[j])) * e.head_w[col + j];
                 const size_t o = pix * e.ldc + col;
+                if (e.gate) {
+                    const uint4* g4 = reinterpret_cast<const uint4*>(e.gate + o);
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const uint4 gv = g4[h];
+                        const __nv_bfloat16* gb = reinterpret_cast<const __nv_bfloat16*>(&gv);
+#pragma unroll
+                        for (int j = 0; j < 8; ++j)
+                            if (!(__bfloat162float(gb[j]) > 0.0f)) f[h * 8 + j] = 0.0f;
+                    }
+                }
                 if (e.c16) {
                     uint4 out[2];
                     __nv_bfloat16* ob = reinterpret_cast<__nv_bfloat16*>(out);
@@ -1012,6 +1023,17 @@ __global__ void __launch_bounds__(kConvThreads, kFan ? fan_ctas(BN) : 1) tc_conv
                         for (int jj = 0; jj < 16; ++jj)
                             hz += __bfloat162float(__float2bfloat16_rn(f[jj])) * e.head_w[c0 + jj];
                     const size_t o = pix * e.ldc + n0 + c0;
+                    if (e.gate) {
+                        const uint4* g4 = reinterpret_cast<const uint4*>(e.gate + o);
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            const uint4 gv = g4[h];
+                            const __nv_bfloat16* gb = reinterpret_cast<const __nv_bfloat16*>(&gv);
+#pragma unroll
+                            for (int j = 0; j < 8; ++j)
+                                if (!(__bfloat162float(gb[j]) > 0.0f)) f[h * 8 + j] = 0.0f;
+                        }
+                    }
                     if (e.c16) {
                         uint4 out[2];
                         __nv_bfloat16* ob = reinterpret_cast<__nv_bfloat16*>(out);
@@ -1054,6 +1076,188 @@ __global__ void __launch_bounds__(kConvThreads, kFan ? fan_ctas(BN) : 1) tc_conv
                     __syncwarp();                                         // the stage is free again
                 }
             }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 1)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kCols) : "memory");
+}
+
+// ------------------------------------------------------------------ weight gradient
+// dW[(tap, ci)][n] = sum over pixels of x[pixel + tap][ci] * dz[pixel][n]: a contraction over
+// pixels whose operands both lie channel-contiguous in memory, so both are read MN-major
+// (tcgen05's transposed operands): a TMA box of 64 pixels x CA channels at a tap's offset lands
+// in shared memory as rows of CA channels, which is the canonical MN-major tile (CA 64, 32 or 16
+// channels: 128-, 64- or 32-byte swizzle; 8 pixels per swizzle atom, the atoms of a tile one
+// after the other along the channels). The border reads TMA's zero fill, the convolution's
+// padding. No im2col rows are formed and nothing is transposed in memory: at batch 64 of
+// 128 x 128 the 14 layers took 12.2 ms as im2col, two transposes and a GEMM.
+//
+// An "atom" is one (tap, CA-channel chunk); 128 / CA atoms make an M tile of 128 weight rows. A
+// CTA takes a group of up to 256 / N M tiles (256 TMEM columns, two CTAs per SM) and a slice of
+// the pixel boxes: per box it loads dz once and each M tile's atoms through a ring, so dz is
+// read once per group, and every x element nine times, from L2. At the end it adds its tiles
+// to gw with FP32 atomics. Roles: warp 0 loads (its lanes issue a tile's atoms together), one
+// lane of warp 1 issues the MMAs, warps 2..5 read the accumulators. Waits are bounded and give
+// up when another role has aborted.
+struct WgradArgs {
+    int nb0, nb1;               // CA-channel chunks of the sources
+    int tiles_x, tiles_y;       // 64-pixel boxes per image row / column
+    int tw, th;
+    int boxes;                  // all images' boxes
+    int natoms, mtiles;         // 9 (nb0 + nb1); M tiles over them
+    int per_group, groups, slices;
+    int cin_out, ch_valid;
+    float* gw;
+    uint32_t* err;
+};
+constexpr int kWgPix = 64;
+__host__ __device__ constexpr int wg_a_stages(int n) { return n == 32 ? 6 : n == 64 ? 5 : n == 128 ? 4 : 2; }
+__host__ __device__ constexpr int wg_b_stages(int n) { return n <= 64 ? 3 : 2; }
+
+// MN-major descriptor: atoms of CA channels (CA * 2 bytes a pixel row) one box apart along M or
+// N (the leading offset), 8-pixel groups 8 rows apart along K (the stride offset).
+template <int CA>
+__device__ __forceinline__ uint64_t desc_mn(uint32_t addr) {
+    constexpr uint32_t row = CA * 2;
+    uint64_t d = (uint64_t)((addr >> 4) & 0x3FFFu);
+    d |= (uint64_t)(((kWgPix * row) >> 4) & 0x3FFFu) << 16;
+    d |= (uint64_t)(((8 * row) >> 4) & 0x3FFFu) << 32;
+    d |= (uint64_t)1 << 46;
+    d |= (uint64_t)(CA == 64 ? 2 : CA == 32 ? 4 : 6) << 61;
+    return d;
+}
+
+template <int N, int CA>
+__global__ void __launch_bounds__(kConvThreads, 2) tc_wgrad_kernel(const __grid_constant__ CUtensorMap map0,
+                                                                   const __grid_constant__ CUtensorMap map1,
+                                                                   const __grid_constant__ CUtensorMap mapZ,
+                                                                   const WgradArgs a) {
+    constexpr int kA = wg_a_stages(N), kB = wg_b_stages(N), kApt = 128 / CA, CB = N >= 64 ? 64 : 32;
+    constexpr uint32_t kAtom = kWgPix * CA * 2, kABytes = kWgPix * 128 * 2, kBBytes = kWgPix * N * 2;
+    constexpr uint32_t kCols = 256;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    uint8_t* sA = smem;
+    uint8_t* sB = smem + kA * kABytes;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sB + kB * kBBytes);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * (kA + kB) + 1);
+    __shared__ int s_abort;
+    volatile int* abort_flag = &s_abort;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    auto a_full = [&](int s) { return smem_u32(&bars[s]); };
+    auto a_empty = [&](int s) { return smem_u32(&bars[kA + s]); };
+    auto b_full = [&](int s) { return smem_u32(&bars[2 * kA + s]); };
+    auto b_empty = [&](int s) { return smem_u32(&bars[2 * kA + kB + s]); };
+    const uint32_t done = smem_u32(&bars[2 * (kA + kB)]);
+    // this CTA's M tiles [m0, m0 + nm) and boxes [k0, k1)
+    const int group = (int)blockIdx.x % a.groups, slice = (int)blockIdx.x / a.groups;
+    const int m0 = group * a.per_group, nm = min(a.per_group, a.mtiles - m0);
+    const int k0 = (int)((long long)a.boxes * slice / a.slices), k1 = (int)((long long)a.boxes * (slice + 1) / a.slices);
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < kA; ++s) { mbar_init(a_full(s), 1); mbar_init(a_empty(s), 1); }
+        for (int s = 0; s < kB; ++s) { mbar_init(b_full(s), 1); mbar_init(b_empty(s), 1); }
+        mbar_init(done, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        s_abort = 0;
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                     "r"(kCols)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+
+    if (warp == 0) {
+        // every lane waits for the slot; lane 0 arms its barrier before the lanes issue the copies
+        const int nchunk = a.nb0 + a.nb1;
+        uint32_t ia = 0, ib = 0;
+        bool ok = true;
+        for (int k = k0; ok && k < k1; ++k, ++ib) {
+            const int x = (k % a.tiles_x) * a.tw, y = ((k / a.tiles_x) % a.tiles_y) * a.th, b = k / (a.tiles_x * a.tiles_y);
+            const int sb = (int)(ib % kB);
+            ok = __all_sync(0xffffffffu, mbar_wait_or_abort(b_empty(sb), ((ib / kB) & 1u) ^ 1u, abort_flag));
+            if (!ok) break;
+            if (lane == 0) mbar_expect_tx(b_full(sb), kBBytes);
+            __syncwarp();
+            if (lane < N / CB) tma_load_4d(smem_u32(sB + sb * kBBytes) + lane * kWgPix * CB * 2, &mapZ, lane * CB, x, y, b, b_full(sb));
+            for (int m = 0; m < nm; ++m, ++ia) {
+                const int sa = (int)(ia % kA);
+                ok = __all_sync(0xffffffffu, mbar_wait_or_abort(a_empty(sa), ((ia / kA) & 1u) ^ 1u, abort_flag));
+                if (!ok) break;
+                const int j0 = (m0 + m) * kApt, nat = min(kApt, a.natoms - j0);
+                if (lane == 0) mbar_expect_tx(a_full(sa), (uint32_t)nat * kAtom);
+                __syncwarp();
+                if (lane < nat) {
+                    const int j = j0 + lane, tap = j / nchunk, c = j % nchunk;
+                    const bool second = c >= a.nb0;
+                    tma_load_4d(smem_u32(sA + sa * kABytes) + lane * kAtom, second ? &map1 : &map0,
+                                (second ? c - a.nb0 : c) * CA, x + tap % 3 - 1, y + tap / 3 - 1, b, a_full(sa));
+                }
+            }
+        }
+        if (!ok && lane == 0) { atomicOr(a.err, DEV_GUARD); s_abort = 1; }
+        // the copies issued must land before the CTA can leave
+        if (lane == 0) {
+            for (uint32_t i = ia > (uint32_t)kA ? ia - kA : 0; i < ia; ++i) mbar_wait(a_full((int)(i % kA)), (i / kA) & 1u);
+            for (uint32_t i = ib > (uint32_t)kB ? ib - kB : 0; i < ib; ++i) mbar_wait(b_full((int)(i % kB)), (i / kB) & 1u);
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {
+            constexpr uint32_t idesc = instr_desc(N) | (1u << 15) | (1u << 16);      // A and B MN-major
+            uint32_t ia = 0, ib = 0;
+            bool ok = true;
+            for (int k = k0; ok && k < k1; ++k, ++ib) {
+                const int sb = (int)(ib % kB);
+                ok = mbar_wait_or_abort(b_full(sb), (ib / kB) & 1u, abort_flag);
+                const uint64_t db = desc_mn<CB>(smem_u32(sB + sb * kBBytes));
+                for (int m = 0; ok && m < nm; ++m, ++ia) {
+                    const int sa = (int)(ia % kA);
+                    ok = mbar_wait_or_abort(a_full(sa), (ia / kA) & 1u, abort_flag);
+                    if (!ok) break;
+                    tc_fence_after();
+                    const uint64_t da = desc_mn<CA>(smem_u32(sA + sa * kABytes));
+#pragma unroll
+                    for (int q = 0; q < kWgPix / 16; ++q)       // 16 pixels: two 8-row groups further
+                        tc_mma(tmem + (uint32_t)(m * N), da + (uint64_t)(q * ((16 * CA * 2) >> 4)),
+                               db + (uint64_t)(q * ((16 * CB * 2) >> 4)), idesc, (k > k0 || q > 0) ? 1u : 0u);
+                    tc_commit(a_empty(sa));
+                }
+                tc_commit(b_empty(sb));
+            }
+            if (!ok) { atomicOr(a.err, DEV_GUARD); s_abort = 1; }
+            tc_commit(done);
+        }
+    } else {
+        const int q = warp & 3, r = q * 32 + lane;
+        const bool ok = __all_sync(0xffffffffu, mbar_wait_or_abort(done, 0, abort_flag)) && !*abort_flag;
+        tc_fence_after();
+        if (__all_sync(0xffffffffu, ok) && k1 > k0) {
+            const int nchunk = a.nb0 + a.nb1;
+            for (int m = 0; m < nm; ++m) {
+                const int j = (m0 + m) * kApt + r / CA, ch = r % CA, tap = j / nchunk, c = j % nchunk;
+                const bool real = j < a.natoms && (a.ch_valid == 0 || ch < a.ch_valid);
+                float* row = a.gw + (size_t)(tap * a.cin_out + c * CA + ch) * N;
+#pragma unroll 1
+                for (int c0 = 0; c0 < N; c0 += 32) {
+                    uint32_t v[32];
+                    tmem_ld32(tmem + (uint32_t)(m * N + c0) + ((uint32_t)(q * 32) << 16), v);
+                    if (real)
+#pragma unroll
+                        for (int h = 0; h < 8; ++h)
+                            atomicAdd(reinterpret_cast<float4*>(row + c0) + h,
+                                      make_float4(__uint_as_float(v[4 * h]), __uint_as_float(v[4 * h + 1]),
+                                                  __uint_as_float(v[4 * h + 2]), __uint_as_float(v[4 * h + 3])));
+                }
+            }
+        } else if (!ok && lane == 0) {
+            atomicOr(a.err, DEV_GUARD);
         }
     }
     tc_fence_before();
@@ -1114,8 +1318,26 @@ bool make_map_nhwc(CUtensorMap* m, const void* base, int B, int H, int W, int C,
     const cuuint32_t box[4] = {(cuuint32_t)cb, (cuuint32_t)tw, (cuuint32_t)th, 1};
     const cuuint32_t elem[4] = {1, 1, 1, 1};
     return fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, elem,
-              CU_TENSOR_MAP_INTERLEAVE_NONE, cb == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
+              CU_TENSOR_MAP_INTERLEAVE_NONE,
+              cb == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : cb == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B,
               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+template <int N, int CA>
+int launch_wgrad(const CUtensorMap& m0, const CUtensorMap& m1, const CUtensorMap& mz, const WgradArgs& a, cudaStream_t s) {
+    const size_t smem = 1024 + wg_a_stages(N) * kWgPix * 128 * 2 + wg_b_stages(N) * kWgPix * N * 2 +
+                        (2 * (wg_a_stages(N) + wg_b_stages(N)) + 1) * 8 + 16;
+    static bool attr = false;
+    if (!attr) {
+        if (cudaFuncSetAttribute(tc_wgrad_kernel<N, CA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+                cudaSuccess ||
+            cudaFuncSetAttribute(tc_wgrad_kernel<N, CA>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                 cudaSharedmemCarveoutMaxShared) != cudaSuccess)
+            return RN_ERR_CUDA;
+        attr = true;
+    }
+    tc_wgrad_kernel<N, CA><<<a.groups * a.slices, kConvThreads, smem, s>>>(m0, m1, mz, a);
+    return cudaGetLastError() == cudaSuccess ? RN_OK : RN_ERR_CUDA;
 }
 
 template <int BN, int CB, int kT>
@@ -1283,7 +1505,8 @@ int tc_conv3x3(const tc::ConvSrc* src, int nsrc, int B, int H, int W, const __nv
         cin += src[i].C;
     }
     if (ldw < 9 * cin || ldw % 8 || ((uintptr_t)w % 16)) return fail(st, RN_ERR_INVALID, "tc_conv3x3: weight stride %d", ldw);
-    if (epi.atomic || epi.gate) return fail(st, RN_ERR_INVALID, "tc_conv3x3: no atomic or gated epilogue");
+    if (epi.atomic || (epi.gate && (!epi.c16 || epi.c32 || up16 || epi.head_out)))
+        return fail(st, RN_ERR_INVALID, "tc_conv3x3: no atomic epilogue, and a gated one has a BF16 output alone");
     if (epi.head_out && (N != 32 || !epi.head_w || !epi.head_b || up16))
         return fail(st, RN_ERR_INVALID, "tc_conv3x3: the fused head needs N 32, its weights and no upsampled copy");
     int bn = (N == 32 || N == 64 || N == 128 || N == 256) ? N : 128;
@@ -1415,6 +1638,61 @@ int tc_conv3x3(const tc::ConvSrc* src, int nsrc, int B, int H, int W, const __nv
     }
 #undef RN_CONV_CASE
     if (rc != RN_OK) return cuda_fail(st, cudaGetLastError(), "tc_conv_kernel");
+    return RN_OK;
+}
+
+int tc_wgrad3x3(const tc::ConvSrc* src, int nsrc, int B, int H, int W, const __nv_bfloat16* dz, int N, float* gw,
+                int cin_out, int ch_valid, uint32_t* err, cudaStream_t s, rn_status* st) {
+    const tc::ConvTiling t = tc::conv_tiling(H, W);
+    if (nsrc < 1 || nsrc > 2 || !src || !dz || !gw || B <= 0 || !t.ok)
+        return fail(st, RN_ERR_INVALID, "tc_wgrad3x3: %dx%dx%d, %d sources", B, H, W, nsrc);
+    if (N != 32 && N != 64 && N != 128 && N != 256) return fail(st, RN_ERR_INVALID, "tc_wgrad3x3 N %d", N);
+    int ca = 64;
+    for (int i = 0; i < nsrc; ++i)
+        while (ca >= 16 && src[i].C % ca) ca /= 2;
+    if (ca < 16) return fail(st, RN_ERR_INVALID, "tc_wgrad3x3: source channels");
+    // 64-pixel boxes: tw x th with tw a power of two dividing W, th dividing H
+    const int tw = std::min(1 << t.tw_log2, tc::kWgPix), th = tc::kWgPix / tw;
+    CUtensorMap m[2], mz;
+    for (int i = 0; i < nsrc; ++i)
+        if (!tc::make_map_nhwc(&m[i], src[i].ptr, B, H, W, src[i].C, tw, th, ca))
+            return fail(st, RN_ERR_CUDA, "cuTensorMapEncodeTiled (activation) failed");
+    if (nsrc == 1) m[1] = m[0];
+    if (!tc::make_map_nhwc(&mz, dz, B, H, W, N, tw, th, N >= 64 ? 64 : 32))
+        return fail(st, RN_ERR_CUDA, "cuTensorMapEncodeTiled (gradient) failed");
+    tc::WgradArgs a{};
+    a.nb0 = src[0].C / ca;
+    a.nb1 = nsrc > 1 ? src[1].C / ca : 0;
+    a.tw = tw; a.th = th;
+    a.tiles_x = W / tw; a.tiles_y = H / th;
+    a.boxes = B * a.tiles_x * a.tiles_y;
+    a.natoms = 9 * (a.nb0 + a.nb1);
+    a.mtiles = (a.natoms * ca + 127) / 128;
+    // groups of equal size, at most 256 TMEM columns; pixel slices so that the items fill two
+    // CTAs an SM once
+    a.groups = (a.mtiles + 256 / N - 1) / (256 / N);
+    a.per_group = (a.mtiles + a.groups - 1) / a.groups;
+    a.groups = (a.mtiles + a.per_group - 1) / a.per_group;
+    a.slices = std::max(1, std::min(a.boxes, 2 * ctx().sm_count / a.groups));
+    a.cin_out = cin_out;
+    a.ch_valid = ch_valid;
+    a.gw = gw;
+    a.err = err;
+    int rc = RN_ERR_INVALID;
+#define RN_WGRAD_CASE(NV)                                                            \
+    case NV:                                                                         \
+        rc = ca == 64   ? tc::launch_wgrad<NV, 64>(m[0], m[1], mz, a, s)             \
+             : ca == 32 ? tc::launch_wgrad<NV, 32>(m[0], m[1], mz, a, s)             \
+                        : tc::launch_wgrad<NV, 16>(m[0], m[1], mz, a, s);            \
+        break;
+    switch (N) {
+        RN_WGRAD_CASE(32)
+        RN_WGRAD_CASE(64)
+        RN_WGRAD_CASE(128)
+        RN_WGRAD_CASE(256)
+    }
+#undef RN_WGRAD_CASE
+    if (rc != RN_OK) return cuda_fail(st, cudaGetLastError(), "tc_wgrad_kernel");
     return RN_OK;
 }
 

@@ -14,7 +14,8 @@ struct Epilogue {
     float* c32;                      // FP32 output (split K: accumulated with atomics)
     __nv_bfloat16* c16;              // BF16 output
     const float* bias;               // [N] or null
-    const __nv_bfloat16* gate;       // [M][ldc]: output zeroed where gate <= 0 (ReLU backward), or null
+    const __nv_bfloat16* gate;       // [M][ldc]: output zeroed where gate is not > 0 (ReLU backward), or null
+                                     // (convolutions: with a BF16 output alone)
     int relu;
     int atomic;
     int k_per_split;                 // K range of one grid.z slice (a multiple of 64)
@@ -55,6 +56,16 @@ ConvTiling conv_tiling(int H, int W);
 // up16, when set, also receives the output upsampled 2x (nearest) at (2H, 2W).
 int tc_conv3x3(const tc::ConvSrc* src, int nsrc, int B, int H, int W, const __nv_bfloat16* w, int ldw, int N,
                const tc::Epilogue& epi, __nv_bfloat16* up16, cudaStream_t s, rn_status* st);
+
+// Weight gradient of such a convolution, from the activations in place (no im2col rows, no
+// transposes): gw[k][n] += sum over pixels of src[pixel + tap][ci] * dz[pixel][n], with
+// k = tap * cin_out + ci, FP32 row stride N, added atomically (the caller zeroes gw). The
+// sources' channels are concatenated; cin_out and ch_valid: the weights' input channels and how
+// many of a chunk's stored channels they have (a padded input: cin_out = ch_valid < C; else
+// cin_out = sum of src[i].C and ch_valid = 0). dz NHWC BF16 [B][H][W][N], N 32, 64, 128 or 256;
+// each C a multiple of 16; H and W as conv_tiling takes them.
+int tc_wgrad3x3(const tc::ConvSrc* src, int nsrc, int B, int H, int W, const __nv_bfloat16* dz, int N, float* gw,
+                int cin_out, int ch_valid, uint32_t* err, cudaStream_t s, rn_status* st);
 
 // C (M x N, row stride ldc) = P (M x K, row stride ldp) * Q (N x K, row stride ldq)^T.
 // M % 128 == 0, N in {32, 64, 128, 256} or a multiple of 128, K % (64 * splits) == 0;

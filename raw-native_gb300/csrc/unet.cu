@@ -11,12 +11,18 @@
 //   level 0            d0a = conv([e0, up d1]; 96->32)   d0 = conv(d0a; 32->32)
 //   head               out = sigmoid(1x1 conv(d0; 32->1))
 // Every 3x3 convolution is followed by ReLU; pooling is a 2x2 average, upsampling nearest.
-// Activations are NHWC BF16. A convolution is a GEMM of its im2col rows (the concat and the
-// upsample are read in place, never materialized) with the weights [Cout][9 Cin]:
+// Activations are NHWC BF16. A convolution is a GEMM of its im2col rows with the weights
+// [Cout][9 Cin], formed implicitly (gemm_tc.cu) where every level's size can be tiled:
 //   forward  Y = im2col(X) W^T (+ bias, ReLU in the epilogue);
 //   wgrad    dW^T = im2col(X)^T dZ (split over pixels, FP32 atomics);
 //   dgrad    dX = im2col(dZ) W'^T with W'[ci][tap', co] = W[co][8 - tap', ci] (the flipped,
-//            transposed kernel), routed back to the sources (2x2 sums for an upsampled one).
+//            transposed kernel).
+// Backward, implicit form: a layer whose input is another layer's output alone writes that
+// layer's dZ (gated, BF16) from the dgrad epilogue. The three concatenated layers leave dX in
+// FP32; one pass sums the upsampled half's 2x2 blocks into its producer's dZ, and the skip half
+// waits for the pooled tensor's gradient, with which one pass forms the encoder layer's dZ. At
+// batch 64 of 128 x 128 a step took 26.1 ms with separate zeroing, routing, pooling, gating and
+// column-sum passes over FP32 accumulators of every tensor.
 // Loss: mean squared error of the sigmoid output; optimizer: Adam on FP32 master weights,
 // which refreshes the BF16 copies the GEMMs read.
 #include "gemm_tc.h"
@@ -161,58 +167,170 @@ __global__ void gate_kernel(const float* __restrict__ dout, const bf16* __restri
         dz[i] = __float2bfloat16_rn(__bfloat162float(out[i]) > 0.0f ? dout[i] : 0.0f);
 }
 
-// db[c] += sum over rows of dZ[m][c] (C <= 256; blocks of 256 threads over row chunks).
-__global__ void colsum_kernel(const bf16* __restrict__ dz, size_t M, int C, float* __restrict__ db) {
-    const int c = threadIdx.x;
-    if (c >= C) return;
-    float s = 0.0f;
-    for (size_t m = blockIdx.x; m < M; m += gridDim.x) s += __bfloat162float(dz[m * C + c]);
-    atomicAdd(db + c, s);
+// db[c] += sum over rows of dZ[m][c], C a multiple of 8 up to 256: a thread keeps the sums of
+// eight channels over every (blocks x 256 / (C / 8))-th row, 16 bytes a load, then the block
+// adds its rows up in shared memory. Bound by HBM: 67 MB (level 0, batch 64 of 128 x 128) in
+// 19 us; a thread a channel over 256 blocks took 2.2 ms.
+__global__ void __launch_bounds__(256) colsum_kernel(const bf16* __restrict__ dz, size_t M, int C, float* __restrict__ db) {
+    const int G = C / 8, g = threadIdx.x % G, r = threadIdx.x / G, R = 256 / G;
+    float s[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+    for (size_t m = (size_t)blockIdx.x * R + r; m < M; m += (size_t)gridDim.x * R) {
+        const uint4 v = *reinterpret_cast<const uint4*>(dz + m * C + g * 8);
+        const bf16* h = reinterpret_cast<const bf16*>(&v);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) s[j] += __bfloat162float(h[j]);
+    }
+    __shared__ float part[256][9];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) part[threadIdx.x][j] = s[j];
+    __syncthreads();
+    if ((int)threadIdx.x < C) {
+        float t = 0.0f;
+        for (int q = 0; q < R; ++q) t += part[q * G + threadIdx.x / 8][threadIdx.x % 8];
+        atomicAdd(db + threadIdx.x, t);
+    }
 }
 
-// The head: out = sigmoid(d0 . wh + bh); with a target also the loss, dOut(d0) and the head's
-// gradients. C = 32 channels, one thread per pixel.
+// dZ of a layer whose output is read upsampled by a concatenated layer: columns [off, off + C) of
+// that layer's dX [B][2h][2w][ld] summed over 2x2 blocks, gated by the output. Eight channels a
+// thread.
+__global__ void up_gate_kernel(const float* __restrict__ dx, int ld, int off, int C, int B, int h, int w,
+                               const bf16* __restrict__ out, bf16* __restrict__ dz) {
+    const int G = C / 8;
+    const size_t total = (size_t)B * h * w * G;
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
+        const int c = (int)(i % G) * 8;
+        const size_t p = i / G;
+        const int x = (int)(p % w);
+        const size_t row = p / w;                               // b * h + y
+        const float* q = dx + (2 * row * (2 * (size_t)w) + 2 * x) * ld + off + c;
+        const size_t down = 2 * (size_t)w * ld;
+        const uint4 gv = *reinterpret_cast<const uint4*>(out + p * C + c);
+        const bf16* gb = reinterpret_cast<const bf16*>(&gv);
+        uint4 o;
+        bf16* ob = reinterpret_cast<bf16*>(&o);
+#pragma unroll
+        for (int v = 0; v < 2; ++v) {
+            const float4 a = *reinterpret_cast<const float4*>(q + 4 * v), b = *reinterpret_cast<const float4*>(q + ld + 4 * v);
+            const float4 d = *reinterpret_cast<const float4*>(q + down + 4 * v);
+            const float4 e = *reinterpret_cast<const float4*>(q + down + ld + 4 * v);
+            const float s[4] = {a.x + b.x + d.x + e.x, a.y + b.y + d.y + e.y, a.z + b.z + d.z + e.z, a.w + b.w + d.w + e.w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                ob[4 * v + j] = __float2bfloat16_rn(__bfloat162float(gb[4 * v + j]) > 0.0f ? s[j] : 0.0f);
+        }
+        *reinterpret_cast<uint4*>(dz + p * C + c) = o;
+    }
+}
+
+// dZ of an encoder layer whose output goes to a skip connection and to the pool: the first C
+// columns of the concatenated layer's dX [B][H][W][ld] plus a quarter of the pooled tensor's
+// gradient [B][H/2][W/2][C], gated by the output. Eight channels a thread.
+__global__ void skip_pool_gate_kernel(const float* __restrict__ dx, int ld, const float* __restrict__ dlo, int C, int B,
+                                      int H, int W, const bf16* __restrict__ out, bf16* __restrict__ dz) {
+    const int G = C / 8;
+    const size_t total = (size_t)B * H * W * G;
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
+        const int c = (int)(i % G) * 8;
+        const size_t p = i / G;
+        const int x = (int)(p % W), y = (int)((p / W) % H);
+        const size_t b = p / ((size_t)W * H);
+        const float* q = dx + p * ld + c;
+        const float* lo = dlo + ((b * (H / 2) + y / 2) * (W / 2) + x / 2) * C + c;
+        const uint4 gv = *reinterpret_cast<const uint4*>(out + p * C + c);
+        const bf16* gb = reinterpret_cast<const bf16*>(&gv);
+        uint4 o;
+        bf16* ob = reinterpret_cast<bf16*>(&o);
+#pragma unroll
+        for (int v = 0; v < 2; ++v) {
+            const float4 a = *reinterpret_cast<const float4*>(q + 4 * v), l = *reinterpret_cast<const float4*>(lo + 4 * v);
+            const float s[4] = {a.x + 0.25f * l.x, a.y + 0.25f * l.y, a.z + 0.25f * l.z, a.w + 0.25f * l.w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                ob[4 * v + j] = __float2bfloat16_rn(__bfloat162float(gb[4 * v + j]) > 0.0f ? s[j] : 0.0f);
+        }
+        *reinterpret_cast<uint4*>(dz + p * C + c) = o;
+    }
+}
+
+// The head's sigmoid of one pixel's 32 channels (f receives them).
+__device__ __forceinline__ float head_pixel(const bf16* __restrict__ d0, const float* __restrict__ wh, float bh, float (&f)[32]) {
+    const uint4* p = reinterpret_cast<const uint4*>(d0);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const uint4 v = p[q];
+        const bf16* h = reinterpret_cast<const bf16*>(&v);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) f[q * 8 + j] = __bfloat162float(h[j]);
+    }
+    float z = bh;
+#pragma unroll
+    for (int c = 0; c < 32; ++c) z += f[c] * wh[c];
+    return 1.0f / (1.0f + __expf(-z));
+}
+
+// The head: out = sigmoid(d0 . wh + bh). C = 32 channels, one thread per pixel.
 __global__ void head_kernel(const bf16* __restrict__ d0, const float* __restrict__ wh, const float* __restrict__ bh,
-                            size_t M, float* __restrict__ out, const float* __restrict__ target, float inv_m,
-                            float* __restrict__ dd0, float* __restrict__ gwh, float* __restrict__ gbh,
-                            float* __restrict__ loss) {
-    __shared__ float s_gw[32], s_gb, s_loss;
-    if (threadIdx.x < 32) s_gw[threadIdx.x] = 0.0f;
-    if (threadIdx.x == 0) { s_gb = 0.0f; s_loss = 0.0f; }
-    __syncthreads();
+                            size_t M, float* __restrict__ out) {
     const size_t m = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (m < M) {
-        float f[32];
-        const uint4* p = reinterpret_cast<const uint4*>(d0 + m * 32);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const uint4 v = p[q];
-            const bf16* h = reinterpret_cast<const bf16*>(&v);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) f[q * 8 + j] = __bfloat162float(h[j]);
-        }
-        float z = bh[0];
-#pragma unroll
-        for (int c = 0; c < 32; ++c) z += f[c] * wh[c];
-        const float s = 1.0f / (1.0f + __expf(-z));
-        if (out) out[m] = s;
-        if (target) {
-            const float diff = s - target[m];
-            const float dz = 2.0f * diff * s * (1.0f - s) * inv_m;
-            atomicAdd(&s_loss, diff * diff);
-            atomicAdd(&s_gb, dz);
-#pragma unroll
-            for (int c = 0; c < 32; ++c) {
-                dd0[m * 32 + c] = dz * wh[c];
-                atomicAdd(&s_gw[c], dz * f[c]);
-            }
-        }
-    }
+    if (m >= M) return;
+    float f[32];
+    out[m] = head_pixel(d0 + m * 32, wh, bh[0], f);
+}
+
+// The head in training: the loss, the head's gradients and dZ of the last layer (its output's
+// gradient dz_head * wh gated by the output, BF16). Each thread keeps its pixels' 34 sums in
+// registers; a warp adds them up by shuffles at its end, so the pixels cost no atomics (one
+// shared-memory atomic a pixel and channel took 0.72 ms at batch 64 of 128 x 128).
+__global__ void __launch_bounds__(256) head_train_kernel(const bf16* __restrict__ d0, const float* __restrict__ wh,
+                                                         const float* __restrict__ bh, size_t M,
+                                                         const float* __restrict__ target, float inv_m,
+                                                         bf16* __restrict__ dz, float* __restrict__ gwh,
+                                                         float* __restrict__ gbh, float* __restrict__ loss) {
+    __shared__ float s_wh[32], s_sum[34];
+    if (threadIdx.x < 32) s_wh[threadIdx.x] = wh[threadIdx.x];
+    if (threadIdx.x < 34) s_sum[threadIdx.x] = 0.0f;
     __syncthreads();
-    if (target) {
-        if (threadIdx.x < 32) atomicAdd(gwh + threadIdx.x, s_gw[threadIdx.x]);
-        if (threadIdx.x == 0) { atomicAdd(gbh, s_gb); atomicAdd(loss, s_loss); }
+    const float b = bh[0];
+    float gw[32], gb = 0.0f, ls = 0.0f;
+#pragma unroll
+    for (int c = 0; c < 32; ++c) gw[c] = 0.0f;
+    for (size_t m = (size_t)blockIdx.x * blockDim.x + threadIdx.x; m < M; m += (size_t)gridDim.x * blockDim.x) {
+        float f[32];
+        const float s = head_pixel(d0 + m * 32, s_wh, b, f);
+        const float diff = s - target[m];
+        const float g = 2.0f * diff * s * (1.0f - s) * inv_m;
+        ls += diff * diff;
+        gb += g;
+        uint4 o[4];
+        bf16* ob = reinterpret_cast<bf16*>(o);
+#pragma unroll
+        for (int c = 0; c < 32; ++c) {
+            gw[c] += g * f[c];
+            ob[c] = __float2bfloat16_rn(f[c] > 0.0f ? g * s_wh[c] : 0.0f);
+        }
+        uint4* d = reinterpret_cast<uint4*>(dz + m * 32);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) d[q] = o[q];
     }
+    const int lane = threadIdx.x & 31;
+    float mine = 0.0f;                     // lane c: the warp's sum of channel c
+#pragma unroll
+    for (int c = 0; c < 32; ++c) {
+        float t = gw[c];
+        for (int o = 16; o; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (lane == c) mine = t;
+    }
+    for (int o = 16; o; o >>= 1) {
+        gb += __shfl_xor_sync(0xffffffffu, gb, o);
+        ls += __shfl_xor_sync(0xffffffffu, ls, o);
+    }
+    atomicAdd(&s_sum[lane], mine);
+    if (lane == 0) { atomicAdd(&s_sum[32], gb); atomicAdd(&s_sum[33], ls); }
+    __syncthreads();
+    if (threadIdx.x < 32) atomicAdd(gwh + threadIdx.x, s_sum[threadIdx.x]);
+    if (threadIdx.x == 32) atomicAdd(gbh, s_sum[32]);
+    if (threadIdx.x == 33) atomicAdd(loss, s_sum[33]);
 }
 
 // fp32 features [M][5] -> bf16 [M][C] (C = 8, 16 or 32; channels 5.. zero)
@@ -473,7 +591,9 @@ struct rn_unet {
     size_t Tn[T_COUNT];   // elements
     int Tlevel[T_COUNT], TC[T_COUNT];
     bf16 *at, *dzt, *dz, *bcol;   // scratch: A^T, dZ^T, dZ, im2col(dZ)
-    float* dx;                    // scratch: dgrad output [M][cin_pad]
+    float* dx;                    // scratch: dgrad output [M][cin_pad] (implicit: a pooled tensor's gradient)
+    bf16* dz2;                    // implicit: the other layer's dZ (a dgrad reads one and writes one)
+    float* dcat[kLayers];         // implicit: dX of the three concatenated layers [M][cin_pad]
     float* loss;                  // device scalar
     float* host_loss;             // pinned: loss, gradient norm, clip scale
     float* gstats;                // device: see clip_kernel
@@ -556,21 +676,16 @@ int forward_all(rn_unet* u, cudaStream_t s, rn_status* st, float* head_out = nul
     return RN_OK;
 }
 
+// Explicit form: dT[l + 1] gated into dZ (the last layer's comes from the head), the layer's
+// weight gradient from its im2col rows, and dX routed into its sources' accumulators.
 int conv_backward(rn_unet* u, int l, cudaStream_t s, rn_status* st) {
     auto& Ly = u->L[l];
     const LayerSpec& sp = kSpec[l];
     const int H = u->H >> Ly.level, W = u->W >> Ly.level;
     const size_t M = pixels(u, Ly.level);
     // dZ: the gradient at the pre-activation
-    gate_kernel<<<grid_for(M * Ly.cout), 256, 0, s>>>(u->dT[l + 1], u->T[l + 1], M * Ly.cout, u->dz);
-    colsum_kernel<<<256, 256, 0, s>>>(u->dz, M, Ly.cout, Ly.gb);
-    if (u->implicit) {
-        // the forward left no im2col rows: form this layer's now (one shared buffer)
-        Im2col a{u->T[sp.s0.tensor], u->TC[sp.s0.tensor], sp.s0.up, nullptr, 0, 0, u->B, H, W, Ly.kpad, Ly.A};
-        if (sp.nsrc == 2) { a.s1 = u->T[sp.s1.tensor]; a.c1 = u->TC[sp.s1.tensor]; a.up1 = sp.s1.up; }
-        if (l == 0) { a.c0 = kInC; a.ld0 = u->TC[T_IN]; }
-        im2col_kernel<<<grid_for(M * (Ly.kpad / 8)), 256, 0, s>>>(a);
-    }
+    if (l != kLayers - 1) gate_kernel<<<grid_for(M * Ly.cout), 256, 0, s>>>(u->dT[l + 1], u->T[l + 1], M * Ly.cout, u->dz);
+    colsum_kernel<<<2 * ctx().sm_count, 256, 0, s>>>(u->dz, M, Ly.cout, Ly.gb);
     // wgrad: dW^T [kpad][cout] = A^T (kpad x M) * (dZ^T (cout x M))^T
     transpose_kernel<<<dim3(Ly.kpad / 32, (unsigned)(M / 32)), dim3(32, 8), 0, s>>>(Ly.A, (int)M, Ly.kpad, u->at);
     transpose_kernel<<<dim3(Ly.cout / 32, (unsigned)(M / 32)), dim3(32, 8), 0, s>>>(u->dz, (int)M, Ly.cout, u->dzt);
@@ -588,19 +703,55 @@ int conv_backward(rn_unet* u, int l, cudaStream_t s, rn_status* st) {
     ed.ldc = Ly.cin_pad;
     ed.c32 = u->dx;
     ed.err = ctx().dev_error;
-    if (u->implicit) {
-        const tc::ConvSrc src{u->dz, Ly.cout};
-        RN_TRY(tc_conv3x3(&src, 1, u->B, H, W, Ly.wt, Ly.kpad_t, Ly.cin_pad, ed, nullptr, s, st));
-    } else {
-        Im2col a{u->dz, Ly.cout, 0, nullptr, 0, 0, u->B, H, W, Ly.kpad_t, u->bcol};
-        im2col_kernel<<<grid_for(M * (Ly.kpad_t / 8)), 256, 0, s>>>(a);
-        RN_TRY(tc_gemm(u->bcol, Ly.kpad_t, Ly.wt, Ly.kpad_t, (int)M, Ly.cin_pad, Ly.kpad_t, 1, ed, s, st));
-    }
+    Im2col a{u->dz, Ly.cout, 0, nullptr, 0, 0, u->B, H, W, Ly.kpad_t, u->bcol};
+    im2col_kernel<<<grid_for(M * (Ly.kpad_t / 8)), 256, 0, s>>>(a);
+    RN_TRY(tc_gemm(u->bcol, Ly.kpad_t, Ly.wt, Ly.kpad_t, (int)M, Ly.cin_pad, Ly.kpad_t, 1, ed, s, st));
     const int c0 = u->TC[sp.s0.tensor];
     route_kernel<<<grid_for(M * c0), 256, 0, s>>>(u->dx, Ly.cin_pad, 0, c0, sp.s0.up, u->B, H, W, u->dT[sp.s0.tensor]);
     if (sp.nsrc == 2)
         route_kernel<<<grid_for(M * u->TC[sp.s1.tensor]), 256, 0, s>>>(u->dx, Ly.cin_pad, c0, u->TC[sp.s1.tensor],
                                                                          sp.s1.up, u->B, H, W, u->dT[sp.s1.tensor]);
+    return RN_OK;
+}
+
+// Implicit form: layer l's dZ is in u->dz (dz2 is free). Leaves layer l - 1's in u->dz.
+int conv_backward_implicit(rn_unet* u, int l, cudaStream_t s, rn_status* st) {
+    auto& Ly = u->L[l];
+    const LayerSpec& sp = kSpec[l];
+    const int H = u->H >> Ly.level, W = u->W >> Ly.level;
+    const size_t M = pixels(u, Ly.level);
+    colsum_kernel<<<2 * ctx().sm_count, 256, 0, s>>>(u->dz, M, Ly.cout, Ly.gb);
+    tc::ConvSrc src[2] = {{u->T[sp.s0.tensor], u->TC[sp.s0.tensor]}, {nullptr, 0}};
+    if (sp.nsrc == 2) src[1] = {sp.s1.up ? u->UT[sp.s1.tensor] : u->T[sp.s1.tensor], u->TC[sp.s1.tensor]};
+    RN_TRY(tc_wgrad3x3(src, sp.nsrc, u->B, H, W, u->dz, Ly.cout, Ly.gw, Ly.cin, l == 0 ? kInC : 0, ctx().dev_error, s, st));
+    if (l == 0) return RN_OK;                          // the input needs no gradient
+    const tc::ConvSrc dsrc{u->dz, Ly.cout};
+    tc::Epilogue e{};
+    e.err = ctx().dev_error;
+    const bool pooled = l == 2 || l == 4 || l == 6;
+    if (sp.nsrc == 1 && !pooled) {
+        // the input is layer l - 1's output and has no other reader: its dZ from the epilogue
+        e.ldc = Ly.cin_pad;
+        e.c16 = u->dz2;
+        e.gate = u->T[l];
+        RN_TRY(tc_conv3x3(&dsrc, 1, u->B, H, W, Ly.wt, Ly.kpad_t, Ly.cin_pad, e, nullptr, s, st));
+    } else {
+        float* dx = pooled ? u->dx : u->dcat[l];
+        e.ldc = Ly.cin_pad;
+        e.c32 = dx;
+        RN_TRY(tc_conv3x3(&dsrc, 1, u->B, H, W, Ly.wt, Ly.kpad_t, Ly.cin_pad, e, nullptr, s, st));
+        const int C = u->TC[l];                        // layer l - 1's output: the upsampled half, or the pool's input
+        if (pooled) {
+            // the skip half of that output's other reader: layer 12, 10 or 8
+            const int cat = 14 - l;
+            skip_pool_gate_kernel<<<grid_for(4 * M * (C / 8)), 256, 0, s>>>(u->dcat[cat], u->L[cat].cin_pad, dx, C, u->B,
+                                                                           2 * H, 2 * W, u->T[l], u->dz2);
+        } else {
+            up_gate_kernel<<<grid_for(M / 4 * (C / 8)), 256, 0, s>>>(dx, Ly.cin_pad, u->TC[sp.s0.tensor], C, u->B, H / 2,
+                                                                    W / 2, u->T[l], u->dz2);
+        }
+    }
+    std::swap(u->dz, u->dz2);
     return RN_OK;
 }
 
@@ -699,12 +850,12 @@ int rn_unet_create(int batch, int height, int width, uint64_t seed, uint32_t fla
         max_a = std::max(max_a, M * Ly.kpad);
         max_dz = std::max(max_dz, M * Ly.cout);
         max_bcol = std::max(max_bcol, M * Ly.kpad_t);
-        max_dx = std::max(max_dx, M * Ly.cin_pad);
+        if (!u->implicit || l == 2 || l == 4 || l == 6) max_dx = std::max(max_dx, M * Ly.cin_pad);
     }
     max_at = max_a;
     if (u->inference || u->implicit) {   // the layers run in order: one im2col buffer serves all
-        // (implicit inference forms no im2col rows at all)
-        const size_t need = (u->implicit && u->inference) ? 8 : max_a;
+        // (the implicit form makes no im2col rows at all)
+        const size_t need = u->implicit ? 8 : max_a;
         bf16* shared = nullptr;
         if (ualloc(u, (void**)&shared, need * 2, st)) return bail(RN_ERR_NO_MEMORY);
         for (auto& Ly : u->L) Ly.A = shared;
@@ -728,7 +879,7 @@ int rn_unet_create(int batch, int height, int width, uint64_t seed, uint32_t fla
         u->TC[t] = (t == T_IN && u->implicit) ? (u->W % 128 == 0 ? 16 : 32) : tch[t];
         u->Tn[t] = pixels(u, tlevel[t]) * u->TC[t];
         if (ualloc(u, (void**)&u->T[t], u->Tn[t] * 2, st) ||
-            (!u->inference && ualloc(u, (void**)&u->dT[t], u->Tn[t] * 4, st)))
+            (!u->inference && !u->implicit && ualloc(u, (void**)&u->dT[t], u->Tn[t] * 4, st)))
             return bail(RN_ERR_NO_MEMORY);
     }
     if (u->implicit) {
@@ -739,11 +890,18 @@ int rn_unet_create(int batch, int height, int width, uint64_t seed, uint32_t fla
         for (int t : {8, 10, 12})            // b3, d2, d1: read upsampled by d2a, d1a, d0a
             if (ualloc(u, (void**)&u->UT[t], pixels(u, u->Tlevel[t] - 1) * u->TC[t] * 2, st))
                 return bail(RN_ERR_NO_MEMORY);
-    if (!u->inference &&
-        (ualloc(u, (void**)&u->at, max_at * 2, st) || ualloc(u, (void**)&u->dzt, max_dz * 2, st) ||
-         ualloc(u, (void**)&u->dz, max_dz * 2, st) || ualloc(u, (void**)&u->bcol, (u->implicit ? 8 : max_bcol) * 2, st) ||
-         ualloc(u, (void**)&u->dx, max_dx * 4, st)))
+    if (!u->inference && (ualloc(u, (void**)&u->dz, max_dz * 2, st) || ualloc(u, (void**)&u->dx, max_dx * 4, st)))
         return bail(RN_ERR_NO_MEMORY);
+    if (!u->inference && !u->implicit &&
+        (ualloc(u, (void**)&u->at, max_at * 2, st) || ualloc(u, (void**)&u->dzt, max_dz * 2, st) ||
+         ualloc(u, (void**)&u->bcol, max_bcol * 2, st)))
+        return bail(RN_ERR_NO_MEMORY);
+    if (!u->inference && u->implicit) {
+        if (ualloc(u, (void**)&u->dz2, max_dz * 2, st)) return bail(RN_ERR_NO_MEMORY);
+        for (int l : {8, 10, 12})
+            if (ualloc(u, (void**)&u->dcat[l], pixels(u, u->L[l].level) * u->L[l].cin_pad * 4, st))
+                return bail(RN_ERR_NO_MEMORY);
+    }
     if (cudaMallocHost((void**)&u->host_loss, 16) != cudaSuccess) return bail(fail(st, RN_ERR_NO_MEMORY, "pinned loss"));
     std::memset(u->host_loss, 0, 16);
     if (ualloc(u, (void**)&u->gstats, 16, st)) return bail(RN_ERR_NO_MEMORY);
@@ -791,8 +949,7 @@ int rn_unet_forward(rn_unet* u, const float* input, int batch, float* output, rn
         RN_TRY(forward_all(u, s, st, output));         // the head in the last layer's epilogue
     } else {
         RN_TRY(forward_all(u, s, st));
-        head_kernel<<<(unsigned)((M + 255) / 256), 256, 0, s>>>(u->T[14], u->wh, u->bh, M, output, nullptr, 0.0f,
-                                                               nullptr, nullptr, nullptr, nullptr);
+        head_kernel<<<(unsigned)((M + 255) / 256), 256, 0, s>>>(u->T[14], u->wh, u->bh, M, output);
     }
     RN_CUDA(cudaGetLastError(), st);
     return ok(st);
@@ -809,7 +966,8 @@ int rn_unet_backward(rn_unet* u, const float* input, const float* target, int ba
     input_kernel<<<grid_for(M), 256, 0, s>>>(input, M, u->TC[T_IN], u->T[T_IN]);
     RN_TRY(forward_all(u, s, st));
     // zero the gradient accumulators
-    for (int t = 0; t < T_COUNT; ++t) RN_CUDA(cudaMemsetAsync(u->dT[t], 0, u->Tn[t] * 4, s), st);
+    if (!u->implicit)
+        for (int t = 0; t < T_COUNT; ++t) RN_CUDA(cudaMemsetAsync(u->dT[t], 0, u->Tn[t] * 4, s), st);
     for (int l = 0; l < kLayers; ++l) {
         RN_CUDA(cudaMemsetAsync(u->L[l].gw, 0, (size_t)u->L[l].kpad * u->L[l].cout * 4, s), st);
         RN_CUDA(cudaMemsetAsync(u->L[l].gb, 0, (size_t)u->L[l].cout * 4, s), st);
@@ -817,9 +975,13 @@ int rn_unet_backward(rn_unet* u, const float* input, const float* target, int ba
     RN_CUDA(cudaMemsetAsync(u->gwh, 0, 32 * 4, s), st);
     RN_CUDA(cudaMemsetAsync(u->gbh, 0, 4, s), st);
     RN_CUDA(cudaMemsetAsync(u->loss, 0, 4, s), st);
-    head_kernel<<<(unsigned)((M + 255) / 256), 256, 0, s>>>(u->T[14], u->wh, u->bh, M, nullptr, target, 1.0f / (float)M,
-                                                           u->dT[14], u->gwh, u->gbh, u->loss);
+    head_train_kernel<<<2 * ctx().sm_count, 256, 0, s>>>(u->T[14], u->wh, u->bh, M, target, 1.0f / (float)M, u->dz, u->gwh,
+                                                         u->gbh, u->loss);
     for (int l = kLayers - 1; l >= 0; --l) {
+        if (u->implicit) {
+            RN_TRY(conv_backward_implicit(u, l, s, st));
+            continue;
+        }
         RN_TRY(conv_backward(u, l, s, st));
         // pooled tensors feed encoder levels: their gradients flow back through the pool
         if (l == 6) pool_back_kernel<<<grid_for(u->Tn[6]), 256, 0, s>>>(u->dT[T_P2], u->B, u->H >> 2, u->W >> 2, 128, u->dT[6]);
@@ -964,8 +1126,7 @@ int rn_surrogate_ao(rn_unet* u, const rn_gbuf* g, const float* depth, const rn_a
         RN_TRY(forward_all(u, s, st, pr));             // the head in the last layer's epilogue
     } else {
         RN_TRY(forward_all(u, s, st));
-        head_kernel<<<(unsigned)((npad + 255) / 256), 256, 0, s>>>(u->T[14], u->wh, u->bh, npad, pr, nullptr, 0.0f,
-                                                                  nullptr, nullptr, nullptr, nullptr);
+        head_kernel<<<(unsigned)((npad + 255) / 256), 256, 0, s>>>(u->T[14], u->wh, u->bh, npad, pr);
     }
     // 4. the band test, 5. the fallback trace, 6. the composite
     band_kernel<<<dim3(tx, ty), kTile * kTile, 0, s>>>(pr, u->W, a4, g->mask, w, h, k, tf, fbm, counts, fb_list);

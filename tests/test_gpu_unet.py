@@ -200,3 +200,11 @@ def test_unet_step_in_halves_and_data_parallel_average(rn):
     r0.apply(1e-3)
     r1.apply(1e-3)
     assert np.array_equal(r0.get_params(), r1.get_params())
+
+
+@pytest.mark.parametrize("B,H,W", [(1, 128, 64), (1, 256, 96), (1, 512, 16), (3, 128, 384)])
+def test_implicit_gradients_match_torch_over_box_shapes(rn, B, H, W):
+    """The implicit backward where its weight gradients' 64-pixel boxes are whole rows, several
+    rows and 2-pixel columns, and with both paddings of the input's channels: the same
+    comparison and bounds as above."""
+    test_unet_gradients_match_torch(rn, B, H, W, False)
