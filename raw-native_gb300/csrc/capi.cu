@@ -702,12 +702,12 @@ int rn_gtao(const rn_gbuf* g, const float* camera, float radius, int slices, int
     void *vp, *vn, *vd;
     RN_TRY(ws_get(WS_VPOS, np * 12, &vp, st));
     RN_TRY(ws_get(WS_VNRM, np * 12, &vn, st));
-    RN_TRY(ws_get(WS_VDEPTH, np * 4, &vd, st));
+    RN_TRY(ws_get(WS_VDEPTH, gtao_depth_cells(g->w, g->h) * sizeof(float2), &vd, st));
     float* d_ao;
     RN_TRY(stage_out(ao, np, dev, WS_GTAO, &d_ao, st));
     const M4 view = view_matrix(camera);
     if (launch_gtao(g->w, g->h, sg.pos, sg.nrm, sg.mask, view.m, camera[9], radius, slices, steps, (float*)vp,
-                    (float*)vn, (float*)vd, d_ao, c.stream) != RN_OK)
+                    (float*)vn, (float2*)vd, d_ao, c.stream) != RN_OK)
         return cuda_fail(st, cudaGetLastError(), "gtao_kernel");
     if (dev) return ok(st);
     RN_TRY(copy_back(ao, d_ao, np, st));

@@ -272,8 +272,9 @@ int launch_motion(int w, int h, const float* pos, const uint8_t* mask, const flo
 // ---------------------------------------------------------------- GTAO (gtao.cu)
 // The view-space G-buffer (view16: the camera's row-major view matrix) into vpos/vnrm/vdepth,
 // then GTAO (radius, slices, steps; fovy and aspect w / h of the camera) into out.
+size_t gtao_depth_cells(int w, int h);     // float2 cells of the padded depth plane
 int launch_gtao(int w, int h, const float* pos, const float* nrm, const uint8_t* mask, const float* view16,
-                float fovy, float radius, int slices, int steps, float* vpos, float* vnrm, float* vdepth, float* out,
+                float fovy, float radius, int slices, int steps, float* vpos, float* vnrm, float2* vdepth, float* out,
                 cudaStream_t s);
 
 // ---------------------------------------------------------------- G-buffer

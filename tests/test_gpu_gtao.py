@@ -55,3 +55,19 @@ def test_gtao_judged_by_the_traced_ao(rn, oracle):
             assert not (ctl.mean() <= 0.05 and np.percentile(ctl, 95) <= 0.15)      # the control fails
         rec = rn.reconcile(a, ref, mask, 0.12, error_map=False)
         assert rec.pixels == int(mask.sum()) and rec.rmse > 0
+
+
+@pytest.mark.parametrize("w,h,slices,steps,radius", [(3, 2, 3, 5, 0.5), (17, 33, 1, 1, 0.5), (97, 61, 7, 11, 3.0),
+                                                     (161, 90, 5, 24, 40.0)])
+def test_gtao_edges_of_the_depth_plane(rn, oracle, w, h, slices, steps, radius):
+    """Frames smaller than a block, step counts that are no powers of two, and radii whose samples
+    leave the frame on every side (the padded plane's clamped border), within the same rule. Frames
+    this small allow no pixel off, so a tenth of a percent is none of them."""
+    cam = CAMERAS["near"]
+    _, pos, nrm, mask = _gbuffer(oracle, cam, w, h)
+    got = rn.gtao(rn.GBuffer(pos, nrm, mask), cam, radius, slices, steps)
+    vp, vn, vd = oracle.view_gbuffer(pos, nrm, mask, cam)
+    want = oracle.gtao(vp, vn, vd, cam[9], radius, slices, steps)
+    d = np.abs(got.astype(np.float64) - want)
+    assert bool((got[mask == 0] == 1.0).all())
+    assert (d > 1e-3).sum() <= 1e-3 * mask.sum(), (int((d > 1e-3).sum()), float(d.max()))
