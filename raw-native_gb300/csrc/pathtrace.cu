@@ -362,7 +362,7 @@ struct Lobe {
 __device__ __forceinline__ float km_of(const Bsdf& m, float b, float eavg, float kd) {
     return fadd(fmul(m.metallic, kms(fadd(b, fdiv(fsub(1.0f, b), 21.0f)), eavg)), fmul(fsub(1.0f, m.metallic), kd));
 }
-__device__ __noinline__ void lobe_setup(const PtParams& P, const Bsdf& m, float woz, Lobe& L) {
+__device__ __forceinline__ void lobe_core(const PtParams& P, const Bsdf& m, float woz, Lobe& L) {
     L.m = m;
     L.ps = lobe_prob(m);
     const float kd = fdiv(fsub(1.0f, m.metallic), kPiF);
@@ -392,9 +392,10 @@ __device__ __noinline__ void lobe_setup(const PtParams& P, const Bsdf& m, float 
     L.omesa = fsub(1.0f, esa);
     L.km = mk(km_of(m, m.base.x, ea, L.kd), km_of(m, m.base.y, ea, L.kd), km_of(m, m.base.z, ea, L.kd));
 }
+__device__ __noinline__ void lobe_setup(const PtParams& P, const Bsdf& m, float woz, Lobe& L) { lobe_core(P, m, woz, L); }
 // evalBsdf / evalLegacy (f cos and pdf) and lambertCos of one (wo, wi) pair.
 struct Eval { v3 fcos; float pdf; v3 lam; };
-__device__ __noinline__ Eval eval_lobe(const PtParams& P, const Lobe& L, v3 wo, v3 wi, bool dropCosine) {
+__device__ __forceinline__ Eval eval_core(const PtParams& P, const Lobe& L, v3 wo, v3 wi, bool dropCosine) {
     const v3 z = mk(0.0f, 0.0f, 0.0f);
     Eval r{z, 0.0f, z};
     if (wo.z <= 0.0f || wi.z <= 0.0f) return r;
@@ -439,6 +440,9 @@ __device__ __noinline__ Eval eval_lobe(const PtParams& P, const Lobe& L, v3 wo, 
     r.lam = scale(lam, cosI);
     return r;
 }
+__device__ __noinline__ Eval eval_lobe(const PtParams& P, const Lobe& L, v3 wo, v3 wi, bool dropCosine) {
+    return eval_core(P, L, wo, wi, dropCosine);
+}
 __device__ __forceinline__ v3 spec_albedo(const Bsdf& m, float cosO) {
     if (lobe_prob(m) <= 0.0f) return mk(0.0f, 0.0f, 0.0f);
     const float x1 = clampf(fsub(1.0f, cosO), 0.0f, 1.0f), fw = fmul(fmul(fmul(fmul(x1, x1), x1), x1), x1);
@@ -467,7 +471,7 @@ __device__ __forceinline__ v3 tri_corner(const PtParams& P, int t, int k) { retu
 
 // The surface at the closest hit (triangle tri at t along o + t d): the hit's barycentrics,
 // position, normals, texture coordinates, texel and material (rt_pt_ctx.hpp:18-60).
-__device__ __noinline__ void surface_of(const PtParams& P, v3 o, v3 d, int tri, float t, Surf& x) {
+__device__ __forceinline__ void surface_core(const PtParams& P, v3 o, v3 d, int tri, float t, Surf& x) {
     const v3 a = tri_corner(P, tri, 0), b = tri_corner(P, tri, 1), c = tri_corner(P, tri, 2);
     float tt, u, v;
     hit_tri_uv(make_wray(o, d), a, b, c, tt, u, v);      // the winner's u, v (its t is the walk's)
@@ -494,6 +498,9 @@ __device__ __noinline__ void surface_of(const PtParams& P, v3 o, v3 d, int tri, 
     if (dot(x.ng, d) > 0.0f) x.ng = scale(x.ng, -1.0f);
     if (dot(x.n, x.ng) < 0.0f) x.n = scale(x.n, -1.0f);
     (void)tt;
+}
+__device__ __noinline__ void surface_of(const PtParams& P, v3 o, v3 d, int tri, float t, Surf& x) {
+    surface_core(P, o, d, tri, t, x);
 }
 __device__ __noinline__ bool hit(const PtParams& P, v3 o, v3 d, float tmax, Surf& x) {
     if (!P.has_geometry) return false;
@@ -788,13 +795,12 @@ __device__ __forceinline__ uint32_t wave_reserve(uint32_t* ctr, uint32_t n) {
     return base + incl - n;
 }
 
-// path_finish and store_sample from the slot's arrays.
-__device__ void wave_finish(const PtParams& P, const WaveBufs& W, uint32_t i) {
+// path_finish and store_sample from the slot's arrays; L and R as the pass has them.
+__device__ __forceinline__ void wave_finish(const PtParams& P, const WaveBufs& W, uint32_t i, const v3& L, const v3& R) {
     using namespace wave;
     Sample o;
-    o.L = wld3(W, OL, i); o.D = wld3(W, OD, i); o.S = wld3(W, OS, i); o.E = wld3(W, OE, i);
+    o.L = L; o.D = wld3(W, OD, i); o.S = wld3(W, OS, i); o.E = wld3(W, OE, i);
     o.alb = wld3(W, OALB, i); o.nrm = wld3(W, ONRM, i); o.dAlb = wld3(W, ODALB, i); o.sAlb = wld3(W, OSALB, i);
-    const v3 R = wld3(W, wave::R, i);
     o.D = add(o.D, mulv(wld3(W, WD, i), R));
     if (!(P.controls & RN_PT_AOV_DROP_SPECULAR_INDIRECT)) o.S = add(o.S, mulv(wld3(W, WS, i), R));
     if (P.controls & RN_PT_AOV_EMISSION_TO_DIFFUSE) { o.D = add(o.D, o.E); o.E = mk(0.0f, 0.0f, 0.0f); }
@@ -814,130 +820,146 @@ __device__ void wave_start(const PtParams& P, const WaveBufs& W, uint32_t i, uin
     wu(W, UB, i) = 0; wu(W, UPX, i) = px; wu(W, USMP, i) = smp; wu(W, UJ, i) = j;
 }
 
-// One bounce after its closest hit, for a slot in M_TRACE (path_bounce from the hit on):
-// returns the slot's next mode; next-event estimation leaves its flags in *fl and its
-// shadow rays in the ray arguments.
-__device__ __noinline__ uint32_t wave_bounce(const PtParams& P, const WaveBufs& W, uint32_t i, uint32_t& fl,
-                                             v3& sun_o, v3& em_o, v3& em_d, float& em_t) {
+// What a shade pass reads of a slot, loaded at once before anything is written: the passes
+// are bound by the latency of these loads, and one after another (as the estimate, the
+// emission and the bounce come to need them) they were ten round trips a pass.
+struct SlotIn {
+    v3 ro, rd, T, tw, L, R;
+    float prev, ht;
+    uint32_t b, px, smp;
+    int tri;
+};
+
+// One bounce after its closest hit, for a slot in M_TRACE (path_bounce from the hit on; L and R
+// are updated in s, everything else is stored): returns the slot's next mode; next-event
+// estimation leaves its flags in *fl and its shadow rays in the ray arguments. The lobe is
+// evaluated for its three incoming directions by one copy of the code in a loop, the lobe
+// itself in registers: as three out-of-line calls it went through local memory each time.
+__device__ __forceinline__ uint32_t wave_bounce(const PtParams& P, const WaveBufs& W, uint32_t i, SlotIn& s, uint32_t& fl,
+                                                v3& sun_o, v3& em_o, v3& em_d, float& em_t) {
     using namespace wave;
-    const uint32_t b = wu(W, UB, i);
+    const uint32_t b = s.b;
     if (b > P.max_bounces) return M_FRESH;
     const bool dc = (P.controls & RN_PT_DROP_LAMBERT_COSINE) != 0;
-    const int tri = (int)wu(W, UTRI, i);
-    const v3 ro = wld3(W, RO, i), rd = wld3(W, RD, i);
-    v3 T = wld3(W, wave::T, i), tw = wld3(W, TW, i);
-    if (tri < 0) {
-        wst3(W, OL, i, add(wld3(W, OL, i), mulv(T, P.sky)));
-        if (b == 0) wst3(W, OE, i, P.sky); else wst3(W, wave::R, i, add(wld3(W, wave::R, i), mulv(tw, P.sky)));
+    if (s.tri < 0) {
+        s.L = add(s.L, mulv(s.T, P.sky));
+        if (b == 0) wst3(W, OE, i, P.sky); else s.R = add(s.R, mulv(s.tw, P.sky));
         return M_FRESH;
     }
     Surf x0;
-    surface_of(P, ro, rd, tri, wf(W, HT, i), x0);
+    surface_core(P, s.ro, s.rd, s.tri, s.ht, x0);
     const Bsdf bs{x0.base, __ldg(x0.m + 1), __ldg(x0.m + 2), __ldg(x0.m + 3), (P.controls & RN_PT_LEGACY_LOBE_V2) != 0};
+    const v3 Le = mk(__ldg(x0.m + 4), __ldg(x0.m + 5), __ldg(x0.m + 6));
     if (b == 0) {
         wst3(W, OALB, i, x0.base); wst3(W, ONRM, i, x0.n);
         wst3(W, ODALB, i, scale(x0.base, fsub(1.0f, bs.metallic)));
-        wst3(W, OSALB, i, spec_albedo(bs, clampf(-dot(x0.n, rd), 0.0f, 1.0f)));
+        wst3(W, OSALB, i, spec_albedo(bs, clampf(-dot(x0.n, s.rd), 0.0f, 1.0f)));
     }
-    const v3 Le = mk(__ldg(x0.m + 4), __ldg(x0.m + 5), __ldg(x0.m + 6));
     if (maxc(Le) > 0.0f) {
         float w = 1.0f;
         if (b > 0 && !(P.controls & RN_PT_MIS_WEIGHT_ONE)) {
-            const float pp = wf(W, PREV, i);
-            const float cosL = fabsf(dot(x0.ng, rd)), pl = fdiv(fmul(x0.t, x0.t), fmul(cosL, P.area));
+            const float pp = s.prev;
+            const float cosL = fabsf(dot(x0.ng, s.rd)), pl = fdiv(fmul(x0.t, x0.t), fmul(cosL, P.area));
             w = fdiv(fmul(pp, pp), fadd(fmul(pp, pp), fmul(pl, pl)));
         }
-        wst3(W, OL, i, add(wld3(W, OL, i), scale(mulv(T, Le), w)));
-        if (b == 0) wst3(W, OE, i, Le); else wst3(W, wave::R, i, add(wld3(W, wave::R, i), scale(mulv(tw, Le), w)));
+        s.L = add(s.L, scale(mulv(s.T, Le), w));
+        if (b == 0) wst3(W, OE, i, Le); else s.R = add(s.R, scale(mulv(s.tw, Le), w));
     }
     if (b == P.max_bounces) return M_FRESH;
     const Frame fr = basis(x0.n);
-    const v3 woL = to_local(fr, scale(rd, -1.0f));
+    const v3 woL = to_local(fr, scale(s.rd, -1.0f));
     if (woL.z <= 0.0f) return M_FRESH;
     const uint32_t base = 2 + b * 4;
+    wst3(W, TP, i, s.T);
+    wst3(W, TWP, i, s.tw);
     Lobe lb;
-    lobe_setup(P, bs, woL.z, lb);
+    lobe_core(P, bs, woL.z, lb);
     // next-event estimation (nee) up to its shadow rays: the terms each adds when its ray
-    // reaches the light
+    // reaches the light; then the sampled direction
     fl = F_NEE | (b == 0 ? F_B0 : 0u);
-    if (maxc(P.sun_irr) > 0.0f) {
-        const v3 l = P.sun_dir, lL = to_local(fr, l);
-        const Eval e = eval_lobe(P, lb, woL, lL, dc);
-        if (maxc(e.fcos) > 0.0f) {
+#pragma unroll 1
+    for (int k = 0; k < 3; ++k) {
+        v3 l, lL;
+        float pl = 0.0f, dist = 0.0f, rr = 0.0f;
+        int et = 0;
+        if (k == 0) {
+            if (!(maxc(P.sun_irr) > 0.0f)) continue;
+            l = P.sun_dir;
+            lL = to_local(fr, l);
+        } else if (k == 1) {
+            if (P.nemit == 0) continue;
+            const R2 a = rand2(P, s.px, s.smp, base + 2), bb = rand2(P, s.px, s.smp, base + 3);
+            const float target = fmul(a.a, P.area);
+            uint32_t lo = 0, hi = P.nemit;              // std::upper_bound: the first cdf > target
+            while (lo < hi) {
+                const uint32_t mid = lo + (hi - lo) / 2;
+                if (target < __ldg(P.cdf + mid)) hi = mid; else lo = mid + 1;
+            }
+            et = (int)__ldg(P.emit + (lo < P.nemit - 1 ? lo : P.nemit - 1));
+            const v3 ta = tri_corner(P, et, 0), tb = tri_corner(P, et, 1), tc = tri_corner(P, et, 2);
+            const float su = fsqrt(a.b);
+            const v3 q = add(add(scale(ta, fsub(1.0f, su)), scale(tb, fmul(su, fsub(1.0f, bb.a)))), scale(tc, fmul(su, bb.a)));
+            const v3 to = sub(q, x0.p);
+            dist = length(to);
+            l = scale(to, frcp(dist));
+            lL = to_local(fr, l);
+            const float cosL = fabsf(dot(normalize(cross(sub(tb, ta), sub(tc, ta))), l));
+            if (!(cosL > 0.0f)) continue;
+            pl = fdiv(fmul(dist, dist), fmul(cosL, P.area));
+        } else {
+            const R2 u = rand2(P, s.px, s.smp, base), r = rand2(P, s.px, s.smp, base + 1);
+            rr = r.b;
+            if (!sample_bsdf(P, bs, woL, r.a, u.a, u.kb, lL)) return M_END;
+        }
+        const Eval e = eval_core(P, lb, woL, lL, dc);
+        if (k == 0) {
+            if (!(maxc(e.fcos) > 0.0f)) continue;
             wst3(W, LSUN, i, mulv(e.fcos, P.sun_irr));
             wst3(W, DSUN, i, mulv(e.lam, P.sun_irr));
             sun_o = offset_of(x0, l);
             fl |= F_SUN;
-        }
-    }
-    if (P.nemit != 0) {
-        const R2 a = rand2(P, wu(W, UPX, i), wu(W, USMP, i), base + 2), bb = rand2(P, wu(W, UPX, i), wu(W, USMP, i), base + 3);
-        const float target = fmul(a.a, P.area);
-        uint32_t lo = 0, hi = P.nemit;              // std::upper_bound: the first cdf > target
-        while (lo < hi) {
-            const uint32_t mid = lo + (hi - lo) / 2;
-            if (target < __ldg(P.cdf + mid)) hi = mid; else lo = mid + 1;
-        }
-        const uint32_t k = lo < P.nemit - 1 ? lo : P.nemit - 1;
-        const int et = (int)__ldg(P.emit + k);
-        const v3 ta = tri_corner(P, et, 0), tb = tri_corner(P, et, 1), tc = tri_corner(P, et, 2);
-        const float su = fsqrt(a.b);
-        const v3 q = add(add(scale(ta, fsub(1.0f, su)), scale(tb, fmul(su, fsub(1.0f, bb.a)))), scale(tc, fmul(su, bb.a)));
-        const v3 to = sub(q, x0.p);
-        const float dist = length(to);
-        const v3 l = scale(to, frcp(dist)), lL = to_local(fr, l);
-        const float cosL = fabsf(dot(normalize(cross(sub(tb, ta), sub(tc, ta))), l));
-        if (cosL > 0.0f) {
-            const float pl = fdiv(fmul(dist, dist), fmul(cosL, P.area));
-            const Eval e = eval_lobe(P, lb, woL, lL, dc);
-            if (maxc(e.fcos) > 0.0f) {
-                const float w = (P.controls & RN_PT_MIS_WEIGHT_ONE)
-                                    ? 1.0f
-                                    : fdiv(fmul(pl, pl), fadd(fmul(pl, pl), fmul(e.pdf, e.pdf)));
-                const float* em = P.mat + 7 * (size_t)__ldg(P.tritex + et) + 4;
-                const v3 Lem = mk(__ldg(em), __ldg(em + 1), __ldg(em + 2));
-                const float wp = fdiv(w, pl);
-                wst3(W, DEM, i, scale(mulv(e.lam, Lem), wp));
-                wst3(W, LEM, i, scale(mulv(e.fcos, Lem), wp));
-                em_o = offset_of(x0, l);
-                em_d = l;
-                em_t = fmul(dist, fsub(1.0f, 1e-3f));
-                fl |= F_EM;
+        } else if (k == 1) {
+            if (!(maxc(e.fcos) > 0.0f)) continue;
+            const float w = (P.controls & RN_PT_MIS_WEIGHT_ONE)
+                                ? 1.0f
+                                : fdiv(fmul(pl, pl), fadd(fmul(pl, pl), fmul(e.pdf, e.pdf)));
+            const float* em = P.mat + 7 * (size_t)__ldg(P.tritex + et) + 4;
+            const v3 Lem = mk(__ldg(em), __ldg(em + 1), __ldg(em + 2));
+            const float wp = fdiv(w, pl);
+            wst3(W, DEM, i, scale(mulv(e.lam, Lem), wp));
+            wst3(W, LEM, i, scale(mulv(e.fcos, Lem), wp));
+            em_o = offset_of(x0, l);
+            em_d = l;
+            em_t = fmul(dist, fsub(1.0f, 1e-3f));
+            fl |= F_EM;
+        } else {
+            if (e.pdf <= 0.0f) return M_END;
+            const float ip = frcp(e.pdf);
+            const v3 step = scale(e.fcos, ip);
+            v3 T = mulv(s.T, step), tw = s.tw;
+            if (b == 0) {
+                const v3 wd = scale(e.lam, ip);
+                wst3(W, WD, i, wd);
+                wst3(W, WS, i, sub(step, wd));
+            } else {
+                tw = mulv(tw, step);
             }
+            if (P.rr && b >= 3) {
+                const float q = smin(0.95f, maxc(T));
+                if (rr >= q) return M_END;
+                const float iq = frcp(q);
+                T = scale(T, iq);
+                tw = scale(tw, iq);
+            }
+            const v3 wi = to_world(fr, lL);
+            wst3(W, wave::T, i, T);
+            wst3(W, TW, i, tw);
+            wf(W, PREV, i) = e.pdf;
+            wst3(W, RO, i, offset_of(x0, wi));
+            wst3(W, RD, i, wi);
+            wu(W, UB, i) = b + 1;
         }
     }
-    wst3(W, TP, i, T);
-    wst3(W, TWP, i, tw);
-    // the sampled direction
-    const R2 u = rand2(P, wu(W, UPX, i), wu(W, USMP, i), base), r = rand2(P, wu(W, UPX, i), wu(W, USMP, i), base + 1);
-    v3 wiL;
-    if (!sample_bsdf(P, bs, woL, r.a, u.a, u.kb, wiL)) return M_END;
-    const Eval e = eval_lobe(P, lb, woL, wiL, dc);
-    if (e.pdf <= 0.0f) return M_END;
-    const float ip = frcp(e.pdf);
-    const v3 step = scale(e.fcos, ip);
-    T = mulv(T, step);
-    if (b == 0) {
-        const v3 wd = scale(e.lam, ip);
-        wst3(W, WD, i, wd);
-        wst3(W, WS, i, sub(step, wd));
-    } else {
-        tw = mulv(tw, step);
-    }
-    if (P.rr && b >= 3) {
-        const float q = smin(0.95f, maxc(T));
-        if (r.b >= q) return M_END;
-        const float iq = frcp(q);
-        T = scale(T, iq);
-        tw = scale(tw, iq);
-    }
-    const v3 wi = to_world(fr, wiL);
-    wst3(W, wave::T, i, T);
-    wst3(W, TW, i, tw);
-    wf(W, PREV, i) = e.pdf;
-    wst3(W, RO, i, offset_of(x0, wi));
-    wst3(W, RD, i, wi);
-    wu(W, UB, i) = b + 1;
     return M_TRACE;
 }
 
@@ -950,29 +972,42 @@ __global__ void __launch_bounds__(128, kMinBlocks) pt_wave_shade(const PtParams 
     const bool in = i < W.Q;
     uint32_t fl = in ? wu(W, UFL, i) : (uint32_t)M_IDLE;
     uint32_t mode = fl & 3u;
-    // 1. the last bounce's estimate, its shadow rays now traced (nee's sums, then the
-    //    bounce's use of them: L += T Ln, then D and S at bounce 0 or R += tw Ln)
-    if (fl & F_NEE) {
-        v3 L = mk(0.0f, 0.0f, 0.0f), diff = L;
-        if ((fl & F_SUN) && W.vis[i]) { L = add(L, wld3(W, LSUN, i)); diff = add(diff, wld3(W, DSUN, i)); }
-        if ((fl & F_EM) && W.vis[W.Q + i]) { diff = add(diff, wld3(W, DEM, i)); L = add(L, wld3(W, LEM, i)); }
-        wst3(W, OL, i, add(wld3(W, OL, i), mulv(wld3(W, TP, i), L)));
-        if (fl & F_B0) { wst3(W, OD, i, diff); wst3(W, OS, i, sub(L, diff)); }
-        else wst3(W, wave::R, i, add(wld3(W, wave::R, i), mulv(wld3(W, TWP, i), L)));
+    // 1. the slot's state, in one round of loads
+    const bool trace = mode == M_TRACE, path = trace || mode == M_END;
+    SlotIn s;
+    if (path) { s.L = wld3(W, OL, i); s.R = wld3(W, wave::R, i); }
+    if (trace) {
+        s.b = wu(W, UB, i); s.px = wu(W, UPX, i); s.smp = wu(W, USMP, i); s.tri = (int)wu(W, UTRI, i);
+        s.ht = wf(W, HT, i); s.prev = wf(W, PREV, i);
+        s.ro = wld3(W, RO, i); s.rd = wld3(W, RD, i);
+        s.T = wld3(W, wave::T, i); s.tw = wld3(W, TW, i);
+    }
+    //    the last bounce's estimate, its shadow rays now traced (nee's sums, then the bounce's
+    //    use of them: L += T Ln, then D and S at bounce 0 or R += tw Ln). Slots with an estimate
+    //    are in M_TRACE or M_END.
+    if (path && (fl & F_NEE)) {
+        const v3 z = mk(0.0f, 0.0f, 0.0f), tp = wld3(W, TP, i), twp = wld3(W, TWP, i);
+        const uint8_t vs = (fl & F_SUN) ? W.vis[i] : 0, ve = (fl & F_EM) ? W.vis[W.Q + i] : 0;
+        const v3 ls = (fl & F_SUN) ? wld3(W, LSUN, i) : z, le = (fl & F_EM) ? wld3(W, LEM, i) : z;
+        const bool b0 = (fl & F_B0) != 0;            // the diffuse parts are used at bounce 0 alone
+        const v3 ds = b0 && (fl & F_SUN) ? wld3(W, DSUN, i) : z, de = b0 && (fl & F_EM) ? wld3(W, DEM, i) : z;
+        v3 L = z, diff = z;
+        if (vs) { L = add(L, ls); diff = add(diff, ds); }
+        if (ve) { diff = add(diff, de); L = add(L, le); }
+        s.L = add(s.L, mulv(tp, L));
+        if (b0) { wst3(W, OD, i, diff); wst3(W, OS, i, sub(L, diff)); }
+        else s.R = add(s.R, mulv(twp, L));
     }
     // 2. the bounce after the closest hit, or the end of a path that ended after its estimate
     uint32_t nfl = 0;
     v3 sun_o = mk(0.0f, 0.0f, 0.0f), em_o = sun_o, em_d = sun_o;
     float em_t = 0.0f;
-    if (mode == M_TRACE) {
-        mode = wave_bounce(P, W, i, nfl, sun_o, em_o, em_d, em_t);
-        // a path that ended before any estimate (a miss, the bounce limit, a surface seen
-        // from behind) is finished now; one that ended after it (M_END) in the next pass
-        if (mode == M_FRESH) wave_finish(P, W, i);
-    } else if (mode == M_END) {
-        wave_finish(P, W, i);
-        mode = M_FRESH;
-    }
+    if (trace) mode = wave_bounce(P, W, i, s, nfl, sun_o, em_o, em_d, em_t);
+    else if (path) mode = M_FRESH;
+    // a path that ended before any estimate (a miss, the bounce limit, a surface seen from
+    // behind) is finished now; one that ended after it (M_END) in the next pass
+    if (path && mode == M_FRESH) wave_finish(P, W, i, s.L, s.R);
+    else if (path) { wst3(W, OL, i, s.L); wst3(W, wave::R, i, s.R); }
     // 3. free slots take the next items (one atomic a warp per round)
     const uint32_t tiles_x = (P.w + kTileW - 1) / kTileW, tiles_y = (P.h + kTileH - 1) / kTileH;
     const uint32_t ntiles = tiles_x * tiles_y;

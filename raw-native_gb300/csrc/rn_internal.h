@@ -78,7 +78,7 @@ struct Tune {
     int trace_pool_sort = 0;    // ... the queue ordered by the walks' direction octant (at most 16 spp)
     int pt_regen = 4;           // path tracer: persistent threads regenerating paths, blocks of 128 per SM (0: one thread a sample)
     int pt_wave = 1024;         // path tracer: the wavefront form over this many x 1024 path slots (0: off)
-    int pt_shade_blocks = 6;    // ... its shade kernel's resident blocks of 128 per SM (register budget)
+    int pt_shade_blocks = 4;    // ... its shade kernel's resident blocks of 128 per SM (register budget)
     int pt_slice = 0;           // path tracer: samples per slice at most (0: as many as 2 GiB of terms hold)
 };
 constexpr uint32_t kSmallScene = 1u << 16;
