@@ -7,10 +7,10 @@
 // 24 taps of each pixel read it from there: per pixel the pass moves 12 B of position, 12 B
 // of normal, 1 B of mask and 4 B of output through HBM, the halo's re-reads hit L2.
 //
-// Sample angle: std::lround(std::cos(a) * rad) only changes when the host's cos differs from
-// the device's by enough to cross a half-integer. With |cos_host - cos_dev| <= 8 ulp and
-// rad <= 6 the product moves by < 3.5e-6, so only taps within 8e-6 of a half-integer consult
-// the host-libm correction table (about 2e-5 of them).
+// Bound by instruction issue (95 % of cycles), so each tap's offset and its occlusion are
+// decided by the cheapest arithmetic that can be trusted away from their thresholds, and by the
+// reference's exact operations near them (tap_offset, ssao_tile): 2560 x 1440, 24 taps:
+// 409 -> 195 us, 480 M -> 206 M warp instructions; the image is the same bits.
 #include "ssao_device.cuh"
 
 namespace rn {
