@@ -217,9 +217,11 @@ __global__ void rs_scatter(const uint32_t* __restrict__ kin, const uint32_t* __r
 // rt_bvh.cpp:68-77 (leafBox) and :134-139.
 __global__ void make_leaves(const float* __restrict__ tris, const uint32_t* __restrict__ order, uint32_t n,
                             float* __restrict__ box, int32_t* __restrict__ left, int32_t* __restrict__ right,
-                            int32_t* __restrict__ tri, float* __restrict__ cbox, int32_t* __restrict__ cl) {
+                            int32_t* __restrict__ tri, uint32_t* __restrict__ count, float* __restrict__ cbox,
+                            int32_t* __restrict__ cl) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
+    if (i + 1 < n) tri[n + i] = -1;              // internal node n + i: the rounds write the rest of it
     const uint32_t t = order[i];
     const float* v = tris + (size_t)t * 9;
     float lo[3], hi[3];
@@ -231,16 +233,9 @@ __global__ void make_leaves(const float* __restrict__ tris, const uint32_t* __re
         cbox[(size_t)i * 6 + a] = lo[a]; cbox[(size_t)i * 6 + 3 + a] = hi[a];
     }
     left[i] = -1; right[i] = -1; tri[i] = (int32_t)t;
+    count[i] = 1;
     cl[i] = (int32_t)i;
 }
-__global__ void init_internal(uint32_t n, float* __restrict__ box, int32_t* __restrict__ left,
-                              int32_t* __restrict__ right, int32_t* __restrict__ tri) {
-    const uint32_t i = n + blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= 2 * n - 1) return;
-    for (int a = 0; a < 6; ++a) box[(size_t)i * 6 + a] = 0.0f;
-    left[i] = -1; right[i] = -1; tri[i] = -1;
-}
-
 // ------------------------------------------------------------------ PLOC rounds
 struct RoundState {
     uint32_t m;          // clusters in the current round
@@ -367,7 +362,8 @@ __global__ void ploc_scatter(const RoundState* __restrict__ st, const int32_t* _
                              int32_t* __restrict__ clo0, int32_t* __restrict__ clo1,
                              const float* __restrict__ cb0, const float* __restrict__ cb1,
                              float* __restrict__ cbo0, float* __restrict__ cbo1,
-                             float* __restrict__ box, int32_t* __restrict__ left, int32_t* __restrict__ right) {
+                             float* __restrict__ box, int32_t* __restrict__ left, int32_t* __restrict__ right,
+                             uint32_t* count) {
     const uint32_t m = st->m;
     if (m <= st->stop || st->merges == 0 || blockIdx.x * (uint32_t)kTile >= m) return;
     const bool p = st->parity != 0;
@@ -398,8 +394,10 @@ __global__ void ploc_scatter(const RoundState* __restrict__ st, const int32_t* _
                 float nb6[6];
                 for (int a = 0; a < 3; ++a) { nb6[a] = smin(A[a], B[a]); nb6[3 + a] = smax(A[3 + a], B[3 + a]); }
                 for (int a = 0; a < 6; ++a) { box[(size_t)id * 6 + a] = nb6[a]; cbo[(size_t)pos * 6 + a] = nb6[a]; }
-                left[id] = cl[i];
-                right[id] = cl[j];
+                const int32_t ci = cl[i], cj = cl[j];
+                left[id] = ci;
+                right[id] = cj;
+                count[id] = count[ci] + count[cj];
                 clo[pos] = (int32_t)id;
             } else {
                 for (int a = 0; a < 6; ++a) cbo[(size_t)pos * 6 + a] = cb[(size_t)i * 6 + a];
@@ -410,7 +408,7 @@ __global__ void ploc_scatter(const RoundState* __restrict__ st, const int32_t* _
     }
 }
 // The round's flags, their prefix sum and the scatter in one launch (ploc_count + ploc_top +
-// ploc_scatter + ploc_commit): a tile of kTile positions per block, tiles handed out by a
+// ploc_scatter + ploc_commit): a tile of kMergeTile positions per block, tiles handed out by a
 // ticket so that every tile a block waits on is already running, and the prefix across tiles
 // by decoupled look-back (Merrill and Garland, 2016): each tile publishes its total, then
 // adds its predecessors' totals back to the first one that published its inclusive prefix.
@@ -420,6 +418,9 @@ __global__ void ploc_scatter(const RoundState* __restrict__ st, const int32_t* _
 // counted per launch, `launch` numbering this build's merge launches: a block that starts
 // after the commit takes a ticket past the round's tiles and leaves). Every wait is bounded:
 // a tile that gives up sets DEV_GUARD and publishes anyway, and the build fails.
+// Two positions a thread: with eight, one after another, a launch took 24 us however few
+// clusters were left (each position's loads wait for the last one's stores) and 50 us at 744k.
+constexpr int kMergeItems = 2, kMergeTile = kThreads * kMergeItems;
 constexpr uint64_t kLookOut = (1ull << 28) - 1;
 constexpr int kLookSpin = 1 << 22;
 __device__ __forceinline__ uint64_t look_load(const unsigned long long* p) {
@@ -433,7 +434,7 @@ __device__ __forceinline__ void look_store(unsigned long long* p, uint64_t v) {
 __global__ void ploc_merge(RoundState* st, const int32_t* __restrict__ nn, unsigned long long* look, uint32_t* ticket,
                            uint32_t launch, int32_t* __restrict__ cl0, int32_t* __restrict__ cl1, float* __restrict__ cb0,
                            float* __restrict__ cb1, float* __restrict__ box, int32_t* __restrict__ left,
-                           int32_t* __restrict__ right) {
+                           int32_t* __restrict__ right, uint32_t* count) {
     __shared__ uint32_t s_m, s_next, s_parity, s_rounds, s_stop, s_tile;
     __shared__ unsigned long long s_prefix;
     if (threadIdx.x == 0) {
@@ -443,48 +444,55 @@ __global__ void ploc_merge(RoundState* st, const int32_t* __restrict__ nn, unsig
     }
     __syncthreads();
     const uint32_t m = s_m, tile = s_tile;
-    const uint32_t ntiles = (m + kTile - 1) / kTile;
+    const uint32_t ntiles = (m + kMergeTile - 1) / kMergeTile;
     if (m <= s_stop || tile >= ntiles) return;
     const bool p = s_parity != 0;
     const int32_t* cl = p ? cl1 : cl0;
     int32_t* clo = p ? cl0 : cl1;
     const float* cb = p ? cb1 : cb0;
     float* cbo = p ? cb0 : cb1;
-    const uint32_t base = tile * kTile + threadIdx.x * kItems;
-    uint32_t o[kItems], g[kItems];
+    const uint32_t base = tile * kMergeTile + threadIdx.x * kMergeItems;
+    uint32_t o[kMergeItems], g[kMergeItems];
     unsigned long long s = 0;
-    for (int k = 0; k < kItems; ++k) {
+#pragma unroll
+    for (int k = 0; k < kMergeItems; ++k) {
         o[k] = g[k] = 0;
         if (base + k < m) ploc_flags(nn, base + k, o[k], g[k]);
         s += (unsigned long long)o[k] | ((unsigned long long)g[k] << 32);
     }
     unsigned long long tot;
     const unsigned long long ex = block_exclusive_scan<unsigned long long>(s, tot);
-    if (threadIdx.x == 0) {
+    if (threadIdx.x < 32) {
+        // one warp looks back: 32 predecessors' words at a time, summed up to the nearest
+        // inclusive prefix (a thread that walked back one word after another took 30 us and more
+        // over the 363 tiles of a 744k-triangle round)
+        const int lane = (int)threadIdx.x;
         const uint64_t tag = (uint64_t)(s_rounds & 63u) << 58;
         const uint64_t agg = (tot & 0xFFFFFFFFull) | ((tot >> 32) << 28);
         uint64_t prefix = 0;
-        if (tile == 0) {
-            look_store(look, tag | (2ull << 56) | agg);
-        } else {
-            look_store(look + tile, tag | (1ull << 56) | agg);
+        if (tile > 0) {
+            if (lane == 0) look_store(look + tile, tag | (1ull << 56) | agg);
             bool ok = true;
-            for (int k = (int)tile - 1; k >= 0;) {
-                uint64_t w = 0;
+            for (int k = (int)tile - 1 - lane;; k -= 32) {
+                uint64_t w = 2ull << 56;                       // before the first tile: a zero prefix
                 int spin = 0;
                 for (; spin < kLookSpin; ++spin) {
-                    w = look_load(look + k);
-                    if ((w >> 58) == (tag >> 58) && ((w >> 56) & 3u) != 0) break;
-                    if (spin > 64) __nanosleep(64);
+                    const bool there = k < 0 || ((w = look_load(look + k)) >> 58 == tag >> 58 && ((w >> 56) & 3u) != 0);
+                    if (__all_sync(0xffffffffu, there)) break;
+                    if (spin > 16) __nanosleep(64);
                 }
                 if (spin == kLookSpin) { ok = false; break; }
-                prefix += w & ((1ull << 56) - 1);
-                if (((w >> 56) & 3u) == 2u) break;
-                --k;
+                const unsigned full = __ballot_sync(0xffffffffu, ((w >> 56) & 3u) == 2u);
+                const int last = full ? __ffs(full) - 1 : 31;
+                uint64_t v = lane <= last ? w & ((1ull << 56) - 1) : 0;
+                for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+                prefix += v;
+                if (full) break;
             }
-            if (!ok) atomicOr(&st->error, DEV_GUARD);
-            look_store(look + tile, tag | (2ull << 56) | ((prefix + agg) & ((1ull << 56) - 1)));
+            if (!ok && lane == 0) atomicOr(&st->error, DEV_GUARD);
         }
+        if (lane == 0) {
+        look_store(look + tile, tag | (2ull << 56) | ((prefix + agg) & ((1ull << 56) - 1)));
         // back to the block's form: survivors in the low half, merges in the high half
         s_prefix = (prefix & kLookOut) | ((prefix >> 28) << 32);
         if (tile == ntiles - 1) {
@@ -502,57 +510,76 @@ __global__ void ploc_merge(RoundState* st, const int32_t* __restrict__ nn, unsig
                 st->rounds = s_rounds + 1;
             }
         }
+        }
     }
     __syncthreads();
+    // every position's clusters are read before anything is written
+    float A[kMergeItems][6], B[kMergeItems][6];
+    int32_t ci[kMergeItems], cj[kMergeItems];
+    uint32_t ct[kMergeItems];
+#pragma unroll
+    for (int k = 0; k < kMergeItems; ++k) {
+        const uint32_t i = base + k;
+        if (!(i < m && o[k])) continue;
+        ci[k] = __ldg(cl + i);
+        for (int a = 0; a < 6; ++a) A[k][a] = __ldg(cb + (size_t)i * 6 + a);
+        if (g[k]) {
+            const int32_t j = nn[i];
+            cj[k] = __ldg(cl + j);
+            for (int a = 0; a < 6; ++a) B[k][a] = __ldg(cb + (size_t)j * 6 + a);
+            ct[k] = __ldg(count + ci[k]) + __ldg(count + cj[k]);
+        }
+    }
     unsigned long long run = ex + s_prefix;
     const uint32_t next = s_next;
-    for (int k = 0; k < kItems; ++k) {
-        const uint32_t i = base + k;
-        if (i < m && o[k]) {
+#pragma unroll
+    for (int k = 0; k < kMergeItems; ++k) {
+        if (base + k < m && o[k]) {
             const uint32_t pos = (uint32_t)(run & 0xFFFFFFFFull);
             if (g[k]) {
                 const uint32_t id = next + (uint32_t)(run >> 32);
-                const int32_t j = nn[i];
-                const float* A = cb + (size_t)i * 6;
-                const float* B = cb + (size_t)j * 6;
-                float nb6[6];
-                for (int a = 0; a < 3; ++a) { nb6[a] = smin(A[a], B[a]); nb6[3 + a] = smax(A[3 + a], B[3 + a]); }
-                for (int a = 0; a < 6; ++a) { box[(size_t)id * 6 + a] = nb6[a]; cbo[(size_t)pos * 6 + a] = nb6[a]; }
-                left[id] = cl[i];
-                right[id] = cl[j];
-                clo[pos] = (int32_t)id;
-            } else {
-                for (int a = 0; a < 6; ++a) cbo[(size_t)pos * 6 + a] = cb[(size_t)i * 6 + a];
-                clo[pos] = cl[i];
+                for (int a = 0; a < 3; ++a) {
+                    A[k][a] = smin(A[k][a], B[k][a]);
+                    A[k][3 + a] = smax(A[k][3 + a], B[k][3 + a]);
+                }
+                for (int a = 0; a < 6; ++a) box[(size_t)id * 6 + a] = A[k][a];
+                left[id] = ci[k];
+                right[id] = cj[k];
+                count[id] = ct[k];
+                ci[k] = (int32_t)id;
             }
+            for (int a = 0; a < 6; ++a) cbo[(size_t)pos * 6 + a] = A[k][a];
+            clo[pos] = ci[k];
         }
         run += (unsigned long long)o[k] | ((unsigned long long)g[k] << 32);
     }
 }
 
-// The remaining rounds in one block, once few clusters are left: the round's three steps
+// The remaining rounds in one block on global memory, down to kTailShared clusters
+// (ploc_tail_shared takes the rest): the round's three steps
 // (nearest neighbours, the flags' prefix sum, the scatter) are separated by block barriers
 // instead of kernel launches, and the round state lives in shared memory. Each thread takes
 // a contiguous run of positions, so the prefix sum runs in position order and node ids,
 // cluster order and boxes are ploc_nn / ploc_scatter's exactly. At most max_rounds rounds
 // (a bound, not a wait: every round either merges or sets DEV_PLOC_NO_MERGE and stops).
 constexpr int kTailThreads = 1024;
+constexpr int kTailShared = 4096;       // clusters ploc_tail_shared keeps in shared memory
 __global__ void __launch_bounds__(kTailThreads) ploc_tail(RoundState* st, int32_t* __restrict__ cl0,
                                                           int32_t* __restrict__ cl1, float* __restrict__ cb0,
                                                           float* __restrict__ cb1, int32_t* __restrict__ nn,
                                                           float* __restrict__ box, int32_t* __restrict__ left,
-                                                          int32_t* __restrict__ right, int R, uint32_t max_rounds,
-                                                          uint32_t tail_max) {
+                                                          int32_t* __restrict__ right, uint32_t* count, int R,
+                                                          uint32_t max_rounds, uint32_t tail_max) {
     __shared__ uint32_t s_m, s_next, s_parity, s_rounds, s_error;
     __shared__ unsigned long long warp_tot[kTailThreads / 32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid == 0) { s_m = st->m; s_next = st->next; s_parity = st->parity; s_rounds = st->rounds; s_error = 0; }
     __syncthreads();
     // launched after every batch of rounds: nothing to do until the rounds reach the threshold
-    if (s_m <= 1 || s_m > tail_max) return;
+    if (s_m <= (uint32_t)kTailShared || s_m > tail_max) return;
     for (uint32_t guard = 0; guard < max_rounds; ++guard) {
         const uint32_t m = s_m;
-        if (m <= 1 || s_error) break;
+        if (m <= (uint32_t)kTailShared || s_error) break;
         const bool p = s_parity != 0;
         const float* cb = p ? cb1 : cb0;
         float* cbo = p ? cb0 : cb1;
@@ -622,8 +649,10 @@ __global__ void __launch_bounds__(kTailThreads) ploc_tail(RoundState* st, int32_
                     float nb6[6];
                     for (int a = 0; a < 3; ++a) { nb6[a] = smin(A[a], B[a]); nb6[3 + a] = smax(A[3 + a], B[3 + a]); }
                     for (int a = 0; a < 6; ++a) { box[(size_t)id * 6 + a] = nb6[a]; cbo[(size_t)pos * 6 + a] = nb6[a]; }
-                    left[id] = cl[i];
-                    right[id] = cl[j];
+                    const int32_t ci = cl[i], cj = cl[j];
+                    left[id] = ci;
+                    right[id] = cj;
+                    count[id] = count[ci] + count[cj];
                     clo[pos] = (int32_t)id;
                 } else {
                     for (int a = 0; a < 6; ++a) cbo[(size_t)pos * 6 + a] = cb[(size_t)i * 6 + a];
@@ -643,10 +672,165 @@ __global__ void __launch_bounds__(kTailThreads) ploc_tail(RoundState* st, int32_
     }
     if (tid == 0) {
         st->m = s_m; st->next = s_next; st->parity = s_parity; st->rounds = s_rounds;
-        st->root = s_m == 1 ? (s_parity ? cl1 : cl0)[0] : -1;
         if (s_error) st->error |= s_error;
-        else if (s_m > 1) st->error |= DEV_GUARD;
+        else if (s_m > (uint32_t)kTailShared) st->error |= DEV_GUARD;
     }
+}
+
+// The last rounds with every cluster in shared memory (boxes by component, node ids, subtree
+// counts, nearest neighbours: 147 KB for 4,096 clusters), in one block. A round is four barriers
+// apart: neighbours; flags and their warp scans; the survivors formed in registers; written back
+// over the same arrays. Bound by latency (some forty rounds, most of few clusters): on global
+// memory the same rounds took 310 us from 4,096 clusters, here TAIL_NOW. Node ids, cluster
+// order and boxes are ploc_nn's and ploc_merge's exactly: each thread takes a contiguous run of
+// positions, so the prefix sum runs in position order.
+__global__ void __launch_bounds__(kTailThreads) ploc_tail_shared(RoundState* st, const int32_t* __restrict__ cl0,
+                                                                 const int32_t* __restrict__ cl1,
+                                                                 const float* __restrict__ cb0,
+                                                                 const float* __restrict__ cb1, float* __restrict__ box,
+                                                                 int32_t* __restrict__ left, int32_t* __restrict__ right,
+                                                                 uint32_t* count, int R, uint32_t max_rounds) {
+    constexpr int kRun = kTailShared / kTailThreads;
+    extern __shared__ float tail_smem[];
+    float* sb[6];
+    for (int a = 0; a < 6; ++a) sb[a] = tail_smem + a * kTailShared;
+    int32_t* scl = reinterpret_cast<int32_t*>(tail_smem + 6 * kTailShared);
+    uint32_t* sct = reinterpret_cast<uint32_t*>(scl + kTailShared);
+    int32_t* snn = reinterpret_cast<int32_t*>(sct + kTailShared);
+    __shared__ unsigned long long warp_tot[kTailThreads / 32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    uint32_t m = st->m, next = st->next, rounds = st->rounds;
+    // launched after every batch of rounds: nothing to do until they are down to what fits
+    if (m <= 1 || m > (uint32_t)kTailShared) return;
+    {
+        const bool p = st->parity != 0;
+        const float* cb = p ? cb1 : cb0;
+        const int32_t* cl = p ? cl1 : cl0;
+        for (uint32_t i = tid; i < m; i += kTailThreads) {
+            for (int a = 0; a < 6; ++a) sb[a][i] = cb[(size_t)i * 6 + a];
+            const int32_t c = cl[i];
+            scl[i] = c;
+            sct[i] = count[c];
+        }
+    }
+    __syncthreads();
+    uint32_t error = 0;
+    for (uint32_t guard = 0; guard < max_rounds && m > 1; ++guard) {      // m, next, rounds: the same in every thread
+        // 2^tl threads a cluster where there are fewer clusters than threads: each takes every
+        // 2^tl-th candidate and a shuffle finds the smallest distance, the lowest position among
+        // equals (the order of the comparisons decides nothing else)
+        int tl = 0;
+        while (tl < 4 && (m << (tl + 1)) <= (uint32_t)kTailThreads) ++tl;
+        const int sub = tid & ((1 << tl) - 1);
+        for (uint32_t i0 = 0; i0 < m; i0 += (uint32_t)kTailThreads >> tl) {
+            const uint32_t i = i0 + ((uint32_t)tid >> tl);
+            float best = FLT_MAX;
+            int arg = -1;
+            if (i < m) {
+                const float a0 = sb[0][i], a1 = sb[1][i], a2 = sb[2][i], a3 = sb[3][i], a4 = sb[4][i], a5 = sb[5][i];
+                const int ii = (int)i;
+                const int j0 = ii - R > 0 ? ii - R : 0, j1 = ii + R < (int)m - 1 ? ii + R : (int)m - 1;
+#pragma unroll 4
+                for (int j = j0 + sub; j <= j1; j += 1 << tl) {
+                    if (j == ii) continue;
+                    const float d = ploc_area(smin(a0, sb[0][j]), smin(a1, sb[1][j]), smin(a2, sb[2][j]), smax(a3, sb[3][j]),
+                                              smax(a4, sb[4][j]), smax(a5, sb[5][j]));
+                    if (d < best) { best = d; arg = j; }
+                }
+            }
+            for (int o = 1; o < (1 << tl); o <<= 1) {
+                const float ob = __shfl_xor_sync(0xffffffffu, best, o);
+                const int oa = __shfl_xor_sync(0xffffffffu, arg, o);
+                if (oa >= 0 && (ob < best || arg < 0 || (ob == best && oa < arg))) { best = ob; arg = oa; }
+            }
+            if (i < m && sub == 0) snn[i] = arg;
+        }
+        __syncthreads();
+        const uint32_t chunk = (m + kTailThreads - 1) / kTailThreads;
+        const uint32_t b0 = min(m, (uint32_t)tid * chunk), nrun = min(m, b0 + chunk) - b0;
+        uint32_t flags = 0;                       // two bits a position: survives, merges
+        unsigned long long s = 0;
+#pragma unroll
+        for (int k = 0; k < kRun; ++k)
+            if ((uint32_t)k < nrun) {
+                uint32_t o, g;
+                ploc_flags(snn, b0 + k, o, g);
+                flags |= (o | (g << 1)) << (2 * k);
+                s += (unsigned long long)o | ((unsigned long long)g << 32);
+            }
+        unsigned long long x = s;
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned long long y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (lane == 31) warp_tot[warp] = x;
+        __syncthreads();
+        // every warp scans the warps' totals for itself
+        unsigned long long w = warp_tot[lane];
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned long long y = __shfl_up_sync(0xffffffffu, w, o);
+            if (lane >= o) w += y;
+        }
+        const unsigned long long total = __shfl_sync(0xffffffffu, w, 31);
+        const unsigned long long upto = __shfl_sync(0xffffffffu, w, warp > 0 ? warp - 1 : 0);
+        const uint32_t merges = (uint32_t)(total >> 32);
+        if (merges == 0) { error = DEV_PLOC_NO_MERGE; break; }
+        const unsigned long long run = (warp == 0 ? 0ull : upto) + x - s;
+        // this thread's survivors, in registers until every thread has read its clusters
+        uint32_t pos = (uint32_t)(run & 0xFFFFFFFFull), id = next + (uint32_t)(run >> 32);
+        const uint32_t pos0 = pos;
+        float nb[kRun][6];
+        int32_t ncl[kRun];
+        uint32_t nct[kRun];
+#pragma unroll
+        for (int k = 0; k < kRun; ++k) {
+            if (!((flags >> (2 * k)) & 1u)) continue;
+            const uint32_t i = b0 + k;
+            for (int a = 0; a < 6; ++a) nb[k][a] = sb[a][i];
+            ncl[k] = scl[i];
+            nct[k] = sct[i];
+            if ((flags >> (2 * k)) & 2u) {
+                const int32_t j = snn[i];
+                for (int a = 0; a < 3; ++a) { nb[k][a] = smin(nb[k][a], sb[a][j]); nb[k][3 + a] = smax(nb[k][3 + a], sb[3 + a][j]); }
+                for (int a = 0; a < 6; ++a) box[(size_t)id * 6 + a] = nb[k][a];
+                left[id] = ncl[k];
+                right[id] = scl[j];
+                nct[k] += sct[j];
+                count[id] = nct[k];
+                ncl[k] = (int32_t)id;
+                ++id;
+            }
+        }
+        __syncthreads();
+        pos = pos0;
+#pragma unroll
+        for (int k = 0; k < kRun; ++k) {
+            if (!((flags >> (2 * k)) & 1u)) continue;
+            for (int a = 0; a < 6; ++a) sb[a][pos] = nb[k][a];
+            scl[pos] = ncl[k];
+            sct[pos] = nct[k];
+            ++pos;
+        }
+        next += merges;
+        m = (uint32_t)(total & 0xFFFFFFFFull);
+        ++rounds;
+        __syncthreads();
+    }
+    if (tid == 0) {
+        st->m = m; st->next = next; st->rounds = rounds;
+        st->root = m == 1 ? scl[0] : -1;
+        if (error) st->error |= error;
+        else if (m > 1) st->error |= DEV_GUARD;
+    }
+}
+cudaError_t launch_tail_shared(cudaStream_t s, RoundState* st, const int32_t* cl0, const int32_t* cl1, const float* cb0,
+                               const float* cb1, float* box, int32_t* left, int32_t* right, uint32_t* count, int R,
+                               uint32_t max_rounds) {
+    constexpr size_t smem = (size_t)kTailShared * 9 * 4;
+    const cudaError_t e = cudaFuncSetAttribute(ploc_tail_shared, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    ploc_tail_shared<<<1, kTailThreads, smem, s>>>(st, cl0, cl1, cb0, cb1, box, left, right, count, R, max_rounds);
+    return cudaGetLastError();
 }
 
 // The remaining rounds in one thread-block cluster of C CTAs (C x 1024 threads on C SMs),
@@ -662,7 +846,7 @@ __global__ void __launch_bounds__(kTailThreads) ploc_tail_cluster(RoundState* st
                                                                   int32_t* __restrict__ cl1, float* __restrict__ cb0,
                                                                   float* __restrict__ cb1, int32_t* __restrict__ nn,
                                                                   float* __restrict__ box, int32_t* __restrict__ left,
-                                                                  int32_t* __restrict__ right, int R,
+                                                                  int32_t* __restrict__ right, uint32_t* count, int R,
                                                                   uint32_t max_rounds, uint32_t tail_max) {
     cg::cluster_group cluster = cg::this_cluster();
     __shared__ uint32_t s_m, s_next, s_parity, s_rounds, s_error;
@@ -764,8 +948,10 @@ __global__ void __launch_bounds__(kTailThreads) ploc_tail_cluster(RoundState* st
                         nb6[3 + a] = smax(__ldcg(A + 3 + a), __ldcg(B + 3 + a));
                     }
                     for (int a = 0; a < 6; ++a) { box[(size_t)id * 6 + a] = nb6[a]; cbo[(size_t)pos * 6 + a] = nb6[a]; }
-                    left[id] = __ldcg(cl + i);
-                    right[id] = __ldcg(cl + j);
+                    const int32_t ci = __ldcg(cl + i), cj = __ldcg(cl + j);
+                    left[id] = ci;
+                    right[id] = cj;
+                    count[id] = __ldcg(count + ci) + __ldcg(count + cj);
                     clo[pos] = (int32_t)id;
                 } else {
                     for (int a = 0; a < 6; ++a) cbo[(size_t)pos * 6 + a] = __ldcg(cb + (size_t)i * 6 + a);
@@ -794,8 +980,8 @@ __global__ void __launch_bounds__(kTailThreads) ploc_tail_cluster(RoundState* st
 
 template <int C>
 cudaError_t launch_tail_cluster(cudaStream_t s, RoundState* st, int32_t* cl0, int32_t* cl1, float* cb0, float* cb1,
-                                int32_t* nn, float* box, int32_t* left, int32_t* right, int R, uint32_t max_rounds,
-                                uint32_t tail_max) {
+                                int32_t* nn, float* box, int32_t* left, int32_t* right, uint32_t* count, int R,
+                                uint32_t max_rounds, uint32_t tail_max) {
     if (C > 8) {
         const cudaError_t e = cudaFuncSetAttribute(ploc_tail_cluster<C>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         if (e != cudaSuccess) return e;
@@ -811,8 +997,8 @@ cudaError_t launch_tail_cluster(cudaStream_t s, RoundState* st, int32_t* cl0, in
     at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, ploc_tail_cluster<C>, st, cl0, cl1, cb0, cb1, nn, box, left, right, R, max_rounds,
-                              tail_max);
+    return cudaLaunchKernelEx(&cfg, ploc_tail_cluster<C>, st, cl0, cl1, cb0, cb1, nn, box, left, right, count, R,
+                              max_rounds, tail_max);
 }
 
 __global__ void ploc_commit(RoundState* st) {
@@ -838,34 +1024,6 @@ __global__ void export_nodes9(uint32_t count, const float* __restrict__ box, con
 }
 
 // ------------------------------------------------------------------ collapse to 4-wide
-__global__ void set_parents(uint32_t n, const int32_t* __restrict__ left, const int32_t* __restrict__ right,
-                            int32_t* __restrict__ parent) {
-    const uint32_t i = n + blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= 2 * n - 1) return;
-    parent[left[i]] = (int32_t)i;
-    parent[right[i]] = (int32_t)i;
-}
-// Subtree leaf counts, bottom-up: the second child to arrive at a node computes it.
-__global__ void subtree_counts(uint32_t n, const int32_t* __restrict__ left, const int32_t* __restrict__ right,
-                               const int32_t* __restrict__ parent, uint32_t* __restrict__ visits,
-                               uint32_t* count, uint32_t* err) {
-    const uint32_t leaf = blockIdx.x * blockDim.x + threadIdx.x;
-    if (leaf >= n) return;
-    volatile uint32_t* vcount = count;
-    vcount[leaf] = 1;
-    int32_t c = (int32_t)leaf;
-    for (uint32_t guard = 0; guard < 2 * n; ++guard) {
-        const int32_t p = parent[c];
-        if (p < 0) return;
-        __threadfence();
-        if (atomicAdd(&visits[p], 1u) == 0) return;   // the sibling is not done yet
-        __threadfence();
-        vcount[p] = vcount[left[p]] + vcount[right[p]];
-        c = p;
-    }
-    atomicOr(err, DEV_GUARD);
-}
-
 struct Task { int32_t bnode, wnode; };
 
 __device__ __forceinline__ float box_area(const float* b) {
@@ -885,81 +1043,118 @@ __device__ __forceinline__ void padded(const float* b, float* lo, float* hi) {
     }
 }
 
-// Reserve `n` consecutive slots of a global counter for each lane of the warp (every lane
-// calls it; `am` is the full warp) with one atomic for the warp: returns the lane's first
-// slot. The counters hand out node ids, queue positions and leaf
-// triangle ranges; their order does not matter to any answer (the tree is the same), and
-// one atomic per warp instead of one per child keeps a level of millions of tasks from
-// queueing on three addresses.
-__device__ __forceinline__ uint32_t warp_reserve(uint32_t* ctr, uint32_t n, unsigned am) {
+// Reserve `nodes` consecutive node ids and `tris` consecutive leaf triangles for each lane of
+// the full warp with one 64-bit atomic for the warp (node ids in the low half): returns the
+// lane's first of each. Their order does not matter to any answer (the tree is the same), and one
+// atomic per warp instead of one per child keeps a level of millions of tasks from queueing on
+// its address.
+__device__ __forceinline__ unsigned long long warp_reserve(unsigned long long* ctr, uint32_t nodes, uint32_t tris) {
     const int lane = threadIdx.x & 31;
-    uint32_t incl = n;
+    const unsigned long long n = (unsigned long long)nodes | ((unsigned long long)tris << 32);
+    unsigned long long incl = n;
     for (int off = 1; off < 32; off <<= 1) {
-        const uint32_t y = __shfl_up_sync(am, incl, off);
+        const unsigned long long y = __shfl_up_sync(0xffffffffu, incl, off);
         if (lane >= off) incl += y;
     }
-    const int last = 31 - __clz(am);
-    const uint32_t total = __shfl_sync(am, incl, last);
-    uint32_t base = 0;
-    if (lane == last && total) base = atomicAdd(ctr, total);
-    base = __shfl_sync(am, base, last);
+    unsigned long long base = 0;
+    if (lane == 31 && incl) base = atomicAdd(ctr, incl);
+    base = __shfl_sync(0xffffffffu, base, 31);
     return base + incl - n;
 }
+
+// The collapse's counters. A level's tasks are the nodes made by the level before it, so a
+// child's place in the next level's queue is its node id less `base`, the count of nodes when
+// the level began.
+struct CollapseCtr {
+    uint32_t tasks;              // of the current level
+    uint32_t base;               // nodes when it began
+    unsigned long long made;     // nodes (low half) and leaf triangles (high half) so far
+    uint32_t err, depth, done, pad;
+};
+static_assert(sizeof(CollapseCtr) == 32, "CollapseCtr layout");
 
 // One level's tasks in[0, m), strided: this thread's warp takes bases first, first + step, ...
 // (first and step warp-uniform), so whole warps step together and every lane takes part in
 // the reservations; lanes past the end reserve nothing. `in` and `out` carry no __restrict__:
 // the single-block form reads in one level what it wrote in the previous one.
 __device__ __forceinline__ void collapse_tasks(const Task* in, uint32_t m, uint32_t first, uint32_t step, Task* out,
-                                               uint32_t* nout, uint32_t out_cap, uint32_t* node_ctr,
-                                               uint32_t node_cap, uint32_t* tri_ctr,
+                                               uint32_t out_cap, CollapseCtr* ctr, uint32_t qbase, uint32_t node_cap,
                                                const float* __restrict__ box, const int32_t* __restrict__ left,
                                                const int32_t* __restrict__ right, const int32_t* __restrict__ tri,
                                                const uint32_t* __restrict__ count, const float* __restrict__ tris,
                                                Node4* __restrict__ nodes, LeafTri* __restrict__ leaf,
-                                               uint32_t leaf_max, uint32_t* err) {
+                                               uint32_t leaf_max) {
     const uint32_t lane = threadIdx.x & 31u;
     for (uint32_t base = first; base < m; base += step) {
         const uint32_t t = base + lane;
         const bool valid = t < m;
         const Task task = valid ? in[t] : Task{0, 0};
-        int32_t C[4];
+        // up to four children: the two of the binary node, then the largest (by surface) that is
+        // no leaf yet replaced by its two, twice. A child's record (box, count, children,
+        // triangle) is read in one go, so a task is five dependent reads, one reservation and the
+        // leaves' triangles; each in its own loop they were some twenty, 31 us a level.
+        struct Child { float b[6]; uint32_t cnt; int32_t node, l, r, tri; };
+        auto child = [&](int32_t c) {
+            Child k;
+            k.node = c;
+            const float* q = box + (size_t)c * 6;
+#pragma unroll
+            for (int a = 0; a < 6; ++a) k.b[a] = __ldg(q + a);
+            k.cnt = __ldg(count + c);
+            k.l = __ldg(left + c);
+            k.r = __ldg(right + c);
+            k.tri = __ldg(tri + c);
+            return k;
+        };
+        Child C[4];
         int nc = 0;
-        const int32_t b = task.bnode;
-        if (!valid) {
-            nc = 0;
-        } else if (tri[b] >= 0 || count[b] <= leaf_max) {
-            C[nc++] = b;
-        } else {
-            C[nc++] = left[b];
-            C[nc++] = right[b];
-            while (nc < 4) {
+        if (valid) {
+            const uint32_t whole = __ldg(count + task.bnode);
+            const int32_t l = __ldg(left + task.bnode), r = __ldg(right + task.bnode);
+            if (whole <= leaf_max) {
+                C[0] = child(task.bnode);
+                nc = 1;
+            } else {
+                C[0] = child(l);
+                C[1] = child(r);
+                nc = 2;
+            }
+#pragma unroll
+            for (int step = 2; step < 4; ++step) {
                 int pick = -1;
                 float best = -1.0f;
-                for (int k = 0; k < nc; ++k) {
-                    const int32_t c = C[k];
-                    if (tri[c] >= 0 || count[c] <= leaf_max) continue;
-                    const float a = box_area(box + (size_t)c * 6);
+#pragma unroll
+                for (int k = 0; k < step; ++k) {
+                    if (nc != step || C[k].cnt <= leaf_max) continue;
+                    const float a = box_area(C[k].b);
                     if (a > best) { best = a; pick = k; }
                 }
-                if (pick < 0) break;
-                const int32_t c = C[pick];
-                C[pick] = left[c];
-                C[nc++] = right[c];
+                if (pick < 0) continue;
+                int32_t pl = C[0].l, pr = C[0].r;
+#pragma unroll
+                for (int k = 1; k < step; ++k)
+                    if (k == pick) { pl = C[k].l; pr = C[k].r; }
+                const Child cl = child(pl);
+                C[step] = child(pr);
+#pragma unroll
+                for (int k = 0; k < step; ++k)
+                    if (k == pick) C[k] = cl;
+                nc = step + 1;
             }
         }
         // this task's leaf triangles and interior children, reserved for the warp at once
         uint32_t ntri = 0, nint = 0;
-        for (int k = 0; k < nc; ++k) {
-            const int32_t c = C[k];
-            if (tri[c] >= 0 || count[c] <= leaf_max) ntri += count[c];
-            else ++nint;
-        }
-        uint32_t tri_next = warp_reserve(tri_ctr, ntri, 0xffffffffu);
-        uint32_t id_next = warp_reserve(node_ctr, nint, 0xffffffffu);
-        uint32_t q_next = warp_reserve(nout, nint, 0xffffffffu);
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (k < nc) {
+                if (C[k].cnt <= leaf_max) ntri += C[k].cnt;
+                else ++nint;
+            }
+        const unsigned long long got = warp_reserve(&ctr->made, nint, ntri);
+        uint32_t id_next = (uint32_t)got, tri_next = (uint32_t)(got >> 32);
         if (!valid) continue;
         Node4 nd;
+#pragma unroll
         for (int k = 0; k < 4; ++k) {
             nd.lox[k] = nd.loy[k] = nd.loz[k] = 1e30f;
             nd.hix[k] = nd.hiy[k] = nd.hiz[k] = -1e30f;
@@ -967,42 +1162,50 @@ __device__ __forceinline__ void collapse_tasks(const Task* in, uint32_t m, uint3
             nd.meta[k] = 0;
         }
         nd.meta[0] = nc;
-        for (int k = 0; k < nc; ++k) {
-            const int32_t c = C[k];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (k >= nc) continue;
             float lo[3], hi[3];
-            padded(box + (size_t)c * 6, lo, hi);
+            padded(C[k].b, lo, hi);
             nd.lox[k] = lo[0]; nd.loy[k] = lo[1]; nd.loz[k] = lo[2];
             nd.hix[k] = hi[0]; nd.hiy[k] = hi[1]; nd.hiz[k] = hi[2];
-            if (tri[c] >= 0 || count[c] <= leaf_max) {
-                const uint32_t cnt = count[c];
+            if (C[k].cnt <= leaf_max) {
                 const uint32_t first = tri_next;
-                tri_next += cnt;
-                // the subtree's leaves, left to right
-                int32_t stack[2 * kLeafCap];
-                int sp = 0, w = 0;
-                stack[sp++] = c;
-                while (sp > 0) {
-                    const int32_t x = stack[--sp];
-                    if (tri[x] >= 0) {
-                        const float* v = tris + (size_t)tri[x] * 9;
-                        LeafTri lt;
-                        lt.ax = v[0]; lt.bx = v[3]; lt.cx = v[6]; lt.id = __int_as_float(tri[x]);
-                        lt.ay = v[1]; lt.by = v[4]; lt.cy = v[7]; lt.pad0 = 0.0f;
-                        lt.az = v[2]; lt.bz = v[5]; lt.cz = v[8]; lt.pad1 = 0.0f;
-                        leaf[first + w++] = lt;
-                    } else if (sp + 2 <= 2 * kLeafCap) {
-                        stack[sp++] = right[x];
-                        stack[sp++] = left[x];
-                    } else {
-                        atomicOr(err, DEV_STACK_OVERFLOW);
+                tri_next += C[k].cnt;
+                auto put = [&](uint32_t at, int32_t tr) {
+                    const float* v = tris + (size_t)tr * 9;
+                    LeafTri lt;
+                    lt.ax = v[0]; lt.bx = v[3]; lt.cx = v[6]; lt.id = __int_as_float(tr);
+                    lt.ay = v[1]; lt.by = v[4]; lt.cy = v[7]; lt.pad0 = 0.0f;
+                    lt.az = v[2]; lt.bz = v[5]; lt.cz = v[8]; lt.pad1 = 0.0f;
+                    leaf[at] = lt;
+                };
+                if (C[k].cnt == 1) {
+                    put(first, C[k].tri);
+                } else {
+                    // the subtree's leaves, left to right
+                    int32_t stack[2 * kLeafCap];
+                    int sp = 0;
+                    uint32_t w = 0;
+                    stack[sp++] = C[k].node;
+                    while (sp > 0) {
+                        const int32_t x = stack[--sp];
+                        if (tri[x] >= 0) {
+                            put(first + w++, tri[x]);
+                        } else if (sp + 2 <= 2 * kLeafCap) {
+                            stack[sp++] = right[x];
+                            stack[sp++] = left[x];
+                        } else {
+                            atomicOr(&ctr->err, DEV_STACK_OVERFLOW);
+                        }
                     }
                 }
-                nd.child[k] = ~(int32_t)((first << 3) | (cnt - 1));
+                nd.child[k] = ~(int32_t)((first << 3) | (C[k].cnt - 1));
             } else {
                 const uint32_t id = id_next++;
-                const uint32_t q = q_next++;
-                if (id >= node_cap || q >= out_cap) { atomicOr(err, DEV_QUEUE_OVERFLOW); nd.child[k] = 0; continue; }
-                out[q] = Task{c, (int32_t)id};
+                const uint32_t q = id - qbase;
+                if (id >= node_cap || q >= out_cap) { atomicOr(&ctr->err, DEV_QUEUE_OVERFLOW); nd.child[k] = kNoChild; continue; }
+                out[q] = Task{C[k].node, (int32_t)id};
                 nd.child[k] = (int32_t)id;
             }
         }
@@ -1010,36 +1213,41 @@ __device__ __forceinline__ void collapse_tasks(const Task* in, uint32_t m, uint3
     }
 }
 
+// Between two levels: count the level just processed if it had tasks (the 4-wide depth), make
+// its output the next input.
+__device__ __forceinline__ void collapse_advance(volatile CollapseCtr* c) {
+    const uint32_t made = (uint32_t)c->made;
+    if (c->tasks > 0) c->depth = c->depth + 1;
+    c->tasks = made - c->base;
+    c->base = made;
+}
 // One level over the whole grid: a fixed grid strides over the level's tasks, whose count
-// is read on the device.
-__global__ void collapse_level(const Task* in, const uint32_t* __restrict__ nin, Task* out,
-                               uint32_t* __restrict__ nout, uint32_t out_cap, uint32_t* __restrict__ node_ctr,
-                               uint32_t node_cap, uint32_t* __restrict__ tri_ctr,
-                               const float* __restrict__ box, const int32_t* __restrict__ left,
-                               const int32_t* __restrict__ right, const int32_t* __restrict__ tri,
-                               const uint32_t* __restrict__ count, const float* __restrict__ tris,
-                               Node4* __restrict__ nodes, LeafTri* __restrict__ leaf, uint32_t leaf_max,
-                               uint32_t* err) {
-    collapse_tasks(in, *nin, blockIdx.x * blockDim.x + (threadIdx.x & ~31u), gridDim.x * blockDim.x, out, nout,
-                   out_cap, node_ctr, node_cap, tri_ctr, box, left, right, tri, count, tris, nodes, leaf, leaf_max,
-                   err);
+// is read on the device; the last block to finish advances the counters.
+__global__ void __launch_bounds__(128) collapse_level(const Task* in, Task* out, uint32_t out_cap, CollapseCtr* ctr,
+                                                      uint32_t node_cap, const float* __restrict__ box,
+                                                      const int32_t* __restrict__ left, const int32_t* __restrict__ right,
+                                                      const int32_t* __restrict__ tri, const uint32_t* __restrict__ count,
+                                                      const float* __restrict__ tris, Node4* __restrict__ nodes,
+                                                      LeafTri* __restrict__ leaf, uint32_t leaf_max) {
+    collapse_tasks(in, ctr->tasks, blockIdx.x * blockDim.x + (threadIdx.x & ~31u), gridDim.x * blockDim.x, out, out_cap,
+                   ctr, ctr->base, node_cap, box, left, right, tri, count, tris, nodes, leaf, leaf_max);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(&ctr->done, 1u) == gridDim.x - 1) {
+            __threadfence();
+            ctr->done = 0;
+            collapse_advance(ctr);
+        }
+    }
 }
-
-// Between two levels: count the level just processed if it had tasks (ctr[5], the 4-wide
-// depth), make its output the next input (ctr[0] = ctr[1]) and restart the output count.
-__device__ __forceinline__ void collapse_advance(uint32_t* ctr) {
-    if (ctr[0] > 0) ++ctr[5];
-    ctr[0] = ctr[1];
-    ctr[1] = 0;
-}
-__global__ void collapse_next(uint32_t* ctr) { collapse_advance(ctr); }
 
 // The whole collapse in one block, for small trees: the levels are separated by block
 // barriers instead of launches and host reads (the same tasks, reservations and nodes as
-// collapse_level / collapse_next). At most max_levels levels (a bound: a level left over
+// collapse_level). At most max_levels levels (a bound: a level left over
 // shows as a task count above zero, which the host reports).
-constexpr int kCollapseThreads = 1024;
-__global__ void __launch_bounds__(kCollapseThreads) collapse_block(Task* q0, Task* q1, uint32_t* ctr, uint32_t out_cap,
+constexpr int kCollapseThreads = 512;
+__global__ void __launch_bounds__(kCollapseThreads) collapse_block(Task* q0, Task* q1, CollapseCtr* ctr, uint32_t out_cap,
                                                                    uint32_t node_cap, const float* __restrict__ box,
                                                                    const int32_t* __restrict__ left,
                                                                    const int32_t* __restrict__ right,
@@ -1048,16 +1256,19 @@ __global__ void __launch_bounds__(kCollapseThreads) collapse_block(Task* q0, Tas
                                                                    const float* __restrict__ tris,
                                                                    Node4* __restrict__ nodes, LeafTri* __restrict__ leaf,
                                                                    uint32_t leaf_max, uint32_t max_levels) {
-    volatile uint32_t* vctr = ctr;
+    volatile CollapseCtr* vctr = ctr;
     for (uint32_t lv = 0; lv < max_levels; ++lv) {
-        const uint32_t m = vctr[0];
+        const uint32_t m = vctr->tasks, base = vctr->base;
         if (m == 0) break;                       // every thread read the same count after the barrier
         const Task* in = (lv & 1) ? q1 : q0;
         Task* out = (lv & 1) ? q0 : q1;
-        collapse_tasks(in, m, threadIdx.x & ~31u, kCollapseThreads, out, ctr + 1, out_cap, ctr + 2, node_cap, ctr + 3,
-                       box, left, right, tri, count, tris, nodes, leaf, leaf_max, ctr + 4);
+        collapse_tasks(in, m, threadIdx.x & ~31u, kCollapseThreads, out, out_cap, ctr, base, node_cap, box, left, right,
+                       tri, count, tris, nodes, leaf, leaf_max);
         __syncthreads();
-        if (threadIdx.x == 0) collapse_advance(ctr);
+        if (threadIdx.x == 0) {
+            __threadfence();
+            collapse_advance(ctr);
+        }
         __syncthreads();
     }
 }
@@ -1097,8 +1308,9 @@ int ploc_build(const float* d_tris, uint32_t n, int radius, PlocTree* out, cudaS
     const size_t o_bsum = take((size_t)(cdiv(256 * nbs, kTile) + 1) * 8);
     const size_t o_cl0 = take((size_t)n * 4), o_cl1 = take((size_t)n * 4);
     const size_t o_cb0 = take((size_t)n * 24), o_cb1 = take((size_t)n * 24);
+    const size_t o_count = take(N * 4);
     const size_t o_nn = take((size_t)n * 4), o_bs64 = take((size_t)(nbs + 1) * 8);
-    const size_t o_look = take((size_t)(nbs + 1) * 8), o_ticket = take(8);
+    const size_t o_look = take((size_t)(cdiv(n, kMergeTile) + 1) * 8), o_ticket = take(8);
     const size_t o_bounds = take(sizeof(Bounds)), o_state = take(sizeof(RoundState));
     char* mem = nullptr;
     RN_TRY(ws_get(WS_PLOC, off, (void**)&mem, st));
@@ -1107,6 +1319,7 @@ int ploc_build(const float* d_tris, uint32_t n, int radius, PlocTree* out, cudaS
     out->left = (int32_t*)(mem + o_left);
     out->right = (int32_t*)(mem + o_right);
     out->tri = (int32_t*)(mem + o_tri);
+    out->count = (uint32_t*)(mem + o_count);
     float* cent = (float*)(mem + o_cent);
     uint32_t *k0 = (uint32_t*)(mem + o_k0), *v0 = (uint32_t*)(mem + o_v0);
     uint32_t *k1 = (uint32_t*)(mem + o_k1), *v1 = (uint32_t*)(mem + o_v1);
@@ -1136,8 +1349,8 @@ int ploc_build(const float* d_tris, uint32_t n, int radius, PlocTree* out, cudaS
         std::swap(v0, v1);
     }
     // 4: leaves
-    make_leaves<<<cdiv(n, 256), 256, 0, s>>>(d_tris, v0, n, out->box, out->left, out->right, out->tri, cb0, cl0);
-    if (n > 1) init_internal<<<cdiv(n - 1, 256), 256, 0, s>>>(n, out->box, out->left, out->right, out->tri);
+    make_leaves<<<cdiv(n, 256), 256, 0, s>>>(d_tris, v0, n, out->box, out->left, out->right, out->tri, out->count, cb0,
+                                             cl0);
     // 5: rounds, in batches; the host reads the state once per batch. With a tail threshold
     // the launched rounds stop at it (stop) and every batch ends with the tail kernel, which
     // runs the remaining rounds once the state is at or below the threshold and otherwise
@@ -1152,7 +1365,7 @@ int ploc_build(const float* d_tris, uint32_t n, int radius, PlocTree* out, cudaS
     const bool fused = ctx().tune.ploc_fused != 0;
     if (fused) {
         // the look-back words of an earlier build must not pass for this one's
-        RN_CUDA(cudaMemsetAsync(look, 0, (size_t)(nbs + 1) * 8, s), st);
+        RN_CUDA(cudaMemsetAsync(look, 0, (size_t)(cdiv(n, kMergeTile) + 1) * 8, s), st);
         RN_CUDA(cudaMemsetAsync(ticket, 0, 8, s), st);
     }
     uint32_t merge_launch = 0;
@@ -1174,14 +1387,14 @@ int ploc_build(const float* d_tris, uint32_t n, int radius, PlocTree* out, cudaS
                 else
                     ploc_nn_any<<<nbn, kThreads, 0, s>>>(state, cb0, cb1, nn, radius);
                 if (fused) {
-                    ploc_merge<<<nbc, kThreads, 0, s>>>(state, nn, look, ticket, merge_launch++, cl0, cl1, cb0, cb1,
-                                                        out->box, out->left, out->right);
+                    ploc_merge<<<cdiv(m_known, kMergeTile), kThreads, 0, s>>>(state, nn, look, ticket, merge_launch++, cl0, cl1, cb0, cb1,
+                                                        out->box, out->left, out->right, out->count);
                     continue;
                 }
                 ploc_count<<<nbc, kThreads, 0, s>>>(state, nn, bs64);
                 ploc_top<<<1, kThreads, 0, s>>>(state, bs64);
                 ploc_scatter<<<nbc, kThreads, 0, s>>>(state, nn, bs64, cl0, cl1, cl0, cl1, cb0, cb1, cb0, cb1,
-                                                      out->box, out->left, out->right);
+                                                      out->box, out->left, out->right, out->count);
                 ploc_commit<<<1, 1, 0, s>>>(state);
             }
         }
@@ -1191,17 +1404,23 @@ int ploc_build(const float* d_tris, uint32_t n, int radius, PlocTree* out, cudaS
             const uint32_t rounds_max = tail_max + 1;
             cudaError_t le = cudaSuccess;
             if (ctas == 16)
-                le = launch_tail_cluster<16>(s, state, cl0, cl1, cb0, cb1, nn, out->box, out->left, out->right, radius,
-                                             rounds_max, tail_max);
+                le = launch_tail_cluster<16>(s, state, cl0, cl1, cb0, cb1, nn, out->box, out->left, out->right,
+                                             out->count, radius, rounds_max, tail_max);
             else if (ctas == 8)
-                le = launch_tail_cluster<8>(s, state, cl0, cl1, cb0, cb1, nn, out->box, out->left, out->right, radius,
-                                            rounds_max, tail_max);
+                le = launch_tail_cluster<8>(s, state, cl0, cl1, cb0, cb1, nn, out->box, out->left, out->right,
+                                            out->count, radius, rounds_max, tail_max);
             else if (ctas == 4)
-                le = launch_tail_cluster<4>(s, state, cl0, cl1, cb0, cb1, nn, out->box, out->left, out->right, radius,
-                                            rounds_max, tail_max);
-            else
-                ploc_tail<<<1, kTailThreads, 0, s>>>(state, cl0, cl1, cb0, cb1, nn, out->box, out->left, out->right,
-                                                     radius, rounds_max, tail_max);
+                le = launch_tail_cluster<4>(s, state, cl0, cl1, cb0, cb1, nn, out->box, out->left, out->right,
+                                            out->count, radius, rounds_max, tail_max);
+            else {
+                // one block: its clusters in shared memory where they fit (any threshold up to
+                // 4,096), else the rounds on global memory down to that many first
+                if (tail_max > (uint32_t)kTailShared)
+                    ploc_tail<<<1, kTailThreads, 0, s>>>(state, cl0, cl1, cb0, cb1, nn, out->box, out->left, out->right,
+                                                         out->count, radius, rounds_max, tail_max);
+                le = launch_tail_shared(s, state, cl0, cl1, cb0, cb1, out->box, out->left, out->right, out->count, radius,
+                                        rounds_max);
+            }
             RN_CUDA(le, st);
         }
         RN_CUDA(cudaGetLastError(), st);
@@ -1252,61 +1471,54 @@ int collapse_bvh4(const PlocTree& t, const float* d_tris, rn_accel* acc, int lea
     acc->d_tris = (LeafTri*)(block + node_bytes);
     size_t off = 0;
     auto take = [&](size_t bytes) { const size_t o = off; off += (bytes + 255) & ~size_t(255); return o; };
-    const size_t o_parent = take((size_t)N * 4), o_visits = take((size_t)N * 4), o_count = take((size_t)N * 4);
     const size_t o_q0 = take((size_t)n * sizeof(Task)), o_q1 = take((size_t)n * sizeof(Task));
-    const size_t o_ctr = take(8 * 4);
+    const size_t o_ctr = take(sizeof(CollapseCtr));
     char* mem = nullptr;
     RN_TRY(ws_get(WS_COLLAPSE, off, (void**)&mem, st));
-    int32_t* parent = (int32_t*)(mem + o_parent);
-    uint32_t* visits = (uint32_t*)(mem + o_visits);
-    uint32_t* count = (uint32_t*)(mem + o_count);
     Task* q0 = (Task*)(mem + o_q0);
     Task* q1 = (Task*)(mem + o_q1);
-    uint32_t* ctr = (uint32_t*)(mem + o_ctr);   // [0] nin [1] nout [2] nodes [3] tris [4] err
-    RN_CUDA(cudaMemsetAsync(parent, 0xFF, (size_t)N * 4, s), st);
-    RN_CUDA(cudaMemsetAsync(visits, 0, (size_t)N * 4, s), st);
-    RN_CUDA(cudaMemsetAsync(ctr, 0, 8 * 4, s), st);
-    if (n > 1) set_parents<<<cdiv(n - 1, 256), 256, 0, s>>>(n, t.left, t.right, parent);
-    subtree_counts<<<cdiv(n, 256), 256, 0, s>>>(n, t.left, t.right, parent, visits, count, ctr + 4);
+    CollapseCtr* ctr = (CollapseCtr*)(mem + o_ctr);
+    const uint32_t* count = t.count;             // triangles under each node (the rounds keep it)
     const Task root{t.root, 0};
-    const uint32_t init[4] = {1u, 0u, 1u, 0u};
+    CollapseCtr hc{};                            // one task, the root, which is node 0
+    hc.tasks = 1;
+    hc.base = 1;
+    hc.made = 1;
     RN_CUDA(cudaMemcpyAsync(q0, &root, sizeof root, cudaMemcpyHostToDevice, s), st);
-    RN_CUDA(cudaMemcpyAsync(ctr, init, sizeof init, cudaMemcpyHostToDevice, s), st);
+    RN_CUDA(cudaMemcpyAsync(ctr, &hc, sizeof hc, cudaMemcpyHostToDevice, s), st);
     // levels in batches of kLevels per host read; a level after the last one finds no task.
     // Small trees run every level in one block and are read once.
     constexpr int kLevels = 8;
-    const uint32_t grid = std::max(1u, std::min(cdiv(n, 128), (uint32_t)ctx().sm_count * 16u));
+    const uint32_t grid = std::max(1u, std::min(cdiv(n, 128), (uint32_t)ctx().sm_count * 8u));
     uint32_t level_tasks = 1, depth = 0;
-    uint32_t hc[6] = {0, 0, 0, 0, 0, 0};
     if (n <= (uint32_t)ctx().tune.collapse_block) {
         collapse_block<<<1, kCollapseThreads, 0, s>>>(q0, q1, ctr, n, node_cap, t.box, t.left, t.right, t.tri, count,
                                                       d_tris, acc->d_nodes, acc->d_tris, (uint32_t)leaf_max, 4097u);
         RN_CUDA(cudaGetLastError(), st);
-        RN_CUDA(cudaMemcpyAsync(hc, ctr, sizeof hc, cudaMemcpyDeviceToHost, s), st);
+        RN_CUDA(cudaMemcpyAsync(&hc, ctr, sizeof hc, cudaMemcpyDeviceToHost, s), st);
         RN_CUDA(cudaStreamSynchronize(s), st);
-        level_tasks = hc[0];
-        depth = hc[5];
+        level_tasks = hc.tasks;
+        depth = hc.depth;
         if (level_tasks > 0) return fail(st, RN_ERR_BUDGET, "collapse: more than 4096 levels");
     }
     while (level_tasks > 0) {
         if (depth > 4096) return fail(st, RN_ERR_BUDGET, "collapse: more than 4096 levels");
         for (int k = 0; k < kLevels; ++k) {
-            collapse_level<<<grid, 128, 0, s>>>(q0, ctr + 0, q1, ctr + 1, n, ctr + 2, node_cap, ctr + 3, t.box,
-                                                t.left, t.right, t.tri, count, d_tris, acc->d_nodes, acc->d_tris,
-                                                (uint32_t)leaf_max, ctr + 4);
-            collapse_next<<<1, 1, 0, s>>>(ctr);
+            collapse_level<<<grid, 128, 0, s>>>(q0, q1, n, ctr, node_cap, t.box, t.left, t.right, t.tri, count, d_tris,
+                                                acc->d_nodes, acc->d_tris, (uint32_t)leaf_max);
             std::swap(q0, q1);
         }
         RN_CUDA(cudaGetLastError(), st);
-        RN_CUDA(cudaMemcpyAsync(hc, ctr, sizeof hc, cudaMemcpyDeviceToHost, s), st);
+        RN_CUDA(cudaMemcpyAsync(&hc, ctr, sizeof hc, cudaMemcpyDeviceToHost, s), st);
         RN_CUDA(cudaStreamSynchronize(s), st);
-        level_tasks = hc[0];
-        depth = hc[5];
+        level_tasks = hc.tasks;
+        depth = hc.depth;
     }
     RN_CUDA(cudaGetLastError(), st);
-    if (hc[4]) return fail(st, RN_ERR_OVERFLOW, "BVH collapse error word 0x%x", hc[4]);
-    if (hc[3] != n) return fail(st, RN_ERR_STATE, "collapse placed %u of %u triangles", hc[3], n);
-    acc->nodes = hc[2];
+    const uint32_t placed = (uint32_t)(hc.made >> 32);
+    if (hc.err) return fail(st, RN_ERR_OVERFLOW, "BVH collapse error word 0x%x", hc.err);
+    if (placed != n) return fail(st, RN_ERR_STATE, "collapse placed %u of %u triangles", placed, n);
+    acc->nodes = (uint32_t)hc.made;
     acc->depth = depth;
     return ok(st);
 }

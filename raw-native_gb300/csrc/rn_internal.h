@@ -194,6 +194,7 @@ struct PlocTree {
     int32_t* left = nullptr;   // (2n-1)
     int32_t* right = nullptr;  // (2n-1)
     int32_t* tri = nullptr;    // (2n-1)
+    uint32_t* count = nullptr; // (2n-1) triangles under the node
     void* mem = nullptr;       // the workspace block holding the arrays above (not owned)
 };
 int ploc_build(const float* d_tris, uint32_t n, int radius, PlocTree* out, cudaStream_t s, rn_status* st);
