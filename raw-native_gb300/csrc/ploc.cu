@@ -681,7 +681,7 @@ __global__ void __launch_bounds__(kTailThreads) ploc_tail(RoundState* st, int32_
 // counts, nearest neighbours: 147 KB for 4,096 clusters), in one block. A round is four barriers
 // apart: neighbours; flags and their warp scans; the survivors formed in registers; written back
 // over the same arrays. Bound by latency (some forty rounds, most of few clusters): on global
-// memory the same rounds took 310 us from 4,096 clusters, here TAIL_NOW. Node ids, cluster
+// memory the same rounds took 310 us from 4,096 clusters, here 160 us. Node ids, cluster
 // order and boxes are ploc_nn's and ploc_merge's exactly: each thread takes a contiguous run of
 // positions, so the prefix sum runs in position order.
 __global__ void __launch_bounds__(kTailThreads) ploc_tail_shared(RoundState* st, const int32_t* __restrict__ cl0,
@@ -1489,7 +1489,7 @@ int collapse_bvh4(const PlocTree& t, const float* d_tris, rn_accel* acc, int lea
     // levels in batches of kLevels per host read; a level after the last one finds no task.
     // Small trees run every level in one block and are read once.
     constexpr int kLevels = 8;
-    const uint32_t grid = std::max(1u, std::min(cdiv(n, 128), (uint32_t)ctx().sm_count * 8u));
+    const uint32_t grid = std::max(1u, std::min(cdiv(n, 128), (uint32_t)ctx().sm_count * 3u));
     uint32_t level_tasks = 1, depth = 0;
     if (n <= (uint32_t)ctx().tune.collapse_block) {
         collapse_block<<<1, kCollapseThreads, 0, s>>>(q0, q1, ctr, n, node_cap, t.box, t.left, t.right, t.tri, count,
