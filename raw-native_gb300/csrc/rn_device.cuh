@@ -55,6 +55,9 @@ __device__ __forceinline__ uint32_t hash24(uint32_t x, uint32_t y, uint32_t s) {
 // the same value.
 __device__ __forceinline__ float unit24(uint32_t k) { return fmul((float)k, 5.9604644775390625e-8f); }
 
+// 1 + k / 2^24 for the 24-bit k in the low bits of h, less its last bit (5.96e-8 at most).
+__device__ __forceinline__ float one_plus(uint32_t h) { return __uint_as_float(((h >> 1) & 0x7FFFFFu) | 0x3F800000u); }
+
 // The sample angle of 24-bit index k: phi = 6.2831853f * (k / 2^24), as both passes form it.
 __device__ __forceinline__ float sample_angle(uint32_t k) { return fmul(6.2831853f, unit24(k)); }
 

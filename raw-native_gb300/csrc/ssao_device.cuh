@@ -27,9 +27,6 @@ __device__ __forceinline__ int round_fast(float v, float& off) {
     off = fabsf(__fsub_rn(v, __fsub_rn(t, kMagic)));
     return __float_as_int(t) - __float_as_int(kMagic);
 }
-// 1 + k / 2^24 for the 24-bit k in the low bits of h, less its last bit (5.96e-8 at most).
-__device__ __forceinline__ float one_plus(uint32_t h) { return __uint_as_float(((h >> 1) & 0x7FFFFFu) | 0x3F800000u); }
-
 // Sample s's tap offset (ssao.cpp:18-23): lround(cos(a) rad), lround(sin(a) rad) with
 // a = 6.2831853 u, rad = (0.3 + 0.7 u') 6, from the pixel's hash sum `base` + s. An integer that
 // only changes where the product crosses a half, so it is formed from the hardware's sine and

@@ -86,6 +86,15 @@ __device__ __forceinline__ bool slab(float lox, float hix, float loy, float hiy,
 // minima and maxima, one multiply and one compare. hit[k] also says that child k exists: an
 // unused slot holds an inverted box, which only a ray without a finite direction component
 // can pass, and the child word kNoChild.
+__device__ __forceinline__ uint64_t pack2(float a, float b) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void fma2(float& a, float& b, float x, float y, uint64_t m, uint64_t c) {
+    asm("{\n.reg .b64 t;\nmov.b64 t, {%2, %3};\nfma.rn.f32x2 t, t, %4, %5;\nmov.b64 {%0, %1}, t;\n}\n"
+        : "=f"(a), "=f"(b) : "f"(x), "f"(y), "l"(m), "l"(c));
+}
 template <typename L>
 __device__ __forceinline__ void node_test(const char* node, L ld, const Inv& iv, float tmax, int32_t (&CH)[4],
                                           float (&tn)[4], bool (&hit)[4]) {
@@ -93,10 +102,21 @@ __device__ __forceinline__ void node_test(const char* node, L ld, const Inv& iv,
     const float4 ny = ld(node + iv.ny), fy = ld(node + (iv.ny ^ 16u));
     const float4 nz = ld(node + iv.nz), fz = ld(node + (iv.nz ^ 16u));
     const float4 ch = ld(node + 96);
-    hit[0] = slab_nf(nx.x, fx.x, ny.x, fy.x, nz.x, fz.x, iv, tmax, tn[0]);
-    hit[1] = slab_nf(nx.y, fx.y, ny.y, fy.y, nz.y, fz.y, iv, tmax, tn[1]);
-    hit[2] = slab_nf(nx.z, fx.z, ny.z, fy.z, nz.z, fz.z, iv, tmax, tn[2]);
-    hit[3] = slab_nf(nx.w, fx.w, ny.w, fy.w, nz.w, fz.w, iv, tmax, tn[3]);
+    const uint64_t ix = pack2(iv.x, iv.x), iy = pack2(iv.y, iv.y), iz = pack2(iv.z, iv.z);
+    const uint64_t ox = pack2(-iv.ox, -iv.ox), oy = pack2(-iv.oy, -iv.oy), oz = pack2(-iv.oz, -iv.oz);
+    float ax[4], bx[4], ay[4], by[4], az[4], bz[4];
+    fma2(ax[0], ax[1], nx.x, nx.y, ix, ox); fma2(ax[2], ax[3], nx.z, nx.w, ix, ox);
+    fma2(bx[0], bx[1], fx.x, fx.y, ix, ox); fma2(bx[2], bx[3], fx.z, fx.w, ix, ox);
+    fma2(ay[0], ay[1], ny.x, ny.y, iy, oy); fma2(ay[2], ay[3], ny.z, ny.w, iy, oy);
+    fma2(by[0], by[1], fy.x, fy.y, iy, oy); fma2(by[2], by[3], fy.z, fy.w, iy, oy);
+    fma2(az[0], az[1], nz.x, nz.y, iz, oz); fma2(az[2], az[3], nz.z, nz.w, iz, oz);
+    fma2(bz[0], bz[1], fz.x, fz.y, iz, oz); fma2(bz[2], bz[3], fz.z, fz.w, iz, oz);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const float t0 = max3(ax[k], ay[k], fmaxf(az[k], 0.0f)), t1 = min3(bx[k], by[k], fminf(bz[k], tmax));
+        tn[k] = t0;
+        hit[k] = t0 <= t1 * 1.0000008f;
+    }
     CH[0] = __float_as_int(ch.x); CH[1] = __float_as_int(ch.y); CH[2] = __float_as_int(ch.z); CH[3] = __float_as_int(ch.w);
 }
 struct LdGlobal {
@@ -437,25 +457,31 @@ __device__ inline int walk_closest(const Node4* __restrict__ nodes, const LeafTr
     return best_tri;
 }
 
-// The frontier of the warp's packet for AO walks of `radius` (all 32 lanes call it and build
-// it together; o: the lane's ray origin, where `covered`). Returns its size, 0: the walks start
-// at the root, -1: no triangle is within reach.
-__device__ __forceinline__ int tile_frontier(const TraceParams& p, const v3& o, bool covered, const TilePlane& pl,
-                                             Node4* F) {
-    float lo[3] = {3.0e38f, 3.0e38f, 3.0e38f}, hi[3] = {-3.0e38f, -3.0e38f, -3.0e38f}, mag = 0.0f;
+// The bounds of the packet's ray origins (o: the lane's, where `covered`; all 32 lanes call it).
+struct TileBox { float lo[3], hi[3], mag; };
+__device__ __forceinline__ TileBox tile_box(const v3& o, bool covered) {
+    TileBox t{{3.0e38f, 3.0e38f, 3.0e38f}, {-3.0e38f, -3.0e38f, -3.0e38f}, 0.0f};
     if (covered) {
-        lo[0] = hi[0] = o.x; lo[1] = hi[1] = o.y; lo[2] = hi[2] = o.z;
-        mag = fmaxf(fmaxf(fabsf(o.x), fabsf(o.y)), fabsf(o.z));
+        t.lo[0] = t.hi[0] = o.x; t.lo[1] = t.hi[1] = o.y; t.lo[2] = t.hi[2] = o.z;
+        t.mag = fmaxf(fmaxf(fabsf(o.x), fabsf(o.y)), fabsf(o.z));
     }
-    for (int off = 16; off > 0; off >>= 1)
+    for (int off = 16; off > 0; off >>= 1) {
         for (int a = 0; a < 3; ++a) {
-            lo[a] = fminf(lo[a], __shfl_xor_sync(0xffffffffu, lo[a], off));
-            hi[a] = fmaxf(hi[a], __shfl_xor_sync(0xffffffffu, hi[a], off));
+            t.lo[a] = fminf(t.lo[a], __shfl_xor_sync(0xffffffffu, t.lo[a], off));
+            t.hi[a] = fmaxf(t.hi[a], __shfl_xor_sync(0xffffffffu, t.hi[a], off));
         }
-    for (int off = 16; off > 0; off >>= 1) mag = fmaxf(mag, __shfl_xor_sync(0xffffffffu, mag, off));
+        t.mag = fmaxf(t.mag, __shfl_xor_sync(0xffffffffu, t.mag, off));
+    }
+    return t;
+}
+// The frontier of the warp's packet for AO walks of `radius` (all 32 lanes call it and build
+// it together). Returns its size, 0: the walks start at the root, -1: no triangle is within
+// reach.
+__device__ __forceinline__ int tile_frontier(const TraceParams& p, const TileBox& t, const TilePlane& pl, Node4* F) {
+    float lo[3] = {t.lo[0], t.lo[1], t.lo[2]}, hi[3] = {t.hi[0], t.hi[1], t.hi[2]};
     if (lo[0] > hi[0]) return 0;
     // grow by the radius with margin for the rounding of t, |d| and the hit point
-    const float g = p.radius * 1.0001f + 1e-5f * (mag + 1.0f);
+    const float g = p.radius * 1.0001f + 1e-5f * (t.mag + 1.0f);
     for (int a = 0; a < 3; ++a) { lo[a] -= g; hi[a] += g; }
     const int n = build_frontier(p.nodes, lo, hi, pl, F, p.frontier_tail);
     __syncwarp();
@@ -494,8 +520,40 @@ __device__ __forceinline__ v3 sample_direction(const v3& t, const v3& b, const v
     return normalize(add(add(scale(t, lx), scale(b, ly)), scale(n, lz)));
 }
 
-// Whether a walk of this ray has anything to descend into: any of the fn entries of F is
-// entered before tmax.
+// The sieve's rays are rough: the direction to 1e-5 (hardware sine, cosine and roots, no table
+// byte, not normalized: |n| is within a few percent of one), and the entries of F grown by 2e-5
+// of the distance to their farthest corner from any origin of the packet, so that the rough ray
+// enters the grown box wherever the exact ray enters the box.
+__device__ __forceinline__ void grow_entries(Node4* F, int n, const TileBox& t) {
+    const int lane = (int)(threadIdx.x & 31u);
+    if (lane < n) {
+        FrontierBox b = frontier_get(F, lane);
+        float d = 0.0f;
+        for (int a = 0; a < 3; ++a) d += fmaxf(b.hi[a] - t.lo[a], t.hi[a] - b.lo[a]);
+        const float g = 2e-5f * d;
+        for (int a = 0; a < 3; ++a) { b.lo[a] -= g; b.hi[a] += g; }
+        frontier_put(F, lane, b);
+    }
+    __syncwarp();
+}
+__device__ __forceinline__ float sqrt_rough(float x) {
+    float r;
+    asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+// sample_direction to 1e-5, of about unit length. The radius keeps its exact u (the root of a
+// small one would feel its last bit); the angle is taken less pi, where the hardware's sine and
+// cosine are good to 2^-21.
+__device__ __forceinline__ v3 rough_direction(const v3& t, const v3& b, const v3& n, uint32_t ux, uint32_t uy, uint32_t s) {
+    const float u1 = unit24(hash24(ux, uy, 2u * s));
+    const float ang = (one_plus(hash24(ux, uy, 2u * s + 1u)) - 1.5f) * 6.2831853f;
+    const float r = -sqrt_rough(u1), lz = sqrt_rough(1.0f - u1);
+    const float lx = r * __cosf(ang), ly = r * __sinf(ang);
+    return mk(__fmaf_rn(t.x, lx, __fmaf_rn(b.x, ly, n.x * lz)), __fmaf_rn(t.y, lx, __fmaf_rn(b.y, ly, n.y * lz)),
+              __fmaf_rn(t.z, lx, __fmaf_rn(b.z, ly, n.z * lz)));
+}
+// Whether a walk along the rough direction d has anything to descend into: any of the fn grown
+// entries of F is entered before tmax.
 __device__ __forceinline__ bool walk_starts(const v3& o, const v3& d, float tmax, const Node4* F, int fn) {
     const Inv iv = make_inv(o, d);
     bool any;
@@ -556,9 +614,16 @@ __device__ __forceinline__ void trace_packet(const TraceParams& p, int x, int y,
     // the sky's at the root, whose live children serve the sieve (the frontier is rebuilt for
     // every packet)
     int fn = 0;
+    bool sieve = false;
     if (p.has_geometry && (p.want_sky || p.frontier)) {
         const TilePlane pl = tile_plane(n, origin, m != 0, covered);
-        fn = p.want_sky ? root_frontier(p.nodes, pl, F) : tile_frontier(p, origin, m != 0, pl, F);
+        const TileBox tb = tile_box(origin, m != 0);
+        fn = p.want_sky ? root_frontier(p.nodes, pl, F) : tile_frontier(p, tb, pl, F);
+        // the sieve needs normals of about unit length (its rough rays are not normalized)
+        const float n2 = n.x * n.x + n.y * n.y + n.z * n.z;
+        sieve = !kCount && fn > 0 && skip == 0 && __all_sync(0xffffffffu, !m || (n2 > 0.9f && n2 < 1.1f));
+        if (!kCount && fn > 0 && skip > 0) --skip;
+        if (sieve) grow_entries(F, fn, tb);
     }
     int open = 0, freec = 0;
     bool lit = true;
@@ -586,26 +651,18 @@ __device__ __forceinline__ void trace_packet(const TraceParams& p, int x, int y,
         open = freec = p.spp;
         if (kCount && m) { cn.rays += p.spp; if (p.want_sky) cn.sky += p.spp; }
     }
-    bool sieve = !kCount && fn > 0 && skip == 0;
-    if (!kCount && fn > 0 && skip > 0) --skip;
     for (int s0 = first; s0 < slots; s0 += kChunk) {
         const int nslot = min(kChunk, slots - s0), nsamp = min(kChunk, p.spp - s0);
         uint64_t todo = m ? (nslot == 64 ? ~0ull : (1ull << nslot) - 1ull) : 0ull;
         if (sieve && nsamp > 0) {
             uint64_t keep = todo;
-            if (m) {
-                fetch(s0);
-                for (int k = 0; k < nsamp; ++k) {
-                    const uint32_t k2 = k2n;
-                    const int cb = cbn;
-                    if (k + 1 < nsamp) fetch(s0 + k + 1);
-                    if (!walk_starts(origin, direction(s0 + k, k2, cb), tfar_h, F, fn)) {
+            if (m)
+                for (int k = 0; k < nsamp; ++k)
+                    if (!walk_starts(origin, rough_direction(t, b, n, ux, uy, (uint32_t)(s0 + k)), 1.1f * tfar_h, F, fn)) {
                         keep &= ~(1ull << k);
                         ++open;
                         ++freec;
                     }
-                }
-            }
             todo = keep;
             const unsigned left = __reduce_add_sync(0xffffffffu, (unsigned)__popcll(keep));
             if (left * kSieveDen > (unsigned)(nsamp * __popc(covered)) * kSieveNum) {
