@@ -361,39 +361,40 @@ __global__ void __launch_bounds__(kConvThreads, 1) tc_conv_kernel(const __grid_c
     const uint32_t tmem = *tmem_slot;
 
     if (warp == 0) {
-        // lane s < kSt owns stage s: it issues K steps kc = s, s + kSt, ... of this CTA's
-        // sequence (items blockIdx.x, + gridDim.x, ...; nkb steps each), waiting for each
-        // previous use of its stage in order, so the stages fill in parallel
-        if (lane < kSt) {
-            const int my_items = a.items > (int)blockIdx.x ? (a.items - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
-            const uint32_t total = (uint32_t)my_items * (uint32_t)nkb;
-            uint32_t last = 0xFFFFFFFFu;
-            for (uint32_t kc = lane; kc < total; kc += kSt) {
-                const uint32_t ph = (kc / kSt) & 1u;
-                if (!mbar_wait_or_abort(empty(lane), ph ^ 1u, abort_flag)) {
-                    atomicOr(e.err, DEV_GUARD);
-                    s_abort = 1;
-                    break;
+        // The warp fills the stages in order, all lanes waiting for the same one: lane 0 arms its
+        // barrier, lanes 0 .. kT - 1 issue a tile's box each, lane kT the weights'. (A lane per
+        // stage, each waiting for its own, held one another up: a lane suspended in try_wait
+        // keeps the warp from the lane whose stage is free.) Stage, phase, tap and channel block
+        // are kept by increment.
+        uint32_t issued = 0, ph = 0;
+        int s = 0;
+        bool ok = true;
+        for (int item = blockIdx.x; ok && item < a.items; item += gridDim.x) {
+            const int group = item / a.n_slices, n0 = (item % a.n_slices) * BN;
+            const int tile = group * kT + (lane < kT ? lane : 0);
+            const int tx = tile % a.tiles_x, ty = (tile / a.tiles_x) % a.tiles_y, b = tile / (a.tiles_x * a.tiles_y);
+            for (int tap = 0; ok && tap < 9; ++tap) {
+                const int x = tx * tw + tap % 3 - 1, y = ty * th + tap / 3 - 1;
+                for (int r = 0; r < per_tap; ++r) {
+                    ok = __all_sync(0xffffffffu, mbar_wait_or_abort(empty(s), ph ^ 1u, abort_flag));
+                    if (!ok) break;
+                    if (lane == 0) mbar_expect_tx(full(s), kT * kABytes + kBBytes);
+                    __syncwarp();
+                    const bool second = r >= nb0;
+                    const int cb = second ? r - nb0 : r;
+                    if (lane < kT)
+                        tma_load_4d(smem_u32(sA + (s * kT + lane) * kABytes), second ? &map1 : &map0, cb * CB, x, y, b, full(s));
+                    else if (lane == kT)
+                        tma_load_2d(smem_u32(sB + s * kBBytes), &mapW, tap * a.cin + (second ? a.C0 : 0) + cb * CB, n0, full(s));
+                    ++issued;
+                    if (++s == kSt) { s = 0; ph ^= 1u; }
                 }
-                const int item = (int)blockIdx.x + (int)(kc / nkb) * (int)gridDim.x, kb = (int)(kc % nkb);
-                const int group = item / a.n_slices, n0 = (item % a.n_slices) * BN;
-                const int tap = kb / per_tap, r = kb % per_tap;
-                const bool second = r >= nb0;
-                const int cb = second ? r - nb0 : r;
-                mbar_expect_tx(full(lane), kT * kABytes + kBBytes);
-                for (int t = 0; t < kT; ++t) {
-                    const int tile = group * kT + t;
-                    const int tx = tile % a.tiles_x, ty = (tile / a.tiles_x) % a.tiles_y, b = tile / (a.tiles_x * a.tiles_y);
-                    tma_load_4d(smem_u32(sA + (lane * kT + t) * kABytes), second ? &map1 : &map0, cb * CB,
-                                tx * tw + tap % 3 - 1, ty * th + tap / 3 - 1, b, full(lane));
-                }
-                tma_load_2d(smem_u32(sB + lane * kBBytes), &mapW, tap * a.cin + (second ? a.C0 : 0) + cb * CB, n0,
-                            full(lane));
-                last = kc;
             }
-            // the copies this lane issued must land before the CTA can leave
-            if (last != 0xFFFFFFFFu) mbar_wait(full(lane), (last / kSt) & 1u);
         }
+        if (!ok && lane == 0) { atomicOr(e.err, DEV_GUARD); s_abort = 1; }
+        // the copies issued must land before the CTA can leave
+        if (lane == 0)
+            for (uint32_t k = issued > (uint32_t)kSt ? issued - kSt : 0; k < issued; ++k) mbar_wait(full((int)(k % kSt)), (k / kSt) & 1u);
     } else if (warp == 1) {
         if (lane == 0) {
             const uint32_t idesc = instr_desc(BN);
