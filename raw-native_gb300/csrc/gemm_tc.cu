@@ -6,7 +6,7 @@
 //   - warp 0, lane 0: TMA producer. Each 64-wide K step loads a 128 x 64 tile of P and a
 //     BN x 64 tile of Q (cp.async.bulk.tensor, 128-byte swizzle) into one of 4 shared-memory
 //     stages and signals the stage's "full" mbarrier with the byte count;
-//   - warp 1, lane 0: MMA issuer. Per stage, four tcgen05.mma.kind::f16 (M 128, N BN, K 16)
+//   - warp 1: MMA issuer (an elected lane). Per stage, four tcgen05.mma.kind::f16 (M 128, N BN, K 16)
 //     accumulate into a BN-column TMEM accumulator; tcgen05.commit releases the stage
 //     ("empty" mbarrier) when its MMAs have read it, and a final commit signals "done";
 //   - all four warps: epilogue. Each thread owns one row (its warp's TMEM lane quarter),
@@ -28,6 +28,15 @@ constexpr int kStages = 4, kThreads = 128;
 constexpr uint32_t kSpin = 1u << 24;      // try_wait rounds before a wait gives up
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+// The thread's warp in its block, known to be the same for the whole warp.
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(*reinterpret_cast<uint64_t*>(&a)), "l"(*reinterpret_cast<uint64_t*>(&b)));
+    return *reinterpret_cast<float2*>(&r);
+}
 
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
@@ -81,14 +90,20 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map
 __host__ __device__ constexpr uint32_t instr_desc(int n) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
 }
+// Issued by a whole warp, one elected lane executing (the same lane each time): the warp stays
+// convergent, so the operands can be formed in the uniform registers that the instruction
+// reads. From a branch of one lane a row-ring MMA cost 84 to 130 cycles where the tensor pipe
+// needs 35 to 60 (64 + 128 -> 64 channels at 1088 x 1920: 643 us so, 362 convergent).
 __device__ __forceinline__ void tc_mma(uint32_t tmem, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
-        "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem),
+        "{\n.reg .pred p, e;\nelect.sync _|e, 0xffffffff;\nsetp.ne.b32 p, %4, 0;\n@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem),
         "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
         : "memory");
 }
 __device__ __forceinline__ void tc_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+    asm volatile(
+        "{\n.reg .pred e;\nelect.sync _|e, 0xffffffff;\n@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n" ::"r"(bar)
+        : "memory");
 }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
@@ -148,7 +163,7 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const __grid_const
     uint64_t* bars = reinterpret_cast<uint64_t*>(sB + kStages * kBBytes);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kStages + 1);
     __shared__ int s_abort;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     const int m0 = blockIdx.x * kBM, n0 = blockIdx.y * BN;
     const int kbeg = blockIdx.z * e.k_per_split, nkb = e.k_per_split / kBK;
     auto full = [&](int s) { return smem_u32(&bars[s]); };
@@ -170,7 +185,7 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const __grid_const
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = *tmem_slot;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
 
     const uint32_t spin = e.spin ? e.spin : kSpin;
     if (warp == 0 && lane == 0) {
@@ -189,13 +204,16 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const __grid_const
         // the copies this thread issued must land before the CTA can leave
         for (int kb = issued > kStages ? issued - kStages : 0; kb < issued; ++kb)
             mbar_wait(full(kb % kStages), (uint32_t)(kb / kStages) & 1u, spin);
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1) {
         // MMA issuer
         const uint32_t idesc = instr_desc(BN);
         for (int kb = 0; kb < nkb; ++kb) {
             const int s = kb % kStages;
             const uint32_t ph = (uint32_t)(kb / kStages) & 1u;
-            if (!mbar_wait(full(s), ph, spin)) { atomicOr(e.err, DEV_GUARD); s_abort = 1; break; }
+            if (!__all_sync(0xffffffffu, mbar_wait(full(s), ph, spin))) {
+                if (lane == 0) { atomicOr(e.err, DEV_GUARD); s_abort = 1; }
+                break;
+            }
             tc_fence_after();
             const uint32_t a0 = smem_u32(sA + s * kABytes), b0 = smem_u32(sB + s * kBBytes);
 #pragma unroll
@@ -271,8 +289,8 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const __grid_const
 // one K step (64: 128-byte rows and swizzle; 32: 64-byte rows and swizzle); a K step is
 // (tap, source, channel block), taps outermost, matching the weights' column order
 // tap * Cin + ci. Roles (6 warps):
-//   - warp 0, lane 0: TMA producer over all items' K steps, through a ring of kSt stages;
-//   - warp 1, lane 0: MMA issuer; item i accumulates into TMEM buffer i & 1 (2 x BN columns),
+//   - warp 0: TMA producer over all items' K steps, through a ring of kSt stages;
+//   - warp 1: MMA issuer (an elected lane); item i accumulates into TMEM buffer i & 1 (2 x BN columns),
 //     so the MMAs of item i + 1 run while the epilogue drains item i;
 //   - warps 2..5: epilogue; warp w reads TMEM lanes 32 (w % 4) .. +31 (its row quarter),
 //     then releases the buffer.
@@ -332,7 +350,7 @@ __global__ void __launch_bounds__(kConvThreads, 1) tc_conv_kernel(const __grid_c
     __shared__ int s_abort;
     __shared__ float s_bias[512];       // the bias of every output channel, staged once
     volatile int* abort_flag = &s_abort;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     const int tw = 1 << a.tw_log2, th = kBM >> a.tw_log2;
     const int nb0 = a.C0 / CB, nb1 = a.nsrc > 1 ? a.C1 / CB : 0, per_tap = nb0 + nb1;
     const int nkb = 9 * per_tap;
@@ -358,7 +376,7 @@ __global__ void __launch_bounds__(kConvThreads, 1) tc_conv_kernel(const __grid_c
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = *tmem_slot;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
 
     if (warp == 0) {
         // The warp fills the stages in order, all lanes waiting for the same one: lane 0 arms its
@@ -396,44 +414,40 @@ __global__ void __launch_bounds__(kConvThreads, 1) tc_conv_kernel(const __grid_c
         if (lane == 0)
             for (uint32_t k = issued > (uint32_t)kSt ? issued - kSt : 0; k < issued; ++k) mbar_wait(full((int)(k % kSt)), (k / kSt) & 1u);
     } else if (warp == 1) {
-        if (lane == 0) {
-            const uint32_t idesc = instr_desc(BN);
-            uint32_t kc = 0, i = 0;
-            for (int item = blockIdx.x; item < a.items && !*abort_flag; item += gridDim.x, ++i) {
-                const uint32_t buf = i & 1u, use = i >> 1;
-                if (!mbar_wait_or_abort(acc_empty(buf), (use & 1u) ^ 1u, abort_flag)) {
-                    atomicOr(e.err, DEV_GUARD);
-                    s_abort = 1;
-                    break;
-                }
+        const uint32_t idesc = instr_desc(BN);
+        uint32_t ph = 0, i = 0;
+        int s = 0;
+        bool ok = true;
+        for (int item = blockIdx.x; item < a.items; item += gridDim.x, ++i) {
+            const uint32_t buf = i & 1u, use = i >> 1;
+            ok = __all_sync(0xffffffffu, mbar_wait_or_abort(acc_empty(buf), (use & 1u) ^ 1u, abort_flag));
+            if (!ok) break;
+            tc_fence_after();
+            const uint32_t acc = tmem + buf * kT * BN;
+            for (int kb = 0; kb < nkb; ++kb) {
+                ok = __all_sync(0xffffffffu, mbar_wait_or_abort(full(s), ph, abort_flag));
+                if (!ok) break;
                 tc_fence_after();
-                const uint32_t acc = tmem + buf * kT * BN;
-                bool ok = true;
-                for (int kb = 0; kb < nkb; ++kb, ++kc) {
-                    const int s = kc % kSt;
-                    const uint32_t ph = (kc / kSt) & 1u;
-                    if (!mbar_wait_or_abort(full(s), ph, abort_flag)) { ok = false; break; }
-                    tc_fence_after();
-                    const uint32_t b0 = smem_u32(sB + s * kBBytes);
+                const uint32_t b0 = smem_u32(sB + s * kBBytes);
 #pragma unroll
-                    for (int k = 0; k < CB / 16; ++k) {
-                        const uint64_t db = CB == 64 ? smem_desc(b0 + k * 32) : smem_desc64(b0 + k * 32);
+                for (int k = 0; k < CB / 16; ++k) {
+                    const uint64_t db = CB == 64 ? smem_desc(b0 + k * 32) : smem_desc64(b0 + k * 32);
 #pragma unroll
-                        for (int t = 0; t < kT; ++t) {
-                            const uint32_t a0 = smem_u32(sA + (s * kT + t) * kABytes);
-                            const uint64_t da = CB == 64 ? smem_desc(a0 + k * 32) : smem_desc64(a0 + k * 32);
-                            tc_mma(acc + (uint32_t)(t * BN), da, db, idesc, (kb | k) != 0 ? 1u : 0u);
-                        }
+                    for (int t = 0; t < kT; ++t) {
+                        const uint32_t a0 = smem_u32(sA + (s * kT + t) * kABytes);
+                        const uint64_t da = CB == 64 ? smem_desc(a0 + k * 32) : smem_desc64(a0 + k * 32);
+                        tc_mma(acc + (uint32_t)(t * BN), da, db, idesc, (kb | k) != 0 ? 1u : 0u);
                     }
-                    tc_commit(empty(s));
                 }
-                if (!ok) {
-                    atomicOr(e.err, DEV_GUARD);
-                    s_abort = 1;
-                    break;
-                }
-                tc_commit(acc_full(buf));
+                tc_commit(empty(s));
+                if (++s == kSt) { s = 0; ph ^= 1u; }
             }
+            if (!ok) break;
+            tc_commit(acc_full(buf));
+        }
+        if (!ok && lane == 0) {
+            atomicOr(e.err, DEV_GUARD);
+            s_abort = 1;
         }
     } else {
         // epilogue warps 2..5: TMEM lane quarter q = warp % 4 holds rows 32 q .. 32 q + 31
@@ -529,13 +543,17 @@ __global__ void __launch_bounds__(kConvThreads, 1) tc_conv_kernel(const __grid_c
 // of output rows [y0, y1); the CTA loads the chunk's input rows y0 - 1 .. y1 one at a time,
 // each as ONE TMA box per source holding 136 pixels (x0 - 1 .. x0 + 134) of every input
 // channel, into a ring of row slots. Output row y reads the slots of rows y - 1, y, y + 1
-// in place, each tap's A operand starting 16 bytes (one pixel) further along its row: every
-// input row crosses from L2 once per chunk instead of three times. Layouts are the
-// no-swizzle K-major canonical form: 8 rows x 16 bytes (8 channels) per core matrix, core
-// matrices 128 bytes apart along M (pixels) and one channel group apart along K (136 x 16
-// bytes for A, N x 16 bytes for B). The weights are loaded once per CTA. K order (tap
-// outermost, then channel) and the K16 steps are tc_conv_kernel's, so the two kernels give
-// identical results.
+// in place, each tap's A operand starting one pixel further along its row: every input row
+// crosses from L2 once per chunk instead of three times. A source's row lies in the slot as
+// chunks of 64, 32 or 16 channels (the widest that divides its channel count), each a K-major
+// tile of 136 pixel rows of 128, 64 or 32 bytes with the swizzle of that width: one box per
+// chunk, and a tap's shift moves the operand's start by one pixel row, the swizzle following
+// the address.
+// The weights are loaded once per CTA, in the no-swizzle K-major canonical form: 8 rows x 16
+// bytes per core matrix, core matrices 128 bytes apart along N and one channel group (N x 16
+// bytes) apart along K. K order (tap outermost, then channel) and the K16 steps are
+// tc_conv_kernel's, so the two kernels give identical results. Rows whose A operands go on to
+// TMEM (kTA) stay in the no-swizzle form, a 136 x 16-byte group per 8 channels.
 constexpr int kHaloW = 136;                        // box width: 128 + 2 halo, rounded for alignment
 constexpr uint32_t kHaloGroup = kHaloW * 16;       // bytes of one 8-channel group of a row slot
 
@@ -544,6 +562,16 @@ __device__ __forceinline__ uint64_t desc_plain(uint32_t addr, uint32_t lbo, uint
     d |= (uint64_t)((lbo >> 4) & 0x3FFFu) << 16;      // leading byte offset: next core matrix along K
     d |= (uint64_t)((sbo >> 4) & 0x3FFFu) << 32;      // stride byte offset: next 8 rows along M / N
     d |= (uint64_t)1 << 46;                           // descriptor version; layout 0: no swizzle
+    return d;
+}
+// Pixel rows of cb channels (64, 32 or 16) with the swizzle of that width, 8-row atoms one
+// after the other. The start may be any pixel row or 32-byte step of a tile: the swizzle
+// is a function of the address.
+__device__ __forceinline__ uint64_t desc_rows(uint32_t addr, int cb) {
+    uint64_t d = (uint64_t)((addr >> 4) & 0x3FFFu);
+    d |= (uint64_t)cb << 32;                          // stride byte offset: 8 rows x 2 cb bytes, in 16-byte units
+    d |= (uint64_t)1 << 46;
+    d |= (uint64_t)(cb == 64 ? 2 : cb == 32 ? 4 : 6) << 61;
     return d;
 }
 __device__ __forceinline__ void tma_load_5d(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, int c3, int c4,
@@ -563,13 +591,14 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map
 // tcgen05.cp of a 128-row x 256-bit matrix (128 pixels x 16 BF16 channels, K-major, the
 // descriptor's canonical layout) from shared memory into TMEM columns [taddr, taddr + 8).
 __device__ __forceinline__ void tc_cp_128x256b(uint32_t taddr, uint64_t sdesc) {
-    asm volatile("tcgen05.cp.cta_group::1.128x256b [%0], %1;" ::"r"(taddr), "l"(sdesc) : "memory");
+    asm volatile("{\n.reg .pred e;\nelect.sync _|e, 0xffffffff;\n@e tcgen05.cp.cta_group::1.128x256b [%0], %1;\n}\n" ::"r"(taddr), "l"(sdesc)
+                 : "memory");
 }
 // tcgen05.mma.kind::f16 with the A operand read from TMEM (128 lanes = M rows, K in columns).
 __device__ __forceinline__ void tc_mma_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t b, uint32_t idesc,
                                           uint32_t accumulate) {
     asm volatile(
-        "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(tmem_d),
+        "{\n.reg .pred p, e;\nelect.sync _|e, 0xffffffff;\nsetp.ne.b32 p, %4, 0;\n@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(tmem_d),
         "r"(tmem_a), "l"(b), "r"(idesc), "r"(accumulate)
         : "memory");
 }
@@ -584,12 +613,14 @@ constexpr uint32_t kTaRowCols = 3 * 2 * 8;         // taps x K steps (at most 32
 
 struct HaloArgs {
     int nsrc, C0, C1, cin;
+    int cb0, cb1;               // the sources' channel chunks in a row slot (64, 32 or 16)
     int B, H, W;
     int chunk, chunks_y;        // output rows per work item; items per strip column
     int items;                  // n_slices x slice_items
     int n_slices, slice_items;  // output-channel slices of BN (fan-out; else 1) and items per slice,
                                 // (W / 128) x chunks_y x B
     int stages;                 // row slots in the ring (>= 4; fan-out >= 2)
+    int sets;                   // sets of four epilogue warps, taking the output rows in turn (1 or 2)
     uint32_t a_bytes, b_bytes;  // one row slot (all sources), the resident weights
     __nv_bfloat16* up16;
 };
@@ -626,26 +657,67 @@ __device__ __forceinline__ HaloItem halo_item(const HaloArgs& a, int item) {
 // both forms give the same values (0 + x = x; at most the sign of an all-zero sum differs).
 // Each row slot in shared memory is read by the MMAs of its own input row only; the row's A
 // operand crosses from shared memory three times (dx) instead of nine.
-constexpr int kFanMaxAcc = 8;   // accumulator slots (BN 32: 8; BN 64: 4)
-constexpr int kFanCases = 6;    // which of a load's three output rows exist
-// Fan-out accumulator ring and residency: 256 TMEM columns (eight rows' accumulators at BN
-// 32, four at BN 64) and two CTAs per SM. Three CTAs of a four-row ring at BN 32 (128
-// columns, 96 registers) measured slower on every layer (32 -> 32 at 1088 x 1920: 94.0 us
-// against 88.7).
-__host__ __device__ constexpr int fan_acc(int bn) { return 256 / bn; }
-__host__ __device__ constexpr int fan_ctas(int bn) { return 2; }
-// The MMAs of one K16 step of one load in fan-out form: n pieces (two where the accumulator
-// ring wraps), each (accumulator address, instruction descriptor, B offset in 16-byte units).
-struct FanPlan { uint4 p[2]; int n, pad0, pad1, pad2; };
-// Static shared memory of tc_conv_halo_kernel<BN>, rounded up: the bias (512 floats), the
-// abort flag, the epilogue's stage (4 warps x 32 pixels x BN BF16 channels) and the fan-out
-// MMA plans.
-__host__ __device__ constexpr size_t halo_static_smem(int bn) {
-    return 2048 + 64 + (size_t)4 * 32 * bn * 2 + sizeof(FanPlan) * kFanCases * kFanMaxAcc;
+// Accumulator ring and residency: 256 TMEM columns (eight rows' accumulators at BN 32, four at
+// BN 64) and two CTAs per SM where shared memory allows two; else all 512 columns (kWide), which
+// halves the loads whose MMAs split at the ring's wrap (64 -> 64 at 1088 x 1920 131 -> 112 us,
+// 64 + 128 -> 64 354 -> 338, 32 + 64 -> 32 at 2176 x 3840 408 -> 393; but one wide CTA where
+// two would fit: 32 -> 32 at 2176 x 3840 173 -> 221).
+constexpr int kFanMaxAcc = 16;
+__host__ __device__ constexpr int fan_cols(bool wide) { return wide ? 512 : 256; }
+// Static shared memory of tc_conv_halo_kernel, rounded up: the bias (512 floats) and the abort
+// flag; and the epilogue's stage (a set's four warps x 32 pixels x BN BF16 channels).
+constexpr size_t kHaloStatic = 2048 + 64;
+__host__ __device__ constexpr size_t halo_stage(int bn, int sets) { return (size_t)sets * 4 * 32 * bn * 2; }
+constexpr int kFanThreads = 320;    // two sets of epilogue warps
+
+// One load's MMAs in fan-out form for sources of C0 and C1 channels (C1: 0 with one source),
+// every operand a base descriptor plus a constant. The row ring's pace is the MMA warp's: its
+// instructions come cold from the cache at each row, beside eight epilogue warps, and a loop's
+// branch costs as much as an MMA, so a tap's steps are straight line and the three shifts loop
+// around them. Measured at 2176 x 3840, 16 -> 32 channels / 32 + 64 -> 32, and at 1088 x 1920,
+// 64 + 128 -> 64: loops over chunks and steps 184 / 615 / 446 us, all shifts unrolled
+// 145 / 422 / 375, this 144 / 408 / 354.
+struct FanRow {
+    uint64_t a0, a1;            // the sources' descriptors at the row's first pixel
+    uint64_t b0, b1;            // B at each piece's first row
+    uint32_t acc0, acc1, id0, id1;
+    bool split;                 // a second piece
+};
+__device__ __forceinline__ uint64_t desc_add(uint64_t d, uint32_t n) {      // the address field is in the low word
+    return (d & 0xFFFFFFFF00000000ull) | ((uint32_t)d + n);
+}
+__host__ __device__ constexpr int chunk_channels(int C) { return C % 64 == 0 ? 64 : C % 32 == 0 ? 32 : 16; }
+template <int BN, int C0, int C1>
+__device__ __forceinline__ void fan_row(const FanRow& f) {
+    constexpr uint32_t b_grp = 3u * BN;                                     // 16-byte units, as all here
+    auto step = [&](bool split, uint32_t xa0, uint32_t xa1, uint32_t xb) {
+#pragma unroll
+        for (int q = 0; q < (C0 + C1) / 16; ++q) {
+            const bool first = q * 16 < C0;
+            const int ch = first ? q * 16 : q * 16 - C0, cb = first ? chunk_channels(C0) : chunk_channels(C1 ? C1 : 16);
+            const uint32_t oa = (uint32_t)(ch / cb * kHaloW * (cb >> 3) + ch % cb / 8), ob = (uint32_t)(2 * q) * b_grp + xb;
+            const uint64_t da = first ? desc_add(f.a0, oa + xa0) : desc_add(f.a1, oa + xa1);
+            tc_mma(f.acc0, da, desc_add(f.b0, ob), f.id0, 1u);
+            if (split) tc_mma(f.acc1, da, desc_add(f.b1, ob), f.id1, 1u);
+        }
+    };
+    auto run = [&](bool split) {
+        constexpr uint32_t p0 = chunk_channels(C0) >> 3, p1 = chunk_channels(C1 ? C1 : 16) >> 3, pb = (C0 + C1) / 8 * b_grp;
+#pragma unroll 1
+        for (uint32_t dx = 0; dx < 3; ++dx) step(split, dx * p0, dx * p1, dx * pb);
+    };
+    if (f.split) run(true);
+    else run(false);
 }
 
-template <int BN, bool kTA, bool kFan>
-__global__ void __launch_bounds__(kConvThreads, kFan ? fan_ctas(BN) : 1) tc_conv_halo_kernel(const __grid_constant__ CUtensorMap map0,
+// Bytes of one row slot (C1: 0 with one source).
+__host__ __device__ constexpr uint32_t halo_slot(int C0, int C1, bool ta) {
+    return ta ? ((uint32_t)(C0 + C1) * 2u * kHaloW + 1023u) & ~1023u
+              : (((uint32_t)C0 * 2u * kHaloW + 1023u) & ~1023u) + (((uint32_t)C1 * 2u * kHaloW + 1023u) & ~1023u);
+}
+
+template <int BN, bool kTA, bool kFan, bool kWide>
+__global__ void __launch_bounds__(kFan ? kFanThreads : kConvThreads, kFan && !kWide ? 2 : 1) tc_conv_halo_kernel(const __grid_constant__ CUtensorMap map0,
                                                                        const __grid_constant__ CUtensorMap map1,
                                                                        const __grid_constant__ CUtensorMap mapW,
                                                                        const HaloArgs a, const Epilogue e) {
@@ -655,23 +727,23 @@ __global__ void __launch_bounds__(kConvThreads, kFan ? fan_ctas(BN) : 1) tc_conv
     // epilogue; four measured no faster), then (kTA) the ring of input rows' A operands; a
     // power of two. Fan-out: a ring of 256 / BN accumulators.
     static_assert(!(kTA && kFan), "one form at a time");
-    static_assert(!kFan || (3 * BN <= 256 && 256 / BN <= kFanMaxAcc), "three rows' accumulators in one MMA");
-    constexpr uint32_t kAcc = kFan ? (uint32_t)fan_acc(BN) : 2u;
-    constexpr uint32_t kCols = (kTA || kFan) ? 256u : kAcc * BN;
+    static_assert(!kFan || (3 * BN <= 256 && 512 / BN <= kFanMaxAcc), "three rows' accumulators in one MMA");
+    constexpr uint32_t kAcc = kFan ? (uint32_t)(fan_cols(kWide) / BN) : 2u;
+    constexpr uint32_t kCols = kTA ? 256u : kAcc * BN;
     static_assert(!kTA || 2 * BN + kTaSlots * kTaRowCols <= 256, "the TMEM ring fits");
     const int kSt = a.stages;
     uint8_t* sB = smem;
     uint8_t* sA = smem + ((a.b_bytes + 1023) & ~1023u);
-    const uint32_t a_stride = (a.a_bytes + 1023) & ~1023u;
+    const uint32_t a_stride = halo_slot(a.C0, a.C1, kTA);
     // full[kSt], empty[kSt], acc_full[8], acc_empty[8], w (weights landed), wfree (the weights'
     // last MMAs done: a slice's weights may be replaced)
-    uint64_t* bars = reinterpret_cast<uint64_t*>(sA + kSt * a_stride);
+    uint4* s_stage = reinterpret_cast<uint4*>(sA + kSt * a_stride);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sA + kSt * a_stride + halo_stage(BN, a.sets));
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kSt + 2 * kFanMaxAcc + 2);
     __shared__ int s_abort;
-    __shared__ float s_bias[512];       // the bias of every output channel, staged once
-    __shared__ FanPlan s_fan[kFanCases][kFanMaxAcc];
+    __shared__ __align__(16) float s_bias[512];       // the bias of every output channel, staged once
     volatile int* abort_flag = &s_abort;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     auto full = [&](int s) { return smem_u32(&bars[s]); };
     auto empty = [&](int s) { return smem_u32(&bars[kSt + s]); };
     auto acc_full = [&](int b) { return smem_u32(&bars[2 * kSt + b]); };
@@ -700,8 +772,26 @@ __global__ void __launch_bounds__(kConvThreads, kFan ? fan_ctas(BN) : 1) tc_conv
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = *tmem_slot;
-    const uint32_t src1_off = (uint32_t)(a.C0 / 8) * kHaloGroup;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+    // the second source's place in a row slot (the swizzled tiles start on 1024 bytes)
+    const uint32_t src1_off = kTA ? (uint32_t)(a.C0 / 8) * kHaloGroup : ((uint32_t)a.C0 * 2u * kHaloW + 1023u) & ~1023u;
+    const int nch0 = kTA ? 0 : a.C0 / a.cb0, nch1 = kTA || a.nsrc < 2 ? 0 : a.C1 / a.cb1;
+    // the K16 steps of the tap dx pixels along a row, in channel order: mma(A's descriptor);
+    // da0, da1: the sources' descriptors at the row's first pixel
+    auto each_step = [&](uint64_t da0, uint64_t da1, int dx, auto&& mma) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int cb = i ? a.cb1 : a.cb0;
+            uint64_t da = (i ? da1 : da0) + (uint64_t)(dx * (cb >> 3));       // one pixel: 2 cb bytes
+            for (int c = i ? nch1 : nch0; c > 0; --c) {
+                for (int k = 0; k < cb; k += 16) {
+                    mma(da);
+                    da += 2;                                                  // 16 channels: 32 bytes
+                }
+                da += (uint64_t)((kHaloW - 1) * (cb >> 3));                   // the next chunk's tile
+            }
+        }
+    };
     if (kFan) {
         // fan-out accumulators start at zero and every MMA adds to them: each epilogue warp
         // clears its lane quarter of the ring now and of each row again once it has read it
@@ -749,8 +839,17 @@ __global__ void __launch_bounds__(kConvThreads, kFan ? fan_ctas(BN) : 1) tc_conv
                     }
                     mbar_expect_tx(full(s), a.a_bytes);
                     const uint32_t dst = smem_u32(sA + s * a_stride);
-                    tma_load_5d(dst, &map0, 0, it.tx * 128 - 1, it.y0 + r, it.b, 0, full(s));
-                    if (a.nsrc > 1) tma_load_5d(dst + src1_off, &map1, 0, it.tx * 128 - 1, it.y0 + r, it.b, 0, full(s));
+                    if (kTA) {
+                        tma_load_5d(dst, &map0, 0, it.tx * 128 - 1, it.y0 + r, it.b, 0, full(s));
+                        if (a.nsrc > 1) tma_load_5d(dst + src1_off, &map1, 0, it.tx * 128 - 1, it.y0 + r, it.b, 0, full(s));
+                    } else {
+                        for (int c = 0; c < nch0; ++c)
+                            tma_load_4d(dst + (uint32_t)(c * a.cb0 * 2 * kHaloW), &map0, c * a.cb0, it.tx * 128 - 1, it.y0 + r,
+                                        it.b, full(s));
+                        for (int c = 0; c < nch1; ++c)
+                            tma_load_4d(dst + src1_off + (uint32_t)(c * a.cb1 * 2 * kHaloW), &map1, c * a.cb1,
+                                        it.tx * 128 - 1, it.y0 + r, it.b, full(s));
+                    }
                     if (++s == kSt) { s = 0; ph ^= 1u; }
                 }
             }
@@ -759,217 +858,196 @@ __global__ void __launch_bounds__(kConvThreads, kFan ? fan_ctas(BN) : 1) tc_conv
             mbar_wait(wbar, wfree_ph);      // the last weights load (one more than the reloads)
         }
     } else if (warp == 1 && kFan) {
-        // The MMAs of a load depend only on which of its three output rows exist (the load's
-        // case: lo = max(0, k - 2) - k and hi = min(rows - 1, k) - k, six cases) and on the
-        // ring residue of its row k, so the warp tabulates them once: per case and residue the
-        // one or two pieces (two where the ring wraps) of every K16 step, each an accumulator
-        // address, an instruction descriptor (N) and the offset of its first B row (vertical
-        // tap k - h for its top row h, in 16-byte units). The issuing thread then spends two
-        // shared loads per load instead of forming pieces: it is blocked while the tensor
-        // pipe takes each MMA, so its other work adds directly to the layer's time.
-        for (int e_ = lane; e_ < kFanCases * (int)kAcc; e_ += 32) {
-            const int cs = e_ / (int)kAcc, r = e_ % (int)kAcc;
-            const int lo = cs == 0 ? 0 : cs <= 2 ? -1 : -2;                       // relative to k
-            const int hi = cs == 0 || cs == 1 || cs == 3 ? 0 : cs == 2 || cs == 4 ? -1 : -2;
-            // ring index of row k + x is r + x (mod kAcc); the piece holding the top row first
-            FanPlan& pl = s_fan[cs][r];
-            int n = 0;
-            for (int h = hi; h >= lo;) {
-                const uint32_t ih = (uint32_t)(r + h + (int)kAcc) % kAcc;
-                const int b = max(lo, h - (int)ih);
-                pl.p[n++] = make_uint4(tmem + (kAcc - 1u - ih) * BN, instr_desc((h - b + 1) * BN), (uint32_t)(-h * BN), 0u);
-                h = b - 1;
-            }
-            pl.n = n;
-        }
-        __syncwarp();
-        if (lane == 0) {
-            const int q16 = a.cin / 16, G = a.cin / 8;
-            const uint32_t b_grp = 3u * BN * 16u;                         // next channel group of B (LBO)
-            const uint64_t db0 = desc_plain(smem_u32(sB), b_grp, 128);
-            const uint64_t dq_a = (2u * kHaloGroup) >> 4;                 // the next 16 channels of A
-            const uint64_t dq_b = (2u * b_grp) >> 4;                      // ... of B
-            const uint64_t dx_b = ((uint32_t)G * b_grp) >> 4;             // the next horizontal tap of B
-            bool ok = mbar_wait_or_abort(wbar, 0, abort_flag);
-            int wslice = (int)blockIdx.x % a.n_slices;
-            uint32_t w_ph = 0;
-            uint32_t i0 = 0;            // output rows of earlier items
-            // the current load's ring slot, its phase and its shared-memory row (kept by increment)
-            int slot = 0;
-            uint32_t phase = 0, row_smem = smem_u32(sA);
-            // Descriptors are affine in their address (the 14-bit field holds address / 16, and
-            // no offset here carries out of it): every MMA is a base descriptor plus a constant.
-            for (int item = blockIdx.x; ok && item < a.items && !*abort_flag; item += gridDim.x) {
-                const HaloItem it = halo_item(a, item);
-                if (it.slice != wslice) {
-                    // the next slice's weights: once this slice's MMAs have read theirs
-                    tc_commit(wfree);
-                    w_ph ^= 1u;
-                    if (!mbar_wait_or_abort(wbar, w_ph, abort_flag)) { ok = false; break; }
-                    wslice = it.slice;
-                }
-                // load k is input row y0 - 1 + k; it feeds output rows k - 2 .. k of the item
-                for (int k = 0; ok && k <= it.rows + 1; ++k) {
-                    const int lo = max(0, k - 2) - k, hi = min(it.rows - 1, k) - k;
-                    const int cs = -lo * (1 - lo) / 2 - hi;               // (0,0) 0; (-1,0) 1; (-1,-1) 2; (-2,0) 3; ...
-                    const FanPlan& pl = s_fan[cs][(i0 + (uint32_t)k) % kAcc];
-                    const uint4 c0 = pl.p[0], c1 = pl.p[1];
-                    const int nc = pl.n;
-                    if (hi == 0) {
-                        // output row k's first load: its accumulator must be free
-                        const uint32_t i = i0 + (uint32_t)k;
-                        if (!mbar_wait_or_abort(acc_empty(i % kAcc), ((i / kAcc) & 1u) ^ 1u, abort_flag)) {
-                            ok = false;
-                            break;
-                        }
-                    }
-                    if (!mbar_wait_or_abort(full(slot), phase, abort_flag)) { ok = false; break; }
-                    tc_fence_after();
-                    const uint64_t da_row = desc_plain(row_smem, kHaloGroup, 128);
-#pragma unroll
-                    for (int dx = 0; dx < 3; ++dx) {
-                        uint64_t da = da_row + (uint64_t)dx;                      // one pixel: 16 bytes
-                        uint64_t db = db0 + (uint64_t)dx * dx_b;
-                        for (int q = 0; q < q16; ++q) {
-                            tc_mma(c0.x, da, db + c0.z, c0.y, 1u);
-                            if (nc > 1) tc_mma(c1.x, da, db + c1.z, c1.y, 1u);
-                            da += dq_a;
-                            db += dq_b;
-                        }
-                    }
-                    // the row slot is free once its MMAs have read it; output row k - 2 is complete
-                    tc_commit(empty(slot));
-                    if (k >= 2) tc_commit(acc_full((i0 + (uint32_t)(k - 2)) % kAcc));
-                    if (++slot == kSt) {
-                        slot = 0;
-                        phase ^= 1u;
-                        row_smem = smem_u32(sA);
-                    } else {
-                        row_smem += a_stride;
-                    }
-                }
+        const int G = a.cin / 8;
+        const uint32_t b_grp = 3u * BN * 16u;                         // next channel group of B (LBO)
+        const uint64_t db0 = desc_plain(smem_u32(sB), b_grp, 128);
+        const uint64_t dq_b = (2u * b_grp) >> 4;                      // the next 16 channels of B
+        const uint64_t dx_b = ((uint32_t)G * b_grp) >> 4;             // the next horizontal tap of B
+        bool ok = __all_sync(0xffffffffu, mbar_wait_or_abort(wbar, 0, abort_flag));
+        int wslice = (int)blockIdx.x % a.n_slices;
+        uint32_t w_ph = 0;
+        uint32_t i0 = 0;            // output rows of earlier items
+        // the current load's ring slot, its phase and its shared-memory row (kept by increment)
+        int slot = 0;
+        uint32_t phase = 0, row_smem = smem_u32(sA);
+        // Descriptors are affine in their address (the 14-bit field holds address / 16, and
+        // no offset here carries out of it): every MMA is a base descriptor plus a constant.
+        for (int item = blockIdx.x; ok && item < a.items; item += gridDim.x) {
+            const HaloItem it = halo_item(a, item);
+            if (it.slice != wslice) {
+                // the next slice's weights: once this slice's MMAs have read theirs
+                tc_commit(wfree);
+                w_ph ^= 1u;
+                ok = __all_sync(0xffffffffu, mbar_wait_or_abort(wbar, w_ph, abort_flag));
                 if (!ok) break;
-                i0 += (uint32_t)it.rows;
+                wslice = it.slice;
             }
-            if (!ok) {
-                atomicOr(e.err, DEV_GUARD);
-                s_abort = 1;
+            // load k is input row y0 - 1 + k; it feeds output rows k - 2 .. k of the item
+            for (int k = 0; k <= it.rows + 1; ++k) {
+                // the output rows that exist, lo .. hi of them: one piece with the top row first
+                // and, where the ring wraps below it, a second; each an accumulator address, N
+                // and the offset of its first B row (vertical tap k - h for its top row h)
+                const int lo = max(0, k - 2), hi = min(it.rows - 1, k);
+                const uint32_t ih = (i0 + (uint32_t)hi) % kAcc;
+                const int n = hi - lo + 1, n0 = min(n, (int)ih + 1), n1 = n - n0;
+                const uint32_t acc0 = tmem + (kAcc - 1u - ih) * BN, acc1 = tmem;   // the wrapped piece: ring index kAcc - 1
+                const uint32_t id0 = instr_desc(n0 * BN), id1 = instr_desc(n1 * BN);
+                const uint64_t b0 = db0 + (uint64_t)((k - hi) * BN), b1 = b0 + (uint64_t)(n0 * BN);
+                if (hi == k) {
+                    // output row k's first load: its accumulator must be free
+                    const uint32_t i = i0 + (uint32_t)k;
+                    ok = __all_sync(0xffffffffu, mbar_wait_or_abort(acc_empty(i % kAcc), ((i / kAcc) & 1u) ^ 1u, abort_flag));
+                    if (!ok) break;
+                }
+                ok = __all_sync(0xffffffffu, mbar_wait_or_abort(full(slot), phase, abort_flag));
+                if (!ok) break;
+                tc_fence_after();
+                const uint64_t da0 = desc_rows(row_smem, a.cb0), da1 = desc_rows(row_smem + src1_off, a.cb1);
+                // the channel counts of the U-Net's layers whose weights fit; any other runs the
+                // general loops
+                const FanRow fr{da0, da1, b0, b1, acc0, acc1, id0, id1, n1 != 0};
+                if (a.C0 == 32 && a.C1 == 0) fan_row<BN, 32, 0>(fr);
+                else if (a.C0 == 16 && a.C1 == 0) fan_row<BN, 16, 0>(fr);
+                else if (a.C0 == 64 && a.C1 == 0) fan_row<BN, 64, 0>(fr);
+                else if (a.C0 == 128 && a.C1 == 0) fan_row<BN, 128, 0>(fr);
+                else if (a.C0 == 32 && a.C1 == 64) fan_row<BN, 32, 64>(fr);
+                else if (a.C0 == 64 && a.C1 == 128) fan_row<BN, 64, 128>(fr);
+                else {
+#pragma unroll 1
+                    for (int dx = 0; dx < 3; ++dx) {
+                        uint64_t db = (uint64_t)dx * dx_b;
+                        each_step(da0, da1, dx, [&](uint64_t da) {
+                            tc_mma(acc0, da, b0 + db, id0, 1u);
+                            if (n1) tc_mma(acc1, da, b1 + db, id1, 1u);
+                            db += dq_b;
+                        });
+                    }
+                }
+                // the row slot is free once its MMAs have read it; output row k - 2 is complete
+                tc_commit(empty(slot));
+                if (k >= 2) tc_commit(acc_full((i0 + (uint32_t)(k - 2)) % kAcc));
+                if (++slot == kSt) {
+                    slot = 0;
+                    phase ^= 1u;
+                    row_smem = smem_u32(sA);
+                } else {
+                    row_smem += a_stride;
+                }
             }
+            if (!ok) break;
+            i0 += (uint32_t)it.rows;
+        }
+        if (!ok && lane == 0) {
+            atomicOr(e.err, DEV_GUARD);
+            s_abort = 1;
         }
     } else if (warp == 1 && kTA) {
-        if (lane == 0) {
-            const uint32_t idesc = instr_desc(BN);
-            const uint32_t b0 = smem_u32(sB);
-            const int q16 = a.cin / 16, g_tap = a.cin / 8;
-            const uint32_t ta0 = tmem + 2u * BN;
-            bool ok = mbar_wait_or_abort(wbar, 0, abort_flag);
-            uint32_t base = 0, i = 0;   // ring index of the item's first load; output rows so far
-            for (int item = blockIdx.x; ok && item < a.items && !*abort_flag; item += gridDim.x) {
-                const HaloItem it = halo_item(a, item);
-                for (int j = 0; ok && j < it.rows; ++j, ++i) {
-                    // output row y0 + j reads loads j, j + 1, j + 2 of the item
-                    const uint32_t buf = i % kAcc, use = i / kAcc;
-                    // row i - 2's MMAs are done once its accumulator is free again: the TMEM
-                    // slots they read may be overwritten
-                    if (!mbar_wait_or_abort(acc_empty(buf), (use & 1u) ^ 1u, abort_flag)) { ok = false; break; }
-                    if (j == 0 && i > 0) {
-                        // a new item reloads three rows: the previous row's MMAs must be done too
-                        const uint32_t pi = i - 1;
-                        if (!mbar_wait_or_abort(acc_full(pi % kAcc), (pi / kAcc) & 1u, abort_flag)) { ok = false; break; }
-                    }
-                    for (int d = (j == 0 ? 0 : 2); d < 3 && ok; ++d) {
-                        const uint32_t k = base + (uint32_t)(j + d);
-                        ok = mbar_wait_or_abort(full(k % kSt), (k / kSt) & 1u, abort_flag);
-                        if (!ok) break;
-                        tc_fence_after();
-                        const uint32_t row = smem_u32(sA + (k % kSt) * a_stride);
-                        const uint32_t slot = ta0 + (k % kTaSlots) * kTaRowCols;
-                        for (int dx = 0; dx < 3; ++dx)
-                            for (int q = 0; q < q16; ++q)
-                                tc_cp_128x256b(slot + (uint32_t)(dx * q16 + q) * 8u,
-                                               desc_plain(row + (uint32_t)dx * 16u + (uint32_t)(2 * q) * kHaloGroup,
-                                                          kHaloGroup, 128));
-                        // the shared-memory slot is free once its copies have run
-                        tc_commit(empty(k % kSt));
-                    }
-                    if (!ok) break;
-                    const uint32_t acc = tmem + buf * BN;
-                    for (int t = 0; t < 9; ++t) {
-                        const uint32_t k = base + (uint32_t)(j + t / 3);
-                        const uint32_t slot = ta0 + (k % kTaSlots) * kTaRowCols + (uint32_t)((t % 3) * q16) * 8u;
-                        for (int q = 0; q < q16; ++q) {
-                            const uint64_t db = desc_plain(b0 + (uint32_t)(t * g_tap + 2 * q) * (BN * 16), BN * 16, 128);
-                            tc_mma_ta(acc, slot + (uint32_t)q * 8u, db, idesc, (t | q) != 0 ? 1u : 0u);
-                        }
-                    }
-                    tc_commit(acc_full(buf));
+        const uint32_t idesc = instr_desc(BN);
+        const uint32_t b0 = smem_u32(sB);
+        const int q16 = a.cin / 16, g_tap = a.cin / 8;
+        const uint32_t ta0 = tmem + 2u * BN;
+        bool ok = __all_sync(0xffffffffu, mbar_wait_or_abort(wbar, 0, abort_flag));
+        uint32_t base = 0, i = 0;   // ring index of the item's first load; output rows so far
+        for (int item = blockIdx.x; ok && item < a.items; item += gridDim.x) {
+            const HaloItem it = halo_item(a, item);
+            for (int j = 0; ok && j < it.rows; ++j, ++i) {
+                // output row y0 + j reads loads j, j + 1, j + 2 of the item
+                const uint32_t buf = i % kAcc, use = i / kAcc;
+                // row i - 2's MMAs are done once its accumulator is free again: the TMEM
+                // slots they read may be overwritten
+                if (!__all_sync(0xffffffffu, mbar_wait_or_abort(acc_empty(buf), (use & 1u) ^ 1u, abort_flag))) { ok = false; break; }
+                if (j == 0 && i > 0) {
+                    // a new item reloads three rows: the previous row's MMAs must be done too
+                    const uint32_t pi = i - 1;
+                    if (!__all_sync(0xffffffffu, mbar_wait_or_abort(acc_full(pi % kAcc), (pi / kAcc) & 1u, abort_flag))) { ok = false; break; }
                 }
-                if (!ok) break;
-                base += (uint32_t)it.rows + 2;
-            }
-            if (!ok) {
-                atomicOr(e.err, DEV_GUARD);
-                s_abort = 1;
-            }
-        }
-    } else if (warp == 1) {
-        if (lane == 0) {
-            const uint32_t idesc = instr_desc(BN);
-            const int q16 = a.cin / 16, g_tap = a.cin / 8;
-            const uint64_t db0 = desc_plain(smem_u32(sB), BN * 16, 128);
-            const uint64_t dq_a = (2u * kHaloGroup) >> 4;                 // the next 16 channels of A
-            const uint64_t dq_b = (2u * BN * 16u) >> 4;                   // ... of B
-            const uint64_t dtap_b = ((uint32_t)g_tap * BN * 16u) >> 4;    // the next tap of B
-            bool ok = mbar_wait_or_abort(wbar, 0, abort_flag);
-            uint32_t base = 0, i = 0;   // ring index of the item's first load; output rows so far
-            for (int item = blockIdx.x; ok && item < a.items && !*abort_flag; item += gridDim.x) {
-                const HaloItem it = halo_item(a, item);
-                for (int j = 0; ok && j < it.rows; ++j, ++i) {
-                    // output row y0 + j reads loads j, j + 1, j + 2 of the item
-                    const uint32_t buf = i % kAcc, use = i / kAcc;
-                    if (!mbar_wait_or_abort(acc_empty(buf), (use & 1u) ^ 1u, abort_flag)) { ok = false; break; }
-                    uint32_t row_addr[3];
-                    for (int d = 0; d < 3 && ok; ++d) {
-                        const uint32_t k = base + (uint32_t)(j + d);
-                        ok = mbar_wait_or_abort(full(k % kSt), (k / kSt) & 1u, abort_flag);
-                        row_addr[d] = smem_u32(sA + (k % kSt) * a_stride);
-                    }
+                for (int d = (j == 0 ? 0 : 2); d < 3 && ok; ++d) {
+                    const uint32_t k = base + (uint32_t)(j + d);
+                    ok = __all_sync(0xffffffffu, mbar_wait_or_abort(full(k % kSt), (k / kSt) & 1u, abort_flag));
                     if (!ok) break;
                     tc_fence_after();
-                    const uint32_t acc = tmem + buf * BN;
-                    // a descriptor is affine in its address (the 14-bit field holds address / 16
-                    // and no offset here carries out of it): each MMA's operands are the row's or
-                    // the weights' base descriptor plus a constant, so the issuing thread spends
-                    // a few instructions per MMA instead of forming two descriptors
-                    const uint64_t da_row[3] = {desc_plain(row_addr[0], kHaloGroup, 128),
-                                                desc_plain(row_addr[1], kHaloGroup, 128),
-                                                desc_plain(row_addr[2], kHaloGroup, 128)};
-                    uint64_t db_tap = db0;
-#pragma unroll
-                    for (int t = 0; t < 9; ++t) {
-                        uint64_t da = da_row[t / 3] + (uint64_t)(t % 3);        // one pixel: 16 bytes
-                        uint64_t db = db_tap;
-                        for (int q = 0; q < q16; ++q) {
-                            tc_mma(acc, da, db, idesc, (t | q) != 0 ? 1u : 0u);
-                            da += dq_a;
-                            db += dq_b;
-                        }
-                        db_tap += dtap_b;
-                    }
-                    tc_commit(acc_full(buf));
-                    // load j (input row y0 + j - 1) has no later reader
-                    tc_commit(empty((base + (uint32_t)j) % kSt));
+                    const uint32_t row = smem_u32(sA + (k % kSt) * a_stride);
+                    const uint32_t slot = ta0 + (k % kTaSlots) * kTaRowCols;
+                    for (int dx = 0; dx < 3; ++dx)
+                        for (int q = 0; q < q16; ++q)
+                            tc_cp_128x256b(slot + (uint32_t)(dx * q16 + q) * 8u,
+                                           desc_plain(row + (uint32_t)dx * 16u + (uint32_t)(2 * q) * kHaloGroup,
+                                                      kHaloGroup, 128));
+                    // the shared-memory slot is free once its copies have run
+                    tc_commit(empty(k % kSt));
                 }
                 if (!ok) break;
-                // the item's last two loads
-                tc_commit(empty((base + (uint32_t)it.rows) % kSt));
-                tc_commit(empty((base + (uint32_t)it.rows + 1) % kSt));
-                base += (uint32_t)it.rows + 2;
+                const uint32_t acc = tmem + buf * BN;
+                for (int t = 0; t < 9; ++t) {
+                    const uint32_t k = base + (uint32_t)(j + t / 3);
+                    const uint32_t slot = ta0 + (k % kTaSlots) * kTaRowCols + (uint32_t)((t % 3) * q16) * 8u;
+                    for (int q = 0; q < q16; ++q) {
+                        const uint64_t db = desc_plain(b0 + (uint32_t)(t * g_tap + 2 * q) * (BN * 16), BN * 16, 128);
+                        tc_mma_ta(acc, slot + (uint32_t)q * 8u, db, idesc, (t | q) != 0 ? 1u : 0u);
+                    }
+                }
+                tc_commit(acc_full(buf));
             }
-            if (!ok) {
-                atomicOr(e.err, DEV_GUARD);
-                s_abort = 1;
+            if (!ok) break;
+            base += (uint32_t)it.rows + 2;
+        }
+        if (!ok && lane == 0) {
+            atomicOr(e.err, DEV_GUARD);
+            s_abort = 1;
+        }
+    } else if (warp == 1) {
+        const uint32_t idesc = instr_desc(BN);
+        const int g_tap = a.cin / 8;
+        const uint64_t db0 = desc_plain(smem_u32(sB), BN * 16, 128);
+        const uint64_t dq_b = (2u * BN * 16u) >> 4;                   // the next 16 channels of B
+        const uint64_t dtap_b = ((uint32_t)g_tap * BN * 16u) >> 4;    // the next tap of B
+        bool ok = __all_sync(0xffffffffu, mbar_wait_or_abort(wbar, 0, abort_flag));
+        uint32_t base = 0, i = 0;   // ring index of the item's first load; output rows so far
+        for (int item = blockIdx.x; ok && item < a.items; item += gridDim.x) {
+            const HaloItem it = halo_item(a, item);
+            for (int j = 0; ok && j < it.rows; ++j, ++i) {
+                // output row y0 + j reads loads j, j + 1, j + 2 of the item
+                const uint32_t buf = i % kAcc, use = i / kAcc;
+                if (!__all_sync(0xffffffffu, mbar_wait_or_abort(acc_empty(buf), (use & 1u) ^ 1u, abort_flag))) { ok = false; break; }
+                uint32_t row_addr[3];
+                for (int d = 0; d < 3 && ok; ++d) {
+                    const uint32_t k = base + (uint32_t)(j + d);
+                    ok = __all_sync(0xffffffffu, mbar_wait_or_abort(full(k % kSt), (k / kSt) & 1u, abort_flag));
+                    row_addr[d] = smem_u32(sA + (k % kSt) * a_stride);
+                }
+                if (!ok) break;
+                tc_fence_after();
+                const uint32_t acc = tmem + buf * BN;
+                // a descriptor is affine in its address (the 14-bit field holds address / 16
+                // and no offset here carries out of it): each MMA's operands are the row's or
+                // the weights' base descriptor plus a constant, so the issuing thread spends
+                // a few instructions per MMA instead of forming two descriptors
+                uint64_t db_tap = db0;
+                uint32_t add = 0;
+#pragma unroll
+                for (int t = 0; t < 9; ++t) {
+                    const uint32_t row = row_addr[t / 3];
+                    uint64_t db = db_tap;
+                    each_step(desc_rows(row, a.cb0), desc_rows(row + src1_off, a.cb1), t % 3, [&](uint64_t da) {
+                        tc_mma(acc, da, db, idesc, add);
+                        add = 1u;
+                        db += dq_b;
+                    });
+                    db_tap += dtap_b;
+                }
+                tc_commit(acc_full(buf));
+                // load j (input row y0 + j - 1) has no later reader
+                tc_commit(empty((base + (uint32_t)j) % kSt));
             }
+            if (!ok) break;
+            // the item's last two loads
+            tc_commit(empty((base + (uint32_t)it.rows) % kSt));
+            tc_commit(empty((base + (uint32_t)it.rows + 1) % kSt));
+            base += (uint32_t)it.rows + 2;
+        }
+        if (!ok && lane == 0) {
+            atomicOr(e.err, DEV_GUARD);
+            s_abort = 1;
         }
     } else {
         const int q = warp & 3;
@@ -981,14 +1059,18 @@ __global__ void __launch_bounds__(kConvThreads, kFan ? fan_ctas(BN) : 1) tc_conv
         // quarter-warp's eight 16-byte accesses then fall in eight different bank groups
         // both when lanes write their own pixels and when they read consecutive chunks.
         constexpr int kCh = BN / 8;
-        __shared__ __align__(16) uint4 s_stage[4][32 * kCh];
-        uint4* stage = s_stage[q];
+        uint4* stage = s_stage + (warp - 2) * 32 * kCh;
+        // One set's row takes it 1,300 cycles from the accumulator to the last store, all of it
+        // latency: two sets in turn (16 -> 32 at 2176 x 3840 173 -> 144 us with the second, 32 ->
+        // 32 202 -> 174, 32 -> 64 at 1088 x 1920 111 -> 88).
+        const int set = (warp - 2) >> 2;
         auto slot = [](int p, int c) { return p * kCh + (c ^ ((kCh == 4 ? (p >> 1) : p) & (kCh - 1))); };
         uint32_t i = 0;
         bool ok = true;
         for (int item = blockIdx.x; ok && item < a.items; item += gridDim.x) {
             const HaloItem it = halo_item(a, item);
             for (int j = 0; j < it.rows; ++j, ++i) {
+                if (a.sets == 2 && (int)(i & 1u) != set) continue;
                 const uint32_t buf = i % kAcc, use = i / kAcc;
                 ok = __all_sync(0xffffffffu, mbar_wait_or_abort(acc_full(buf), use & 1u, abort_flag));
                 if (!ok) {
@@ -1001,52 +1083,69 @@ __global__ void __launch_bounds__(kConvThreads, kFan ? fan_ctas(BN) : 1) tc_conv
                 const uint32_t tbase = tmem + acc_col(i) + ((uint32_t)(q * 32) << 16);
                 const int n0 = it.slice * BN;                  // the item's first output channel
                 float hz = e.head_out ? e.head_b[0] : 0.0f;
-                // the row's BN columns in one TMEM load and one wait
-                uint32_t vv[BN];
-                if constexpr (BN == 64) tmem_ld64(tbase, vv);
-                else tmem_ld32(tbase, vv);
-                if (kFan)                                      // the row's next use starts from zero
+                const bool plain = !e.head_out && !e.c32;
+                const __nv_bfloat16* gate = e.gate ? e.gate + pix * e.ldc + n0 : nullptr;
 #pragma unroll
-                    for (int c32 = 0; c32 < BN; c32 += 32) tmem_zero32(tbase + (uint32_t)c32);
+                for (int c32 = 0; c32 < BN; c32 += 32) {
+                    // 32 columns in one TMEM load and one wait
+                    uint32_t vv[32];
+                    tmem_ld32(tbase + (uint32_t)c32, vv);
+                    if (kFan) tmem_zero32(tbase + (uint32_t)c32);      // the row's next use starts from zero
+                    if (plain) {
+                        // two channels an instruction: bias added in FP32, then rounded, then
+                        // ReLU and gate on the rounded pair (the same values: rounding keeps the
+                        // sign, and a gated value is zero either way)
 #pragma unroll
-                for (int c0 = 0; c0 < BN; c0 += 16) {
-                    const uint32_t* v = vv + c0;
-                    float f[16];
+                        for (int c8 = 0; c8 < 32; c8 += 8) {
+                            uint4 out, gv;
+                            uint32_t* ob = reinterpret_cast<uint32_t*>(&out);
+                            if (gate) gv = *reinterpret_cast<const uint4*>(gate + c32 + c8);
 #pragma unroll
-                    for (int jj = 0; jj < 16; ++jj) {
-                        float t = __uint_as_float(v[jj]);
-                        if (e.bias) t += s_bias[n0 + c0 + jj];
-                        if (e.relu) t = fmaxf(t, 0.0f);
-                        f[jj] = t;
-                    }
-                    if (e.head_out)
+                            for (int h = 0; h < 4; ++h) {
+                                float2 t = make_float2(__uint_as_float(vv[c8 + 2 * h]), __uint_as_float(vv[c8 + 2 * h + 1]));
+                                if (e.bias) t = add2(t, *reinterpret_cast<const float2*>(s_bias + n0 + c32 + c8 + 2 * h));
+                                __nv_bfloat162 o2 = __floats2bfloat162_rn(t.x, t.y);
+                                if (e.relu) o2 = __hmax2(o2, __floats2bfloat162_rn(0.0f, 0.0f));
+                                ob[h] = *reinterpret_cast<uint32_t*>(&o2);
+                            }
+                            if (gate) {
+                                const uint32_t* g = reinterpret_cast<const uint32_t*>(&gv);
 #pragma unroll
-                        for (int jj = 0; jj < 16; ++jj)
-                            hz += __bfloat162float(__float2bfloat16_rn(f[jj])) * e.head_w[c0 + jj];
-                    const size_t o = pix * e.ldc + n0 + c0;
-                    if (e.gate) {
-                        const uint4* g4 = reinterpret_cast<const uint4*>(e.gate + o);
-#pragma unroll
-                        for (int h = 0; h < 2; ++h) {
-                            const uint4 gv = g4[h];
-                            const __nv_bfloat16* gb = reinterpret_cast<const __nv_bfloat16*>(&gv);
-#pragma unroll
-                            for (int j = 0; j < 8; ++j)
-                                if (!(__bfloat162float(gb[j]) > 0.0f)) f[h * 8 + j] = 0.0f;
+                                for (int h = 0; h < 4; ++h)
+                                    ob[h] &= __hgt2_mask(*reinterpret_cast<const __nv_bfloat162*>(g + h), __floats2bfloat162_rn(0.0f, 0.0f));
+                            }
+                            stage[slot(lane, (c32 + c8) / 8)] = out;
                         }
+                        continue;
                     }
-                    if (e.c16) {
-                        uint4 out[2];
-                        __nv_bfloat16* ob = reinterpret_cast<__nv_bfloat16*>(out);
 #pragma unroll
-                        for (int jj = 0; jj < 16; ++jj) ob[jj] = __float2bfloat16_rn(f[jj]);
-                        stage[slot(lane, c0 / 8)] = out[0];
-                        stage[slot(lane, c0 / 8 + 1)] = out[1];
-                    }
-                    if (e.c32) {
-                        float4* d4 = reinterpret_cast<float4*>(e.c32 + o);
+                    for (int c0 = c32; c0 < c32 + 32; c0 += 16) {
+                        const uint32_t* v = vv + (c0 - c32);
+                        float f[16];
 #pragma unroll
-                        for (int h = 0; h < 4; ++h) d4[h] = make_float4(f[4 * h], f[4 * h + 1], f[4 * h + 2], f[4 * h + 3]);
+                        for (int jj = 0; jj < 16; ++jj) {
+                            float t = __uint_as_float(v[jj]);
+                            if (e.bias) t += s_bias[n0 + c0 + jj];
+                            if (e.relu) t = fmaxf(t, 0.0f);
+                            f[jj] = t;
+                        }
+                        if (e.head_out)
+#pragma unroll
+                            for (int jj = 0; jj < 16; ++jj)
+                                hz += __bfloat162float(__float2bfloat16_rn(f[jj])) * e.head_w[c0 + jj];
+                        if (e.c16) {
+                            uint4 out[2];
+                            __nv_bfloat16* ob = reinterpret_cast<__nv_bfloat16*>(out);
+#pragma unroll
+                            for (int jj = 0; jj < 16; ++jj) ob[jj] = __float2bfloat16_rn(f[jj]);
+                            stage[slot(lane, c0 / 8)] = out[0];
+                            stage[slot(lane, c0 / 8 + 1)] = out[1];
+                        }
+                        if (e.c32) {
+                            float4* d4 = reinterpret_cast<float4*>(e.c32 + pix * e.ldc + n0 + c0);
+#pragma unroll
+                            for (int h = 0; h < 4; ++h) d4[h] = make_float4(f[4 * h], f[4 * h + 1], f[4 * h + 2], f[4 * h + 3]);
+                        }
                     }
                 }
                 if (e.head_out) e.head_out[pix] = 1.0f / (1.0f + __expf(-hz));
@@ -1058,11 +1157,11 @@ __global__ void __launch_bounds__(kConvThreads, kFan ? fan_ctas(BN) : 1) tc_conv
                 if (lane == 0) mbar_arrive(acc_empty(buf));
                 if (e.c16) {
                     const size_t pix0 = pix - lane;                       // the warp's first pixel
-#pragma unroll 1
-                    for (int k = 0; k < kCh; ++k) {
-                        const int idx = k * 32 + lane, p = idx / kCh, c = idx % kCh;
-                        *reinterpret_cast<uint4*>(e.c16 + (pix0 + p) * e.ldc + n0 + c * 8) = stage[slot(p, c)];
-                    }
+                    __nv_bfloat16* d = e.c16 + (pix0 + lane / kCh) * e.ldc + n0 + lane % kCh * 8;
+                    const size_t dk = (size_t)(32 / kCh) * e.ldc;
+#pragma unroll
+                    for (int k = 0; k < kCh; ++k, d += dk)
+                        *reinterpret_cast<uint4*>(d) = stage[slot(k * (32 / kCh) + lane / kCh, lane % kCh)];
                     if (a.up16) {
                         // rows 2y and 2y + 1 of the 2x copy: 64 pixels, each source pixel twice
                         const size_t up0 = ((size_t)it.b * 2 * a.H + 2 * y) * (2 * a.W) + 2 * (x - lane);
@@ -1146,7 +1245,7 @@ __global__ void __launch_bounds__(kConvThreads, 2) tc_wgrad_kernel(const __grid_
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * (kA + kB) + 1);
     __shared__ int s_abort;
     volatile int* abort_flag = &s_abort;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     auto a_full = [&](int s) { return smem_u32(&bars[s]); };
     auto a_empty = [&](int s) { return smem_u32(&bars[kA + s]); };
     auto b_full = [&](int s) { return smem_u32(&bars[2 * kA + s]); };
@@ -1173,7 +1272,7 @@ __global__ void __launch_bounds__(kConvThreads, 2) tc_wgrad_kernel(const __grid_
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = *tmem_slot;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
 
     if (warp == 0) {
         // every lane waits for the slot; lane 0 arms its barrier before the lanes issue the copies
@@ -1210,31 +1309,29 @@ __global__ void __launch_bounds__(kConvThreads, 2) tc_wgrad_kernel(const __grid_
             for (uint32_t i = ib > (uint32_t)kB ? ib - kB : 0; i < ib; ++i) mbar_wait(b_full((int)(i % kB)), (i / kB) & 1u);
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            constexpr uint32_t idesc = instr_desc(N) | (1u << 15) | (1u << 16);      // A and B MN-major
-            uint32_t ia = 0, ib = 0;
-            bool ok = true;
-            for (int k = k0; ok && k < k1; ++k, ++ib) {
-                const int sb = (int)(ib % kB);
-                ok = mbar_wait_or_abort(b_full(sb), (ib / kB) & 1u, abort_flag);
-                const uint64_t db = desc_mn<CB>(smem_u32(sB + sb * kBBytes));
-                for (int m = 0; ok && m < nm; ++m, ++ia) {
-                    const int sa = (int)(ia % kA);
-                    ok = mbar_wait_or_abort(a_full(sa), (ia / kA) & 1u, abort_flag);
-                    if (!ok) break;
-                    tc_fence_after();
-                    const uint64_t da = desc_mn<CA>(smem_u32(sA + sa * kABytes));
+        constexpr uint32_t idesc = instr_desc(N) | (1u << 15) | (1u << 16);      // A and B MN-major
+        uint32_t ia = 0, ib = 0;
+        bool ok = true;
+        for (int k = k0; ok && k < k1; ++k, ++ib) {
+            const int sb = (int)(ib % kB);
+            ok = __all_sync(0xffffffffu, mbar_wait_or_abort(b_full(sb), (ib / kB) & 1u, abort_flag));
+            const uint64_t db = desc_mn<CB>(smem_u32(sB + sb * kBBytes));
+            for (int m = 0; ok && m < nm; ++m, ++ia) {
+                const int sa = (int)(ia % kA);
+                ok = __all_sync(0xffffffffu, mbar_wait_or_abort(a_full(sa), (ia / kA) & 1u, abort_flag));
+                if (!ok) break;
+                tc_fence_after();
+                const uint64_t da = desc_mn<CA>(smem_u32(sA + sa * kABytes));
 #pragma unroll
-                    for (int q = 0; q < kWgPix / 16; ++q)       // 16 pixels: two 8-row groups further
-                        tc_mma(tmem + (uint32_t)(m * N), da + (uint64_t)(q * ((16 * CA * 2) >> 4)),
-                               db + (uint64_t)(q * ((16 * CB * 2) >> 4)), idesc, (k > k0 || q > 0) ? 1u : 0u);
-                    tc_commit(a_empty(sa));
-                }
-                tc_commit(b_empty(sb));
+                for (int q = 0; q < kWgPix / 16; ++q)       // 16 pixels: two 8-row groups further
+                    tc_mma(tmem + (uint32_t)(m * N), da + (uint64_t)(q * ((16 * CA * 2) >> 4)),
+                           db + (uint64_t)(q * ((16 * CB * 2) >> 4)), idesc, (k > k0 || q > 0) ? 1u : 0u);
+                tc_commit(a_empty(sa));
             }
-            if (!ok) { atomicOr(a.err, DEV_GUARD); s_abort = 1; }
-            tc_commit(done);
+            tc_commit(b_empty(sb));
         }
+        if (!ok && lane == 0) { atomicOr(a.err, DEV_GUARD); s_abort = 1; }
+        tc_commit(done);
     } else {
         const int q = warp & 3, r = q * 32 + lane;
         const bool ok = __all_sync(0xffffffffu, mbar_wait_or_abort(done, 0, abort_flag)) && !*abort_flag;
@@ -1366,7 +1463,7 @@ int launch_conv(const CUtensorMap& m0, const CUtensorMap& m1, const CUtensorMap&
 }
 
 
-// The row box of one source: a 5-D view of the NHWC tensor, (8 channels, W, H, B, C / 8
+// The row box of one source for kTA: a 5-D view of the NHWC tensor, (8 channels, W, H, B, C / 8
 // groups), read in boxes of 8 x 136 x 1 x 1 x C/8 without swizzle (the channel groups
 // outermost in shared memory).
 bool make_map_halo(CUtensorMap* m, const void* base, int B, int H, int W, int C) {
@@ -1408,14 +1505,14 @@ bool make_map_wfan(CUtensorMap* m, const void* base, int N, int ldw, int cin, in
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int BN, bool kTA, bool kFan>
+template <int BN, bool kTA, bool kFan, bool kWide>
 int launch_conv_halo(const CUtensorMap& m0, const CUtensorMap& m1, const CUtensorMap& mw, const HaloArgs& a,
                      const Epilogue& e, size_t smem, cudaStream_t s) {
     static size_t attr = 0;
     if (attr < smem) {
-        if (cudaFuncSetAttribute(tc_conv_halo_kernel<BN, kTA, kFan>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        if (cudaFuncSetAttribute(tc_conv_halo_kernel<BN, kTA, kFan, kWide>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)smem) != cudaSuccess ||
-            cudaFuncSetAttribute(tc_conv_halo_kernel<BN, kTA, kFan>, cudaFuncAttributePreferredSharedMemoryCarveout,
+            cudaFuncSetAttribute(tc_conv_halo_kernel<BN, kTA, kFan, kWide>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                  cudaSharedmemCarveoutMaxShared) != cudaSuccess)
             return RN_ERR_CUDA;
         attr = smem;
@@ -1424,11 +1521,11 @@ int launch_conv_halo(const CUtensorMap& m0, const CUtensorMap& m1, const CUtenso
     cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, ctx().device);
     // co-resident CTAs: shared memory (dynamic, static and 1 KB reserved) and TMEM (512
     // columns an SM) both have to fit
-    const int tmem_cols = kTA ? 256 : kFan ? fan_acc(BN) * BN : 2 * BN;
-    const int per_cta = (int)(smem + halo_static_smem(BN) + 1024);
+    const int tmem_cols = kTA ? 256 : kFan ? fan_cols(kWide) : 2 * BN;
+    const int per_cta = (int)(smem + kHaloStatic + 1024);
     const int per_sm = std::max(1, std::min(std::min(smem_sm / per_cta, 512 / tmem_cols), 3));
     const int ctas = std::min(a.items, per_sm * ctx().sm_count);
-    tc_conv_halo_kernel<BN, kTA, kFan><<<ctas, kConvThreads, smem, s>>>(m0, m1, mw, a, e);
+    tc_conv_halo_kernel<BN, kTA, kFan, kWide><<<ctas, 64 + 128 * a.sets, smem, s>>>(m0, m1, mw, a, e);
     return cudaGetLastError() == cudaSuccess ? RN_OK : RN_ERR_CUDA;
 }
 
@@ -1526,14 +1623,17 @@ int tc_conv3x3(const tc::ConvSrc* src, int nsrc, int B, int H, int W, const __nv
     const bool one_slice = N == 32 || N == 64;
     if ((ctx().tune.conv_halo || !all32) && ring_shape && (one_slice || (fan && N % 32 == 0 && N <= 512))) {
         const uint32_t a_bytes = (uint32_t)cin / 8 * tc::kHaloGroup;
-        const uint32_t a_stride = (a_bytes + 1023) & ~1023u;
+        // a row slot; two swizzled sources each start on 1024 bytes
+        const uint32_t a_stride = tc::halo_slot(src[0].C, nsrc > 1 ? src[1].C : 0, ta);
+        auto chunk = [](int C) { return C % 64 == 0 ? 64 : C % 32 == 0 ? 32 : 16; };
         const size_t bars = (size_t)(2 * 8 + 2 * tc::kFanMaxAcc + 2) * 8 + 16;
         int bn = one_slice && (N == 32 || !fan || ctx().tune.conv_fan_bn == 64) ? N : 32, stages = 0;
         uint32_t b_bytes = 0, b_pad = 0;
+        int sets = 1;
         auto fit = [&](int bnf) {
             b_bytes = (uint32_t)bnf * 9 * cin * 2;
             b_pad = (b_bytes + 1023) & ~1023u;
-            const size_t stat = tc::halo_static_smem(bnf);
+            const size_t stat = tc::kHaloStatic + tc::halo_stage(bnf, 1);
             if (!fan) {
                 // dynamic shared memory: 227 KB a block less the kernel's static arrays (the
                 // bias, the abort flag and the epilogue's BF16 stage of 4 x 32 pixels x N)
@@ -1543,11 +1643,13 @@ int tc_conv3x3(const tc::ConvSrc* src, int nsrc, int B, int H, int W, const __nv
             // fan-out: a slot is busy only until its own MMAs have run: four at most (4, 6 and 8
             // measured alike); two CTAs per SM (228 KB less 1 KB reserved each) where two slots
             // fit, else one CTA with the whole 227 KB of a block
-            const size_t fixed = stat + 1024 + bars + b_pad;
-            for (const size_t cta : {(size_t)228 * 1024 / 2 - 1024, (size_t)227 * 1024}) {
-                const size_t room = cta > fixed ? (cta - fixed) / a_stride : 0;
-                if (room >= 2) return (int)std::min<size_t>(4, room);
-            }
+            for (const size_t cta : {(size_t)228 * 1024 / 2 - 1024, (size_t)227 * 1024})
+                for (sets = 2; sets >= 1; --sets) {
+                    const size_t fixed = tc::kHaloStatic + tc::halo_stage(bnf, sets) + 1024 + bars + b_pad;
+                    const size_t room = cta > fixed ? (cta - fixed) / a_stride : 0;
+                    if (room >= 2) return (int)std::min<size_t>(4, room);
+                }
+            sets = 1;
             return 0;
         };
         stages = fit(bn);
@@ -1557,12 +1659,15 @@ int tc_conv3x3(const tc::ConvSrc* src, int nsrc, int B, int H, int W, const __nv
         }
         CUtensorMap hm[2], hw;
         bool maps = stages >= (fan ? 2 : 4) && (fan || one_slice);
-        for (int i = 0; maps && i < nsrc; ++i) maps = tc::make_map_halo(&hm[i], src[i].ptr, B, H, W, src[i].C);
+        for (int i = 0; maps && i < nsrc; ++i)
+            maps = ta ? tc::make_map_halo(&hm[i], src[i].ptr, B, H, W, src[i].C)
+                      : tc::make_map_nhwc(&hm[i], src[i].ptr, B, H, W, src[i].C, tc::kHaloW, 1, chunk(src[i].C));
         if (maps && nsrc == 1) hm[1] = hm[0];
         maps = maps && (fan ? tc::make_map_wfan(&hw, w, N, ldw, cin, bn) : tc::make_map_wgroups(&hw, w, N, ldw, 9 * cin / 8));
         if (maps) {
             tc::HaloArgs h{};
             h.nsrc = nsrc; h.C0 = src[0].C; h.C1 = nsrc > 1 ? src[1].C : 0; h.cin = cin;
+            h.cb0 = chunk(src[0].C); h.cb1 = nsrc > 1 ? chunk(src[1].C) : 16;
             h.B = B; h.H = H; h.W = W;
             // chunks of 16 output rows (2 halo rows re-read per chunk), fewer where that leaves
             // less than two items per SM
@@ -1573,14 +1678,18 @@ int tc_conv3x3(const tc::ConvSrc* src, int nsrc, int B, int H, int W, const __nv
             h.slice_items = (W / 128) * h.chunks_y * B;
             h.items = h.n_slices * h.slice_items;
             h.stages = stages;
+            h.sets = sets;
             h.a_bytes = a_bytes; h.b_bytes = b_bytes;
             h.up16 = up16;
-            const size_t smem = 1024 + b_pad + (size_t)stages * a_stride + bars;
-            const int rc = ta    ? tc::launch_conv_halo<32, true, false>(hm[0], hm[1], hw, h, epi, smem, s)
-                         : fan   ? (bn == 32 ? tc::launch_conv_halo<32, false, true>(hm[0], hm[1], hw, h, epi, smem, s)
-                                             : tc::launch_conv_halo<64, false, true>(hm[0], hm[1], hw, h, epi, smem, s))
-                         : N == 32 ? tc::launch_conv_halo<32, false, false>(hm[0], hm[1], hw, h, epi, smem, s)
-                                   : tc::launch_conv_halo<64, false, false>(hm[0], hm[1], hw, h, epi, smem, s);
+            const size_t smem = 1024 + b_pad + (size_t)stages * a_stride + tc::halo_stage(bn, sets) + bars;
+            const bool wide = smem + tc::kHaloStatic + 1024 > (size_t)228 * 1024 / 2;      // one CTA per SM
+            const int rc = ta    ? tc::launch_conv_halo<32, true, false, false>(hm[0], hm[1], hw, h, epi, smem, s)
+                         : fan && wide ? (bn == 32 ? tc::launch_conv_halo<32, false, true, true>(hm[0], hm[1], hw, h, epi, smem, s)
+                                                   : tc::launch_conv_halo<64, false, true, true>(hm[0], hm[1], hw, h, epi, smem, s))
+                         : fan   ? (bn == 32 ? tc::launch_conv_halo<32, false, true, false>(hm[0], hm[1], hw, h, epi, smem, s)
+                                             : tc::launch_conv_halo<64, false, true, false>(hm[0], hm[1], hw, h, epi, smem, s))
+                         : N == 32 ? tc::launch_conv_halo<32, false, false, false>(hm[0], hm[1], hw, h, epi, smem, s)
+                                   : tc::launch_conv_halo<64, false, false, false>(hm[0], hm[1], hw, h, epi, smem, s);
             if (rc != RN_OK) return cuda_fail(st, cudaGetLastError(), "tc_conv_halo_kernel");
             return RN_OK;
         }

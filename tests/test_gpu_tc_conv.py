@@ -186,3 +186,37 @@ def test_conv_fan_slices_of_32_match(rn, B, H, W, c0, c1, N):
     finally:
         rn.tune_set("conv_fan", saved[0])
         rn.tune_set("conv_fan_bn", saved[1])
+
+
+@pytest.mark.parametrize("B,H,W,c0,c1,N", [(1, 5, 128, 48, 0, 32), (1, 9, 256, 16, 64, 64), (1, 17, 128, 112, 0, 32),
+                                            (2, 7, 128, 64, 128, 64), (1, 18, 384, 96, 32, 32), (1, 3, 128, 128, 0, 128),
+                                            (1, 20, 256, 32, 64, 32), (1, 33, 128, 64, 0, 64), (2, 2, 128, 16, 0, 32)])
+def test_conv_row_tiles_over_channel_chunks(rn, B, H, W, c0, c1, N):
+    """A row slot holds each source as chunks of 64, 32 or 16 channels, each with the swizzle of
+    its width, and a tap's shift moves an operand's start by a pixel row: one chunk and several,
+    sources of different widths, the channel counts with their own straight-line steps and
+    others, one and two CTAs per SM, against the FP32 convolution of the same BF16 values (FP32
+    accumulation of at most 9 x 192 products: 1e-3 of the largest output) and bit for bit
+    against the row-by-row form (or, where that does not fit, the per-tap kernel)."""
+    import torch
+    saved = rn.tune_get("conv_fan")
+    try:
+        g = torch.Generator(device="cuda").manual_seed(B + H + W + 3 * c0 + c1 + N)
+        x0 = torch.randn(B, H, W, c0, device="cuda", generator=g).to(torch.bfloat16)
+        x1 = torch.randn(B, H, W, c1, device="cuda", generator=g).to(torch.bfloat16) if c1 else None
+        cin = c0 + c1
+        w = (torch.randn(N, 9 * cin, device="cuda", generator=g) / (9 * cin) ** 0.5).to(torch.bfloat16)
+        bias = torch.randn(N, device="cuda", generator=g)
+        outs = []
+        for fan in (0, 1):
+            rn.tune_set("conv_fan", fan)
+            f = rn.tc_conv3x3(x0, w, x1, bias=bias, relu=False)
+            o = rn.tc_conv3x3(x0, w, x1, bias=bias, relu=True, out_dtype=torch.bfloat16)
+            torch.cuda.synchronize()
+            outs.append((f.clone(), o.clone()))
+        ref = _ref(x0, x1, w, bias, False)
+        assert (outs[1][0] - ref).abs().max().item() <= 1e-3 * ref.abs().max().item()
+        for a, b in zip(*outs):
+            assert torch.equal(a, b)
+    finally:
+        rn.tune_set("conv_fan", saved)
