@@ -231,7 +231,6 @@ int rn_batch_run(rn_batch* b, rn_reconcile_result* results, rn_status* st) {
     Context& c = ctx();
     if (b->device != c.device) return fail(st, RN_ERR_STATE, "batch belongs to device %d", b->device);
     RN_CUDA(cudaGraphLaunch(b->exec, c.stream), st);
-    RN_CUDA(cudaStreamSynchronize(c.stream), st);
     RN_TRY(check_device_error(st, "rn_batch_run"));
     if (results)
         for (int v = 0; v < b->nviews; ++v) {

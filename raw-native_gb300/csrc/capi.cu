@@ -244,6 +244,8 @@ int ensure_ctx(rn_status* st) {
     c.stream = c.own_stream;
     RN_CUDA(cudaMalloc((void**)&c.dev_error, 64), st);
     RN_CUDA(cudaMemsetAsync(c.dev_error, 0, 64, c.stream), st);
+    RN_CUDA(cudaHostAlloc((void**)&c.back, sizeof(Readback), cudaHostAllocMapped | cudaHostAllocPortable), st);
+    *c.back = Readback{};
     // the library's own pool for accelerators (rebuilt per scene, often per frame): a freed
     // accelerator's memory stays mapped for the next build instead of going back to the driver
     cudaMemPoolProps pp = {};
@@ -278,11 +280,21 @@ int ws_get(Slot s, size_t bytes, void** out, rn_status* st) {
     return RN_OK;
 }
 
-int check_device_error(rn_status* st, const char* where) {
+int queue_device_error(rn_status* st) {
     Context& c = ctx();
-    uint32_t word = 0;
-    RN_CUDA(cudaMemcpyAsync(&word, c.dev_error, 4, cudaMemcpyDeviceToHost, c.stream), st);
-    RN_CUDA(cudaStreamSynchronize(c.stream), st);
+    RN_CUDA(cudaMemcpyAsync(&c.back->dev_error, c.dev_error, 4, cudaMemcpyDeviceToHost, c.stream), st);
+    return RN_OK;
+}
+
+int check_device_error(rn_status* st, const char* where) {
+    RN_TRY(queue_device_error(st));
+    RN_CUDA(cudaStreamSynchronize(ctx().stream), st);
+    return judge_device_error(st, where);
+}
+
+int judge_device_error(rn_status* st, const char* where) {
+    Context& c = ctx();
+    const uint32_t word = c.back->dev_error;
     if (word) {
         RN_CUDA(cudaMemsetAsync(c.dev_error, 0, 4, c.stream), st);
         const int code = (word & (DEV_STACK_OVERFLOW | DEV_QUEUE_OVERFLOW)) ? RN_ERR_OVERFLOW : RN_ERR_BUDGET;
@@ -383,6 +395,25 @@ int do_visibility(const StagedGbuf& g, int w, int h, const rn_accel* accel, int 
 
 void fill_result(const RecOut& r, float tolerance, rn_reconcile_result* out);
 
+// An accelerator over device triangles in two steps: the build queued (a small scene's whole
+// build without a host read; a larger one is done when this returns), and, once the stream has
+// been synchronised, its outcome.
+int start_accel(const float* d_tris, uint32_t ntri, rn_accel** out, PlocTree* tree, rn_status* st) {
+    Context& c = ctx();
+    rn_accel* acc = *out = new rn_accel();
+    acc->device = c.device;
+    // the tree only prunes (every hit is the triangle test's): its shape is a tuning choice
+    RN_TRY(ploc_build(d_tris, ntri, c.tune.accel_radius, tree, c.stream, st, true));
+    return collapse_bvh4(*tree, d_tris, acc, ntri < kSmallScene ? c.tune.accel_leaf_small : c.tune.accel_leaf, c.stream, st);
+}
+int finish_accel(rn_accel* acc, PlocTree* tree, rn_status* st) {
+    RN_TRY(collapse_finish(*tree, acc, st));
+    ploc_free(tree);
+    if (acc->depth * 3 + 2 > 96)
+        return fail(st, RN_ERR_OVERFLOW, "BVH depth %u needs more than the traversal's 96-entry stack", acc->depth);
+    return RN_OK;
+}
+
 // The device address of a pinned, mapped host buffer (nullptr for any other kind).
 void* mapped(const void* p) {
     cudaPointerAttributes a;
@@ -422,12 +453,10 @@ int direct_frame(const rn_gbuf* g, const rn_accel* accel, int spp, float radius,
     const uint8_t* corr = (flags & RN_DEVICE_TRIG) ? nullptr : c.trig_corr;
     if (launch_ssao(w, h, mirror_pos(m, np), mirror_nrm(m, np), mirror_mask(m, np), ss_samples, radius, corr,
                     (float*)mapped(h_ss), mirror_ao(m, np), h_err ? (float*)mapped(h_err) : nullptr,
-                    (RecPartial*)parts, (RecOut*)ro, c.stream) != RN_OK)
+                    (RecPartial*)parts, (RecOut*)ro, c.stream, &c.back->rec) != RN_OK)
         return cuda_fail(st, cudaGetLastError(), "ssao_kernel (fused reconcile)");
-    RecOut r;
-    RN_CUDA(cudaMemcpyAsync(&r, ro, sizeof r, cudaMemcpyDeviceToHost, c.stream), st);
     RN_TRY(check_device_error(st, "rn_ao_frame"));
-    fill_result(r, tolerance, out);
+    fill_result(c.back->rec, tolerance, out);
     return ok(st);
 }
 
@@ -602,21 +631,14 @@ int rn_accel_build(const float* tris, uint32_t ntri, int flags, rn_accel** out, 
     const bool dev = (flags & RN_DEVICE_PTRS) != 0;
     const float* d_tris = nullptr;
     RN_TRY(stage_in(tris, (size_t)ntri * 9, dev, WS_TRIS_IN, &d_tris, st));
-    rn_accel* acc = new rn_accel();
-    acc->device = c.device;
+    rn_accel* acc = nullptr;
     PlocTree tree;
-    // the tree only prunes (every hit is the triangle test's): its shape is a tuning choice
-    int rc = ploc_build(d_tris, ntri, c.tune.accel_radius, &tree, c.stream, st);
-    if (rc == RN_OK)
-        rc = collapse_bvh4(tree, d_tris, acc, ntri < kSmallScene ? c.tune.accel_leaf_small : c.tune.accel_leaf,
-                           c.stream, st);
+    int rc = start_accel(d_tris, ntri, &acc, &tree, st);
     if (rc == RN_OK) {
         cudaError_t e = cudaStreamSynchronize(c.stream);
         if (e != cudaSuccess) rc = cuda_fail(st, e, "rn_accel_build");
     }
-    ploc_free(&tree);
-    if (rc == RN_OK && acc->depth * 3 + 2 > 96)
-        rc = fail(st, RN_ERR_OVERFLOW, "BVH depth %u needs more than the traversal's 96-entry stack", acc->depth);
+    if (rc == RN_OK) rc = finish_accel(acc, &tree, st);
     if (rc != RN_OK) { rn_accel_free(acc); return rc; }
     *out = acc;
     return ok(st);
@@ -739,13 +761,11 @@ int rn_reconcile(const float* approx, const float* truth, const uint8_t* mask, i
     void *parts = nullptr, *ro = nullptr;
     RN_TRY(ws_get(WS_PARTIALS, (size_t)nb * sizeof(RecPartial), &parts, st));
     RN_TRY(ws_get(WS_COUNTERS, sizeof(RecOut), &ro, st));
-    const cudaError_t le = launch_reconcile(d_a, d_t, d_m, np, d_e, (RecPartial*)parts, nb, (RecOut*)ro, c.stream);
+    const cudaError_t le = launch_reconcile(d_a, d_t, d_m, np, d_e, (RecPartial*)parts, nb, (RecOut*)ro, c.stream, &c.back->rec);
     if (le != cudaSuccess) return cuda_fail(st, le, "reconcile_kernel");
-    RecOut r;
-    RN_CUDA(cudaMemcpyAsync(&r, ro, sizeof r, cudaMemcpyDeviceToHost, c.stream), st);
     if (!dev) RN_TRY(copy_back(err, d_e, np, st));
     RN_CUDA(cudaStreamSynchronize(c.stream), st);
-    fill_result(r, tolerance, out);
+    fill_result(c.back->rec, tolerance, out);
     return ok(st);
 }
 
@@ -783,10 +803,8 @@ int rn_ao_frame(const rn_gbuf* g, const rn_accel* accel, int spp, float radius, 
     RN_TRY(ws_get(WS_COUNTERS, sizeof(RecOut), &ro, st));
     const uint8_t* corr = (flags & RN_DEVICE_TRIG) ? nullptr : c.trig_corr;
     if (launch_ssao(g->w, g->h, sg.pos, sg.nrm, sg.mask, ss_samples, radius, corr, d_ss, d_ao, d_err,
-                    (RecPartial*)parts, (RecOut*)ro, c.stream) != RN_OK)
+                    (RecPartial*)parts, (RecOut*)ro, c.stream, &c.back->rec) != RN_OK)
         return cuda_fail(st, cudaGetLastError(), "ssao_kernel (fused reconcile)");
-    RecOut r;
-    RN_CUDA(cudaMemcpyAsync(&r, ro, sizeof r, cudaMemcpyDeviceToHost, c.stream), st);
     if (!dev) {
         RN_TRY(copy_back(ao, d_ao, np, st));
         if (flags & RN_SKY) { RN_TRY(copy_back(sky, d_sky, np, st)); RN_TRY(copy_back(sun, d_sun, np, st)); }
@@ -794,7 +812,7 @@ int rn_ao_frame(const rn_gbuf* g, const rn_accel* accel, int spp, float radius, 
         if (err) RN_TRY(copy_back(err, d_err, np, st));
     }
     RN_TRY(check_device_error(st, "rn_ao_frame"));
-    fill_result(r, tolerance, out);
+    fill_result(c.back->rec, tolerance, out);
     return ok(st);
 }
 
@@ -850,6 +868,20 @@ int rn_render_frame(const rn_frame_scene* sc, const float* camera, const float* 
     unsigned* d_valid = (unsigned*)((char*)small + 128);
     RN_CUDA(cudaMemcpyAsync(d_vp, vp.m, 64, cudaMemcpyHostToDevice, c.stream), st);
     RN_CUDA(cudaMemsetAsync(d_valid, 0, 8, c.stream), st);
+    // The accelerator is built per frame from the scene's triangles, as the rtao pass does. Its
+    // build is queued before the rasterizer, whose bin count the host waits for: one stop serves
+    // both. Only this stream reads it: at the end its block goes back behind the frame's work.
+    struct Build {
+        rn_accel* acc = nullptr;
+        PlocTree tree;
+        cudaStream_t s;
+        ~Build() {
+            if (acc && acc->d_nodes) cudaFreeAsync(acc->d_nodes, s);
+            delete acc;
+        }
+    } build;
+    build.s = c.stream;
+    if (o.rtao) RN_TRY(start_accel(d_tris, sc->ntri, &build.acc, &build.tree, st));
     size_t pairs = (size_t)8 * sc->ntri + 1024;
     for (int attempt = 0; attempt < 2; ++attempt) {
         const size_t bytes = raster_scratch_bytes(sc->ntri, np, pairs);
@@ -867,25 +899,21 @@ int rn_render_frame(const rn_frame_scene* sc, const float* camera, const float* 
                            sc->has_light ? sc->light_dir[2] : 0.0f};
     const float li = sc->has_light ? sc->light_intensity : 1.0f;
     StagedGbuf sg{d_pos, d_nrm, d_mask};
-    rn_accel* acc = nullptr;
-    RecOut r{};
     if (o.rtao) {
-        // the accelerator is built per frame from the scene's triangles, as the rtao pass does
-        RN_TRY(rn_accel_build(d_tris, sc->ntri, RN_DEVICE_PTRS, &acc, st));
+        // a build still queued has at least two triangles, and the rasterizer has synchronised since
+        RN_TRY(finish_accel(build.acc, &build.tree, st));
         const float tl[3] = {-ldir[0], -ldir[1], -ldir[2]};
-        int rc = do_visibility(sg, w, h, acc, o.spp, o.radius, tl, model == 2 ? RN_SKY : 0, d_ao, d_sky, d_sun, st);
+        int rc = do_visibility(sg, w, h, build.acc, o.spp, o.radius, tl, model == 2 ? RN_SKY : 0, d_ao, d_sky, d_sun, st);
         if (rc == RN_OK) {
             const int nb = ssao_blocks(w, h);
             void *parts = nullptr, *ro = nullptr;
             rc = ws_get(WS_PARTIALS, (size_t)nb * sizeof(RecPartial), &parts, st);
             if (rc == RN_OK) rc = ws_get(WS_COUNTERS, sizeof(RecOut), &ro, st);
             if (rc == RN_OK && launch_ssao(w, h, d_pos, d_nrm, d_mask, o.ss_samples, o.radius, c.trig_corr, d_ss, d_ao,
-                                           d_err, (RecPartial*)parts, (RecOut*)ro, c.stream) != RN_OK)
+                                           d_err, (RecPartial*)parts, (RecOut*)ro, c.stream, &c.back->rec) != RN_OK)
                 rc = cuda_fail(st, cudaGetLastError(), "ssao_kernel (fused reconcile)");
-            if (rc == RN_OK && cudaMemcpyAsync(&r, ro, sizeof r, cudaMemcpyDeviceToHost, c.stream) != cudaSuccess)
-                rc = cuda_fail(st, cudaGetLastError(), "reconcile read-back");
         }
-        if (rc != RN_OK) { cudaStreamSynchronize(c.stream); rn_accel_free(acc); return rc; }
+        if (rc != RN_OK) { cudaStreamSynchronize(c.stream); return rc; }
     } else {
         if (launch_ssao(w, h, d_pos, d_nrm, d_mask, o.ss_samples, o.radius, c.trig_corr, d_ss, nullptr, nullptr,
                         nullptr, nullptr, c.stream) != RN_OK)
@@ -896,7 +924,7 @@ int rn_render_frame(const rn_frame_scene* sc, const float* camera, const float* 
     int rc = launch_shade(w, h, d_nrm, d_alb, d_mask, model, light_ao, d_sun, ldir, li, d_frame, d_hdr, c.stream);
     if (rc == RN_OK)
         rc = launch_motion(w, h, d_pos, d_mask, vp.m, prev_view_proj ? prev_view_proj : vp.m, d_mot, d_valid, c.stream);
-    unsigned counts[2] = {0, 0};
+    uint32_t* counts = c.back->counts;
     if (rc == RN_OK && cudaMemcpyAsync(counts, d_valid, 8, cudaMemcpyDeviceToHost, c.stream) != cudaSuccess)
         rc = cuda_fail(st, cudaGetLastError(), "motion counts");
     if (rc == RN_OK && !dev) {
@@ -911,12 +939,12 @@ int rn_render_frame(const rn_frame_scene* sc, const float* camera, const float* 
             if (rc == RN_OK && x.h && x.d && cudaMemcpyAsync(x.h, x.d, x.bytes, cudaMemcpyDeviceToHost, c.stream) != cudaSuccess)
                 rc = cuda_fail(st, cudaGetLastError(), "frame read-back");
     }
+    if (rc == RN_OK) rc = queue_device_error(st);
     const cudaError_t e = cudaStreamSynchronize(c.stream);
-    if (acc) rn_accel_free(acc);
     if (rc != RN_OK) return rc;
     if (e != cudaSuccess) return cuda_fail(st, e, "rn_render_frame");
-    RN_TRY(check_device_error(st, "rn_render_frame"));
-    if (o.rtao) fill_result(r, o.tolerance, &out->rec);
+    RN_TRY(judge_device_error(st, "rn_render_frame"));
+    if (o.rtao) fill_result(c.back->rec, o.tolerance, &out->rec);
     else out->rec = rn_reconcile_result{0.0f, 0.0f, 0, 0, 0.0};
     out->motion_valid = (int)counts[0];
     out->motion_total = (int)counts[1];

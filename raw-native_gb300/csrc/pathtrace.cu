@@ -1412,8 +1412,9 @@ int rn_pathtrace(const rn_ptscene* s, const rn_pt_desc* d, int flags, rn_pt_out*
                 }
                 if ((pass & 7) == 7) {
                     uint32_t live = 0;
-                    RN_CUDA(cudaMemcpyAsync(&live, W.ctr + 1, 4, cudaMemcpyDeviceToHost, c.stream), st);
+                    RN_CUDA(cudaMemcpyAsync(&c.back->word, W.ctr + 1, 4, cudaMemcpyDeviceToHost, c.stream), st);
                     RN_CUDA(cudaStreamSynchronize(c.stream), st);
+                    live = c.back->word;
                     done = live == 0;
                 }
                 if (!done) {

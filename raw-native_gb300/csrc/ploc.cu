@@ -1255,8 +1255,21 @@ __global__ void __launch_bounds__(kCollapseThreads) collapse_block(Task* q0, Tas
                                                                    const uint32_t* __restrict__ count,
                                                                    const float* __restrict__ tris,
                                                                    Node4* __restrict__ nodes, LeafTri* __restrict__ leaf,
-                                                                   uint32_t leaf_max, uint32_t max_levels) {
+                                                                   uint32_t leaf_max, uint32_t max_levels,
+                                                                   const RoundState* __restrict__ tree) {
     volatile CollapseCtr* vctr = ctr;
+    if (tree) {             // queued behind its build: the root is on the device, if the build ended well
+        if (threadIdx.x == 0) {
+            CollapseCtr c{};
+            c.tasks = tree->error == 0 && tree->m == 1 && tree->root >= 0 ? 1u : 0u;
+            c.base = 1;
+            c.made = 1;
+            *ctr = c;
+            q0[0] = Task{tree->root, 0};
+            __threadfence();
+        }
+        __syncthreads();
+    }
     for (uint32_t lv = 0; lv < max_levels; ++lv) {
         const uint32_t m = vctr->tasks, base = vctr->base;
         if (m == 0) break;                       // every thread read the same count after the barrier
@@ -1290,7 +1303,23 @@ int scan_exclusive_u32(const uint32_t* in, uint32_t* out, uint32_t n, uint32_t* 
 }
 
 // ------------------------------------------------------------------ host drivers
-int ploc_build(const float* d_tris, uint32_t n, int radius, PlocTree* out, cudaStream_t s, rn_status* st) {
+// The tail kernel alone builds the tree and collapse_block collapses it.
+bool ploc_one_batch(uint32_t n) {
+    const Tune& t = ctx().tune;
+    return n > 1 && t.ploc_tail > 1 && n <= (uint32_t)t.ploc_tail && t.ploc_tail_ctas == 1 && n <= (uint32_t)t.collapse_block;
+}
+
+static int judge_rounds(const RoundState& hs, uint32_t n, rn_status* st) {
+    if (hs.error & DEV_PLOC_NO_MERGE)
+        return fail(st, RN_ERR_STATE, "PLOC round %u made no merge (%u clusters)", hs.rounds, hs.m);
+    if ((hs.error & DEV_GUARD) || hs.m != 1) return fail(st, RN_ERR_BUDGET, "PLOC: rounds left %u clusters", hs.m);
+    if (hs.next != 2 * n - 1)
+        return fail(st, RN_ERR_STATE, "PLOC made %u nodes, expected %u", hs.next, 2 * n - 1);
+    return RN_OK;
+}
+
+int ploc_build(const float* d_tris, uint32_t n, int radius, PlocTree* out, cudaStream_t s, rn_status* st, bool deferred) {
+    deferred = deferred && ploc_one_batch(n);
     *out = PlocTree{};
     out->n = n;
     if (n == 0) return ok(st);
@@ -1424,8 +1453,14 @@ int ploc_build(const float* d_tris, uint32_t n, int radius, PlocTree* out, cudaS
             RN_CUDA(le, st);
         }
         RN_CUDA(cudaGetLastError(), st);
-        RN_CUDA(cudaMemcpyAsync(&hs, state, sizeof hs, cudaMemcpyDeviceToHost, s), st);
+        static_assert(sizeof(RoundState) <= sizeof(Readback::ploc), "the read-back area holds the state");
+        RN_CUDA(cudaMemcpyAsync(ctx().back->ploc, state, sizeof hs, cudaMemcpyDeviceToHost, s), st);
+        if (deferred) {
+            out->state = state;
+            return ok(st);
+        }
         RN_CUDA(cudaStreamSynchronize(s), st);
+        memcpy(&hs, ctx().back->ploc, sizeof hs);
         if (hs.error & DEV_PLOC_NO_MERGE)
             return fail(st, RN_ERR_STATE, "PLOC round %u made no merge (%u clusters)", hs.rounds, hs.m);
         if (hs.error & DEV_GUARD) return fail(st, RN_ERR_BUDGET, "PLOC: rounds left %u clusters", hs.m);
@@ -1436,8 +1471,9 @@ int ploc_build(const float* d_tris, uint32_t n, int radius, PlocTree* out, cudaS
         return fail(st, RN_ERR_STATE, "PLOC made %u nodes, expected %u", hs.next, 2 * n - 1);
     int32_t root = tail_root;                // the tail kernels leave the root in the state
     if (root < 0 || n == 1) {
-        RN_CUDA(cudaMemcpyAsync(&root, hs.parity ? cl1 : cl0, 4, cudaMemcpyDeviceToHost, s), st);
+        RN_CUDA(cudaMemcpyAsync(&ctx().back->word, hs.parity ? cl1 : cl0, 4, cudaMemcpyDeviceToHost, s), st);
         RN_CUDA(cudaStreamSynchronize(s), st);
+        root = (int32_t)ctx().back->word;
     }
     out->root = root;
     out->rounds = hs.rounds;
@@ -1451,6 +1487,15 @@ int ploc_export(const PlocTree& t, int32_t* d_nodes9, cudaStream_t s, rn_status*
     const uint32_t N = 2 * t.n - 1;
     export_nodes9<<<cdiv(N, 256), 256, 0, s>>>(N, t.box, t.left, t.right, t.tri, d_nodes9);
     RN_CUDA(cudaGetLastError(), st);
+    return ok(st);
+}
+
+static int judge_collapse(const CollapseCtr& hc, rn_accel* acc, rn_status* st) {
+    const uint32_t placed = (uint32_t)(hc.made >> 32);
+    if (hc.err) return fail(st, RN_ERR_OVERFLOW, "BVH collapse error word 0x%x", hc.err);
+    if (placed != acc->ntri) return fail(st, RN_ERR_STATE, "collapse placed %u of %u triangles", placed, acc->ntri);
+    acc->nodes = (uint32_t)hc.made;
+    acc->depth = hc.depth;
     return ok(st);
 }
 
@@ -1484,8 +1529,24 @@ int collapse_bvh4(const PlocTree& t, const float* d_tris, rn_accel* acc, int lea
     hc.tasks = 1;
     hc.base = 1;
     hc.made = 1;
+    if (t.state) {
+        // the build is still queued: so is the collapse, with its counters behind it
+        collapse_block<<<1, kCollapseThreads, 0, s>>>(q0, q1, ctr, n, node_cap, t.box, t.left, t.right, t.tri, count, d_tris,
+                                                      acc->d_nodes, acc->d_tris, (uint32_t)leaf_max, 4097u,
+                                                      (const RoundState*)t.state);
+        RN_CUDA(cudaGetLastError(), st);
+        RN_CUDA(cudaMemcpyAsync(ctx().back->collapse, ctr, sizeof hc, cudaMemcpyDeviceToHost, s), st);
+        return ok(st);
+    }
     RN_CUDA(cudaMemcpyAsync(q0, &root, sizeof root, cudaMemcpyHostToDevice, s), st);
     RN_CUDA(cudaMemcpyAsync(ctr, &hc, sizeof hc, cudaMemcpyHostToDevice, s), st);
+    static_assert(sizeof hc <= sizeof(Readback::collapse), "the read-back area holds the counters");
+    auto read = [&]() -> int {
+        RN_CUDA(cudaMemcpyAsync(ctx().back->collapse, ctr, sizeof hc, cudaMemcpyDeviceToHost, s), st);
+        RN_CUDA(cudaStreamSynchronize(s), st);
+        memcpy(&hc, ctx().back->collapse, sizeof hc);
+        return RN_OK;
+    };
     // levels in batches of kLevels per host read; a level after the last one finds no task.
     // Small trees run every level in one block and are read once.
     constexpr int kLevels = 8;
@@ -1493,10 +1554,10 @@ int collapse_bvh4(const PlocTree& t, const float* d_tris, rn_accel* acc, int lea
     uint32_t level_tasks = 1, depth = 0;
     if (n <= (uint32_t)ctx().tune.collapse_block) {
         collapse_block<<<1, kCollapseThreads, 0, s>>>(q0, q1, ctr, n, node_cap, t.box, t.left, t.right, t.tri, count,
-                                                      d_tris, acc->d_nodes, acc->d_tris, (uint32_t)leaf_max, 4097u);
+                                                      d_tris, acc->d_nodes, acc->d_tris, (uint32_t)leaf_max, 4097u,
+                                                      nullptr);
         RN_CUDA(cudaGetLastError(), st);
-        RN_CUDA(cudaMemcpyAsync(&hc, ctr, sizeof hc, cudaMemcpyDeviceToHost, s), st);
-        RN_CUDA(cudaStreamSynchronize(s), st);
+        RN_TRY(read());
         level_tasks = hc.tasks;
         depth = hc.depth;
         if (level_tasks > 0) return fail(st, RN_ERR_BUDGET, "collapse: more than 4096 levels");
@@ -1509,18 +1570,24 @@ int collapse_bvh4(const PlocTree& t, const float* d_tris, rn_accel* acc, int lea
             std::swap(q0, q1);
         }
         RN_CUDA(cudaGetLastError(), st);
-        RN_CUDA(cudaMemcpyAsync(&hc, ctr, sizeof hc, cudaMemcpyDeviceToHost, s), st);
-        RN_CUDA(cudaStreamSynchronize(s), st);
+        RN_TRY(read());
         level_tasks = hc.tasks;
         depth = hc.depth;
     }
     RN_CUDA(cudaGetLastError(), st);
-    const uint32_t placed = (uint32_t)(hc.made >> 32);
-    if (hc.err) return fail(st, RN_ERR_OVERFLOW, "BVH collapse error word 0x%x", hc.err);
-    if (placed != n) return fail(st, RN_ERR_STATE, "collapse placed %u of %u triangles", placed, n);
-    acc->nodes = (uint32_t)hc.made;
-    acc->depth = depth;
-    return ok(st);
+    return judge_collapse(hc, acc, st);
+}
+
+int collapse_finish(const PlocTree& t, rn_accel* acc, rn_status* st) {
+    if (!t.state) return ok(st);
+    RoundState hs;
+    CollapseCtr hc;
+    memcpy(&hs, ctx().back->ploc, sizeof hs);
+    memcpy(&hc, ctx().back->collapse, sizeof hc);
+    RN_TRY(judge_rounds(hs, t.n, st));
+    acc->rounds = hs.rounds;
+    if (hc.tasks > 0) return fail(st, RN_ERR_BUDGET, "collapse: more than 4096 levels");
+    return judge_collapse(hc, acc, st);
 }
 
 }  // namespace rn

@@ -256,9 +256,10 @@ int launch_raster(const float* tris, const float* nrm, uint32_t ntri, const floa
         raster_setup<<<(ntri + 127) / 128, 128, 0, s>>>(tris, nrm, ntri, d_vp, nearZ, w, h, recs);
         count_tiles<<<(nrec + 255) / 256, 256, 0, s>>>(recs, nrec, cnt);
         scan_exclusive_u32(cnt, ofs, nrec, bsum, total, s);
-        if (cudaMemcpyAsync(&npairs, total, 4, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+        if (cudaMemcpyAsync(&ctx().back->word, total, 4, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
             cudaStreamSynchronize(s) != cudaSuccess)
             return RN_ERR_CUDA;
+        npairs = ctx().back->word;
         if (npairs > cap) { *pairs_needed = npairs; return RN_ERR_NO_MEMORY; }
         // records of 8 bins and more on average: a thread a pair (the built-in scene's 28 records
         // over a 512 x 512 frame took 45 us with a thread a record); else a thread a record

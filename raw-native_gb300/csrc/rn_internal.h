@@ -83,6 +83,12 @@ struct Tune {
 };
 constexpr uint32_t kSmallScene = 1u << 16;
 
+// What calls read back from the device, in pinned host memory that kernels write and copies
+// land in without a stop (a copy to pageable memory returns only when it is done, and the
+// stream idles until the next launch). One host thread calls at a time, and every call reads
+// its own fields after its own synchronisation.
+struct Readback;
+
 struct Context {
     bool ready = false;
     Tune tune;
@@ -92,6 +98,7 @@ struct Context {
     cudaStream_t own_stream = nullptr;  // the library's own stream
     uint8_t* trig_corr = nullptr;       // 2^24 bytes: host-libm correction per sample angle
     uint32_t* dev_error = nullptr;      // one DeviceError word
+    Readback* back = nullptr;           // pinned and mapped
     cudaMemPool_t accel_pool = nullptr; // the accelerators' memory: freed blocks kept for reuse (up to 4 GiB)
     DevBuf ws[WS_COUNT];
 };
@@ -118,8 +125,11 @@ int cuda_fail(rn_status* st, cudaError_t e, const char* what);
 int ensure_ctx(rn_status* st);
 // A workspace buffer of at least `bytes`.
 int ws_get(Slot s, size_t bytes, void** out, rn_status* st);
-// Read and clear the device error word (synchronizes the stream).
+// Read and clear the device error word (synchronizes the stream); or in two steps around a
+// call's own synchronisation: the copy queued, and the word judged once it has landed.
 int check_device_error(rn_status* st, const char* where);
+int queue_device_error(rn_status* st);
+int judge_device_error(rn_status* st, const char* where);
 
 // ---------------------------------------------------------------- sampler table
 int build_trig_correction(Context& c, rn_status* st);
@@ -137,13 +147,22 @@ struct RecOut {       // the reduction's device-side result
     uint32_t done;    // blocks finished (the last block reduces, then resets it to 0)
     uint32_t pad;
 };
+struct Readback {
+    RecOut rec;                 // written by the reduction's last block
+    uint32_t counts[3];
+    float mean;
+    uint32_t dev_error, word;
+    alignas(16) unsigned char ploc[48], collapse[32];
+};
 // Returns the launch's error (read once with cudaGetLastError, so the caller reports it).
+// host_out: a mapped host copy of the result (or null).
 cudaError_t launch_reconcile(const float* approx, const float* truth, const uint8_t* mask, size_t npx,
-                             float* err, RecPartial* partials, int nblocks, RecOut* out, cudaStream_t s);
+                             float* err, RecPartial* partials, int nblocks, RecOut* out, cudaStream_t s,
+                             RecOut* host_out = nullptr);
 int reconcile_blocks(size_t npx);
 int launch_ssao(int w, int h, const float* pos, const float* nrm, const uint8_t* mask, int samples,
                 float radius, const uint8_t* corr, float* ao, const float* truth, float* err,
-                RecPartial* partials, RecOut* out, cudaStream_t s);
+                RecPartial* partials, RecOut* out, cudaStream_t s, RecOut* host_out = nullptr);
 int ssao_blocks(int w, int h);
 
 // ---------------------------------------------------------------- accelerator
@@ -196,12 +215,20 @@ struct PlocTree {
     int32_t* tri = nullptr;    // (2n-1)
     uint32_t* count = nullptr; // (2n-1) triangles under the node
     void* mem = nullptr;       // the workspace block holding the arrays above (not owned)
+    const void* state = nullptr;   // a build queued and not yet read: its round state on the device
 };
-int ploc_build(const float* d_tris, uint32_t n, int radius, PlocTree* out, cudaStream_t s, rn_status* st);
+// deferred: a build of one batch (few triangles) is queued whole, its state copied to the
+// read-back area, and out->state set instead of root and rounds; collapse_finish judges it.
+int ploc_build(const float* d_tris, uint32_t n, int radius, PlocTree* out, cudaStream_t s, rn_status* st,
+               bool deferred = false);
+bool ploc_one_batch(uint32_t n);
 void ploc_free(PlocTree* t);
 int ploc_export(const PlocTree& t, int32_t* d_nodes9, cudaStream_t s, rn_status* st);
 int collapse_bvh4(const PlocTree& t, const float* d_tris, rn_accel* acc, int leaf_max, cudaStream_t s,
                   rn_status* st);
+// After the stream has been synchronised behind collapse_bvh4 of a deferred tree: its errors,
+// counts and depth.
+int collapse_finish(const PlocTree& t, rn_accel* acc, rn_status* st);
 
 // ---------------------------------------------------------------- traversal
 struct TraceParams {

@@ -33,7 +33,7 @@ struct RecAcc {
 // Every thread of the block must call it.
 template <int kThreads>
 __device__ void rec_block_finish(const RecAcc& a, RecPartial* __restrict__ parts, RecOut* out, uint32_t block,
-                                 uint32_t nblocks) {
+                                 uint32_t nblocks, RecOut* host_out = nullptr) {
     __shared__ double s_sum[kThreads / 32];
     __shared__ float s_max[kThreads / 32];
     __shared__ int s_n[kThreads / 32];
@@ -88,6 +88,11 @@ __device__ void rec_block_finish(const RecAcc& a, RecPartial* __restrict__ parts
         out->max = bm;
         out->n = bn;
         out->done = 0;     // ready for the next launch
+        if (host_out) {    // mapped host memory: there once the launch has completed
+            host_out->sum = bs;
+            host_out->max = bm;
+            host_out->n = bn;
+        }
     }
 }
 

@@ -989,7 +989,6 @@ int rn_unet_backward(rn_unet* u, const float* input, const float* target, int ba
         if (l == 2) pool_back_kernel<<<grid_for(u->Tn[2]), 256, 0, s>>>(u->dT[T_P0], u->B, u->H, u->W, 32, u->dT[2]);
     }
     RN_CUDA(cudaMemcpyAsync(u->host_loss, u->loss, 4, cudaMemcpyDeviceToHost, s), st);
-    RN_CUDA(cudaStreamSynchronize(s), st);
     RN_TRY(check_device_error(st, "rn_unet_backward"));
     if (loss) *loss = *u->host_loss / (float)M;
     return ok(st);
@@ -1011,7 +1010,6 @@ int rn_unet_apply(rn_unet* u, float lr, rn_status* st) {
         refresh_weights(u, &a, s);
     }
     RN_CUDA(cudaMemcpyAsync(u->host_loss + 1, u->gstats + 1, 8, cudaMemcpyDeviceToHost, s), st);
-    RN_CUDA(cudaStreamSynchronize(s), st);
     RN_TRY(check_device_error(st, "rn_unet_apply"));
     return ok(st);
 }
@@ -1139,11 +1137,12 @@ int rn_surrogate_ao(rn_unet* u, const rn_gbuf* g, const float* depth, const rn_a
     if (pred_out) RN_CUDA(cudaMemcpy2DAsync(pred_out, (size_t)w * 4, pr, (size_t)u->W * 4, (size_t)w * 4, h,
                                             cudaMemcpyDeviceToDevice, s), st);
     RN_CUDA(cudaGetLastError(), st);
-    unsigned hc[3] = {0, 0, 0};
-    float hm = 0.0f;
-    RN_CUDA(cudaMemcpyAsync(hc, counts, 12, cudaMemcpyDeviceToHost, s), st);
-    RN_CUDA(cudaMemcpyAsync(&hm, mean, 4, cudaMemcpyDeviceToHost, s), st);
+    Readback& back = *ctx().back;
+    RN_CUDA(cudaMemcpyAsync(back.counts, counts, 16, cudaMemcpyDeviceToHost, s), st);     // and the mean behind them
+    static_assert(offsetof(Readback, mean) == offsetof(Readback, counts) + 12, "counts and mean lie as on the device");
     RN_TRY(check_device_error(st, "rn_surrogate_ao"));
+    const uint32_t* hc = back.counts;
+    const float hm = back.mean;
     if (stats) {
         stats->tiles_covered = hc[0];
         stats->tiles_fallback = hc[1];
