@@ -143,6 +143,14 @@ __device__ __forceinline__ uint32_t spread10(uint32_t v) {
     return v;
 }
 // rt_bvh.cpp:123-130: 10-bit quantization min(1023, (x - lo) * s * 1023), code = morton3.
+__device__ __forceinline__ uint32_t morton_code(const float* c, const float* lo, float scale) {
+    uint32_t q[3];
+    for (int k = 0; k < 3; ++k) {
+        const uint32_t v = (uint32_t)fmul(fmul(fsub(c[k], lo[k]), scale), 1023.0f);
+        q[k] = v < 1023u ? v : 1023u;
+    }
+    return (spread10(q[0]) << 2) | (spread10(q[1]) << 1) | spread10(q[2]);
+}
 __global__ void morton_codes(const float* __restrict__ cent, uint32_t n, const Bounds* __restrict__ b,
                              uint32_t* __restrict__ keys, uint32_t* __restrict__ vals) {
     __shared__ float slo[3], sscale;
@@ -154,12 +162,7 @@ __global__ void morton_codes(const float* __restrict__ cent, uint32_t n, const B
     __syncthreads();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    uint32_t q[3];
-    for (int k = 0; k < 3; ++k) {
-        const uint32_t v = (uint32_t)fmul(fmul(fsub(cent[(size_t)i * 3 + k], slo[k]), sscale), 1023.0f);
-        q[k] = v < 1023u ? v : 1023u;
-    }
-    keys[i] = (spread10(q[0]) << 2) | (spread10(q[1]) << 1) | spread10(q[2]);
+    keys[i] = morton_code(cent + (size_t)i * 3, slo, sscale);
     vals[i] = i;
 }
 
@@ -214,15 +217,12 @@ __global__ void rs_scatter(const uint32_t* __restrict__ kin, const uint32_t* __r
 }
 
 // ------------------------------------------------------------------ leaves
-// rt_bvh.cpp:68-77 (leafBox) and :134-139.
-__global__ void make_leaves(const float* __restrict__ tris, const uint32_t* __restrict__ order, uint32_t n,
-                            float* __restrict__ box, int32_t* __restrict__ left, int32_t* __restrict__ right,
-                            int32_t* __restrict__ tri, uint32_t* __restrict__ count, float* __restrict__ cbox,
-                            int32_t* __restrict__ cl) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+// rt_bvh.cpp:68-77 (leafBox) and :134-139: leaf i, of triangle t.
+__device__ __forceinline__ void make_leaf(const float* __restrict__ tris, uint32_t i, uint32_t t, uint32_t n,
+                                          float* __restrict__ box, int32_t* __restrict__ left, int32_t* __restrict__ right,
+                                          int32_t* __restrict__ tri, uint32_t* __restrict__ count, float* __restrict__ cbox,
+                                          int32_t* __restrict__ cl) {
     if (i + 1 < n) tri[n + i] = -1;              // internal node n + i: the rounds write the rest of it
-    const uint32_t t = order[i];
     const float* v = tris + (size_t)t * 9;
     float lo[3], hi[3];
     for (int a = 0; a < 3; ++a) { lo[a] = v[a]; hi[a] = v[a]; }
@@ -236,6 +236,13 @@ __global__ void make_leaves(const float* __restrict__ tris, const uint32_t* __re
     count[i] = 1;
     cl[i] = (int32_t)i;
 }
+__global__ void make_leaves(const float* __restrict__ tris, const uint32_t* __restrict__ order, uint32_t n,
+                            float* __restrict__ box, int32_t* __restrict__ left, int32_t* __restrict__ right,
+                            int32_t* __restrict__ tri, uint32_t* __restrict__ count, float* __restrict__ cbox,
+                            int32_t* __restrict__ cl) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) make_leaf(tris, i, order[i], n, box, left, right, tri, count, cbox, cl);
+}
 // ------------------------------------------------------------------ PLOC rounds
 struct RoundState {
     uint32_t m;          // clusters in the current round
@@ -248,6 +255,72 @@ struct RoundState {
     int32_t root;        // the last cluster, written by the tail kernels when one is left
     uint32_t stop;       // the launched rounds do nothing once m <= stop (the tail's threshold, or 1)
 };
+
+// A small scene's centroids, bounds, codes, their stable sort and its leaves in one block, the
+// round state with them: as separate passes they are 24 launches of a few microseconds each
+// whatever the size. The sort is a bitonic one over (code, index), so equal codes keep their
+// order as in the radix passes. Launch-bound before, one
+// block's latency now (5.9 us at 14 triangles).
+constexpr int kSmallBuild = 4096, kSmallThreads = 1024;
+__global__ void __launch_bounds__(kSmallThreads) small_leaves(const float* __restrict__ tris, uint32_t n,
+                                                              float* __restrict__ box, int32_t* __restrict__ left,
+                                                              int32_t* __restrict__ right, int32_t* __restrict__ tri,
+                                                              uint32_t* __restrict__ count, float* __restrict__ cbox,
+                                                              int32_t* __restrict__ cl, RoundState* state, RoundState init) {
+    __shared__ unsigned long long key[kSmallBuild];
+    __shared__ unsigned slo[3], shi[3];
+    __shared__ float lo[3], scale;
+    constexpr int kPer = kSmallBuild / kSmallThreads;
+    const int tid = threadIdx.x;
+    if (tid < 3) { slo[tid] = f2ord(FLT_MAX); shi[tid] = f2ord(-FLT_MAX); }
+    if (tid == 0) *state = init;
+    __syncthreads();
+    float c[kPer][3];
+    unsigned mn[3], mx[3];
+    for (int k = 0; k < 3; ++k) { mn[k] = f2ord(FLT_MAX); mx[k] = f2ord(-FLT_MAX); }
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+        const uint32_t i = j * kSmallThreads + tid;
+        if (i >= n) continue;
+        const float* t = tris + (size_t)i * 9;
+        const float third = 0.333333343f;
+        for (int k = 0; k < 3; ++k) {
+            c[j][k] = fmul(fadd(fadd(t[k], t[3 + k]), t[6 + k]), third);
+            mn[k] = min(mn[k], f2ord(c[j][k]));
+            mx[k] = max(mx[k], f2ord(c[j][k]));
+        }
+    }
+    for (int k = 0; k < 3; ++k) {
+        const unsigned a = __reduce_min_sync(0xffffffffu, mn[k]), b = __reduce_max_sync(0xffffffffu, mx[k]);
+        if ((tid & 31) == 0) { atomicMin(&slo[k], a); atomicMax(&shi[k], b); }
+    }
+    __syncthreads();
+    if (tid == 0) {
+        float hi[3];
+        for (int k = 0; k < 3; ++k) { lo[k] = ord2f(slo[k]); hi[k] = ord2f(shi[k]); }
+        scale = pow2_scale(smax(fsub(hi[0], lo[0]), smax(fsub(hi[1], lo[1]), fsub(hi[2], lo[2]))));
+    }
+    uint32_t size = 2;
+    while (size < n) size *= 2;                     // at most kSmallBuild
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+        const uint32_t i = j * kSmallThreads + tid;
+        if (i < size) key[i] = i < n ? (unsigned long long)morton_code(c[j], lo, scale) << 32 | i : ~0ull;
+    }
+    for (uint32_t run = 2; run <= size; run *= 2)
+        for (uint32_t d = run / 2; d > 0; d /= 2) {
+            __syncthreads();
+            for (uint32_t e = tid; e < size / 2; e += kSmallThreads) {
+                const uint32_t a = 2 * e - (e & (d - 1)), b = a + d;
+                const unsigned long long x = key[a], y = key[b];
+                if ((x > y) == ((a & run) == 0)) { key[a] = y; key[b] = x; }
+            }
+        }
+    __syncthreads();
+    for (uint32_t i = tid; i < n; i += kSmallThreads)
+        make_leaf(tris, i, (uint32_t)key[i], n, box, left, right, tri, count, cbox, cl);
+}
 
 // rt_bvh.cpp:104-110: 2 (dy (dx + dz) + dz dx), operation for operation.
 __device__ __forceinline__ float ploc_area(float lx, float ly, float lz, float hx, float hy, float hz) {
@@ -1364,35 +1437,42 @@ int ploc_build(const float* d_tris, uint32_t n, int radius, PlocTree* out, cudaS
     Bounds* bounds = (Bounds*)(mem + o_bounds);
     RoundState* state = (RoundState*)(mem + o_state);
 
-    // 1-2: centroids, bounds, codes
-    init_bounds<<<1, 32, 0, s>>>(bounds);
-    centroid_bounds<<<cdiv(n, 256), 256, 0, s>>>(d_tris, n, cent, bounds);
-    morton_codes<<<cdiv(n, 256), 256, 0, s>>>(cent, n, bounds, k0, v0);
-    // 3: four stable 8-bit passes over the 30-bit codes
-    for (int pass = 0; pass < 4; ++pass) {
-        const int shift = 8 * pass;
-        rs_hist<<<nbs, kThreads, 0, s>>>(k0, n, shift, nbs, hist);
-        scan_exclusive_u32(hist, offs, 256 * nbs, bsum, nullptr, s);
-        rs_scatter<<<nbs, kThreads, 0, s>>>(k0, v0, n, shift, nbs, offs, k1, v1);
-        std::swap(k0, k1);
-        std::swap(v0, v1);
-    }
-    // 4: leaves
-    make_leaves<<<cdiv(n, 256), 256, 0, s>>>(d_tris, v0, n, out->box, out->left, out->right, out->tri, out->count, cb0,
-                                             cl0);
-    // 5: rounds, in batches; the host reads the state once per batch. With a tail threshold
-    // the launched rounds stop at it (stop) and every batch ends with the tail kernel, which
-    // runs the remaining rounds once the state is at or below the threshold and otherwise
-    // leaves at once: the batch that reaches the threshold also finishes the tree.
     const uint32_t tail_max = (uint32_t)ctx().tune.ploc_tail;
     RoundState init{};
     init.m = n;
     init.next = n;
     init.root = -1;
     init.stop = tail_max > 1 ? tail_max : 1u;
-    RN_CUDA(cudaMemcpyAsync(state, &init, sizeof init, cudaMemcpyHostToDevice, s), st);
+    // 1-4 in one block for a small scene, up to what one block's shared memory and sort take: an
+    // accelerator over 14 triangles 163 -> 78 us, 500 241 -> 156, 2,000 307 -> 225, 4,096 383 -> 314
+    if (n <= (uint32_t)kSmallBuild) {
+        small_leaves<<<1, kSmallThreads, 0, s>>>(d_tris, n, out->box, out->left, out->right, out->tri, out->count, cb0, cl0,
+                                                 state, init);
+    } else {
+        // 1-2: centroids, bounds, codes
+        init_bounds<<<1, 32, 0, s>>>(bounds);
+        centroid_bounds<<<cdiv(n, 256), 256, 0, s>>>(d_tris, n, cent, bounds);
+        morton_codes<<<cdiv(n, 256), 256, 0, s>>>(cent, n, bounds, k0, v0);
+        // 3: four stable 8-bit passes over the 30-bit codes
+        for (int pass = 0; pass < 4; ++pass) {
+            const int shift = 8 * pass;
+            rs_hist<<<nbs, kThreads, 0, s>>>(k0, n, shift, nbs, hist);
+            scan_exclusive_u32(hist, offs, 256 * nbs, bsum, nullptr, s);
+            rs_scatter<<<nbs, kThreads, 0, s>>>(k0, v0, n, shift, nbs, offs, k1, v1);
+            std::swap(k0, k1);
+            std::swap(v0, v1);
+        }
+        // 4: leaves
+        make_leaves<<<cdiv(n, 256), 256, 0, s>>>(d_tris, v0, n, out->box, out->left, out->right, out->tri, out->count, cb0,
+                                                 cl0);
+        RN_CUDA(cudaMemcpyAsync(state, &init, sizeof init, cudaMemcpyHostToDevice, s), st);
+    }
+    // 5: rounds, in batches; the host reads the state once per batch. With a tail threshold
+    // the launched rounds stop at it (stop) and every batch ends with the tail kernel, which
+    // runs the remaining rounds once the state is at or below the threshold and otherwise
+    // leaves at once: the batch that reaches the threshold also finishes the tree.
     const bool fused = ctx().tune.ploc_fused != 0;
-    if (fused) {
+    if (fused && n > tail_max) {
         // the look-back words of an earlier build must not pass for this one's
         RN_CUDA(cudaMemsetAsync(look, 0, (size_t)(cdiv(n, kMergeTile) + 1) * 8, s), st);
         RN_CUDA(cudaMemsetAsync(ticket, 0, 8, s), st);
@@ -1506,7 +1586,6 @@ int collapse_bvh4(const PlocTree& t, const float* d_tris, rn_accel* acc, int lea
     acc->ntri = n;
     acc->rounds = t.rounds;
     if (n == 0) return ok(st);
-    const uint32_t N = 2 * n - 1;
     const uint32_t node_cap = n;              // every 4-wide node has at least 2 children
     // the accelerator's nodes and leaf triangles in one allocation (rn_accel_free frees d_nodes)
     const size_t node_bytes = ((size_t)node_cap * sizeof(Node4) + 255) & ~size_t(255);

@@ -138,3 +138,24 @@ def test_accel_info(rn, oracle):
     finally:
         for k, v in saved.items():
             rn.tune_set(k, v)
+
+
+@pytest.mark.parametrize("n,dup", [(2, 0), (31, 1), (32, 0), (33, 0), (1023, 3), (1024, 0), (1025, 0), (2048, 2), (4095, 0),
+                                   (4096, 5), (4097, 5)])
+def test_ploc_small_scene_equals_oracle(rn, oracle, n, dup):
+    """Scenes up to 4,096 triangles take their codes, sort and leaves in one block (a bitonic sort
+    padded to a power of two): the oracle's tree node for node around its sizes, with triangles
+    that repeat (equal codes keep their order); and an accelerator over the same triangles,
+    queued with its collapse and read once, counts its nodes and answers rays as the scan does."""
+    tris = oracle.soup(n, 100 + n).copy()
+    if dup:
+        tris[dup:] = tris[np.arange(len(tris) - dup) // (dup + 1)]
+    nodes, root, rounds = rn.build_ploc(tris)
+    want = oracle.ploc(tris)
+    assert np.array_equal(nodes, want[0]) and (root, rounds) == (want[1], want[2])
+    acc = rn.LinearAccel(tris)
+    info = acc.info()
+    assert info["leaf_tris"] == n and 1 <= info["wide_nodes"] <= n
+    rays = random_rays(np.random.default_rng(n), 512)
+    tmax = np.full(512, 40.0, np.float32)
+    assert np.array_equal(rn.occluded(acc, rays, tmax), oracle.occluded_scan(tris, rays, tmax, threads=os.cpu_count() or 1))
