@@ -434,39 +434,77 @@ __global__ void clip_kernel(float* __restrict__ stats, float ratio) {
 // ------------------------------------------------------------------ the surrogate's frame
 constexpr int kSppIn = 4;                 // samples of the traced input
 constexpr int kTile = 16;                 // fallback tiles: 16 x 16 pixels
+constexpr int kBandTiles = 4;             // tiles a block judges together
 constexpr int kDepthBlocks = 512;
 
-// Per-block sums of the covered pixels' depth (FP64) and count, in a fixed order.
-__global__ void depth_partial_kernel(const float* __restrict__ depth, const uint8_t* __restrict__ mask, size_t n,
-                                     double* __restrict__ part_sum, unsigned* __restrict__ part_cnt) {
+// The mean of the covered pixels' depth: FP64 sums per thread and per block in a fixed order;
+// the last block to finish adds the partials, also in a fixed order, and divides (0 without
+// covered pixels). A thread's 60-odd pixels of a 4K frame are a chain of loads unless several
+// are in flight: eight at a time (4K: 60 us and a 39 us one-thread pass over the partials before,
+// 25 us now).
+__global__ void __launch_bounds__(256) depth_mean_kernel(const float* __restrict__ depth, const uint8_t* __restrict__ mask,
+                                                         size_t n, double* part_sum, unsigned* part_cnt, unsigned* ticket,
+                                                         float* __restrict__ mean) {
     double s = 0.0;
     unsigned c = 0;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-        if (mask[i]) { s += (double)depth[i]; ++c; }
-    for (int o = 16; o; o >>= 1) {
-        s += __shfl_xor_sync(0xffffffffu, s, o);
-        c += __shfl_xor_sync(0xffffffffu, c, o);
+    constexpr int kAhead = 8;
+    const size_t stride = (size_t)gridDim.x * blockDim.x;
+    for (size_t i0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += stride * kAhead) {
+        float d[kAhead];
+        bool m[kAhead];
+#pragma unroll
+        for (int k = 0; k < kAhead; ++k) {
+            const size_t i = i0 + stride * k;
+            m[k] = i < n && mask[i];
+            d[k] = i < n ? depth[i] : 0.0f;
+        }
+        // their sum as a float pair (two-sum: what a sum loses goes into lo), then two FP64 additions
+        // instead of eight: FP64 issues at two a clock and SM here
+        float hi = 0.0f, lo = 0.0f;
+#pragma unroll
+        for (int k = 0; k < kAhead; ++k)
+            if (m[k]) {
+                const float t = __fadd_rn(hi, d[k]), b = __fsub_rn(t, hi);
+                lo = __fadd_rn(lo, __fadd_rn(__fsub_rn(hi, __fsub_rn(t, b)), __fsub_rn(d[k], b)));
+                hi = t;
+                ++c;
+            }
+        s += (double)hi + (double)lo;
     }
     __shared__ double ss[8];
     __shared__ unsigned sc[8];
-    if ((threadIdx.x & 31) == 0) { ss[threadIdx.x >> 5] = s; sc[threadIdx.x >> 5] = c; }
-    __syncthreads();
+    __shared__ bool last;
+    auto block_sum = [&](double& t, unsigned& tc) {          // thread 0's, in a fixed order
+        for (int o = 16; o; o >>= 1) {
+            t += __shfl_xor_sync(0xffffffffu, t, o);
+            tc += __shfl_xor_sync(0xffffffffu, tc, o);
+        }
+        if ((threadIdx.x & 31) == 0) { ss[threadIdx.x >> 5] = t; sc[threadIdx.x >> 5] = tc; }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            t = 0.0;
+            tc = 0;
+            for (int k = 0; k < 8; ++k) { t += ss[k]; tc += sc[k]; }
+        }
+    };
+    block_sum(s, c);
     if (threadIdx.x == 0) {
-        double t = 0.0;
-        unsigned tc = 0;
-        for (int k = 0; k < 8; ++k) { t += ss[k]; tc += sc[k]; }
-        part_sum[blockIdx.x] = t;
-        part_cnt[blockIdx.x] = tc;
+        part_sum[blockIdx.x] = s;
+        part_cnt[blockIdx.x] = c;
+        __threadfence();
+        last = atomicAdd(ticket, 1u) == gridDim.x - 1;
     }
-}
-// mean = (float)(sum / count) over the partials in block order (0 without covered pixels).
-__global__ void depth_mean_kernel(const double* __restrict__ part_sum, const unsigned* __restrict__ part_cnt, int nb,
-                                  float* __restrict__ mean) {
-    if (threadIdx.x != 0) return;
-    double t = 0.0;
-    unsigned long long c = 0;
-    for (int k = 0; k < nb; ++k) { t += part_sum[k]; c += part_cnt[k]; }
-    *mean = c ? (float)(t / (double)c) : 0.0f;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    s = 0.0;
+    c = 0;                                                   // at most 2^31 pixels in all
+    for (unsigned k = threadIdx.x; k < gridDim.x; k += blockDim.x) { s += __ldcg(part_sum + k); c += __ldcg(part_cnt + k); }
+    block_sum(s, c);
+    if (threadIdx.x == 0) {
+        *mean = c ? (float)(s / (double)c) : 0.0f;
+        *ticket = 0;                                         // ready for the next launch
+    }
 }
 
 // The network's BF16 input for a w x h frame inside its H x W shape: clamp((depth - mean) /
@@ -475,10 +513,12 @@ __global__ void depth_mean_kernel(const double* __restrict__ part_sum, const uns
 __global__ void features_kernel(const float* __restrict__ depth, const float* __restrict__ nrm,
                                 const uint8_t* __restrict__ mask, const float* __restrict__ ao4, int w, int h, int W,
                                 int H, const float* __restrict__ mean, float radius, int C, bf16* __restrict__ out) {
-    const size_t total = (size_t)W * H;
+    // a block is 256 pixels of a row: no division per pixel
     const float mu = *mean;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        const int x = (int)(i % W), y = (int)(i / W);
+    const int x = blockIdx.x * blockDim.x + threadIdx.x;
+    if (x >= W) return;
+    for (int y = blockIdx.y; y < H; y += gridDim.y) {
+        const size_t i = (size_t)y * W + x;
         float f[5] = {0.0f, 0.0f, 0.0f, 0.0f, 1.0f};
         if (x < w && y < h) {
             const size_t p = (size_t)y * w + x;
@@ -500,7 +540,9 @@ __global__ void features_kernel(const float* __restrict__ depth, const float* __
     }
 }
 
-// One 16 x 16 tile per block: the confidence band test of the prediction's tile mean against
+// Four 16 x 16 tiles per block and step, a tile's steps being one chain of latencies, and the
+// frame's two counts by one atomic a judging warp (a block a tile: 68 us at 4K; a tile a step: 92;
+// four: 46). A tile: the confidence band test of the prediction's tile mean against
 // the 4-spp tile mean (sigma = max(sqrt(sum p (1 - p) / 4) / n, 0.5 / sqrt(4 n)) over the n
 // covered pixels), the tile's flag, and the fallback mask of its pixels.
 __global__ void __launch_bounds__(kTile * kTile) band_kernel(const float* __restrict__ pred, int W,
@@ -509,43 +551,74 @@ __global__ void __launch_bounds__(kTile * kTile) band_kernel(const float* __rest
                                                               uint8_t* __restrict__ tile_flag,
                                                               uint8_t* __restrict__ fb_mask,
                                                               unsigned* __restrict__ counts,
-                                                              uint32_t* __restrict__ fb_list) {
-    const int x = blockIdx.x * kTile + (threadIdx.x % kTile), y = blockIdx.y * kTile + (threadIdx.x / kTile);
-    const bool in = x < w && y < h;
-    const size_t p = (size_t)y * w + x;
-    const bool cov = in && mask[p];
-    float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    if (cov) {
-        const float a = ao4[p];
-        v[0] = 1.0f;
-        v[1] = pred[(size_t)y * W + x];
-        v[2] = a;
-        v[3] = a * (1.0f - a);
-    }
-    __shared__ float red[4][kTile * kTile / 32];
+                                                              uint32_t* __restrict__ fb_list, uint32_t* __restrict__ open,
+                                                              int tx, int tiles) {
+    __shared__ float red[kBandTiles][4][kTile * kTile / 32];
+    __shared__ int s_flag[kBandTiles];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    unsigned covered = 0, flagged = 0;          // of the tiles that this warp judges
+    for (int tile0 = blockIdx.x * kBandTiles; tile0 < tiles; tile0 += gridDim.x * kBandTiles) {
+        float v[kBandTiles][4];
+        size_t p[kBandTiles];
+        unsigned in = 0, cov = 0;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        float t = v[q];
-        for (int o = 16; o; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-        if ((threadIdx.x & 31) == 0) red[q][threadIdx.x >> 5] = t;
+        for (int j = 0; j < kBandTiles; ++j) {
+            const int tile = tile0 + j;
+            const int x = tile % tx * kTile + (threadIdx.x % kTile), y = tile / tx * kTile + (threadIdx.x / kTile);
+            const bool inside = tile < tiles && x < w && y < h;
+            p[j] = (size_t)y * w + x;
+            const bool c = inside && mask[p[j]];
+            const float a = inside ? ao4[p[j]] : 0.0f, q = inside ? pred[(size_t)y * W + x] : 0.0f;
+            in |= (unsigned)inside << j;
+            cov |= (unsigned)c << j;
+            v[j][0] = c ? 1.0f : 0.0f;
+            v[j][1] = c ? q : 0.0f;
+            v[j][2] = c ? a : 0.0f;
+            v[j][3] = c ? a * (1.0f - a) : 0.0f;
+        }
+#pragma unroll
+        for (int j = 0; j < kBandTiles; ++j)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                float t = v[j][q];
+                for (int o = 16; o; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+                if (lane == 0) red[j][q][warp] = t;
+            }
+        __syncthreads();
+        if (lane == 0 && warp < kBandTiles && tile0 + warp < tiles) {
+            float t[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            for (int q = 0; q < 4; ++q)
+                for (int j = 0; j < kTile * kTile / 32; ++j) t[q] += red[warp][q][j];
+            const float n = fmaxf(t[0], 1.0f);
+            const float sigma = fmaxf(sqrtf(fmaxf(t[3], 0.0f) / (float)kSppIn) / n, 0.5f / sqrtf((float)kSppIn * n));
+            const int flag = t[0] > 0.0f && fabsf(t[1] / n - t[2] / n) > k * sigma;
+            tile_flag[tile0 + warp] = (uint8_t)flag;
+            covered += t[0] > 0.0f;
+            flagged += flag;
+            s_flag[warp] = flag;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < kBandTiles; ++j) {
+            if (tile0 + j >= tiles) break;
+            const bool fb = (cov >> j & 1u) && s_flag[j];
+            if (in >> j & 1u) fb_mask[p[j]] = (uint8_t)fb;
+            if (s_flag[j]) {
+                const unsigned peers = __ballot_sync(0xffffffffu, fb);
+                unsigned at = 0;
+                if (lane == 0 && peers) at = atomicAdd(counts + 2, (unsigned)__popc(peers));
+                at = __shfl_sync(0xffffffffu, at, 0) + __popc(peers & ((1u << lane) - 1u));
+                if (fb) {
+                    fb_list[at] = (uint32_t)p[j];
+                    open[p[j]] = 0;             // the fallback pixels' open rays, counted from here
+                }
+            }
+        }
     }
-    __syncthreads();
-    __shared__ int s_flag;
-    if (threadIdx.x == 0) {
-        float t[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-        for (int q = 0; q < 4; ++q)
-            for (int j = 0; j < kTile * kTile / 32; ++j) t[q] += red[q][j];
-        const float n = fmaxf(t[0], 1.0f);
-        const float sigma = fmaxf(sqrtf(fmaxf(t[3], 0.0f) / (float)kSppIn) / n, 0.5f / sqrtf((float)kSppIn * n));
-        const int flag = t[0] > 0.0f && fabsf(t[1] / n - t[2] / n) > k * sigma;
-        tile_flag[blockIdx.y * gridDim.x + blockIdx.x] = (uint8_t)flag;
-        if (t[0] > 0.0f) atomicAdd(counts, 1u);
-        if (flag) atomicAdd(counts + 1, 1u);
-        s_flag = flag;
+    if (lane == 0) {
+        if (covered) atomicAdd(counts, covered);
+        if (flagged) atomicAdd(counts + 1, flagged);
     }
-    __syncthreads();
-    if (in) fb_mask[p] = (uint8_t)(cov && s_flag);
-    if (cov && s_flag) fb_list[atomicAdd(counts + 2, 1u)] = (uint32_t)p;
 }
 
 // ao = 1 off the coverage, the traced AO (open rays / spp, as the trace divides) on fallback
@@ -553,11 +626,16 @@ __global__ void __launch_bounds__(kTile * kTile) band_kernel(const float* __rest
 __global__ void composite_kernel(const float* __restrict__ pred, int W, const uint32_t* __restrict__ open, int spp,
                                  const uint8_t* __restrict__ mask, const uint8_t* __restrict__ fb, int w, int h,
                                  float* __restrict__ ao) {
-    const size_t total = (size_t)w * h;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        const int x = (int)(i % w), y = (int)(i / w);
-        ao[i] = !mask[i] ? 1.0f : fb[i] ? __fdiv_rn((float)open[i], (float)spp) : pred[(size_t)y * W + x];
-    }
+    // a block is 1,024 pixels of a row, four a thread: no division per pixel
+    for (int y = blockIdx.y; y < h; y += gridDim.y)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int x = (blockIdx.x * 4 + j) * blockDim.x + threadIdx.x;
+            if (x >= w) break;
+            const size_t i = (size_t)y * w + x;
+            const float p = pred[(size_t)y * W + x];
+            ao[i] = !mask[i] ? 1.0f : fb[i] ? __fdiv_rn((float)open[i], (float)spp) : p;
+        }
 }
 
 inline unsigned grid_for(size_t n, int block = 256) {
@@ -1100,7 +1178,7 @@ int rn_surrogate_ao(rn_unet* u, const rn_gbuf* g, const float* depth, const rn_a
     RN_TRY(ws_get(WS_SUR_PRED, npad * 4, &p_pred, st));
     RN_TRY(ws_get(WS_SUR_FB, np + (size_t)tx * ty, &p_fb, st));
     RN_TRY(ws_get(WS_SUR_AOFB, np * 8, &p_aofb, st));          // open-ray counts, then the pixel list
-    RN_TRY(ws_get(WS_SUR_STATS, 16 + kDepthBlocks * 12, &p_st, st));
+    RN_TRY(ws_get(WS_SUR_STATS, 16 + kDepthBlocks * 12 + 16, &p_st, st));
     float* a4 = ao4_out ? ao4_out : (float*)p_ao4;
     float* pr = (float*)p_pred;
     uint8_t* fbm = (uint8_t*)p_fb;
@@ -1112,13 +1190,11 @@ int rn_surrogate_ao(rn_unet* u, const rn_gbuf* g, const float* depth, const rn_a
     uint32_t* fb_list = open + np;
     unsigned* pcnt = (unsigned*)(psum + kDepthBlocks);
     RN_CUDA(cudaMemsetAsync(counts, 0, 12, s), st);
-    RN_CUDA(cudaMemsetAsync(open, 0, np * 4, s), st);
     // 1. the 4-spp trace
     RN_TRY(trace_ao_device(g->position, g->normal, g->mask, w, h, accel, kSppIn, radius, a4, st));
     // 2. features straight into the network's input, 3. the network
-    depth_partial_kernel<<<kDepthBlocks, 256, 0, s>>>(depth, g->mask, np, psum, pcnt);
-    depth_mean_kernel<<<1, 32, 0, s>>>(psum, pcnt, kDepthBlocks, mean);
-    features_kernel<<<grid_for(npad), 256, 0, s>>>(depth, g->normal, g->mask, a4, w, h, u->W, u->H, mean, radius,
+    depth_mean_kernel<<<kDepthBlocks, 256, 0, s>>>(depth, g->mask, np, psum, pcnt, pcnt + kDepthBlocks, mean);
+    features_kernel<<<dim3((u->W + 255) / 256, std::min(u->H, 65535)), 256, 0, s>>>(depth, g->normal, g->mask, a4, w, h, u->W, u->H, mean, radius,
                                                     u->TC[T_IN], u->T[T_IN]);
     if (u->implicit) {
         RN_TRY(forward_all(u, s, st, pr));             // the head in the last layer's epilogue
@@ -1127,13 +1203,14 @@ int rn_surrogate_ao(rn_unet* u, const rn_gbuf* g, const float* depth, const rn_a
         head_kernel<<<(unsigned)((npad + 255) / 256), 256, 0, s>>>(u->T[14], u->wh, u->bh, npad, pr);
     }
     // 4. the band test, 5. the fallback trace, 6. the composite
-    band_kernel<<<dim3(tx, ty), kTile * kTile, 0, s>>>(pr, u->W, a4, g->mask, w, h, k, tf, fbm, counts, fb_list);
+    band_kernel<<<std::min((tx * ty + kBandTiles - 1) / kBandTiles, ctx().sm_count * 8), kTile * kTile, 0, s>>>(pr, u->W, a4, g->mask, w, h, k, tf, fbm,
+                                                                                counts, fb_list, open, tx, tx * ty);
     // the fallback pixels' rays, one thread per (pixel, sample): a few tiles' worth of work
     // spreads over the whole GPU instead of a few warps
     const TraceParams tp = ao_trace_params(g->position, g->normal, fbm, w, h, accel, spp_full, radius);
     if (launch_ao_samples(tp, fb_list, counts + 2, open, ctx().sm_count, s) != RN_OK)
         return cuda_fail(st, cudaGetLastError(), "ao_samples_kernel");
-    composite_kernel<<<grid_for(np), 256, 0, s>>>(pr, u->W, open, spp_full, g->mask, fbm, w, h, ao);
+    composite_kernel<<<dim3((w + 1023) / 1024, std::min(h, 65535)), 256, 0, s>>>(pr, u->W, open, spp_full, g->mask, fbm, w, h, ao);
     if (pred_out) RN_CUDA(cudaMemcpy2DAsync(pred_out, (size_t)w * 4, pr, (size_t)u->W * 4, (size_t)w * 4, h,
                                             cudaMemcpyDeviceToDevice, s), st);
     RN_CUDA(cudaGetLastError(), st);
