@@ -513,7 +513,7 @@ __device__ __noinline__ bool hit(const PtParams& P, v3 o, v3 d, float tmax, Surf
 __device__ __noinline__ bool visible(const PtParams& P, v3 p, v3 dir, float tmax) {
     if (!P.has_geometry) return true;
     Counts cn;
-    return walk<false>(P.nodes, P.ltris, p, dir, tmax, tmax, P.err, cn) == 0;
+    return walk<false, kStack, true, false>(P.nodes, P.ltris, p, dir, tmax, tmax, P.err, cn) == 0;
 }
 __device__ __forceinline__ v3 offset_of(const Surf& x, v3 dir) {
     const float e = fmul(2e-4f, fadd(1.0f, smax(fabsf(x.p.x), smax(fabsf(x.p.y), fabsf(x.p.z)))));
@@ -1070,7 +1070,7 @@ __global__ void __launch_bounds__(128) pt_wave_shadow(const PtParams P, const Wa
         bool vis = true;
         if (P.has_geometry) {
             Counts cn;
-            vis = walk<false>(P.nodes, P.ltris, o, d, tmax, tmax, P.err, cn) == 0;
+            vis = walk<false, kStack, true, false>(P.nodes, P.ltris, o, d, tmax, tmax, P.err, cn) == 0;
         }
         W.vis[(size_t)(s & 1u) * W.Q + (s >> 1)] = vis ? 1 : 0;
     }

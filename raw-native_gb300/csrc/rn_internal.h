@@ -166,6 +166,12 @@ int launch_ssao(int w, int h, const float* pos, const float* nrm, const uint8_t*
 int ssao_blocks(int w, int h);
 
 // ---------------------------------------------------------------- accelerator
+// Entries of a warp's frontier (trace_device.cuh), a multiple of 4, at most 32 (a lane an entry):
+// more entries mean walks that start deeper and a longer list for each ray to pass. 12 / 16 / 20 /
+// 24 / 32: six views of 744k triangles 26.98 / 26.42 / 26.24 / 26.17 / 26.94 ms, 3840 x 2160 x 256
+// spp over the built-in scene - / 13.22 / 13.09 / 13.08 / 13.26.
+constexpr int kFrontier = 24;
+
 // A 4-wide BVH node: six 4-float planes of child boxes (SoA) then the 4 child words and
 // per-node metadata. 128 bytes, 16-byte aligned for vector loads. Child word >= 0: index of
 // an interior node; < 0: leaf, ~word = first << 3 | (count - 1) into the leaf triangles.
@@ -251,7 +257,7 @@ struct TraceParams {
     int frontier;         // AO-only walks start from a per-warp frontier (0: from the root)
     int packet_log2;      // log2 of the packet width (pixels per warp row): 2, 3 or 4
     int frontier_tail;    // greedy single-entry steps after the breadth-first frontier build
-    int stack_need;       // entries the walk can push on this tree: 16 + 3 x wide depth
+    int stack_need;       // entries the walk can push on this tree: the frontier + 3 x wide depth
     // copy-through of a G-buffer read from host memory (null: none): every pixel's position,
     // normal, AO and mask are also written to a device buffer laid out as
     // [position w*h*12 B][normal w*h*12 B][ao w*h*4 B][mask w*h B] (mirror_* below)

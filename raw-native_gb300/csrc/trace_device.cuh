@@ -139,7 +139,7 @@ enum : int { HIT_NEAR = 1, HIT_FAR = 2 };
 // kFrontier entries result. AO walks start from it instead of re-descending from the root.
 // The entries are kept in the node layout, four to a group: a walk tests a group exactly as
 // it tests a node.
-constexpr int kFrontier = 16, kFrontierNodes = kFrontier / 4;
+constexpr int kFrontierNodes = kFrontier / 4;
 struct FrontierBox { float lo[3], hi[3]; int32_t word; };
 __device__ __forceinline__ void frontier_put(Node4* F, int e, const FrontierBox& b) {
     Node4& n = F[e >> 2];
@@ -298,7 +298,11 @@ __device__ inline int build_frontier(const Node4* __restrict__ nodes, const floa
 // together, and the triangle test exists once in the code instead of once per position).
 // Either order finds the same answers: boxes are only culled against tmax >= tnear, and a
 // far hit only lowers tmax to tnear.
-template <bool kCount, int kStackN = kStack, bool kLeafPass = true>
+// kNearest: of a node's interior children the nearest is descended into and the others stacked;
+// else the first, without a comparison per child (any order finds the same answers). Short AO
+// rays meet an occluder sooner in the nearest child, the path tracer's shadow rays do not gain
+// what the comparisons cost: FIG.
+template <bool kCount, int kStackN = kStack, bool kLeafPass = true, bool kNearest = true>
 __device__ int walk(const Node4* __restrict__ nodes, const LeafTri* __restrict__ tris, const v3& o, const v3& d,
                     float tnear, float tfar, uint32_t* err, Counts& cn, const Node4* F = nullptr, int fn = 0) {
     const Inv iv = make_inv(o, d);
@@ -340,7 +344,7 @@ __device__ int walk(const Node4* __restrict__ nodes, const LeafTri* __restrict__
                 if (kLeafPass) leaves |= 1u << k;
                 else if (leaf(c)) return true;
             }
-            const bool closer = in && tn[k] < tbest;
+            const bool closer = in && (kNearest ? tn[k] < tbest : nearest < 0);
             const int32_t push = closer ? nearest : c;
             if (in && nearest >= 0) stack[sp++] = push;
             nearest = closer ? c : nearest;
