@@ -1192,13 +1192,15 @@ __global__ void __launch_bounds__(kFan ? kFanThreads : kConvThreads, kFan && !kW
 // channels: 128-, 64- or 32-byte swizzle; 8 pixels per swizzle atom, the atoms of a tile one
 // after the other along the channels). The border reads TMA's zero fill, the convolution's
 // padding. No im2col rows are formed and nothing is transposed in memory: at batch 64 of
-// 128 x 128 the 14 layers took 12.2 ms as im2col, two transposes and a GEMM.
+// 128 x 128 the 14 layers took 12.2 ms as im2col, two transposes and a GEMM, 0.80 ms so.
 //
 // An "atom" is one (tap, CA-channel chunk); 128 / CA atoms make an M tile of 128 weight rows. A
 // CTA takes a group of up to 256 / N M tiles (256 TMEM columns, two CTAs per SM) and a slice of
 // the pixel boxes: per box it loads dz once and each M tile's atoms through a ring, so dz is
 // read once per group, and every x element nine times, from L2. At the end it adds its tiles
-// to gw with FP32 atomics. Roles: warp 0 loads (its lanes issue a tile's atoms together), one
+// to gw with FP32 atomics. The bias gradient, dz's column sums, comes from the same boxes: in the
+// first group's CTAs the epilogue warps, idle until the end, add up each dz box in shared memory
+// before its slot is released (a pass of its own read dz again: 14 passes, 250 us). Roles: warp 0 loads (its lanes issue a tile's atoms together), one
 // lane of warp 1 issues the MMAs, warps 2..5 read the accumulators. Waits are bounded and give
 // up when another role has aborted.
 struct WgradArgs {
@@ -1210,6 +1212,7 @@ struct WgradArgs {
     int per_group, groups, slices;
     int cin_out, ch_valid;
     float* gw;
+    float* gb;                  // column sums of dz, or null
     uint32_t* err;
 };
 constexpr int kWgPix = 64;
@@ -1253,12 +1256,13 @@ __global__ void __launch_bounds__(kConvThreads, 2) tc_wgrad_kernel(const __grid_
     const uint32_t done = smem_u32(&bars[2 * (kA + kB)]);
     // this CTA's M tiles [m0, m0 + nm) and boxes [k0, k1)
     const int group = (int)blockIdx.x % a.groups, slice = (int)blockIdx.x / a.groups;
+    const bool sums = a.gb && group == 0;
     const int m0 = group * a.per_group, nm = min(a.per_group, a.mtiles - m0);
     const int k0 = (int)((long long)a.boxes * slice / a.slices), k1 = (int)((long long)a.boxes * (slice + 1) / a.slices);
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < kA; ++s) { mbar_init(a_full(s), 1); mbar_init(a_empty(s), 1); }
-        for (int s = 0; s < kB; ++s) { mbar_init(b_full(s), 1); mbar_init(b_empty(s), 1); }
+        for (int s = 0; s < kB; ++s) { mbar_init(b_full(s), 1); mbar_init(b_empty(s), sums ? 5 : 1); }
         mbar_init(done, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         s_abort = 0;
@@ -1334,6 +1338,44 @@ __global__ void __launch_bounds__(kConvThreads, 2) tc_wgrad_kernel(const __grid_
         tc_commit(done);
     } else {
         const int q = warp & 3, r = q * 32 + lane;
+        if (sums) {
+            // a thread keeps eight channels (one 16-byte chunk, found by its tile's swizzle) of
+            // every (1024 / N)-th pixel
+            constexpr int kChunks = N / 8, kRows = 128 / kChunks;
+            const int ch = r % kChunks, sub = ch / (CB / 8), j = ch % (CB / 8);
+            float t[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+            uint32_t ib = 0;
+            bool more = true;
+            for (int k = k0; more && k < k1; ++k, ++ib) {
+                const int sb = (int)(ib % kB);
+                more = __all_sync(0xffffffffu, mbar_wait_or_abort(b_full(sb), (ib / kB) & 1u, abort_flag));
+                if (!more) break;
+                const uint8_t* tile = sB + sb * kBBytes + sub * (kWgPix * CB * 2);
+#pragma unroll
+                for (int p0 = 0; p0 < kWgPix; p0 += kRows) {
+                    const int px = p0 + r / kChunks;
+                    const int at = j ^ (CB == 64 ? px & 7 : (px >> 1) & 3);
+                    const uint4 v = *reinterpret_cast<const uint4*>(tile + px * (CB * 2) + at * 16);
+                    const __nv_bfloat16* h = reinterpret_cast<const __nv_bfloat16*>(&v);
+#pragma unroll
+                    for (int c = 0; c < 8; ++c) t[c] += __bfloat162float(h[c]);
+                }
+                // the loads must have returned before the slot's next copy may write it: the copy
+                // is the async proxy's, and without the fence a load queued behind the MMAs'
+                // operand reads can still be under way when the arrival is seen
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(b_empty(sb));
+            }
+            // lanes a multiple of kChunks apart hold the same channels
+#pragma unroll
+            for (int o = kChunks; o < 32; o <<= 1)
+#pragma unroll
+                for (int c = 0; c < 8; ++c) t[c] += __shfl_xor_sync(0xffffffffu, t[c], o);
+            if (more && lane < kChunks)
+#pragma unroll
+                for (int c = 0; c < 8; ++c) atomicAdd(a.gb + ch * 8 + c, t[c]);
+        }
         const bool ok = __all_sync(0xffffffffu, mbar_wait_or_abort(done, 0, abort_flag)) && !*abort_flag;
         tc_fence_after();
         if (__all_sync(0xffffffffu, ok) && k1 > k0) {
@@ -1752,7 +1794,7 @@ int tc_conv3x3(const tc::ConvSrc* src, int nsrc, int B, int H, int W, const __nv
 }
 
 int tc_wgrad3x3(const tc::ConvSrc* src, int nsrc, int B, int H, int W, const __nv_bfloat16* dz, int N, float* gw,
-                int cin_out, int ch_valid, uint32_t* err, cudaStream_t s, rn_status* st) {
+                int cin_out, int ch_valid, float* gb, uint32_t* err, cudaStream_t s, rn_status* st) {
     const tc::ConvTiling t = tc::conv_tiling(H, W);
     if (nsrc < 1 || nsrc > 2 || !src || !dz || !gw || B <= 0 || !t.ok)
         return fail(st, RN_ERR_INVALID, "tc_wgrad3x3: %dx%dx%d, %d sources", B, H, W, nsrc);
@@ -1787,6 +1829,7 @@ int tc_wgrad3x3(const tc::ConvSrc* src, int nsrc, int B, int H, int W, const __n
     a.cin_out = cin_out;
     a.ch_valid = ch_valid;
     a.gw = gw;
+    a.gb = gb;
     a.err = err;
     int rc = RN_ERR_INVALID;
 #define RN_WGRAD_CASE(NV)                                                            \

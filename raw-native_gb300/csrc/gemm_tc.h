@@ -62,10 +62,11 @@ int tc_conv3x3(const tc::ConvSrc* src, int nsrc, int B, int H, int W, const __nv
 // k = tap * cin_out + ci, FP32 row stride N, added atomically (the caller zeroes gw). The
 // sources' channels are concatenated; cin_out and ch_valid: the weights' input channels and how
 // many of a chunk's stored channels they have (a padded input: cin_out = ch_valid < C; else
-// cin_out = sum of src[i].C and ch_valid = 0). dz NHWC BF16 [B][H][W][N], N 32, 64, 128 or 256;
+// cin_out = sum of src[i].C and ch_valid = 0). gb, where not null: gb[n] += sum over pixels of
+// dz[pixel][n], the bias gradient (zeroed by the caller too). dz NHWC BF16 [B][H][W][N], N 32, 64, 128 or 256;
 // each C a multiple of 16; H and W as conv_tiling takes them.
 int tc_wgrad3x3(const tc::ConvSrc* src, int nsrc, int B, int H, int W, const __nv_bfloat16* dz, int N, float* gw,
-                int cin_out, int ch_valid, uint32_t* err, cudaStream_t s, rn_status* st);
+                int cin_out, int ch_valid, float* gb, uint32_t* err, cudaStream_t s, rn_status* st);
 
 // C (M x N, row stride ldc) = P (M x K, row stride ldp) * Q (N x K, row stride ldq)^T.
 // M % 128 == 0, N in {32, 64, 128, 256} or a multiple of 128, K % (64 * splits) == 0;

@@ -170,7 +170,7 @@ __global__ void gate_kernel(const float* __restrict__ dout, const bf16* __restri
 // db[c] += sum over rows of dZ[m][c], C a multiple of 8 up to 256: a thread keeps the sums of
 // eight channels over every (blocks x 256 / (C / 8))-th row, 16 bytes a load, then the block
 // adds its rows up in shared memory. Bound by HBM: 67 MB (level 0, batch 64 of 128 x 128) in
-// 19 us; a thread a channel over 256 blocks took 2.2 ms.
+// 30 us, the 14 layers 0.25 ms; a thread a channel over 256 blocks took 9.5 ms.
 __global__ void __launch_bounds__(256) colsum_kernel(const bf16* __restrict__ dz, size_t M, int C, float* __restrict__ db) {
     const int G = C / 8, g = threadIdx.x % G, r = threadIdx.x / G, R = 256 / G;
     float s[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
@@ -358,41 +358,41 @@ __global__ void expand_w0_kernel(const bf16* __restrict__ wq, int kpad, bf16* __
 
 struct AdamArgs { float lr, b1, b2, eps, c1, c2; const float* scale; };
 
-// Adam on one convolution's weights (master [cout][kpad], gradient stored [kpad][cout],
-// multiplied by the clip factor *a.scale), then its BF16 copies: wq [cout][kpad] and the
-// flipped, transposed wt [cin_pad][kpad_t].
-__global__ void adam_conv_kernel(float* __restrict__ w, float* __restrict__ m, float* __restrict__ v,
-                                 const float* __restrict__ g, int cout, int cin, int kpad, int kpad_t, AdamArgs a,
-                                 bf16* __restrict__ wq, bf16* __restrict__ wt) {
-    const int total = cout * 9 * cin;
-    const float sc = g ? *a.scale : 0.0f;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
-        const int co = i / (9 * cin), k = i % (9 * cin);
-        const size_t wi = (size_t)co * kpad + k;
-        if (g) {
-            const float gr = g[(size_t)k * cout + co] * sc;
-            const float mm = a.b1 * m[wi] + (1.0f - a.b1) * gr;
-            const float vv = a.b2 * v[wi] + (1.0f - a.b2) * gr * gr;
-            m[wi] = mm;
-            v[wi] = vv;
-            w[wi] -= a.lr * (mm * a.c1) / (sqrtf(vv * a.c2) + a.eps);
+// Adam on every parameter array, blockIdx.y the array (a launch per array was 30 launches of 3 to
+// 10 us: 130 us, FIG now). The gradient is multiplied by the clip factor *a.scale (a.scale null:
+// no update, only the BF16 copies). An array of a convolution's weights (master [cout][kpad],
+// gradient stored [kpad][cout]) also gets its BF16 copies: wq [cout][kpad] and the flipped,
+// transposed wt [cin_pad][kpad_t]; a plain vector has wq null.
+struct AdamSeg {
+    float *w, *m, *v;
+    const float* g;
+    bf16 *wq, *wt;
+    int n;                       // values: cout x 9 cin, or the vector's length
+    int cout, cin, kpad, kpad_t;
+};
+__global__ void adam_kernel(const AdamSeg* __restrict__ segs, AdamArgs a) {
+    const AdamSeg sg = segs[blockIdx.y];
+    const float sc = a.scale ? *a.scale : 0.0f;
+    auto update = [&](size_t i, float grad) {
+        const float gr = grad * sc;
+        const float mm = a.b1 * sg.m[i] + (1.0f - a.b1) * gr;
+        const float vv = a.b2 * sg.v[i] + (1.0f - a.b2) * gr * gr;
+        sg.m[i] = mm;
+        sg.v[i] = vv;
+        return sg.w[i] -= a.lr * (mm * a.c1) / (sqrtf(vv * a.c2) + a.eps);
+    };
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < sg.n; i += gridDim.x * blockDim.x) {
+        if (!sg.wq) {
+            if (a.scale) update((size_t)i, sg.g[i]);
+            continue;
         }
-        const bf16 q = __float2bfloat16_rn(w[wi]);
-        wq[wi] = q;
-        const int tap = k / cin, ci = k % cin;
-        wt[(size_t)ci * kpad_t + (size_t)(8 - tap) * cout + co] = q;
+        const int co = i / (9 * sg.cin), k = i % (9 * sg.cin);
+        const size_t wi = (size_t)co * sg.kpad + k;
+        const bf16 q = __float2bfloat16_rn(a.scale ? update(wi, sg.g[(size_t)k * sg.cout + co]) : sg.w[wi]);
+        sg.wq[wi] = q;
+        const int tap = k / sg.cin, ci = k % sg.cin;
+        sg.wt[(size_t)ci * sg.kpad_t + (size_t)(8 - tap) * sg.cout + co] = q;
     }
-}
-__global__ void adam_vec_kernel(float* __restrict__ w, float* __restrict__ m, float* __restrict__ v,
-                                const float* __restrict__ g, int n, AdamArgs a) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float gr = g[i] * *a.scale;
-    const float mm = a.b1 * m[i] + (1.0f - a.b1) * gr;
-    const float vv = a.b2 * v[i] + (1.0f - a.b2) * gr * gr;
-    m[i] = mm;
-    v[i] = vv;
-    w[i] -= a.lr * (mm * a.c1) / (sqrtf(vv * a.c2) + a.eps);
 }
 
 // The squared global gradient norm: blockIdx.y picks one gradient array of the table.
@@ -676,6 +676,8 @@ struct rn_unet {
     float* host_loss;             // pinned: loss, gradient norm, clip scale
     float* gstats;                // device: see clip_kernel
     GradSeg* segs;                // device table of the gradient arrays
+    AdamSeg* adam;                // device table of the parameter arrays
+    int nadam = 0;
     int nsegs = 0;
     std::vector<GradSeg> hsegs;   // the same table on the host (flat gradient copies)
     float clip_ratio = 0.0f;
@@ -798,10 +800,10 @@ int conv_backward_implicit(rn_unet* u, int l, cudaStream_t s, rn_status* st) {
     const LayerSpec& sp = kSpec[l];
     const int H = u->H >> Ly.level, W = u->W >> Ly.level;
     const size_t M = pixels(u, Ly.level);
-    colsum_kernel<<<2 * ctx().sm_count, 256, 0, s>>>(u->dz, M, Ly.cout, Ly.gb);
     tc::ConvSrc src[2] = {{u->T[sp.s0.tensor], u->TC[sp.s0.tensor]}, {nullptr, 0}};
     if (sp.nsrc == 2) src[1] = {sp.s1.up ? u->UT[sp.s1.tensor] : u->T[sp.s1.tensor], u->TC[sp.s1.tensor]};
-    RN_TRY(tc_wgrad3x3(src, sp.nsrc, u->B, H, W, u->dz, Ly.cout, Ly.gw, Ly.cin, l == 0 ? kInC : 0, ctx().dev_error, s, st));
+    RN_TRY(tc_wgrad3x3(src, sp.nsrc, u->B, H, W, u->dz, Ly.cout, Ly.gw, Ly.cin, l == 0 ? kInC : 0, Ly.gb,
+                        ctx().dev_error, s, st));
     if (l == 0) return RN_OK;                          // the input needs no gradient
     const tc::ConvSrc dsrc{u->dz, Ly.cout};
     tc::Epilogue e{};
@@ -834,20 +836,10 @@ int conv_backward_implicit(rn_unet* u, int l, cudaStream_t s, rn_status* st) {
 }
 
 void refresh_weights(rn_unet* u, const AdamArgs* a, cudaStream_t s) {
-    for (int l = 0; l < kLayers; ++l) {
-        auto& Ly = u->L[l];
-        const int n = Ly.cout * 9 * Ly.cin;
-        adam_conv_kernel<<<(n + 255) / 256, 256, 0, s>>>(Ly.w, Ly.m, Ly.v, a ? Ly.gw : nullptr, Ly.cout, Ly.cin,
-                                                        Ly.kpad, Ly.kpad_t, a ? *a : AdamArgs{}, Ly.wq, Ly.wt);
-        if (a) adam_vec_kernel<<<(Ly.cout + 255) / 256, 256, 0, s>>>(Ly.b, Ly.bm, Ly.bv, Ly.gb, Ly.cout, *a);
-    }
+    adam_kernel<<<dim3(ctx().sm_count, u->nadam), 256, 0, s>>>(u->adam, a ? *a : AdamArgs{});
     if (u->wq0)
         expand_w0_kernel<<<(u->L[0].cout * 72 + 255) / 256, 256, 0, s>>>(u->L[0].wq, u->L[0].kpad, u->wq0, u->kpad0,
                                                                           u->L[0].cout, u->TC[T_IN]);
-    if (a) {
-        adam_vec_kernel<<<1, 32, 0, s>>>(u->wh, u->mh, u->vh, u->gwh, 32, *a);
-        adam_vec_kernel<<<1, 32, 0, s>>>(u->bh, u->mbh, u->vbh, u->gbh, 1, *a);
-    }
 }
 
 int check_shape(const rn_unet* u, int batch, rn_status* st) {
@@ -996,6 +988,17 @@ int rn_unet_create(int batch, int height, int width, uint64_t seed, uint32_t fla
         if (ualloc(u, (void**)&u->segs, segs.size() * sizeof(GradSeg), st)) return bail(RN_ERR_NO_MEMORY);
         if (cudaMemcpy(u->segs, segs.data(), segs.size() * sizeof(GradSeg), cudaMemcpyHostToDevice) != cudaSuccess)
             return bail(fail(st, RN_ERR_CUDA, "gradient table upload"));
+        std::vector<AdamSeg> adam;
+        for (auto& Ly : u->L) {
+            adam.push_back({Ly.w, Ly.m, Ly.v, Ly.gw, Ly.wq, Ly.wt, Ly.cout * 9 * Ly.cin, Ly.cout, Ly.cin, Ly.kpad, Ly.kpad_t});
+            adam.push_back({Ly.b, Ly.bm, Ly.bv, Ly.gb, nullptr, nullptr, Ly.cout, 0, 0, 0, 0});
+        }
+        adam.push_back({u->wh, u->mh, u->vh, u->gwh, nullptr, nullptr, 32, 0, 0, 0, 0});
+        adam.push_back({u->bh, u->mbh, u->vbh, u->gbh, nullptr, nullptr, 1, 0, 0, 0, 0});
+        u->nadam = (int)adam.size();
+        if (ualloc(u, (void**)&u->adam, adam.size() * sizeof(AdamSeg), st)) return bail(RN_ERR_NO_MEMORY);
+        if (cudaMemcpy(u->adam, adam.data(), adam.size() * sizeof(AdamSeg), cudaMemcpyHostToDevice) != cudaSuccess)
+            return bail(fail(st, RN_ERR_CUDA, "parameter table upload"));
     }
     refresh_weights(u, nullptr, ctx().stream);
     if (cudaStreamSynchronize(ctx().stream) != cudaSuccess) return bail(cuda_fail(st, cudaGetLastError(), "unet init"));
