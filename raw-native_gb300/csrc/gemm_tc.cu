@@ -288,12 +288,12 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const __grid_const
 // stride of the grid, keeping its barriers and TMEM across items. CB is the channel block of
 // one K step (64: 128-byte rows and swizzle; 32: 64-byte rows and swizzle); a K step is
 // (tap, source, channel block), taps outermost, matching the weights' column order
-// tap * Cin + ci. Roles (6 warps):
+// tap * Cin + ci. Roles (10 warps):
 //   - warp 0: TMA producer over all items' K steps, through a ring of kSt stages;
 //   - warp 1: MMA issuer (an elected lane); item i accumulates into TMEM buffer i & 1 (2 x BN columns),
 //     so the MMAs of item i + 1 run while the epilogue drains item i;
-//   - warps 2..5: epilogue; warp w reads TMEM lanes 32 (w % 4) .. +31 (its row quarter),
-//     then releases the buffer.
+//   - warps 2..9: epilogue, two sets of four; warp w reads TMEM lanes 32 (w % 4) .. +31 (its row
+//     quarter) of its set's columns, then releases the buffer.
 // Every wait is bounded and also gives up when another role has aborted.
 constexpr int kConvThreads = 192;
 
@@ -333,8 +333,11 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 template <int BN, int CB, int kT>
 __host__ __device__ constexpr int conv_stages() { return (CB == 32 ? 8 : 4) / (kT == 2 && BN <= 64 ? 2 : 1); }
 
+constexpr int kTapThreads = 320;                // two sets of four epilogue warps
+constexpr size_t kTapStage = 8 * 128 * 16;      // their stages
+
 template <int BN, int CB, int kT>
-__global__ void __launch_bounds__(kConvThreads, 1) tc_conv_kernel(const __grid_constant__ CUtensorMap map0,
+__global__ void __launch_bounds__(kTapThreads, 2) tc_conv_kernel(const __grid_constant__ CUtensorMap map0,
                                                                   const __grid_constant__ CUtensorMap map1,
                                                                   const __grid_constant__ CUtensorMap mapW,
                                                                   const ConvArgs a, const Epilogue e) {
@@ -345,10 +348,11 @@ __global__ void __launch_bounds__(kConvThreads, 1) tc_conv_kernel(const __grid_c
     constexpr uint32_t kCols = 2 * kT * BN;                  // two buffers of kT accumulators
     uint8_t* sA = smem;                                      // kSt stages of kT A boxes
     uint8_t* sB = smem + kSt * kT * kABytes;
-    uint64_t* bars = reinterpret_cast<uint64_t*>(sB + kSt * kBBytes);
+    uint4* s_stage = reinterpret_cast<uint4*>(sB + kSt * kBBytes);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sB + kSt * kBBytes + kTapStage);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kSt + 4);
     __shared__ int s_abort;
-    __shared__ float s_bias[512];       // the bias of every output channel, staged once
+    __shared__ __align__(16) float s_bias[512];       // the bias of every output channel, staged once
     volatile int* abort_flag = &s_abort;
     const int warp = warp_index(), lane = threadIdx.x & 31;
     const int tw = 1 << a.tw_log2, th = kBM >> a.tw_log2;
@@ -361,7 +365,7 @@ __global__ void __launch_bounds__(kConvThreads, 1) tc_conv_kernel(const __grid_c
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < kSt; ++s) { mbar_init(full(s), 1); mbar_init(empty(s), 1); }
-        for (int b = 0; b < 2; ++b) { mbar_init(acc_full(b), 1); mbar_init(acc_empty(b), 4); }
+        for (int b = 0; b < 2; ++b) { mbar_init(acc_full(b), 1); mbar_init(acc_empty(b), 8); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         s_abort = 0;
     }
@@ -450,9 +454,18 @@ __global__ void __launch_bounds__(kConvThreads, 1) tc_conv_kernel(const __grid_c
             s_abort = 1;
         }
     } else {
-        // epilogue warps 2..5: TMEM lane quarter q = warp % 4 holds rows 32 q .. 32 q + 31
-        const int q = warp & 3;
-        const int r = q * 32 + lane;
+        // epilogue warps 2..9: TMEM lane quarter q = warp % 4 holds rows 32 q .. 32 q + 31. An
+        // item's accumulators are units of 32 columns of a tile, the two sets of four warps taking
+        // them in turn. One set, 16 columns at a time and stored from there in 32-byte pieces, took
+        // longer than the MMAs: 128 -> 128 with its upsampled copy at 544 x 960 309 -> 170 us, 256 ->
+        // 256 at 272 x 480 177 -> 120, 64 -> 128 at 544 x 960 82 -> 68. A BF16
+        // output passes through the warp's stage, 32 pixels of 32 channels, and is stored in
+        // whole sectors: chunk c of pixel p at 4 p + (c ^ (p >> 1) % 4), clear of bank conflicts
+        // both ways.
+        const int q = warp & 3, set = (warp - 2) >> 2;
+        constexpr int kUnits = kT * BN / 32;
+        uint4* stage = s_stage + (warp - 2) * 128;
+        auto slot = [](int p, int c) { return p * 4 + (c ^ ((p >> 1) & 3)); };
         uint32_t i = 0;
         for (int item = blockIdx.x; item < a.items; item += gridDim.x, ++i) {
             const uint32_t buf = i & 1u, use = i >> 1;
@@ -464,70 +477,99 @@ __global__ void __launch_bounds__(kConvThreads, 1) tc_conv_kernel(const __grid_c
             tc_fence_after();
             const int group = item / a.n_slices, n0 = (item % a.n_slices) * BN;
 #pragma unroll 1
-            for (int t = 0; t < kT; ++t) {
-            const int tile = group * kT + t;
-            const int tx = tile % a.tiles_x, ty = (tile / a.tiles_x) % a.tiles_y, b = tile / (a.tiles_x * a.tiles_y);
-            const int y = ty * th + (r >> a.tw_log2), x = tx * tw + (r & (tw - 1));
-            const size_t pix = ((size_t)b * a.H + y) * a.W + x;
-            const uint32_t tbase = tmem + buf * kT * BN + (uint32_t)(t * BN) + ((uint32_t)(q * 32) << 16);
-            float hz = e.head_out ? e.head_b[0] : 0.0f;
-#pragma unroll 1
-            for (int c0 = 0; c0 < BN; c0 += 16) {
-                uint32_t v[16];
-                tmem_ld16(tbase + (uint32_t)c0, v);
-                float f[16];
-                const int col = n0 + c0;
-#pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    float t = __uint_as_float(v[j]);
-                    if (e.bias) t += s_bias[col + j];
-                    if (e.relu) t = fmaxf(t, 0.0f);
-                    f[j] = t;
+            for (int u = set; u < kUnits; u += 2) {
+                const int t = u / (BN / 32), col = n0 + u % (BN / 32) * 32;
+                const int tile = group * kT + t;
+                const int tx = tile % a.tiles_x, ty = (tile / a.tiles_x) % a.tiles_y, b = tile / (a.tiles_x * a.tiles_y);
+                uint32_t v[32];
+                tmem_ld32(tmem + buf * kT * BN + (uint32_t)(u * 32) + ((uint32_t)(q * 32) << 16), v);
+                if (u + 2 >= kUnits) {                        // this warp's last read of the buffer
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(acc_empty(buf));
                 }
-                if (e.head_out)
+                float f[32];
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) hz += __bfloat162float(__float2bfloat16_rn(f[j])) * e.head_w[col + j];
-                const size_t o = pix * e.ldc + col;
-                if (e.gate) {
-                    const uint4* g4 = reinterpret_cast<const uint4*>(e.gate + o);
+                for (int j = 0; j < 32; j += 4) {
+                    float4 bv = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    if (e.bias) bv = *reinterpret_cast<const float4*>(s_bias + col + j);
+                    const float bb[4] = {bv.x, bv.y, bv.z, bv.w};
 #pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        const uint4 gv = g4[h];
-                        const __nv_bfloat16* gb = reinterpret_cast<const __nv_bfloat16*>(&gv);
+                    for (int k = 0; k < 4; ++k) {
+                        float x = __uint_as_float(v[j + k]);
+                        if (e.bias) x += bb[k];
+                        if (e.relu) x = fmaxf(x, 0.0f);
+                        f[j + k] = x;
+                    }
+                }
+                // pixel p of the warp's quarter
+                auto at = [&](int p, int& y, int& x) {
+                    const int r = q * 32 + p;
+                    y = ty * th + (r >> a.tw_log2);
+                    x = tx * tw + (r & (tw - 1));
+                };
+                if (e.c32 || e.head_out) {
+                    int y, x;
+                    at(lane, y, x);
+                    const size_t pix = ((size_t)b * a.H + y) * a.W + x;
+                    if (e.head_out) {                         // N 32: the unit has every channel
+                        float hz = e.head_b[0];
 #pragma unroll
-                        for (int j = 0; j < 8; ++j)
-                            if (!(__bfloat162float(gb[j]) > 0.0f)) f[h * 8 + j] = 0.0f;
+                        for (int j = 0; j < 32; ++j) hz += __bfloat162float(__float2bfloat16_rn(f[j])) * e.head_w[j];
+                        e.head_out[pix] = 1.0f / (1.0f + __expf(-hz));
+                    }
+                    if (e.c32) {
+                        float4* d4 = reinterpret_cast<float4*>(e.c32 + pix * e.ldc + col);
+#pragma unroll
+                        for (int h = 0; h < 8; ++h) d4[h] = make_float4(f[4 * h], f[4 * h + 1], f[4 * h + 2], f[4 * h + 3]);
                     }
                 }
                 if (e.c16) {
-                    uint4 out[2];
-                    __nv_bfloat16* ob = reinterpret_cast<__nv_bfloat16*>(out);
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) ob[j] = __float2bfloat16_rn(f[j]);
-                    uint4* d4 = reinterpret_cast<uint4*>(e.c16 + o);
-                    d4[0] = out[0];
-                    d4[1] = out[1];
-                    if (a.up16) {
+                    for (int c = 0; c < 4; ++c) {
+                        uint4 o;
+                        uint32_t* ob = reinterpret_cast<uint32_t*>(&o);
 #pragma unroll
-                        for (int u = 0; u < 4; ++u) {
-                            const size_t up = ((size_t)b * 2 * a.H + 2 * y + (u >> 1)) * (2 * a.W) + 2 * x + (u & 1);
-                            uint4* d = reinterpret_cast<uint4*>(a.up16 + up * e.ldc + col);
-                            d[0] = out[0];
-                            d[1] = out[1];
+                        for (int h = 0; h < 4; ++h) {
+                            const __nv_bfloat162 o2 = __floats2bfloat162_rn(f[c * 8 + 2 * h], f[c * 8 + 2 * h + 1]);
+                            ob[h] = *reinterpret_cast<const uint32_t*>(&o2);
+                        }
+                        stage[slot(lane, c)] = o;
+                    }
+                    __syncwarp();
+                    const int c = lane & 3;
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        const int p = k * 8 + (lane >> 2);
+                        int y, x;
+                        at(p, y, x);
+                        uint4 o = stage[slot(p, c)];
+                        const size_t off = (((size_t)b * a.H + y) * a.W + x) * e.ldc + col + c * 8;
+                        if (e.gate) {                          // zero where the gate is not positive
+                            const uint4 gv = *reinterpret_cast<const uint4*>(e.gate + off);
+                            const uint32_t* g = reinterpret_cast<const uint32_t*>(&gv);
+                            uint32_t* ob = reinterpret_cast<uint32_t*>(&o);
+#pragma unroll
+                            for (int h = 0; h < 4; ++h)
+                                ob[h] &= __hgt2_mask(*reinterpret_cast<const __nv_bfloat162*>(g + h), __floats2bfloat162_rn(0.0f, 0.0f));
+                        }
+                        *reinterpret_cast<uint4*>(e.c16 + off) = o;
+                        if (a.up16) {                          // nearest 2x: four copies
+                            __nv_bfloat16* d = a.up16 + (((size_t)b * 2 * a.H + 2 * y) * (2 * a.W) + 2 * x) * e.ldc + col + c * 8;
+                            const size_t row = (size_t)2 * a.W * e.ldc;
+                            *reinterpret_cast<uint4*>(d) = o;
+                            *reinterpret_cast<uint4*>(d + e.ldc) = o;
+                            *reinterpret_cast<uint4*>(d + row) = o;
+                            *reinterpret_cast<uint4*>(d + row + e.ldc) = o;
                         }
                     }
-                }
-                if (e.c32) {
-                    float4* d4 = reinterpret_cast<float4*>(e.c32 + o);
-#pragma unroll
-                    for (int h = 0; h < 4; ++h) d4[h] = make_float4(f[4 * h], f[4 * h + 1], f[4 * h + 2], f[4 * h + 3]);
+                    __syncwarp();                              // the stage is free again
                 }
             }
-            if (e.head_out) e.head_out[pix] = 1.0f / (1.0f + __expf(-hz));
+            if (set >= kUnits) {                               // one unit: the second set has none
+                __syncwarp();
+                if (lane == 0) mbar_arrive(acc_empty(buf));
             }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(acc_empty(buf));
         }
     }
     tc_fence_before();
@@ -1484,7 +1526,7 @@ template <int BN, int CB, int kT>
 int launch_conv(const CUtensorMap& m0, const CUtensorMap& m1, const CUtensorMap& mw, const ConvArgs& a,
                 const Epilogue& e, cudaStream_t s) {
     constexpr int kSt = conv_stages<BN, CB, kT>();
-    const size_t smem = 1024 + kSt * (kT * kBM * CB * 2 + BN * CB * 2) + (2 * kSt + 4) * 8 + 16;
+    const size_t smem = 1024 + kSt * (kT * kBM * CB * 2 + BN * CB * 2) + kTapStage + (2 * kSt + 4) * 8 + 16;
     static int per_sm = 0;
     if (!per_sm) {
         if (cudaFuncSetAttribute(tc_conv_kernel<BN, CB, kT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
@@ -1493,14 +1535,14 @@ int launch_conv(const CUtensorMap& m0, const CUtensorMap& m1, const CUtensorMap&
                                  cudaSharedmemCarveoutMaxShared) != cudaSuccess)
             return RN_ERR_CUDA;
         // residency: shared memory (228 KB per SM, 1 KB reserved per CTA), TMEM (512 columns per
-        // SM, 2 x BN per CTA) and at most 3 CTAs of 192 threads and 88 registers
+        // SM, 2 x BN per CTA) and at most 2 CTAs of 320 threads and 96 registers
         int smem_sm = 0;
         cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, ctx().device);
         const int by_smem = smem_sm / (int)(smem + 1024);
-        per_sm = std::max(1, std::min(std::min(by_smem, 512 / (2 * kT * BN)), 3));
+        per_sm = std::max(1, std::min(std::min(by_smem, 512 / (2 * kT * BN)), 2));
     }
     const int ctas = std::min(a.items, per_sm * ctx().sm_count);
-    tc_conv_kernel<BN, CB, kT><<<ctas, kConvThreads, smem, s>>>(m0, m1, mw, a, e);
+    tc_conv_kernel<BN, CB, kT><<<ctas, kTapThreads, smem, s>>>(m0, m1, mw, a, e);
     return cudaGetLastError() == cudaSuccess ? RN_OK : RN_ERR_CUDA;
 }
 
@@ -1760,10 +1802,10 @@ int tc_conv3x3(const tc::ConvSrc* src, int nsrc, int B, int H, int W, const __nv
     const long tiles = (long)a.tiles_x * a.tiles_y * B;
     auto resident = [&](int kt) {
         const int st_n = (cb == 32 ? 8 : 4) / (kt == 2 && bn <= 64 ? 2 : 1);
-        const int smem = 1024 + st_n * (kt * tc::kBM * cb * 2 + bn * cb * 2) + (2 * st_n + 4) * 8 + 16;
+        const int smem = 1024 + st_n * (kt * tc::kBM * cb * 2 + bn * cb * 2) + (int)tc::kTapStage + (2 * st_n + 4) * 8 + 16;
         int smem_sm = 0;
         cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, ctx().device);
-        return std::min(std::min(smem_sm / (smem + 1024), 512 / (2 * kt * bn)), 3);
+        return std::min(std::min(smem_sm / (smem + 1024), 512 / (2 * kt * bn)), 2);
     };
     const bool pair = ctx().tune.conv_pair && tiles % 2 == 0 && bn <= 128 && resident(2) >= std::max(1, resident(1));
     a.items = (int)(tiles / (pair ? 2 : 1)) * a.n_slices;

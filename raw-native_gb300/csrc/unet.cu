@@ -359,7 +359,7 @@ __global__ void expand_w0_kernel(const bf16* __restrict__ wq, int kpad, bf16* __
 struct AdamArgs { float lr, b1, b2, eps, c1, c2; const float* scale; };
 
 // Adam on every parameter array, blockIdx.y the array (a launch per array was 30 launches of 3 to
-// 10 us: 130 us, FIG now). The gradient is multiplied by the clip factor *a.scale (a.scale null:
+// 10 us, 130 us; 43 us now). The gradient is multiplied by the clip factor *a.scale (a.scale null:
 // no update, only the BF16 copies). An array of a convolution's weights (master [cout][kpad],
 // gradient stored [kpad][cout]) also gets its BF16 copies: wq [cout][kpad] and the flipped,
 // transposed wt [cin_pad][kpad_t]; a plain vector has wq null.
