@@ -328,10 +328,11 @@ def run_ours(args):
         "gpu_launches": 2 * args.steps,
         "roofline": {"bound": "hbm", "kernel": "trace_kernel", "achieved": achieved, "peak": peak,
                      "unit": "GB/s", "frac": achieved / peak, "peak_source": peak_kind,
-                     "limit": "instruction issue: the algorithmic node/triangle bytes are served by L1/L2 "
-                              "(the BVH is cache-resident), so frac is cache-served node bandwidth against the "
-                              "HBM peak; dram_frac is the HBM share actually used, issue_active the binding limit's "
-                              "fraction",
+                     "limit": "instruction issue: the algorithmic node/triangle bytes are those of one walk a ray; "
+                              "most are never fetched (a ray that misses the boxes its packet shares in shared "
+                              "memory takes no walk) and L1/L2 serve the rest (the BVH is cache-resident), so frac "
+                              "can pass 1; dram_frac is the HBM share actually used, issue_active the binding "
+                              "limit's fraction",
                      "binding_limit": "instruction issue (ncu smsp__issue_active of the same kernel)",
                      "binding_frac": prof.get("issue_active"),
                      "dram_frac": (traffic / (trace_ms * 1e-3) / 1e9 / peak) if traffic else None,

@@ -876,6 +876,7 @@ int rn_render_frame(const rn_frame_scene* sc, const float* camera, const float* 
         PlocTree tree;
         cudaStream_t s;
         ~Build() {
+            if (tree.state) cudaStreamSynchronize(s);       // left early: its copies must not land in a later call
             if (acc && acc->d_nodes) cudaFreeAsync(acc->d_nodes, s);
             delete acc;
         }

@@ -1721,7 +1721,7 @@ int tc_conv3x3(const tc::ConvSrc* src, int nsrc, int B, int H, int W, const __nv
             if (!fan) {
                 // dynamic shared memory: 227 KB a block less the kernel's static arrays (the
                 // bias, the abort flag and the epilogue's BF16 stage of 4 x 32 pixels x N)
-                const size_t budget = 220 * 1024 - stat;
+                const size_t budget = 224 * 1024 - stat;
                 return (int)std::min<size_t>(8, (budget - std::min<size_t>(budget, b_pad + 2048)) / a_stride);
             }
             // fan-out: a slot is busy only until its own MMAs have run: four at most (4, 6 and 8
