@@ -963,6 +963,11 @@ __device__ __forceinline__ uint32_t wave_bounce(const PtParams& P, const WaveBuf
     return M_TRACE;
 }
 
+// Bound by the latency of the slots' state (DRAM 41 %, issue 39 % of cycles): everything a slot
+// needs is loaded in one round, the surface, lobe and evaluation are inlined, and the lobe is
+// evaluated for the sun's, the emitter's and the sampled direction by one copy of the code in a
+// loop. Lit room at 1920 x 1080, 4 samples: 32.2 -> 24.9 ms (out-of-line calls with their state
+// spilled before); 4, 6 or 8 blocks of 128 threads an SM 24.89 / 25.33 / 26.58 ms.
 template <int kMinBlocks>
 __global__ void __launch_bounds__(128, kMinBlocks) pt_wave_shade(const PtParams P, const WaveBufs W,
                                                                  unsigned long long total) {

