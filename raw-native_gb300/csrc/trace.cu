@@ -31,10 +31,10 @@ using namespace trace_dev;
 // fetches to counts[0..3] (hemisphere rays, nodes, tris, sky continuations); the outputs of
 // the other tiles are left unwritten. "Sky continuations" are the open hemisphere rays whose
 // walk went on past the radius: the same walk serves both queries.
-template <bool kCount, int kMinBlocks, int kStackN, bool kLeafPass>
+template <bool kCount, int kMinBlocks, int kStackN, bool kLeafPass, int kP>
 __global__ void __launch_bounds__(256, kMinBlocks) trace_kernel(const __grid_constant__ TraceParams p, uint32_t* tile_ctr,
                                                                 unsigned long long* counts, uint32_t stride) {
-    const int pl = p.packet_log2, tw = 1 << pl, th = 32 >> pl;
+    const int pl = kP == 0 ? p.packet_log2 : min(p.packet_log2, 5 - kP), tw = 1 << pl, th = (32 >> kP) >> pl;
     const int tiles_x = (p.w + tw - 1) >> pl, tiles_y = (p.h + th - 1) / th;
     const uint32_t ntiles = (uint32_t)tiles_x * tiles_y;
     const unsigned lane = threadIdx.x & 31u;
@@ -49,11 +49,12 @@ __global__ void __launch_bounds__(256, kMinBlocks) trace_kernel(const __grid_con
         if (lane == 0) tile = atomicAdd(tile_ctr, 1u);
         tile = __shfl_sync(0xffffffffu, tile, 0);
         if (tile >= ntiles) break;
-        const int x = ((int)(tile % tiles_x) << pl) + (int)(lane & (tw - 1));
-        const int y = (int)(tile / tiles_x) * th + (int)(lane >> pl);
+        const unsigned px = kP == 0 ? lane : lane & ((32u >> kP) - 1u);
+        const int x = ((int)(tile % tiles_x) << pl) + (int)(px & (tw - 1));
+        const int y = (int)(tile / tiles_x) * th + (int)(px >> pl);
         // no lane leaves the loop body early: the next tile fetch is a full-warp shuffle
         if (kCount && tile % stride != 0) continue;
-        trace_packet<kCount, kStackN, kLeafPass>(p, x, y, x < p.w && y < p.h, toLight, cn, skip, F);
+        trace_packet<kCount, kStackN, kLeafPass, kP>(p, x, y, x < p.w && y < p.h, toLight, cn, skip, F, (int)(lane >> (5 - kP)));
         __syncwarp();                              // the frontier is rebuilt for the next tile
     }
     if (kCount) {
@@ -366,10 +367,28 @@ int launch_ao_samples(const TraceParams& p, const uint32_t* list, const uint32_t
     return cudaGetLastError() == cudaSuccess ? RN_OK : RN_ERR_CUDA;
 }
 
+// Lanes a pixel's samples are shared by (log2). A frame of few packets a warp leaves the last
+// packets' samples, a pixel's one after the other, on few warps; with two or four lanes a pixel
+// the packets are smaller and as many times more. A packet's own work (its frontier, its pixels'
+// frames) is then done more often, which counts where walks are short: a small tree with the sky,
+// where most rays end in the sieve, or few samples a lane. Measured one / two / four lanes, us:
+// 512 x 512 x 64 (2.2 packets a warp) built-in scene with sky 199 / 168 / 184, without 157 / 107 /
+// 87, 146k triangles 3336 / 2693 / 2394 and 1542 / 932 / 782; 256 x 256 x 64 (0.6) 143 / 102 / 75
+// and 2581 / 1461 / 862; 1024 x 768 x 32 (6.7) 212 / 248 / 306, without sky 105 / 100 / 137, 146k
+// 3539 / 3379 / 3360 and 1095 / 937 / 1022; 1283 x 723 x 16 (8) 135 / 169, without 71 / 78, 146k
+// 2046 / 1942 and 633 / 652; 1920 x 1080 x 16 (18) 275 / 355, 146k 4060 / 4068 and 1087 / 1179.
+int lanes_log2(const TraceParams& p, long warps) {
+    const long tw = 1L << p.packet_log2, th = 32 >> p.packet_log2;
+    const double r = (double)(((p.w + tw - 1) / tw) * ((p.h + th - 1) / th)) / (double)warps;
+    const bool deep = p.stack_need >= kFrontier + 3 * 6;       // a tree of six levels and more
+    if (p.spp >= 32 && r < (p.want_sky && !deep ? 1.5 : 3.0)) return 2;
+    return p.spp >= 16 && r < (p.want_sky ? (deep ? 9.0 : 4.5) : (p.spp >= 32 ? 9.0 : 4.0)) ? 1 : 0;
+}
+
 // Residency variants: the register budget decides how many 256-thread blocks share an SM
 // (2: up to 128 registers, 3: 80, 4: 64, with spills to L1). The launch uses enough
 // blocks to fill every SM at that residency; ctx().tune.trace_min_blocks picks the variant.
-// Stack variants: 48 entries where the tree's bound (16 + 3 x wide depth) fits, else 96.
+// Stack variants: 48 entries where the tree's bound (24 + 3 x wide depth) fits, else 96.
 // The counting build (traversal statistics) always uses the 96-entry stack.
 template <int kMB, int kStackN>
 void launch_variant(const TraceParams& p, int sm_count, cudaStream_t s, uint32_t* tile_ctr, unsigned long long* counts,
@@ -377,13 +396,18 @@ void launch_variant(const TraceParams& p, int sm_count, cudaStream_t s, uint32_t
     const int blocks = sm_count * kMB;
     const int pool = ctx().tune.trace_pool;
     if (counts)
-        trace_kernel<true, kMB, kStack, false><<<blocks, 256, 0, s>>>(p, tile_ctr, counts, stride < 1 ? 1 : stride);
+        trace_kernel<true, kMB, kStack, false, 0><<<blocks, 256, 0, s>>>(p, tile_ctr, counts, stride < 1 ? 1 : stride);
     else if (pool > 0 && !p.want_sky)
         trace_ao_pool_kernel<kMB, kStackN><<<blocks, 256, 0, s>>>(p, tile_ctr, pool, ctx().tune.trace_pool_sort);
-    else if (ctx().tune.trace_leaf_pass)
-        trace_kernel<false, kMB, kStackN, true><<<blocks, 256, 0, s>>>(p, tile_ctr, nullptr, 1);
+    else if (ctx().tune.trace_leaf_pass) {
+        switch (lanes_log2(p, 8L * blocks)) {
+            case 2: trace_kernel<false, kMB, kStackN, true, 2><<<blocks, 256, 0, s>>>(p, tile_ctr, nullptr, 1); break;
+            case 1: trace_kernel<false, kMB, kStackN, true, 1><<<blocks, 256, 0, s>>>(p, tile_ctr, nullptr, 1); break;
+            default: trace_kernel<false, kMB, kStackN, true, 0><<<blocks, 256, 0, s>>>(p, tile_ctr, nullptr, 1);
+        }
+    }
     else
-        trace_kernel<false, kMB, kStackN, false><<<blocks, 256, 0, s>>>(p, tile_ctr, nullptr, 1);
+        trace_kernel<false, kMB, kStackN, false, 0><<<blocks, 256, 0, s>>>(p, tile_ctr, nullptr, 1);
 }
 
 template <int kStackN>

@@ -590,23 +590,29 @@ __device__ __forceinline__ bool walk_starts(const v3& o, const v3& d, float tmax
 // built-in scene at 3840 x 2160, 256 spp with sky 25.4 -> 18.9 ms with exact rays in the sieve,
 // 18.0 -> 13.2 with rough ones; views of 744k triangles within 1 % either way (thresholds of
 // 3/8, 5/8, 8/8: 22.0, 19.2 ms, and views 33.6 ms against 33.1).
+// With kP > 0 a packet is 32 >> kP pixels and 1 << kP lanes share each (`part`, the lane's high
+// bits): a part takes a run of the pixel's samples, part 0 the sun as well, and the counts are
+// added up at the end; integers, so the split changes no bit.
 constexpr int kChunk = 64, kSieveNum = 7, kSieveDen = 8, kSieveSkip = 15;
-template <bool kCount, int kStackN = kStack, bool kLeafPass = true>
+template <bool kCount, int kStackN = kStack, bool kLeafPass = true, int kP = 0>
 __device__ __forceinline__ void trace_packet(const TraceParams& p, int x, int y, bool valid, const v3& toLight,
-                                             Counts& cn, int& skip, Node4* F) {
+                                             Counts& cn, int& skip, Node4* F, int part = 0) {
+    const bool lead = kP == 0 || part == 0;        // writes the pixel
+    const int span = kP == 0 ? p.spp : (p.spp + (1 << kP) - 1) >> kP;      // a part's samples: first .. first + mine
+    const int sbase = kP == 0 ? 0 : part * span, mine = kP == 0 ? p.spp : max(0, min(span, p.spp - sbase));
     const float kFar = 1e30f;
     const size_t i = valid ? (size_t)y * p.w + x : 0;
     const uint8_t m = valid ? p.mask[i] : 0;
     v3 P = mk(0.0f, 0.0f, 0.0f), n = P;
     if (valid) { P = load3(p.pos + 3 * i); n = load3(p.nrm + 3 * i); }
-    if (valid && p.mirror) {
+    if (valid && p.mirror && lead) {
         const size_t np = (size_t)p.w * p.h;
         store3(mirror_pos(p.mirror, np) + 3 * i, P);
         store3(mirror_nrm(p.mirror, np) + 3 * i, n);
         mirror_mask(p.mirror, np)[i] = m;
         if (!m) mirror_ao(p.mirror, np)[i] = 1.0f;
     }
-    if (valid && !m) {
+    if (valid && !m && lead) {
         p.ao[i] = 1.0f;
         if (p.want_sky) { p.sky[i] = 1.0f; p.sun[i] = 1.0f; }
     }
@@ -618,7 +624,8 @@ __device__ __forceinline__ void trace_packet(const TraceParams& p, int x, int y,
     const v3 origin = add(P, scale(n, 1e-3f));
     const uint32_t ux = (uint32_t)x, uy = (uint32_t)y;
     const float tfar_h = p.want_sky ? kFar : p.radius;
-    const int slots = p.spp + ((p.want_sky && !p.sun_forced) ? 1 : 0);
+    const bool sun = p.want_sky && !p.sun_forced;
+    const int slots = span + (sun ? 1 : 0);
     // what the packet's rays can reach: AO-only walks start from the entries within the radius,
     // the sky's at the root, whose live children serve the sieve (the frontier is rebuilt for
     // every packet)
@@ -655,19 +662,27 @@ __device__ __forceinline__ void trace_packet(const TraceParams& p, int x, int y,
     };
     // nothing within reach: every hemisphere ray is open and free, only the sun ray is left
     const bool walks = p.has_geometry && fn >= 0;
-    const int first = walks ? 0 : p.spp;
+    const int first = walks ? 0 : span;
     if (!walks) {
-        open = freec = p.spp;
-        if (kCount && m) { cn.rays += p.spp; if (p.want_sky) cn.sky += p.spp; }
+        open = freec = mine;
+        if (kCount && m) { cn.rays += mine; if (p.want_sky) cn.sky += mine; }
     }
     for (int s0 = first; s0 < slots; s0 += kChunk) {
-        const int nslot = min(kChunk, slots - s0), nsamp = min(kChunk, p.spp - s0);
-        uint64_t todo = m ? (nslot == 64 ? ~0ull : (1ull << nslot) - 1ull) : 0ull;
+        const int nslot = min(kChunk, slots - s0), nsamp = min(kChunk, span - s0);
+        uint64_t todo = 0;
+        if (kP == 0) {
+            todo = m ? (nslot == 64 ? ~0ull : (1ull << nslot) - 1ull) : 0ull;
+        } else if (m) {
+            const int nb = min(kChunk, max(0, mine - s0));
+            todo = nb == 64 ? ~0ull : (1ull << nb) - 1ull;
+            if (lead && sun && span - s0 < kChunk) todo |= 1ull << (span - s0);
+        }
         if (sieve && nsamp > 0) {
             uint64_t keep = todo;
             if (m)
                 for (int k = 0; k < nsamp; ++k)
-                    if (!walk_starts(origin, rough_direction(t, b, n, ux, uy, (uint32_t)(s0 + k)), 1.1f * tfar_h, F, fn)) {
+                    if ((kP == 0 || s0 + k < mine) &&
+                        !walk_starts(origin, rough_direction(t, b, n, ux, uy, (uint32_t)(sbase + s0 + k)), 1.1f * tfar_h, F, fn)) {
                         keep &= ~(1ull << k);
                         ++open;
                         ++freec;
@@ -679,17 +694,17 @@ __device__ __forceinline__ void trace_packet(const TraceParams& p, int x, int y,
                 skip = kSieveSkip;
             }
         }
-        if (todo) fetch(s0 + __ffsll((long long)todo) - 1);
+        if (todo) fetch(sbase + s0 + __ffsll((long long)todo) - 1);
         while (todo) {
             const int s = s0 + __ffsll((long long)todo) - 1;
             todo &= todo - 1ull;
             v3 dir;
             float tn, tf;
-            if (s < p.spp) {
+            if (s < span) {
                 const uint32_t k2 = k2n;
                 const int cb = cbn;
-                if (todo) fetch(s0 + __ffsll((long long)todo) - 1);
-                dir = direction(s, k2, cb);
+                if (todo) fetch(sbase + s0 + __ffsll((long long)todo) - 1);
+                dir = direction(sbase + s, k2, cb);
                 tn = p.radius;
                 tf = tfar_h;
             } else {
@@ -697,12 +712,12 @@ __device__ __forceinline__ void trace_packet(const TraceParams& p, int x, int y,
                 tn = tf = kFar;
             }
             // AO-only walks may start from the warp's frontier; the sky and the sun need the root
-            const bool local = s < p.spp && tf == p.radius;
+            const bool local = s < span && tf == p.radius;
             const int h = p.has_geometry
                               ? walk<kCount, kStackN, kLeafPass>(p.nodes, p.tris, origin, dir, tn, tf, p.err_word, cn,
                                                                  local ? F : nullptr, local ? fn : 0)
                               : 0;
-            if (s < p.spp) {
+            if (s < span) {
                 if (kCount) { ++cn.rays; if (p.want_sky && !(h & HIT_NEAR)) ++cn.sky; }
                 if (!(h & HIT_NEAR)) {
                     ++open;
@@ -714,7 +729,12 @@ __device__ __forceinline__ void trace_packet(const TraceParams& p, int x, int y,
         }
         __syncwarp();
     }
-    if (!m) return;
+#pragma unroll
+    for (int o = 16; o >= 32 >> kP; o >>= 1) {     // the parts' counts
+        open += __shfl_xor_sync(0xffffffffu, open, o);
+        freec += __shfl_xor_sync(0xffffffffu, freec, o);
+    }
+    if (!m || !lead) return;
     p.ao[i] = fdiv((float)open, (float)p.spp);
     if (p.mirror) mirror_ao(p.mirror, (size_t)p.w * p.h)[i] = p.ao[i];
     if (p.want_sky) {

@@ -77,3 +77,34 @@ def test_sieve_chunks_against_the_scan(rn, oracle, spp):
     rao, rsky, rsun = oracle.trace(pos, nrm, mask, sc.tris, spp, 2.0, to_light=sc.to_light, threads=THREADS)
     assert np.array_equal(ao, rao) and np.array_equal(sky, rsky) and np.array_equal(sun, rsun)
     assert np.array_equal(rn.compute_rtao(g, acc, spp, 2.0), rao)
+
+
+@pytest.mark.parametrize("spp", [15, 16, 17, 31, 32, 33, 37, 65, 130, 257])
+@pytest.mark.parametrize("small", [True, False])
+def test_small_frames_share_a_pixels_samples(rn, oracle, small, spp):
+    """Frames of few packets give a pixel's samples to two lanes (from 16 samples) or four (from
+    32), a run each, the last one shorter, the sun ray with the first: the oracle's AO, sky and sun
+    bit for bit, on a small tree and a deeper one, in ragged frames and packets of 4, 8 and 16
+    columns."""
+    import scene as scenes
+    if small:
+        sc = scenes.build_test_scene()
+        cam = sc.camera
+    else:
+        sc = scenes.build_synthetic_scene(5, 60, 10, grid=20, half=8.0, subdiv=2)
+        cam = (6.0, 4.0, 5.0, 0.0, 0.5, 0.0, 0.0, 1.0, 0.0, 0.9)
+    tl = (0.3, 0.8, -0.5)
+    acc = rn.LinearAccel(sc.tris)
+    saved = rn.tune_get("trace_packet")
+    try:
+        for (w, h), packet in (((61, 43), 8), ((17, 9), 4), ((33, 3), 16)):
+            rn.tune_set("trace_packet", packet)
+            _, pos, nrm, mask = oracle.rasterize(sc.tris, sc.normals, cam, w, h)
+            g = rn.GBuffer(pos, nrm, mask)
+            want = oracle.trace(pos, nrm, mask, sc.tris, spp, 1.0, to_light=tl, threads=THREADS)
+            got = rn.compute_rt_visibility(g, acc, spp, 1.0, to_light=tl)
+            for a, b in zip(got, want):
+                assert np.array_equal(a, b), (w, h, int((a != b).sum()))
+            assert np.array_equal(rn.compute_rtao(g, acc, spp, 1.0), want[0])
+    finally:
+        rn.tune_set("trace_packet", saved)
