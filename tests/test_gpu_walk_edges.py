@@ -108,3 +108,31 @@ def test_small_frames_share_a_pixels_samples(rn, oracle, small, spp):
             assert np.array_equal(rn.compute_rtao(g, acc, spp, 1.0), want[0])
     finally:
         rn.tune_set("trace_packet", saved)
+
+
+@pytest.mark.parametrize("scale", [1.0, 1e-4, 1e5])
+@pytest.mark.parametrize("length", [1.0, 2e-3, 1e-3, 5e-4, 1e-25])
+def test_rays_along_axes_and_planes(rn, oracle, scale, length):
+    """Directions with one or two zero components (and of every size around the node test's line
+    for short ones) from origins on and off vertices' coordinates, over a soup of several levels at
+    three scales: closest and any-hit answers are the oracle's scans."""
+    rng = np.random.default_rng(7)
+    tris = (oracle.soup(3000, 11) * np.float32(scale)).astype(np.float32)
+    v = tris.reshape(-1, 3)
+    n = 3000
+    o = v[rng.integers(0, len(v), n)].copy()
+    off = rng.random((n, 3)) < 0.5
+    o[off] += (rng.normal(0, 2.0, (n, 3)) * scale).astype(np.float32)[off]
+    d = rng.normal(0, 1, (n, 3))
+    d[np.arange(n), rng.integers(0, 3, n)] = 0.0
+    two = rng.random(n) < 0.5
+    d[two, rng.integers(0, 3, n)[two]] = -0.0
+    d /= np.maximum(np.abs(d).max(1, keepdims=True), 1e-6)
+    rays = np.concatenate([o, d * length], 1).astype(np.float32)
+    tmax = np.where(rng.random(n) < 0.3, 3.0 * scale / length, 1e30).astype(np.float32)
+    acc = rn.LinearAccel(tris)
+    tri, t = rn.closest(acc, rays, tmax)
+    rtri, rt = oracle.closest_scan(tris, rays, tmax, threads=THREADS)
+    assert np.array_equal(tri, rtri), int((tri != rtri).sum())
+    assert np.array_equal(t, rt)
+    assert np.array_equal(rn.occluded(acc, rays, tmax) != 0, oracle.occluded_scan(tris, rays, tmax, threads=THREADS) != 0)
