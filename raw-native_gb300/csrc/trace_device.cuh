@@ -28,33 +28,16 @@ __device__ __forceinline__ float rcp_approx(float x) {
 // ray straight along an axis visits every node (a sample whose u is exactly zero is the normal
 // itself, one in 2^24: 12 ms of one warp over 146k triangles, 800 x 600 x 64 samples 14.9 -> 4.2 ms,
 // 1280 x 720 x 64 16.8 -> 7.3). At 1e27 a plane's distance says on which side of it the origin
-// lies, its rounding 2^-24 |o| of position, inside the boxes' padding; a component below 1e-27
-// moves the ray by less than that over any distance the others leave in the scene.
-__device__ __forceinline__ float inv_clamped(float x) { return fminf(fmaxf(rcp_approx(x), -1e27f), 1e27f); }
+// lies, its rounding 2^-24 |o| of position, inside the boxes' padding, as long as o * inv is finite
+// (|o| up to kFarOrigin; refine_axis beyond); a component below 1e-27 moves the ray by less than
+// that over any distance the others leave in the scene.
+constexpr float kInvMax = 1e27f, kFarOrigin = 3e11f;
+__device__ __forceinline__ float inv_clamped(float x) { return fminf(fmaxf(rcp_approx(x), -kInvMax), kInvMax); }
 // For any direction: a component below 1e-28 that is not zero gives NaN, so that its axis
 // constrains nothing: with its reciprocal one of plane * inv and o * inv could overflow alone
 // and cull a box that the ray enters.
 __device__ __forceinline__ float safe_inv(float x) {
     return fabsf(x) < 1e-28f && x != 0.0f ? __int_as_float(0x7fffffff) : rcp_approx(x);
-}
-
-// The ray's inverse direction, origin x inverse direction, and the byte offset of each axis's
-// near plane in a node (nx, ny, nz: the lo plane for a direction that is not negative, else
-// the hi plane 16 bytes further; the far plane sits at the other of the two), formed once
-// per walk.
-struct Inv { float x, y, z, ox, oy, oz; uint32_t nx, ny, nz; };
-template <bool kUnit = false>        // kUnit: the direction is about of unit length
-__device__ __forceinline__ Inv make_inv(const v3& o, const v3& d) {
-    Inv r;
-    r.x = inv_clamped(d.x); r.y = inv_clamped(d.y); r.z = inv_clamped(d.z);
-    if (!kUnit && !(fmaxf(fmaxf(fabsf(d.x), fabsf(d.y)), fabsf(d.z)) >= 1e-3f)) {
-        r.x = safe_inv(d.x); r.y = safe_inv(d.y); r.z = safe_inv(d.z);
-    }
-    r.ox = o.x * r.x; r.oy = o.y * r.y; r.oz = o.z * r.z;
-    r.nx = (__float_as_uint(r.x) >> 31) * 16u;
-    r.ny = 32u + (__float_as_uint(r.y) >> 31) * 16u;
-    r.nz = 64u + (__float_as_uint(r.z) >> 31) * 16u;
-    return r;
 }
 
 // Three-input maximum and minimum (one instruction each on sm_100 and later); a NaN operand
@@ -67,6 +50,38 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
 __device__ __forceinline__ float min3(float a, float b, float c) {
     float r;
     asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+
+// The ray's inverse direction, origin x inverse direction, and the byte offset of each axis's
+// near plane in a node (nx, ny, nz: the lo plane for a direction that is not negative, else
+// the hi plane 16 bytes further; the far plane sits at the other of the two), formed once
+// per walk.
+struct Inv { float x, y, z, ox, oy, oz; uint32_t nx, ny, nz; };
+// One axis of a ray with a short direction or a far origin. An infinite o * inv of finite
+// factors would put both planes of every box at the same infinity and cull the boxes that
+// the ray enters: NaN instead, and the axis constrains nothing.
+__device__ __forceinline__ void refine_axis(float o, float d, bool is_short, float& inv, float& oi) {
+    if (is_short) { inv = safe_inv(d); oi = o * inv; }
+    if (isinf(oi) && !isinf(o) && !isinf(inv)) inv = oi = __int_as_float(0x7fffffff);
+}
+// kUnit: the direction is about of unit length and the origin not far.
+template <bool kUnit = false>
+__device__ __forceinline__ Inv make_inv(const v3& o, const v3& d) {
+    Inv r;
+    r.x = inv_clamped(d.x); r.y = inv_clamped(d.y); r.z = inv_clamped(d.z);
+    r.ox = o.x * r.x; r.oy = o.y * r.y; r.oz = o.z * r.z;
+    if (!kUnit) {
+        const bool is_short = !(max3(fabsf(d.x), fabsf(d.y), fabsf(d.z)) >= 1e-3f);
+        if (is_short || max3(fabsf(o.x), fabsf(o.y), fabsf(o.z)) > kFarOrigin) {
+            refine_axis(o.x, d.x, is_short, r.x, r.ox);
+            refine_axis(o.y, d.y, is_short, r.y, r.oy);
+            refine_axis(o.z, d.z, is_short, r.z, r.oz);
+        }
+    }
+    r.nx = (__float_as_uint(r.x) >> 31) * 16u;
+    r.ny = 32u + (__float_as_uint(r.y) >> 31) * 16u;
+    r.nz = 64u + (__float_as_uint(r.z) >> 31) * 16u;
     return r;
 }
 
@@ -648,9 +663,10 @@ __device__ __forceinline__ void trace_packet(const TraceParams& p, int x, int y,
         const TilePlane pl = tile_plane(n, origin, m != 0, covered);
         const TileBox tb = tile_box(origin, m != 0);
         fn = p.want_sky ? root_frontier(p.nodes, pl, F) : tile_frontier(p, tb, pl, F);
-        // the sieve needs normals of about unit length (its rough rays are not normalized)
+        // the sieve needs normals of about unit length (its rough rays are not normalized) and
+        // no far origin
         const float n2 = n.x * n.x + n.y * n.y + n.z * n.z;
-        sieve = !kCount && fn > 0 && skip == 0 && __all_sync(0xffffffffu, !m || (n2 > 0.9f && n2 < 1.1f));
+        sieve = !kCount && fn > 0 && skip == 0 && tb.mag <= kFarOrigin && __all_sync(0xffffffffu, !m || (n2 > 0.9f && n2 < 1.1f));
         if (!kCount && fn > 0 && skip > 0) --skip;
         if (sieve) grow_entries(F, fn, tb);
     }

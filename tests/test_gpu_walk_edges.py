@@ -136,3 +136,52 @@ def test_rays_along_axes_and_planes(rn, oracle, scale, length):
     assert np.array_equal(tri, rtri), int((tri != rtri).sum())
     assert np.array_equal(t, rt)
     assert np.array_equal(rn.occluded(acc, rays, tmax) != 0, oracle.occluded_scan(tris, rays, tmax, threads=THREADS) != 0)
+
+
+@pytest.mark.parametrize("log2", [34, 40, 42])
+@pytest.mark.parametrize("length", [1.0, 5e-4])
+def test_rays_along_axes_far_from_the_origin(rn, oracle, log2, length):
+    """The same at coordinates of 2e11 to 6e13, where a coordinate times the reciprocal of a zero
+    component leaves float's range. The scales are powers of two: the vertices stay exact."""
+    scale = np.float32(2.0 ** log2)
+    rng = np.random.default_rng(9)
+    tris = oracle.soup(2000, 12) * scale
+    n = 3000
+    o = tris.reshape(-1, 3)[rng.integers(0, 3 * len(tris), n)].copy()
+    off = rng.random((n, 3)) < 0.5
+    o[off] += (rng.normal(0, 2.0, (n, 3)) * scale).astype(np.float32)[off]
+    d = rng.normal(0, 1, (n, 3))
+    d[np.arange(n), rng.integers(0, 3, n)] = 0.0
+    two = rng.random(n) < 0.5
+    d[two, rng.integers(0, 3, n)[two]] = -0.0
+    d /= np.maximum(np.abs(d).max(1, keepdims=True), 1e-6)
+    rays = np.concatenate([o, d * length], 1).astype(np.float32)
+    tmax = np.where(rng.random(n) < 0.3, 3.0 * scale / length, 1e30).astype(np.float32)
+    acc = rn.LinearAccel(tris)
+    tri, t = rn.closest(acc, rays, tmax)
+    rtri, rt = oracle.closest_scan(tris, rays, tmax, threads=THREADS)
+    assert (rtri >= 0).sum() > n // 20
+    assert np.array_equal(tri, rtri), int((tri != rtri).sum())
+    assert np.array_equal(t, rt)
+    assert np.array_equal(rn.occluded(acc, rays, tmax) != 0, oracle.occluded_scan(tris, rays, tmax, threads=THREADS) != 0)
+
+
+@pytest.mark.parametrize("log2", [34, 40])
+def test_frame_far_from_the_origin(rn, oracle, log2):
+    """AO, sky and a sun with a zero component over the built-in scene at such coordinates: the
+    oracle's planes bit for bit. The positions lie 1/16 off the surface: on it the rounding of t alone
+    decides whether a ray hits its own triangle."""
+    import scene as scenes
+    sc = scenes.build_test_scene()
+    _, pos, nrm, mask = oracle.rasterize(sc.tris, sc.normals, sc.camera, 61, 43)
+    scale = np.float32(2.0 ** log2)
+    tris, pos = sc.tris * scale, (pos + nrm / 16) * scale
+    acc = rn.LinearAccel(tris)
+    g = rn.GBuffer(pos, nrm, mask)
+    for sun in ((0.9, 0.5, 0.0), (0.0, 0.5, 0.9)):
+        want = oracle.trace(pos, nrm, mask, tris, 65, 2.0 * scale, to_light=sun, accel="scan", threads=THREADS)
+        assert (want[2][mask != 0] == 0).sum() > 10
+        got = rn.compute_rt_visibility(g, acc, 65, 2.0 * scale, to_light=sun)
+        for a, b in zip(got, want):
+            assert np.array_equal(a, b), int((a != b).sum())
+    assert np.array_equal(rn.compute_rtao(g, acc, 65, 2.0 * scale), want[0])
