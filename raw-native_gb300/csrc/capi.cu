@@ -214,7 +214,7 @@ int trace_ao_device(const float* pos, const float* nrm, const uint8_t* mask, int
 void apply_tune(TraceParams& p, const rn_accel* accel) {
     const Tune& t = ctx().tune;
     p.frontier = t.trace_frontier && p.spp >= t.trace_frontier_min_spp;
-    p.stack_need = kFrontier + 3 * (int)(accel ? accel->depth : 0);
+    p.stack_need = stack_need(accel ? accel->depth : 0);
     // the frontier's seeds sit under the walk's own pushes: without room for both, walk from the root
     if (p.stack_need > 96) p.frontier = 0;
     p.packet_log2 = packet_log2(t.trace_packet);

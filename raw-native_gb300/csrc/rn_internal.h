@@ -171,6 +171,12 @@ int ssao_blocks(int w, int h);
 // 24 / 32: six views of 744k triangles 26.98 / 26.42 / 26.24 / 26.17 / 26.94 ms, 3840 x 2160 x 256
 // spp over the built-in scene - / 13.22 / 13.09 / 13.08 / 13.26.
 constexpr int kFrontier = 24;
+// Stack entries a walk can hold on a tree of `depth` levels of wide nodes when it starts from a
+// frontier: the other entries, then at most three children of each node that it descends from. The
+// frontier's nodes lie on the second level or below, and a node of the last level has no interior
+// child, so depth - 2 levels push. From the root it is 3 (depth - 1), always less.
+constexpr int stack_need(uint32_t depth) { return kFrontier - 1 + 3 * ((int)depth - 2); }
+
 
 // A 4-wide BVH node: six 4-float planes of child boxes (SoA) then the 4 child words and
 // per-node metadata. 128 bytes, 16-byte aligned for vector loads. Child word >= 0: index of
@@ -257,7 +263,7 @@ struct TraceParams {
     int frontier;         // AO-only walks start from a per-warp frontier (0: from the root)
     int packet_log2;      // log2 of the packet width (pixels per warp row): 2, 3 or 4
     int frontier_tail;    // greedy single-entry steps after the breadth-first frontier build
-    int stack_need;       // entries the walk can push on this tree: the frontier + 3 x wide depth
+    int stack_need;       // entries the walk can push on this tree (rn::stack_need)
     // copy-through of a G-buffer read from host memory (null: none): every pixel's position,
     // normal, AO and mask are also written to a device buffer laid out as
     // [position w*h*12 B][normal w*h*12 B][ao w*h*4 B][mask w*h B] (mirror_* below)

@@ -380,7 +380,7 @@ int launch_ao_samples(const TraceParams& p, const uint32_t* list, const uint32_t
 int lanes_log2(const TraceParams& p, long warps) {
     const long tw = 1L << p.packet_log2, th = 32 >> p.packet_log2;
     const double r = (double)(((p.w + tw - 1) / tw) * ((p.h + th - 1) / th)) / (double)warps;
-    const bool deep = p.stack_need >= kFrontier + 3 * 6;       // a tree of six levels and more
+    const bool deep = p.stack_need >= stack_need(6);           // a tree of six levels and more
     if (p.spp >= 32 && r < (p.want_sky && !deep ? 1.5 : 3.0)) return 2;
     return p.spp >= 16 && r < (p.want_sky ? (deep ? 9.0 : 4.5) : (p.spp >= 32 ? 9.0 : 4.0)) ? 1 : 0;
 }
@@ -388,7 +388,7 @@ int lanes_log2(const TraceParams& p, long warps) {
 // Residency variants: the register budget decides how many 256-thread blocks share an SM
 // (2: up to 128 registers, 3: 80, 4: 64, with spills to L1). The launch uses enough
 // blocks to fill every SM at that residency; ctx().tune.trace_min_blocks picks the variant.
-// Stack variants: 48 entries where the tree's bound (24 + 3 x wide depth) fits, else 96.
+// Stack variants: 48 entries where the tree's bound (17 + 3 x wide depth) fits, else 96.
 // The counting build (traversal statistics) always uses the 96-entry stack.
 template <int kMB, int kStackN>
 void launch_variant(const TraceParams& p, int sm_count, cudaStream_t s, uint32_t* tile_ctr, unsigned long long* counts,

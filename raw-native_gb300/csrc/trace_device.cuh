@@ -340,7 +340,7 @@ __device__ int walk(const Node4* __restrict__ nodes, const LeafTri* __restrict__
     bool wr_ready = false;
     float tmax = tfar;
     int far_hit = 0;
-    int32_t stack[kStackN];
+    int32_t stack[kStackN + 3];          // past kStackN: what the node that passes it pushes
     int sp = 0;
     int32_t cur = 0;                     // the root is always node 0
     // the triangles of leaf word c: true when one is hit nearer than tnear (the walk ends)
@@ -409,9 +409,10 @@ __device__ int walk(const Node4* __restrict__ nodes, const LeafTri* __restrict__
         bool hit[4];
         int32_t CH[4];
         node_test(reinterpret_cast<const char*>(nodes + cur), LdGlobal(), iv, tmax, CH, tn, hit);
-        // a node stacks at most three of its children (the build refuses trees whose depth
-        // could need more than the stack holds)
-        if (sp + 3 > kStackN) { atomicOr(err, DEV_STACK_OVERFLOW); return far_hit; }
+        // a node stacks at most three of its children, one of the last level none: a walk within
+        // stack_need may visit a node with the stack full (the build refuses trees whose depth
+        // could need more)
+        if (sp > kStackN) { atomicOr(err, DEV_STACK_OVERFLOW); return far_hit; }
         nearest = -1;
         tbest = 3.0e38f;
         if (visit(CH, tn, hit)) return HIT_NEAR | HIT_FAR;

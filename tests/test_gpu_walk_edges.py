@@ -185,3 +185,51 @@ def test_frame_far_from_the_origin(rn, oracle, log2):
         for a, b in zip(got, want):
             assert np.array_equal(a, b), int((a != b).sum())
     assert np.array_equal(rn.compute_rtao(g, acc, 65, 2.0 * scale), want[0])
+
+
+def _chain(n):
+    """Triangles around the origin, each 1.5 times as large as the last: a tree of one interior child a
+    node, n / 3 levels deep."""
+    s = 1.5 ** (np.arange(n) - n + 5.0)
+    tris = np.zeros((n, 3, 3))
+    for k in range(3):
+        tris[:, k, k] = s
+    return tris.reshape(n, 9).astype(np.float32)
+
+
+@pytest.mark.parametrize("n", [24, 30, 33, 60, 75, 78, 80, 81, 90])
+def test_deep_trees_trace_from_the_frontier(rn, oracle, n):
+    """Trees of 8 to 30 levels, around the depths at which the frontier's entries and the walk's own
+    no longer fit into stacks of 48 (past 10 levels) and 96 (past 26, where walks start at the
+    root): the oracle's scan bit for bit, and fewer node visits than from the root wherever the
+    frontier runs."""
+    tris = _chain(n)
+    rng = np.random.default_rng(n)
+    h, w = 13, 29
+    pos = (rng.uniform(0.6, 1.0, (h, w, 1)) * np.ones(3) * 1.5 ** 4).astype(np.float32)
+    nrm = np.full((h, w, 3), -1 / np.sqrt(3), np.float32)
+    mask = np.ones((h, w), np.uint8)
+    g = rn.GBuffer(pos, nrm, mask)
+    acc = rn.LinearAccel(tris)
+    keys = ("trace_stack", "trace_frontier", "trace_frontier_min_spp", "trace_pool")
+    saved = {k: rn.tune_get(k) for k in keys}
+    try:
+        rn.tune_set("trace_frontier_min_spp", 1)
+        for radius in (0.5, 3.0):
+            want = oracle.trace(pos, nrm, mask, tris, 15, radius, accel="scan", threads=THREADS)
+            nodes = {}
+            for stack in (48, 96):
+                for frontier in (0, 1):
+                    for pool in (0, 24):
+                        rn.tune_set("trace_stack", stack)
+                        rn.tune_set("trace_frontier", frontier)
+                        rn.tune_set("trace_pool", pool)
+                        assert np.array_equal(rn.compute_rtao(g, acc, 15, radius), want), (stack, frontier, pool)
+                    nodes[frontier] = rn.trace_stats(g, acc, 15, radius)["nodes"]
+            if n <= 80:
+                assert nodes[1] < nodes[0], nodes
+            else:
+                assert nodes[1] == nodes[0], nodes
+    finally:
+        for k, v in saved.items():
+            rn.tune_set(k, v)
