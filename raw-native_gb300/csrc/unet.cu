@@ -441,7 +441,7 @@ constexpr int kDepthBlocks = 512;
 // the last block to finish adds the partials, also in a fixed order, and divides (0 without
 // covered pixels). A thread's 60-odd pixels of a 4K frame are a chain of loads unless several
 // are in flight: eight at a time (4K: 60 us and a 39 us one-thread pass over the partials before,
-// 25 us now).
+// 46 us now, bound by the conversions and additions in FP64).
 __global__ void __launch_bounds__(256) depth_mean_kernel(const float* __restrict__ depth, const uint8_t* __restrict__ mask,
                                                          size_t n, double* part_sum, unsigned* part_cnt, unsigned* ticket,
                                                          float* __restrict__ mean) {
@@ -458,18 +458,12 @@ __global__ void __launch_bounds__(256) depth_mean_kernel(const float* __restrict
             m[k] = i < n && mask[i];
             d[k] = i < n ? depth[i] : 0.0f;
         }
-        // their sum as a float pair (two-sum: what a sum loses goes into lo), then two FP64 additions
-        // instead of eight: FP64 issues at two a clock and SM here
-        float hi = 0.0f, lo = 0.0f;
 #pragma unroll
         for (int k = 0; k < kAhead; ++k)
             if (m[k]) {
-                const float t = __fadd_rn(hi, d[k]), b = __fsub_rn(t, hi);
-                lo = __fadd_rn(lo, __fadd_rn(__fsub_rn(hi, __fsub_rn(t, b)), __fsub_rn(d[k], b)));
-                hi = t;
+                s += (double)d[k];
                 ++c;
             }
-        s += (double)hi + (double)lo;
     }
     __shared__ double ss[8];
     __shared__ unsigned sc[8];

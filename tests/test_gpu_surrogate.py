@@ -100,3 +100,19 @@ def test_trained_surrogate_gains_over_the_method_without_it(rn):
         assert r["sur"] < 0.6 * r["blur"], r
         assert r["sur"] < r["rt64"], r
         assert r["fb"] < 0.05, r
+
+
+@pytest.mark.parametrize("value", [1.0, 3.0e38, float("inf")])
+def test_mean_depth_is_a_64_bit_mean(rn, value):
+    """The mean of the covered pixels' depth is their FP64 mean rounded once, also where a few depths
+    add up to more than the largest float, or to an infinity."""
+    import numpy as np
+    import torch
+    w, h = 640, 352                # several pixels a thread
+    g, depth, acc = _frame(rn, 900124, w, h)
+    m = g.mask.bool()
+    rng = torch.Generator(device="cuda").manual_seed(3)
+    d = value * (1.0 - 2e-3 * torch.rand(h, w, device="cuda", generator=rng)) if value > 1 else depth
+    _, st = rn.surrogate_ao(_net(rn, h, w), g, d.contiguous(), acc, 32)
+    want = np.float32(d[m].double().mean().item())
+    assert np.float32(st["mean_depth"]) == want, (st["mean_depth"], want)
