@@ -329,19 +329,28 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 // A boxes per stage, two TMEM accumulators per buffer), halving the weights' L2 traffic;
 // each tile's MMAs are the same in the same order.
 // Pipeline stages of tc_conv_kernel: 8 of 32 channels or 4 of 64; pairs of tiles with a
-// 64-column or narrower slice take half as many, so that two CTAs still share an SM.
-template <int BN, int CB, int kT>
-__host__ __device__ constexpr int conv_stages() { return (CB == 32 ? 8 : 4) / (kT == 2 && BN <= 64 ? 2 : 1); }
+// 64-column or narrower slice take half as many and single tiles with 64 columns one less, so that
+// two CTAs still share an SM beside the epilogue's stage (96 -> 64 at 136 x 976, single tiles of 32
+// channels: 8 stages and one CTA 49.6 us, 7 and two 31.2).
+__host__ __device__ constexpr int conv_stages(int bn, int cb, int kt) {
+    const int full = cb == 32 ? 8 : 4;
+    return kt == 2 && bn <= 64 ? full / 2 : bn == 64 ? full - 1 : full;
+}
 
 constexpr int kTapThreads = 320;                // two sets of four epilogue warps
 constexpr size_t kTapStage = 8 * 128 * 16;      // their stages
+constexpr size_t kTapStatic = 2048 + 64;        // static shared memory: the bias, the abort flag
+__host__ __device__ constexpr size_t conv_smem(int bn, int cb, int kt) {
+    const int n = conv_stages(bn, cb, kt);
+    return 1024 + (size_t)n * (kt * kBM * cb * 2 + bn * cb * 2) + kTapStage + (2 * n + 4) * 8 + 16;
+}
 
 template <int BN, int CB, int kT>
 __global__ void __launch_bounds__(kTapThreads, 2) tc_conv_kernel(const __grid_constant__ CUtensorMap map0,
                                                                   const __grid_constant__ CUtensorMap map1,
                                                                   const __grid_constant__ CUtensorMap mapW,
                                                                   const ConvArgs a, const Epilogue e) {
-    constexpr int kSt = conv_stages<BN, CB, kT>();
+    constexpr int kSt = conv_stages(BN, CB, kT);
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     constexpr uint32_t kABytes = kBM * CB * 2, kBBytes = BN * CB * 2;
@@ -1525,8 +1534,7 @@ int launch_wgrad(const CUtensorMap& m0, const CUtensorMap& m1, const CUtensorMap
 template <int BN, int CB, int kT>
 int launch_conv(const CUtensorMap& m0, const CUtensorMap& m1, const CUtensorMap& mw, const ConvArgs& a,
                 const Epilogue& e, cudaStream_t s) {
-    constexpr int kSt = conv_stages<BN, CB, kT>();
-    const size_t smem = 1024 + kSt * (kT * kBM * CB * 2 + BN * CB * 2) + kTapStage + (2 * kSt + 4) * 8 + 16;
+    constexpr size_t smem = conv_smem(BN, CB, kT);
     static int per_sm = 0;
     if (!per_sm) {
         if (cudaFuncSetAttribute(tc_conv_kernel<BN, CB, kT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
@@ -1538,7 +1546,7 @@ int launch_conv(const CUtensorMap& m0, const CUtensorMap& m1, const CUtensorMap&
         // SM, 2 x BN per CTA) and at most 2 CTAs of 320 threads and 96 registers
         int smem_sm = 0;
         cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, ctx().device);
-        const int by_smem = smem_sm / (int)(smem + 1024);
+        const int by_smem = smem_sm / (int)(smem + kTapStatic + 1024);
         per_sm = std::max(1, std::min(std::min(by_smem, 512 / (2 * kT * BN)), 2));
     }
     const int ctas = std::min(a.items, per_sm * ctx().sm_count);
@@ -1801,11 +1809,9 @@ int tc_conv3x3(const tc::ConvSrc* src, int nsrc, int B, int H, int W, const __nv
     // the doubled A stages keep as many CTAs per SM as single tiles do
     const long tiles = (long)a.tiles_x * a.tiles_y * B;
     auto resident = [&](int kt) {
-        const int st_n = (cb == 32 ? 8 : 4) / (kt == 2 && bn <= 64 ? 2 : 1);
-        const int smem = 1024 + st_n * (kt * tc::kBM * cb * 2 + bn * cb * 2) + (int)tc::kTapStage + (2 * st_n + 4) * 8 + 16;
         int smem_sm = 0;
         cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, ctx().device);
-        return std::min(std::min(smem_sm / (smem + 1024), 512 / (2 * kt * bn)), 2);
+        return std::min(std::min(smem_sm / (int)(tc::conv_smem(bn, cb, kt) + tc::kTapStatic + 1024), 512 / (2 * kt * bn)), 2);
     };
     const bool pair = ctx().tune.conv_pair && tiles % 2 == 0 && bn <= 128 && resident(2) >= std::max(1, resident(1));
     a.items = (int)(tiles / (pair ? 2 : 1)) * a.n_slices;

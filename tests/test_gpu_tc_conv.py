@@ -220,3 +220,23 @@ def test_conv_row_tiles_over_channel_chunks(rn, B, H, W, c0, c1, N):
             assert torch.equal(a, b)
     finally:
         rn.tune_set("conv_fan", saved)
+
+
+@pytest.mark.parametrize("B,H,W,c0,c1,N", [(1, 24, 48, 96, 0, 64), (3, 8, 16, 128, 0, 64), (1, 8, 16, 32, 32, 64),
+                                            (2, 8, 16, 64, 0, 64), (1, 16, 24, 192, 64, 64)])
+def test_conv_tiles_of_64_output_channels(rn, B, H, W, c0, c1, N):
+    """The per-tap kernel with 64 output channels: single tiles (an odd count of them), whose ring is
+    one stage shorter than a power of two, and pairs, over K loops of 9 to 72 steps."""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(5 * B + H + W + c0 + c1)
+    x0 = torch.randn(B, H, W, c0, device="cuda", generator=g).to(torch.bfloat16)
+    x1 = torch.randn(B, H, W, c1, device="cuda", generator=g).to(torch.bfloat16) if c1 else None
+    cin = c0 + c1
+    w = (torch.randn(N, 9 * cin, device="cuda", generator=g) / (9 * cin) ** 0.5).to(torch.bfloat16)
+    bias = torch.randn(N, device="cuda", generator=g)
+    out = rn.tc_conv3x3(x0, w, x1, bias=bias)
+    ref = _ref(x0, x1, w, bias, False)
+    assert (out - ref).abs().max().item() <= 1e-3 * ref.abs().max().item()
+    o, u = rn.tc_conv3x3(x0, w, x1, bias=bias, upsampled=True)
+    assert torch.equal(o, out.to(torch.bfloat16))
+    assert torch.equal(u, o.repeat_interleave(2, 1).repeat_interleave(2, 2))
