@@ -20,6 +20,7 @@
 #include <cuda_bf16.h>
 #include <algorithm>
 #include <mutex>
+#include <type_traits>
 
 namespace rn {
 namespace tc {
@@ -595,16 +596,18 @@ __global__ void __launch_bounds__(kTapThreads, 2) tc_conv_kernel(const __grid_co
 // each as ONE TMA box per source holding 136 pixels (x0 - 1 .. x0 + 134) of every input
 // channel, into a ring of row slots. Output row y reads the slots of rows y - 1, y, y + 1
 // in place, each tap's A operand starting one pixel further along its row: every input row
-// crosses from L2 once per chunk instead of three times. A source's row lies in the slot as
-// chunks of 64, 32 or 16 channels (the widest that divides its channel count), each a K-major
-// tile of 136 pixel rows of 128, 64 or 32 bytes with the swizzle of that width: one box per
-// chunk, and a tap's shift moves the operand's start by one pixel row, the swizzle following
-// the address.
+// crosses from L2 once per chunk instead of three times. A row in its slot:
+// - fan-out form: a source lies as chunks of 64, 32 or 16 channels (the widest that divides its
+//   channel count), each a K-major tile of 136 pixel rows of 128, 64 or 32 bytes with the swizzle
+//   of that width: one box per chunk, and a tap's shift moves the operand's start by one pixel
+//   row, the swizzle following the address;
+// - row by row: without swizzle, a 136 x 16-byte group per 8 channels, the groups of all sources one
+//   after the other (one box per source), so that one loop takes any channel count: a tap's shift is
+//   16 bytes and a K16 step two groups (48 -> 32 at 272 x 1920 50 us, on swizzled chunks 114).
 // The weights are loaded once per CTA, in the no-swizzle K-major canonical form: 8 rows x 16
 // bytes per core matrix, core matrices 128 bytes apart along N and one channel group (N x 16
 // bytes) apart along K. K order (tap outermost, then channel) and the K16 steps are
-// tc_conv_kernel's, so the two kernels give identical results. Rows whose A operands go on to
-// TMEM (kTA) stay in the no-swizzle form, a 136 x 16-byte group per 8 channels.
+// tc_conv_kernel's, so the two kernels give identical results.
 constexpr int kHaloW = 136;                        // box width: 128 + 2 halo, rounded for alignment
 constexpr uint32_t kHaloGroup = kHaloW * 16;       // bytes of one 8-channel group of a row slot
 
@@ -664,7 +667,9 @@ constexpr uint32_t kTaRowCols = 3 * 2 * 8;         // taps x K steps (at most 32
 
 struct HaloArgs {
     int nsrc, C0, C1, cin;
-    int cb0, cb1;               // the sources' channel chunks in a row slot (64, 32 or 16)
+    int cb0, cb1;               // fan-out: the width of the sources' channel chunks in a row slot (64, 32 or 16)
+    int nch0, nch1;             // and their number (nch1: 0 with one source)
+    int q16;                    // K16 steps of a tap
     int B, H, W;
     int chunk, chunks_y;        // output rows per work item; items per strip column
     int items;                  // n_slices x slice_items
@@ -727,7 +732,8 @@ constexpr int kFanThreads = 320;    // two sets of epilogue warps
 // branch costs as much as an MMA, so a tap's steps are straight line and the three shifts loop
 // around them. Measured at 2176 x 3840, 16 -> 32 channels / 32 + 64 -> 32, and at 1088 x 1920,
 // 64 + 128 -> 64: loops over chunks and steps 184 / 615 / 446 us, all shifts unrolled
-// 145 / 422 / 375, this 144 / 408 / 354.
+// 145 / 422 / 375, this 144 / 408 / 354. They take the channel counts of the U-Net's layers whose
+// weights fit; any other runs loops over its chunks, straight line within one (fan_chunks).
 struct FanRow {
     uint64_t a0, a1;            // the sources' descriptors at the row's first pixel
     uint64_t b0, b1;            // B at each piece's first row
@@ -761,9 +767,39 @@ __device__ __forceinline__ void fan_row(const FanRow& f) {
     else run(false);
 }
 
+// The same for any channel counts: one source's chunks of one tap, the chunk's width fixed in each
+// of three loops (at 272 x 1920 48 -> 32 channels 36.2 us with one loop of a run-time width, 29.1 so, 112
+// -> 64 94.9 and 67.3, 16 + 112 -> 32 101.7 and 62.6). Moves b0 and b1 past the source's steps.
+template <int BN>
+__device__ __forceinline__ void fan_chunks(const FanRow& f, uint64_t a, int cb, int chunks, bool split, uint64_t& b0,
+                                           uint64_t& b1) {
+    constexpr uint32_t kStepB = 2u * 3u * BN;                               // the next 16 channels of B
+    auto steps = [&](auto width) {
+        constexpr int kW = decltype(width)::value;
+#pragma unroll
+        for (int k = 0; k < kW / 16; ++k) {
+            tc_mma(f.acc0, desc_add(a, 2u * k), desc_add(b0, k * kStepB), f.id0, 1u);
+            if (split) tc_mma(f.acc1, desc_add(a, 2u * k), desc_add(b1, k * kStepB), f.id1, 1u);
+        }
+        a = desc_add(a, kHaloW * (kW >> 3));
+        b0 = desc_add(b0, kW / 16 * kStepB);
+        b1 = desc_add(b1, kW / 16 * kStepB);
+    };
+    if (cb == 64) {
+#pragma unroll 1
+        for (int c = 0; c < chunks; ++c) steps(std::integral_constant<int, 64>());
+    } else if (cb == 32) {
+#pragma unroll 2
+        for (int c = 0; c < chunks; ++c) steps(std::integral_constant<int, 32>());
+    } else {
+#pragma unroll 4
+        for (int c = 0; c < chunks; ++c) steps(std::integral_constant<int, 16>());
+    }
+}
+
 // Bytes of one row slot (C1: 0 with one source).
-__host__ __device__ constexpr uint32_t halo_slot(int C0, int C1, bool ta) {
-    return ta ? ((uint32_t)(C0 + C1) * 2u * kHaloW + 1023u) & ~1023u
+__host__ __device__ constexpr uint32_t halo_slot(int C0, int C1, bool fan) {
+    return !fan ? ((uint32_t)(C0 + C1) * 2u * kHaloW + 1023u) & ~1023u
               : (((uint32_t)C0 * 2u * kHaloW + 1023u) & ~1023u) + (((uint32_t)C1 * 2u * kHaloW + 1023u) & ~1023u);
 }
 
@@ -785,9 +821,9 @@ __global__ void __launch_bounds__(kFan ? kFanThreads : kConvThreads, kFan && !kW
     const int kSt = a.stages;
     uint8_t* sB = smem;
     uint8_t* sA = smem + ((a.b_bytes + 1023) & ~1023u);
-    const uint32_t a_stride = halo_slot(a.C0, a.C1, kTA);
-    // full[kSt], empty[kSt], acc_full[8], acc_empty[8], w (weights landed), wfree (the weights'
-    // last MMAs done: a slice's weights may be replaced)
+    const uint32_t a_stride = halo_slot(a.C0, a.C1, kFan);
+    // full[kSt], empty[kSt], acc_full[kFanMaxAcc], acc_empty[kFanMaxAcc], w (weights landed), wfree
+    // (the weights' last MMAs done: a slice's weights may be replaced)
     uint4* s_stage = reinterpret_cast<uint4*>(sA + kSt * a_stride);
     uint64_t* bars = reinterpret_cast<uint64_t*>(sA + kSt * a_stride + halo_stage(BN, a.sets));
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kSt + 2 * kFanMaxAcc + 2);
@@ -825,24 +861,8 @@ __global__ void __launch_bounds__(kFan ? kFanThreads : kConvThreads, kFan && !kW
     tc_fence_after();
     const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     // the second source's place in a row slot (the swizzled tiles start on 1024 bytes)
-    const uint32_t src1_off = kTA ? (uint32_t)(a.C0 / 8) * kHaloGroup : ((uint32_t)a.C0 * 2u * kHaloW + 1023u) & ~1023u;
-    const int nch0 = kTA ? 0 : a.C0 / a.cb0, nch1 = kTA || a.nsrc < 2 ? 0 : a.C1 / a.cb1;
-    // the K16 steps of the tap dx pixels along a row, in channel order: mma(A's descriptor);
-    // da0, da1: the sources' descriptors at the row's first pixel
-    auto each_step = [&](uint64_t da0, uint64_t da1, int dx, auto&& mma) {
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            const int cb = i ? a.cb1 : a.cb0;
-            uint64_t da = (i ? da1 : da0) + (uint64_t)(dx * (cb >> 3));       // one pixel: 2 cb bytes
-            for (int c = i ? nch1 : nch0; c > 0; --c) {
-                for (int k = 0; k < cb; k += 16) {
-                    mma(da);
-                    da += 2;                                                  // 16 channels: 32 bytes
-                }
-                da += (uint64_t)((kHaloW - 1) * (cb >> 3));                   // the next chunk's tile
-            }
-        }
-    };
+    const uint32_t src1_off = !kFan ? (uint32_t)(a.C0 / 8) * kHaloGroup : ((uint32_t)a.C0 * 2u * kHaloW + 1023u) & ~1023u;
+    constexpr uint32_t kStepA = (2u * kHaloGroup) >> 4;               // row by row: the next 16 channels of A
     if (kFan) {
         // fan-out accumulators start at zero and every MMA adds to them: each epilogue warp
         // clears its lane quarter of the ring now and of each row again once it has read it
@@ -890,14 +910,14 @@ __global__ void __launch_bounds__(kFan ? kFanThreads : kConvThreads, kFan && !kW
                     }
                     mbar_expect_tx(full(s), a.a_bytes);
                     const uint32_t dst = smem_u32(sA + s * a_stride);
-                    if (kTA) {
+                    if (!kFan) {
                         tma_load_5d(dst, &map0, 0, it.tx * 128 - 1, it.y0 + r, it.b, 0, full(s));
                         if (a.nsrc > 1) tma_load_5d(dst + src1_off, &map1, 0, it.tx * 128 - 1, it.y0 + r, it.b, 0, full(s));
                     } else {
-                        for (int c = 0; c < nch0; ++c)
+                        for (int c = 0; c < a.nch0; ++c)
                             tma_load_4d(dst + (uint32_t)(c * a.cb0 * 2 * kHaloW), &map0, c * a.cb0, it.tx * 128 - 1, it.y0 + r,
                                         it.b, full(s));
-                        for (int c = 0; c < nch1; ++c)
+                        for (int c = 0; c < a.nch1; ++c)
                             tma_load_4d(dst + src1_off + (uint32_t)(c * a.cb1 * 2 * kHaloW), &map1, c * a.cb1,
                                         it.tx * 128 - 1, it.y0 + r, it.b, full(s));
                     }
@@ -909,11 +929,8 @@ __global__ void __launch_bounds__(kFan ? kFanThreads : kConvThreads, kFan && !kW
             mbar_wait(wbar, wfree_ph);      // the last weights load (one more than the reloads)
         }
     } else if (warp == 1 && kFan) {
-        const int G = a.cin / 8;
         const uint32_t b_grp = 3u * BN * 16u;                         // next channel group of B (LBO)
         const uint64_t db0 = desc_plain(smem_u32(sB), b_grp, 128);
-        const uint64_t dq_b = (2u * b_grp) >> 4;                      // the next 16 channels of B
-        const uint64_t dx_b = ((uint32_t)G * b_grp) >> 4;             // the next horizontal tap of B
         bool ok = __all_sync(0xffffffffu, mbar_wait_or_abort(wbar, 0, abort_flag));
         int wslice = (int)blockIdx.x % a.n_slices;
         uint32_t w_ph = 0;
@@ -953,10 +970,7 @@ __global__ void __launch_bounds__(kFan ? kFanThreads : kConvThreads, kFan && !kW
                 ok = __all_sync(0xffffffffu, mbar_wait_or_abort(full(slot), phase, abort_flag));
                 if (!ok) break;
                 tc_fence_after();
-                const uint64_t da0 = desc_rows(row_smem, a.cb0), da1 = desc_rows(row_smem + src1_off, a.cb1);
-                // the channel counts of the U-Net's layers whose weights fit; any other runs the
-                // general loops
-                const FanRow fr{da0, da1, b0, b1, acc0, acc1, id0, id1, n1 != 0};
+                const FanRow fr{desc_rows(row_smem, a.cb0), desc_rows(row_smem + src1_off, a.cb1), b0, b1, acc0, acc1, id0, id1, n1 != 0};
                 if (a.C0 == 32 && a.C1 == 0) fan_row<BN, 32, 0>(fr);
                 else if (a.C0 == 16 && a.C1 == 0) fan_row<BN, 16, 0>(fr);
                 else if (a.C0 == 64 && a.C1 == 0) fan_row<BN, 64, 0>(fr);
@@ -964,15 +978,16 @@ __global__ void __launch_bounds__(kFan ? kFanThreads : kConvThreads, kFan && !kW
                 else if (a.C0 == 32 && a.C1 == 64) fan_row<BN, 32, 64>(fr);
                 else if (a.C0 == 64 && a.C1 == 128) fan_row<BN, 64, 128>(fr);
                 else {
+                    auto run = [&](bool split) {
+                        uint64_t d0 = b0, d1 = b1;                    // the taps lie one after the other
 #pragma unroll 1
-                    for (int dx = 0; dx < 3; ++dx) {
-                        uint64_t db = (uint64_t)dx * dx_b;
-                        each_step(da0, da1, dx, [&](uint64_t da) {
-                            tc_mma(acc0, da, b0 + db, id0, 1u);
-                            if (n1) tc_mma(acc1, da, b1 + db, id1, 1u);
-                            db += dq_b;
-                        });
-                    }
+                        for (uint32_t dx = 0; dx < 3; ++dx) {
+                            fan_chunks<BN>(fr, desc_add(fr.a0, dx * (uint32_t)(a.cb0 >> 3)), a.cb0, a.nch0, split, d0, d1);
+                            if (a.nch1) fan_chunks<BN>(fr, desc_add(fr.a1, dx * (uint32_t)(a.cb1 >> 3)), a.cb1, a.nch1, split, d0, d1);
+                        }
+                    };
+                    if (n1) run(true);
+                    else run(false);
                 }
                 // the row slot is free once its MMAs have read it; output row k - 2 is complete
                 tc_commit(empty(slot));
@@ -995,7 +1010,7 @@ __global__ void __launch_bounds__(kFan ? kFanThreads : kConvThreads, kFan && !kW
     } else if (warp == 1 && kTA) {
         const uint32_t idesc = instr_desc(BN);
         const uint32_t b0 = smem_u32(sB);
-        const int q16 = a.cin / 16, g_tap = a.cin / 8;
+        const int g_tap = a.cin / 8;
         const uint32_t ta0 = tmem + 2u * BN;
         bool ok = __all_sync(0xffffffffu, mbar_wait_or_abort(wbar, 0, abort_flag));
         uint32_t base = 0, i = 0;   // ring index of the item's first load; output rows so far
@@ -1020,8 +1035,8 @@ __global__ void __launch_bounds__(kFan ? kFanThreads : kConvThreads, kFan && !kW
                     const uint32_t row = smem_u32(sA + (k % kSt) * a_stride);
                     const uint32_t slot = ta0 + (k % kTaSlots) * kTaRowCols;
                     for (int dx = 0; dx < 3; ++dx)
-                        for (int q = 0; q < q16; ++q)
-                            tc_cp_128x256b(slot + (uint32_t)(dx * q16 + q) * 8u,
+                        for (int q = 0; q < a.q16; ++q)
+                            tc_cp_128x256b(slot + (uint32_t)(dx * a.q16 + q) * 8u,
                                            desc_plain(row + (uint32_t)dx * 16u + (uint32_t)(2 * q) * kHaloGroup,
                                                       kHaloGroup, 128));
                     // the shared-memory slot is free once its copies have run
@@ -1031,8 +1046,8 @@ __global__ void __launch_bounds__(kFan ? kFanThreads : kConvThreads, kFan && !kW
                 const uint32_t acc = tmem + buf * BN;
                 for (int t = 0; t < 9; ++t) {
                     const uint32_t k = base + (uint32_t)(j + t / 3);
-                    const uint32_t slot = ta0 + (k % kTaSlots) * kTaRowCols + (uint32_t)((t % 3) * q16) * 8u;
-                    for (int q = 0; q < q16; ++q) {
+                    const uint32_t slot = ta0 + (k % kTaSlots) * kTaRowCols + (uint32_t)((t % 3) * a.q16) * 8u;
+                    for (int q = 0; q < a.q16; ++q) {
                         const uint64_t db = desc_plain(b0 + (uint32_t)(t * g_tap + 2 * q) * (BN * 16), BN * 16, 128);
                         tc_mma_ta(acc, slot + (uint32_t)q * 8u, db, idesc, (t | q) != 0 ? 1u : 0u);
                     }
@@ -1050,8 +1065,8 @@ __global__ void __launch_bounds__(kFan ? kFanThreads : kConvThreads, kFan && !kW
         const uint32_t idesc = instr_desc(BN);
         const int g_tap = a.cin / 8;
         const uint64_t db0 = desc_plain(smem_u32(sB), BN * 16, 128);
-        const uint64_t dq_b = (2u * BN * 16u) >> 4;                   // the next 16 channels of B
-        const uint64_t dtap_b = ((uint32_t)g_tap * BN * 16u) >> 4;    // the next tap of B
+        const uint32_t dq_b = (2u * BN * 16u) >> 4;                   // the next 16 channels of B
+        const uint32_t dtap_b = ((uint32_t)g_tap * BN * 16u) >> 4;    // the next tap of B
         bool ok = __all_sync(0xffffffffu, mbar_wait_or_abort(wbar, 0, abort_flag));
         uint32_t base = 0, i = 0;   // ring index of the item's first load; output rows so far
         for (int item = blockIdx.x; ok && item < a.items; item += gridDim.x) {
@@ -1077,14 +1092,15 @@ __global__ void __launch_bounds__(kFan ? kFanThreads : kConvThreads, kFan && !kW
                 uint32_t add = 0;
 #pragma unroll
                 for (int t = 0; t < 9; ++t) {
-                    const uint32_t row = row_addr[t / 3];
-                    uint64_t db = db_tap;
-                    each_step(desc_rows(row, a.cb0), desc_rows(row + src1_off, a.cb1), t % 3, [&](uint64_t da) {
+                    uint64_t da = desc_plain(row_addr[t / 3] + (uint32_t)(t % 3) * 16u, kHaloGroup, 128), db = db_tap;
+#pragma unroll 4
+                    for (int q = 0; q < a.q16; ++q) {
                         tc_mma(acc, da, db, idesc, add);
                         add = 1u;
-                        db += dq_b;
-                    });
-                    db_tap += dtap_b;
+                        da = desc_add(da, kStepA);
+                        db = desc_add(db, dq_b);
+                    }
+                    db_tap = desc_add(db_tap, dtap_b);
                 }
                 tc_commit(acc_full(buf));
                 // load j (input row y0 + j - 1) has no later reader
@@ -1555,7 +1571,7 @@ int launch_conv(const CUtensorMap& m0, const CUtensorMap& m1, const CUtensorMap&
 }
 
 
-// The row box of one source for kTA: a 5-D view of the NHWC tensor, (8 channels, W, H, B, C / 8
+// The row box of one source without swizzle: a 5-D view of the NHWC tensor, (8 channels, W, H, B, C / 8
 // groups), read in boxes of 8 x 136 x 1 x 1 x C/8 without swizzle (the channel groups
 // outermost in shared memory).
 bool make_map_halo(CUtensorMap* m, const void* base, int B, int H, int W, int C) {
@@ -1716,8 +1732,8 @@ int tc_conv3x3(const tc::ConvSrc* src, int nsrc, int B, int H, int W, const __nv
     if ((ctx().tune.conv_halo || !all32) && ring_shape && (one_slice || (fan && N % 32 == 0 && N <= 512))) {
         const uint32_t a_bytes = (uint32_t)cin / 8 * tc::kHaloGroup;
         // a row slot; two swizzled sources each start on 1024 bytes
-        const uint32_t a_stride = tc::halo_slot(src[0].C, nsrc > 1 ? src[1].C : 0, ta);
-        auto chunk = [](int C) { return C % 64 == 0 ? 64 : C % 32 == 0 ? 32 : 16; };
+        const uint32_t a_stride = tc::halo_slot(src[0].C, nsrc > 1 ? src[1].C : 0, fan);
+        auto chunk = [](int C) { return tc::chunk_channels(C); };
         const size_t bars = (size_t)(2 * 8 + 2 * tc::kFanMaxAcc + 2) * 8 + 16;
         int bn = one_slice && (N == 32 || !fan || ctx().tune.conv_fan_bn == 64) ? N : 32, stages = 0;
         uint32_t b_bytes = 0, b_pad = 0;
@@ -1729,7 +1745,7 @@ int tc_conv3x3(const tc::ConvSrc* src, int nsrc, int B, int H, int W, const __nv
             if (!fan) {
                 // dynamic shared memory: 227 KB a block less the kernel's static arrays (the
                 // bias, the abort flag and the epilogue's BF16 stage of 4 x 32 pixels x N)
-                const size_t budget = 224 * 1024 - stat;
+                const size_t budget = 220 * 1024 - stat;
                 return (int)std::min<size_t>(8, (budget - std::min<size_t>(budget, b_pad + 2048)) / a_stride);
             }
             // fan-out: a slot is busy only until its own MMAs have run: four at most (4, 6 and 8
@@ -1752,14 +1768,16 @@ int tc_conv3x3(const tc::ConvSrc* src, int nsrc, int B, int H, int W, const __nv
         CUtensorMap hm[2], hw;
         bool maps = stages >= (fan ? 2 : 4) && (fan || one_slice);
         for (int i = 0; maps && i < nsrc; ++i)
-            maps = ta ? tc::make_map_halo(&hm[i], src[i].ptr, B, H, W, src[i].C)
-                      : tc::make_map_nhwc(&hm[i], src[i].ptr, B, H, W, src[i].C, tc::kHaloW, 1, chunk(src[i].C));
+            maps = fan ? tc::make_map_nhwc(&hm[i], src[i].ptr, B, H, W, src[i].C, tc::kHaloW, 1, chunk(src[i].C))
+                       : tc::make_map_halo(&hm[i], src[i].ptr, B, H, W, src[i].C);
         if (maps && nsrc == 1) hm[1] = hm[0];
         maps = maps && (fan ? tc::make_map_wfan(&hw, w, N, ldw, cin, bn) : tc::make_map_wgroups(&hw, w, N, ldw, 9 * cin / 8));
         if (maps) {
             tc::HaloArgs h{};
             h.nsrc = nsrc; h.C0 = src[0].C; h.C1 = nsrc > 1 ? src[1].C : 0; h.cin = cin;
             h.cb0 = chunk(src[0].C); h.cb1 = nsrc > 1 ? chunk(src[1].C) : 16;
+            h.nch0 = src[0].C / h.cb0; h.nch1 = nsrc > 1 ? src[1].C / h.cb1 : 0;
+            h.q16 = cin / 16;
             h.B = B; h.H = H; h.W = W;
             // chunks of 16 output rows (2 halo rows re-read per chunk), fewer where that leaves
             // less than two items per SM

@@ -240,3 +240,39 @@ def test_conv_tiles_of_64_output_channels(rn, B, H, W, c0, c1, N):
     o, u = rn.tc_conv3x3(x0, w, x1, bias=bias, upsampled=True)
     assert torch.equal(o, out.to(torch.bfloat16))
     assert torch.equal(u, o.repeat_interleave(2, 1).repeat_interleave(2, 2))
+
+
+@pytest.mark.parametrize("B,H,W,c0,c1,N", [(1, 18, 128, 48, 0, 32), (2, 5, 256, 80, 0, 64), (1, 9, 128, 112, 0, 64),
+                                            (1, 7, 128, 144, 0, 32), (1, 6, 384, 160, 0, 32), (1, 17, 128, 96, 0, 32),
+                                            (1, 4, 128, 192, 0, 64), (1, 8, 128, 16, 112, 32), (1, 3, 256, 112, 16, 64),
+                                            (2, 6, 128, 48, 96, 32), (1, 11, 128, 64, 64, 64), (1, 5, 128, 32, 16, 128)])
+def test_conv_general_channel_counts(rn, B, H, W, c0, c1, N):
+    """Row tiles with channel counts that have no straight-line steps: one to nine chunks of 16, 32 or
+    64 channels a source (the loops' remainders), against the FP32 convolution; and bit for bit
+    against the row-by-row form or the per-tap kernel where one of them takes the shape. What the
+    row-by-row form refuses of 16-channel sources stays refused."""
+    import torch
+    saved = rn.tune_get("conv_fan")
+    try:
+        g = torch.Generator(device="cuda").manual_seed(B + 3 * H + W + 5 * c0 + c1 + N)
+        x0 = torch.randn(B, H, W, c0, device="cuda", generator=g).to(torch.bfloat16)
+        x1 = torch.randn(B, H, W, c1, device="cuda", generator=g).to(torch.bfloat16) if c1 else None
+        cin = c0 + c1
+        w = (torch.randn(N, 9 * cin, device="cuda", generator=g) / (9 * cin) ** 0.5).to(torch.bfloat16)
+        bias = torch.randn(N, device="cuda", generator=g)
+        call = lambda: rn.tc_conv3x3(x0, w, x1, bias=bias)      # noqa: E731
+        rn.tune_set("conv_fan", 1)
+        out = call()
+        ref = _ref(x0, x1, w, bias, False)
+        assert (out - ref).abs().max().item() <= 1e-3 * ref.abs().max().item()
+        rn.tune_set("conv_fan", 0)
+        # weights and four row slots within 220 KB less the epilogue's stage, N in one slice
+        if c0 % 32 or c1 % 32:
+            fits = N <= 64 and 9 * cin * N * 2 + 4 * (-(-cin * 272 // 1024) * 1024) + 2048 <= 220 * 1024 - 2112 - 256 * N
+            if not fits:
+                with pytest.raises(rn.RnError):
+                    call()
+                return
+        assert torch.equal(call(), out)
+    finally:
+        rn.tune_set("conv_fan", saved)
