@@ -354,8 +354,8 @@ int rn_selftest_wait_budget(uint32_t spin_limit, rn_status* st);
  *   accel_leaf_small  1 | 2 | 4 | 8  ... below 65,536 triangles
  *   frame_direct      0 | 1          rn_ao_frame on pinned, mapped host buffers without copies
  *   hybrid_min_blocks 5 | 6 | 8      resident rn_hybrid blocks per SM (register budget)
- *   trace_leaf_pass   0 | 1          rn_ao_visibility: a node's leaf children tested after its
- *                                    four slab tests, in one loop
+ *   trace_leaf_pass   0 | 1          accepted; a node's leaf children are tested after its four
+ *                                    slab tests, in one loop, with either value
  *   conv_tmem_a       0 | 1          row-ring convolutions with at most 32 input and 32 output
  *                                    channels keep each input row's A operands in TMEM
  *   ploc_tail         0|4096|16384|32768|65536|262144  accelerator builds: the PLOC rounds

@@ -24,7 +24,7 @@ Workloads:
   trace/ao       a seeded synthetic scene (2,000 boxes, 500 spheres; 744k triangles),
                  1920 x 1080 orbit view, 64 spp AO only (radius 1)
   trace/large    the 7.88M-triangle scene, one 3840 x 2160 orbit view, 16 spp AO only
-                 (the launch shape jointly, then the walk's leaf pass on the same three)
+                 (the launch shape jointly)
   batch          16 orbit views of the 744k scene in one captured batch (batch_min_blocks)
   ssao           the built-in scene at 4K: SSAO, 24 taps
   conv           the surrogate U-Net: a forward at 1088 x 1920 and a training step on
@@ -121,29 +121,6 @@ def tune_trace(quick: bool, reps: int, log):
         r["score"] = float(np.exp(np.mean([np.log(r["ms"][k] / base[k]) for k in base])))
     best = min(rows, key=lambda r: r["score"])
     _apply(best["cfg"])
-    return best["cfg"], rows
-
-
-def tune_walk(quick: bool, reps: int, log):
-    """The walk's form on the traversal workloads, after the launch shape: leaf children
-    tested inline or in one pass after the slab tests (trace_leaf_pass). Each candidate is
-    checked bit for bit; score: geometric mean of the time ratios to the inline form."""
-    wls = trace_workloads(quick)
-    rn.tune_set("trace_leaf_pass", 0)
-    ref = [fn().clone() for _, fn, _ in wls]
-    rows = []
-    for v in rn.TUNE_KEYS["trace_leaf_pass"]:
-        rn.tune_set("trace_leaf_pass", v)
-        if not all(bool((fn() == r).all()) for (_, fn, _), r in zip(wls, ref)):
-            raise RuntimeError("trace_leaf_pass %d changed a traced result" % v)
-        ms = {name: _time(fn, reps) for name, fn, _ in wls}
-        rows.append(dict(cfg={"trace_leaf_pass": v}, ms=ms))
-        log("trace_leaf_pass %d  %s" % (v, "  ".join("%s %.3f ms" % kv for kv in ms.items())))
-    base = rows[0]["ms"]
-    for r in rows:
-        r["score"] = float(np.exp(np.mean([np.log(r["ms"][k] / base[k]) for k in base])))
-    best = min(rows, key=lambda r: r["score"])
-    rn.tune_set("trace_leaf_pass", best["cfg"]["trace_leaf_pass"])
     return best["cfg"], rows
 
 
@@ -515,7 +492,7 @@ def tune_pt(quick: bool, reps: int, log):
     return best["cfg"], rows
 
 
-STAGES = {"accel": tune_accel, "trace": tune_trace, "walk": tune_walk, "frontier_min_spp": tune_frontier_min_spp,
+STAGES = {"accel": tune_accel, "trace": tune_trace, "frontier_min_spp": tune_frontier_min_spp,
           "frontier_tail": tune_frontier_tail, "batch": tune_batch, "ssao": tune_ssao, "conv": tune_conv,
           "hybrid": tune_hybrid, "ploc_tail": tune_ploc_tail, "pt": tune_pt}
 

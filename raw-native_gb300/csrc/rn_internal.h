@@ -66,7 +66,7 @@ struct Tune {
     int accel_leaf_small = 4;   // ... of those with fewer than kSmallScene triangles
     int frame_direct = 1;       // host-buffer frames: the passes read and write mapped host memory
     int hybrid_min_blocks = 6;  // resident 128-thread hybrid-pass blocks per SM: 5, 6 or 8
-    int trace_leaf_pass = 1;    // traversal: a node's leaf children tested in one loop after its slab tests
+    int trace_leaf_pass = 1;    // kept for tune files: either value runs the leaf pass
     int conv_tmem_a = 0;        // row-ring convolutions of 32 -> 32 or 16 -> 32 channels: A operands kept in TMEM
     int conv_fan = 1;           // row-ring convolutions: each input row's MMAs feed its three output rows (N = 3 x BN)
     int conv_fan_bn = 64;       // ... widest output-channel slice: 64 (where its weights fit, else 32) or 32

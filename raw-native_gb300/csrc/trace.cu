@@ -389,7 +389,10 @@ int lanes_log2(const TraceParams& p, long warps) {
 // (2: up to 128 registers, 3: 80, 4: 64, with spills to L1). The launch uses enough
 // blocks to fill every SM at that residency; ctx().tune.trace_min_blocks picks the variant.
 // Stack variants: 48 entries where the tree's bound (17 + 3 x wide depth) fits, else 96.
-// The counting build (traversal statistics) always uses the 96-entry stack.
+// The counting build (traversal statistics) always uses the 96-entry stack and tests each leaf as
+// its child is met; the others test a node's leaves after its four slab tests (a kernel that tests
+// them as they are met took 0.98 to 1.9 times as long with one lane a pixel, 14 to 744k triangles,
+// and up to 4 times where lanes would share one).
 template <int kMB, int kStackN>
 void launch_variant(const TraceParams& p, int sm_count, cudaStream_t s, uint32_t* tile_ctr, unsigned long long* counts,
                     uint32_t stride) {
@@ -399,15 +402,12 @@ void launch_variant(const TraceParams& p, int sm_count, cudaStream_t s, uint32_t
         trace_kernel<true, kMB, kStack, false, 0><<<blocks, 256, 0, s>>>(p, tile_ctr, counts, stride < 1 ? 1 : stride);
     else if (pool > 0 && !p.want_sky)
         trace_ao_pool_kernel<kMB, kStackN><<<blocks, 256, 0, s>>>(p, tile_ctr, pool, ctx().tune.trace_pool_sort);
-    else if (ctx().tune.trace_leaf_pass) {
+    else
         switch (lanes_log2(p, 8L * blocks)) {
             case 2: trace_kernel<false, kMB, kStackN, true, 2><<<blocks, 256, 0, s>>>(p, tile_ctr, nullptr, 1); break;
             case 1: trace_kernel<false, kMB, kStackN, true, 1><<<blocks, 256, 0, s>>>(p, tile_ctr, nullptr, 1); break;
             default: trace_kernel<false, kMB, kStackN, true, 0><<<blocks, 256, 0, s>>>(p, tile_ctr, nullptr, 1);
         }
-    }
-    else
-        trace_kernel<false, kMB, kStackN, false, 0><<<blocks, 256, 0, s>>>(p, tile_ctr, nullptr, 1);
 }
 
 template <int kStackN>
