@@ -31,7 +31,7 @@ using namespace trace_dev;
 // fetches to counts[0..3] (hemisphere rays, nodes, tris, sky continuations); the outputs of
 // the other tiles are left unwritten. "Sky continuations" are the open hemisphere rays whose
 // walk went on past the radius: the same walk serves both queries.
-template <bool kCount, int kMinBlocks, int kStackN, bool kLeafPass, int kP>
+template <bool kCount, int kMinBlocks, int kStackN, bool kLeafPass, int kP, bool kFew = false>
 __global__ void __launch_bounds__(256, kMinBlocks) trace_kernel(const __grid_constant__ TraceParams p, uint32_t* tile_ctr,
                                                                 unsigned long long* counts, uint32_t stride) {
     const int pl = kP == 0 ? p.packet_log2 : min(p.packet_log2, 5 - kP), tw = 1 << pl, th = (32 >> kP) >> pl;
@@ -54,7 +54,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) trace_kernel(const __grid_con
         const int y = (int)(tile / tiles_x) * th + (int)(px >> pl);
         // no lane leaves the loop body early: the next tile fetch is a full-warp shuffle
         if (kCount && tile % stride != 0) continue;
-        trace_packet<kCount, kStackN, kLeafPass, kP>(p, x, y, x < p.w && y < p.h, toLight, cn, skip, F, (int)(lane >> (5 - kP)));
+        trace_packet<kCount, kStackN, kLeafPass, kP, kFew>(p, x, y, x < p.w && y < p.h, toLight, cn, skip, F, (int)(lane >> (5 - kP)));
         __syncwarp();                              // the frontier is rebuilt for the next tile
     }
     if (kCount) {
@@ -402,6 +402,8 @@ void launch_variant(const TraceParams& p, int sm_count, cudaStream_t s, uint32_t
         trace_kernel<true, kMB, kStack, false, 0><<<blocks, 256, 0, s>>>(p, tile_ctr, counts, stride < 1 ? 1 : stride);
     else if (pool > 0 && !p.want_sky)
         trace_ao_pool_kernel<kMB, kStackN><<<blocks, 256, 0, s>>>(p, tile_ctr, pool, ctx().tune.trace_pool_sort);
+    else if (p.spp <= kFewSpp)
+        trace_kernel<false, kMB, kStackN, true, 0, true><<<blocks, 256, 0, s>>>(p, tile_ctr, nullptr, 1);
     else
         switch (lanes_log2(p, 8L * blocks)) {
             case 2: trace_kernel<false, kMB, kStackN, true, 2><<<blocks, 256, 0, s>>>(p, tile_ctr, nullptr, 1); break;

@@ -227,11 +227,11 @@ __device__ __forceinline__ bool below(const TilePlane& t, float lx, float ly, fl
 // that is an interior node is replaced by its children that overlap Q and are not below the
 // packet's plane, the lanes expanding their entries in
 // parallel (one node fetch per lane, a prefix sum over the lanes for the output slots),
-// while the result stays within kFrontier entries. A round costs one dependent node fetch,
+// while the result stays within `cap` entries (kFrontier at most). A round costs one dependent node fetch,
 // so the build takes about the tree's depth in fetch latencies. Up to `tail` greedy steps
 // follow, each replacing the largest interior entry by its children while the frontier fits.
 __device__ inline int build_frontier(const Node4* __restrict__ nodes, const float* qlo, const float* qhi,
-                                     const TilePlane& pl, Node4* F, int tail) {
+                                     const TilePlane& pl, Node4* F, int cap, int tail) {
     const int lane = (int)(threadIdx.x & 31u);
     int32_t word = 0;                       // lane 0 starts with the root node
     float lo[3] = {0.0f, 0.0f, 0.0f}, hi[3] = {0.0f, 0.0f, 0.0f};
@@ -253,7 +253,7 @@ __device__ inline int build_frontier(const Node4* __restrict__ nodes, const floa
             if (lane >= off) incl += v;
         }
         const int total = __shfl_sync(0xffffffffu, incl, 31);
-        if (!__any_sync(0xffffffffu, inner) || total > kFrontier) break;
+        if (!__any_sync(0xffffffffu, inner) || total > cap) break;
         __syncwarp();                       // every lane has read its entry of the last round
         int pos = incl - c;
         if (inner) {
@@ -291,7 +291,7 @@ __device__ inline int build_frontier(const Node4* __restrict__ nodes, const floa
                     !below(pl, N->lox[k], N->loy[k], N->loz[k], N->hix[k], N->hiy[k], N->hiz[k]))
                     hit |= 1u << k;
         const int c = __popc(__shfl_sync(0xffffffffu, hit, bl));
-        if (n - 1 + c > kFrontier) break;
+        if (n - 1 + c > cap) break;
         __syncwarp();
         if (lane == bl) {
             // the children replace entry bl and append after the last entry; none: the last
@@ -511,14 +511,16 @@ __device__ __forceinline__ TileBox tile_box(const v3& o, bool covered) {
 }
 // The frontier of the warp's packet for AO walks of `radius` (all 32 lanes call it and build
 // it together). Returns its size, 0: the walks start at the root, -1: no triangle is within
-// reach.
+// reach. Below four samples, four entries for each: a round more costs a dependent fetch whatever
+// the samples that start from it (213k triangles, 1920 x 1080, 1 and 3 samples: 284 -> 218 us with
+// the form for few samples below, 449 -> 430 us; 744k, 4 samples: 16 entries 0.5 % slower than 24).
 __device__ __forceinline__ int tile_frontier(const TraceParams& p, const TileBox& t, const TilePlane& pl, Node4* F) {
     float lo[3] = {t.lo[0], t.lo[1], t.lo[2]}, hi[3] = {t.hi[0], t.hi[1], t.hi[2]};
     if (lo[0] > hi[0]) return 0;
     // grow by the radius with margin for the rounding of t, |d| and the hit point
     const float g = p.radius * 1.0001f + 1e-5f * (t.mag + 1.0f);
     for (int a = 0; a < 3; ++a) { lo[a] -= g; hi[a] += g; }
-    const int n = build_frontier(p.nodes, lo, hi, pl, F, p.frontier_tail);
+    const int n = build_frontier(p.nodes, lo, hi, pl, F, p.spp < 4 ? 4 * p.spp : kFrontier, p.frontier_tail);
     __syncwarp();
     return n;
 }
@@ -619,11 +621,14 @@ __device__ __forceinline__ bool walk_starts(const v3& o, const v3& d, float tmax
 // built-in scene at 3840 x 2160, 256 spp with sky 25.4 -> 18.9 ms with exact rays in the sieve,
 // 18.0 -> 13.2 with rough ones; views of 744k triangles within 1 % either way (thresholds of
 // 3/8, 5/8, 8/8: 22.0, 19.2 ms, and views 33.6 ms against 33.1).
+// Few samples (kFew: kFewSpp at most) take none of this: what the packet's rays share then costs
+// more than it saves (built-in scene with sky, 2561 x 1441, 1 sample 155 -> 136 us; from 3 samples
+// on the sieve is the faster one there). AO walks still start from the frontier.
 // With kP > 0 a packet is 32 >> kP pixels and 1 << kP lanes share each (`part`, the lane's high
 // bits): a part takes a run of the pixel's samples, part 0 the sun as well, and the counts are
 // added up at the end; integers, so the split changes no bit.
-constexpr int kChunk = 64, kSieveNum = 7, kSieveDen = 8, kSieveSkip = 15;
-template <bool kCount, int kStackN = kStack, bool kLeafPass = true, int kP = 0>
+constexpr int kChunk = 64, kSieveNum = 7, kSieveDen = 8, kSieveSkip = 15, kFewSpp = 2;
+template <bool kCount, int kStackN = kStack, bool kLeafPass = true, int kP = 0, bool kFew = false>
 __device__ __forceinline__ void trace_packet(const TraceParams& p, int x, int y, bool valid, const v3& toLight,
                                              Counts& cn, int& skip, Node4* F, int part = 0) {
     const bool lead = kP == 0 || part == 0;        // writes the pixel
@@ -660,14 +665,14 @@ __device__ __forceinline__ void trace_packet(const TraceParams& p, int x, int y,
     // every packet)
     int fn = 0;
     bool sieve = false;
-    if (p.has_geometry && (p.want_sky || p.frontier)) {
+    if (p.has_geometry && (kFew ? p.frontier && !p.want_sky : p.want_sky || p.frontier)) {
         const TilePlane pl = tile_plane(n, origin, m != 0, covered);
         const TileBox tb = tile_box(origin, m != 0);
-        fn = p.want_sky ? root_frontier(p.nodes, pl, F) : tile_frontier(p, tb, pl, F);
+        fn = !kFew && p.want_sky ? root_frontier(p.nodes, pl, F) : tile_frontier(p, tb, pl, F);
         // the sieve needs normals of about unit length (its rough rays are not normalized) and
         // no far origin
         const float n2 = n.x * n.x + n.y * n.y + n.z * n.z;
-        sieve = !kCount && fn > 0 && skip == 0 && tb.mag <= kFarOrigin && __all_sync(0xffffffffu, !m || (n2 > 0.9f && n2 < 1.1f));
+        sieve = !kCount && !kFew && fn > 0 && skip == 0 && tb.mag <= kFarOrigin && __all_sync(0xffffffffu, !m || (n2 > 0.9f && n2 < 1.1f));
         if (!kCount && fn > 0 && skip > 0) --skip;
         if (sieve) grow_entries(F, fn, tb);
     }
@@ -697,7 +702,46 @@ __device__ __forceinline__ void trace_packet(const TraceParams& p, int x, int y,
         open = freec = mine;
         if (kCount && m) { cn.rays += mine; if (p.want_sky) cn.sky += mine; }
     }
-    for (int s0 = first; s0 < slots; s0 += kChunk) {
+    // slot s of the part's: a sample's walk, or the sun's; `next`: the sample whose angle to fetch
+    // ahead (-1: none)
+    auto slot = [&](int s, int next) {
+        v3 dir;
+        float tn, tf;
+        if (s < span) {
+            const uint32_t k2 = k2n;
+            const int cb = cbn;
+            if (next >= 0) fetch(next);
+            dir = direction(sbase + s, k2, cb);
+            tn = p.radius;
+            tf = tfar_h;
+        } else {
+            dir = toLight;
+            tn = tf = kFar;
+        }
+        // AO-only walks may start from the warp's frontier; the sky and the sun need the root
+        const bool local = s < span && tf == p.radius;
+        const int h = p.has_geometry
+                          ? walk<kCount, kStackN, kLeafPass>(p.nodes, p.tris, origin, dir, tn, tf, p.err_word, cn,
+                                                             local ? F : nullptr, local ? fn : 0)
+                          : 0;
+        if (s < span) {
+            if (kCount) { ++cn.rays; if (p.want_sky && !(h & HIT_NEAR)) ++cn.sky; }
+            if (!(h & HIT_NEAR)) {
+                ++open;
+                if (!(h & HIT_FAR)) ++freec;
+            }
+        } else {
+            lit = h == 0;
+        }
+    };
+    if (kFew) {
+        if (m && first < slots) {
+            fetch(first);
+            for (int s = first; s < slots; ++s) slot(s, s + 1);
+        }
+        __syncwarp();
+    }
+    for (int s0 = first; !kFew && s0 < slots; s0 += kChunk) {
         const int nslot = min(kChunk, slots - s0), nsamp = min(kChunk, span - s0);
         uint64_t todo = 0;
         if (kP == 0) {
@@ -728,34 +772,7 @@ __device__ __forceinline__ void trace_packet(const TraceParams& p, int x, int y,
         while (todo) {
             const int s = s0 + __ffsll((long long)todo) - 1;
             todo &= todo - 1ull;
-            v3 dir;
-            float tn, tf;
-            if (s < span) {
-                const uint32_t k2 = k2n;
-                const int cb = cbn;
-                if (todo) fetch(sbase + s0 + __ffsll((long long)todo) - 1);
-                dir = direction(sbase + s, k2, cb);
-                tn = p.radius;
-                tf = tfar_h;
-            } else {
-                dir = toLight;
-                tn = tf = kFar;
-            }
-            // AO-only walks may start from the warp's frontier; the sky and the sun need the root
-            const bool local = s < span && tf == p.radius;
-            const int h = p.has_geometry
-                              ? walk<kCount, kStackN, kLeafPass>(p.nodes, p.tris, origin, dir, tn, tf, p.err_word, cn,
-                                                                 local ? F : nullptr, local ? fn : 0)
-                              : 0;
-            if (s < span) {
-                if (kCount) { ++cn.rays; if (p.want_sky && !(h & HIT_NEAR)) ++cn.sky; }
-                if (!(h & HIT_NEAR)) {
-                    ++open;
-                    if (!(h & HIT_FAR)) ++freec;
-                }
-            } else {
-                lit = h == 0;
-            }
+            slot(s, todo ? sbase + s0 + __ffsll((long long)todo) - 1 : -1);
         }
         __syncwarp();
     }

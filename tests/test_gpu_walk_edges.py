@@ -233,3 +233,45 @@ def test_deep_trees_trace_from_the_frontier(rn, oracle, n):
     finally:
         for k, v in saved.items():
             rn.tune_set(k, v)
+
+
+@pytest.mark.parametrize("spp", [1, 2, 3, 4, 5, 6])
+@pytest.mark.parametrize("small", [True, False])
+def test_few_samples_against_the_scan(rn, oracle, small, spp):
+    """One and two samples a pixel run without the sieve, and up to three cap the frontier at four
+    entries a sample: the oracle's AO, sky and sun bit for bit, in ragged frames, packets of 4, 8
+    and 16 columns, with the frontier on and off, and as a view of a batch."""
+    import scene as scenes
+    import torch
+    if small:
+        sc = scenes.build_test_scene()
+        cam = sc.camera
+    else:
+        sc = scenes.build_synthetic_scene(5, 60, 10, grid=20, half=8.0, subdiv=2)
+        cam = (6.0, 4.0, 5.0, 0.0, 0.5, 0.0, 0.0, 1.0, 0.0, 0.9)
+    tl = (0.3, 0.8, -0.5)
+    acc = rn.LinearAccel(sc.tris)
+    keys = ("trace_packet", "trace_frontier", "trace_frontier_min_spp")
+    saved = {k: rn.tune_get(k) for k in keys}
+    try:
+        rn.tune_set("trace_frontier_min_spp", 1)
+        for (w, h), packet in (((61, 43), 8), ((17, 9), 4), ((33, 3), 16)):
+            rn.tune_set("trace_packet", packet)
+            _, pos, nrm, mask = oracle.rasterize(sc.tris, sc.normals, cam, w, h)
+            g = rn.GBuffer(pos, nrm, mask)
+            want = oracle.trace(pos, nrm, mask, sc.tris, spp, 1.0, to_light=tl, threads=THREADS)
+            for frontier in (0, 1):
+                rn.tune_set("trace_frontier", frontier)
+                got = rn.compute_rt_visibility(g, acc, spp, 1.0, to_light=tl)
+                for a, b in zip(got, want):
+                    assert np.array_equal(a, b), (w, h, frontier, int((a != b).sum()))
+                assert np.array_equal(rn.compute_rtao(g, acc, spp, 1.0), want[0]), (w, h, frontier)
+            dg = rn.GBuffer(*[torch.from_numpy(t).cuda() for t in (pos, nrm, mask)])
+            dacc = rn.LinearAccel(torch.from_numpy(sc.tris).cuda())
+            batch = rn.Batch(dacc, [dict(g=dg, spp=spp, radius=1.0, ssao=False)])
+            batch.run()
+            assert np.array_equal(batch.outputs[0]["ao"].cpu().numpy(), want[0]), (w, h)
+            batch.close()
+    finally:
+        for k, v in saved.items():
+            rn.tune_set(k, v)
