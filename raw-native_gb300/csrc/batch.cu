@@ -50,7 +50,8 @@ __device__ __forceinline__ int find_view(const uint32_t* begins, int n, uint32_t
 
 template <int kMinBlocks>
 __global__ void __launch_bounds__(256, kMinBlocks) trace_batch_kernel(const BatchView* __restrict__ views, int nviews,
-                                                                      uint32_t total_tiles, uint32_t* tile_ctr) {
+                                                                      uint32_t total_tiles, uint32_t* tile_ctr,
+                                                                      float short_dir) {
     __shared__ TraceParams sp[kMaxViews];
     __shared__ uint32_t begins[kMaxViews];
     for (int v = threadIdx.x; v < nviews; v += blockDim.x) { sp[v] = views[v].tp; begins[v] = views[v].tile_begin; }
@@ -72,7 +73,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) trace_batch_kernel(const Batc
         const int x = (int)(local % tiles_x) * kTileW + (int)(lane % kTileW);
         const int y = (int)(local / tiles_x) * kTileH + (int)(lane / kTileW);
         const v3 toLight = normalize(mk(p.lx, p.ly, p.lz));
-        trace_dev::trace_packet<false>(p, x, y, x < p.w && y < p.h, toLight, cn, skip, F);
+        trace_dev::trace_packet<false>(p, short_dir, x, y, x < p.w && y < p.h, toLight, cn, skip, F);
         __syncwarp();
     }
 }
@@ -206,9 +207,9 @@ int rn_batch_create(const rn_accel* accel, const rn_view* views, int nviews, int
         cudaMemsetAsync(d_ctr, 0, 4, b->capture);
         cudaMemsetAsync(d_outs, 0, (size_t)nviews * sizeof(RecOut), b->capture);
         const int mb = c.tune.batch_min_blocks;
-        if (mb == 2) trace_batch_kernel<2><<<c.sm_count * 2, 256, 0, b->capture>>>(d_views, nviews, tiles, d_ctr);
-        else if (mb == 4) trace_batch_kernel<4><<<c.sm_count * 4, 256, 0, b->capture>>>(d_views, nviews, tiles, d_ctr);
-        else trace_batch_kernel<3><<<c.sm_count * 3, 256, 0, b->capture>>>(d_views, nviews, tiles, d_ctr);
+        if (mb == 2) trace_batch_kernel<2><<<c.sm_count * 2, 256, 0, b->capture>>>(d_views, nviews, tiles, d_ctr, short_dir(*accel));
+        else if (mb == 4) trace_batch_kernel<4><<<c.sm_count * 4, 256, 0, b->capture>>>(d_views, nviews, tiles, d_ctr, short_dir(*accel));
+        else trace_batch_kernel<3><<<c.sm_count * 3, 256, 0, b->capture>>>(d_views, nviews, tiles, d_ctr, short_dir(*accel));
         if (ssao_blocks_total)
             ssao_batch_kernel<<<ssao_blocks_total, ssao_dev::kThreads, 0, b->capture>>>(d_views, nviews, ss_samples,
                                                                                        d_parts, d_outs);

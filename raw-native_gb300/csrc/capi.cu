@@ -215,6 +215,7 @@ void apply_tune(TraceParams& p, const rn_accel* accel) {
     const Tune& t = ctx().tune;
     p.frontier = t.trace_frontier && p.spp >= t.trace_frontier_min_spp;
     p.stack_need = stack_need(accel ? accel->depth : 0);
+    p.short_dir = accel ? short_dir(*accel) : kShortDir;
     // the frontier's seeds sit under the walk's own pushes: without room for both, walk from the root
     if (p.stack_need > 96) p.frontier = 0;
     p.packet_log2 = packet_log2(t.trace_packet);
@@ -1085,8 +1086,7 @@ int rn_occluded(const rn_accel* accel, const float* rays, const float* t_max, ui
     RN_TRY(stage_in(rays, (size_t)nrays * 6, dev, WS_RAYS, &d_rays, st));
     RN_TRY(stage_in(t_max, (size_t)nrays, dev, WS_TMAX, &d_t, st));
     RN_TRY(stage_out(hit, (size_t)nrays, dev, WS_HITS, &d_hit, st));
-    if (launch_occluded(accel->d_nodes, accel->d_tris, accel->ntri > 0, d_rays, d_t, nrays, d_hit, c.dev_error,
-                        c.stream) != RN_OK)
+    if (launch_occluded(*accel, d_rays, d_t, nrays, d_hit, c.dev_error, c.stream) != RN_OK)
         return cuda_fail(st, cudaGetLastError(), "occluded_kernel");
     if (dev) return ok(st);
     RN_TRY(copy_back(hit, d_hit, nrays, st));
@@ -1111,8 +1111,7 @@ int rn_closest(const rn_accel* accel, const float* rays, const float* t_max, uin
     RN_TRY(stage_in(t_max, (size_t)nrays, dev, WS_TMAX, &d_tm, st));
     RN_TRY(stage_out(tri, (size_t)nrays, dev, WS_CLOSEST_TRI, &d_tri, st));
     RN_TRY(stage_out(t, (size_t)nrays, dev, WS_CLOSEST_T, &d_t, st));
-    if (launch_closest(accel->d_nodes, accel->d_tris, accel->ntri > 0, d_rays, d_tm, nrays, d_tri, d_t, c.dev_error,
-                       c.stream) != RN_OK)
+    if (launch_closest(*accel, d_rays, d_tm, nrays, d_tri, d_t, c.dev_error, c.stream) != RN_OK)
         return cuda_fail(st, cudaGetLastError(), "closest_kernel");
     if (dev) return ok(st);
     RN_TRY(copy_back(tri, d_tri, nrays, st));

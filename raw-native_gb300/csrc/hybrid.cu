@@ -20,14 +20,15 @@ namespace {
 
 using namespace trace_dev;
 
-__global__ void closest_kernel(const Node4* __restrict__ nodes, const LeafTri* __restrict__ tris, int has_geometry,
+__global__ void __launch_bounds__(128, 8) closest_kernel(const Node4* __restrict__ nodes, const LeafTri* __restrict__ tris, int has_geometry,
+                               float short_dir,
                                const float* __restrict__ rays, const float* __restrict__ tmax, uint32_t n,
                                int32_t* __restrict__ tri, float* __restrict__ t_out, uint32_t* err) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const v3 o = load3(rays + (size_t)i * 6), d = load3(rays + (size_t)i * 6 + 3);
     float t = tmax[i];
-    const int id = has_geometry ? walk_closest(nodes, tris, o, d, tmax[i], t, err) : -1;
+    const int id = has_geometry ? walk_closest(nodes, tris, short_dir, o, d, tmax[i], t, err) : -1;
     tri[i] = id;
     t_out[i] = id >= 0 ? t : -1.0f;
 }
@@ -48,6 +49,7 @@ struct HybridArgs {
     const Node4* nodes;
     const LeafTri* tris;
     int has_geometry;
+    float short_dir;
     float ex, ey, ez;     // the eye
     float lx, ly, lz;     // toward the sun (normalized on the device)
     float* lit;           // 1 lit, 0 in shadow, -1 uncovered
@@ -86,21 +88,22 @@ __global__ void __launch_bounds__(128, kMinBlocks) hybrid_kernel(const HybridArg
     const v3 l = normalize(mk(a.lx, a.ly, a.lz));
     Counts cn;
     const bool shadow =
-        a.has_geometry && walk<false>(a.nodes, a.tris, offset_of(pos, ng, l), l, 1e30f, 1e30f, a.err, cn) != 0;
+        a.has_geometry && walk<false>(a.nodes, a.tris, a.short_dir, offset_of(pos, ng, l), l, 1e30f, 1e30f, a.err, cn) != 0;
     a.lit[i] = shadow ? 0.0f : 1.0f;
     const v3 r = sub(d, scale(n, fmul(2.0f, dot(d, n))));
     float t = 1e30f;
-    const int id = a.has_geometry ? walk_closest(a.nodes, a.tris, offset_of(pos, ng, r), r, 1e30f, t, a.err) : -1;
+    const int id = a.has_geometry ? walk_closest(a.nodes, a.tris, a.short_dir, offset_of(pos, ng, r), r, 1e30f, t, a.err) : -1;
     a.refl_tri[i] = id;
     a.refl_t[i] = id >= 0 ? t : -1.0f;
 }
 
 }  // namespace
 
-int launch_closest(const Node4* nodes, const LeafTri* tris, int has_geometry, const float* rays, const float* tmax,
-                   uint32_t n, int32_t* tri, float* t, uint32_t* err, cudaStream_t s) {
+int launch_closest(const rn_accel& accel, const float* rays, const float* tmax, uint32_t n,
+                   int32_t* tri, float* t, uint32_t* err, cudaStream_t s) {
     if (n == 0) return RN_OK;
-    closest_kernel<<<(n + 127) / 128, 128, 0, s>>>(nodes, tris, has_geometry, rays, tmax, n, tri, t, err);
+    closest_kernel<<<(n + 127) / 128, 128, 0, s>>>(accel.d_nodes, accel.d_tris, accel.ntri > 0, short_dir(accel), rays, tmax, n, tri, t,
+                                                      err);
     return cudaGetLastError() == cudaSuccess ? RN_OK : RN_ERR_CUDA;
 }
 
@@ -113,6 +116,7 @@ int launch_hybrid(int w, int h, const float* pos, const float* nrm, const float*
     a.pos = pos; a.nrm = nrm; a.geo = geo_nrm; a.mask = mask;
     a.nodes = accel->d_nodes; a.tris = accel->d_tris;
     a.has_geometry = accel->ntri > 0;
+    a.short_dir = short_dir(*accel);
     a.ex = eye[0]; a.ey = eye[1]; a.ez = eye[2];
     a.lx = to_sun[0]; a.ly = to_sun[1]; a.lz = to_sun[2];
     a.lit = lit; a.refl_tri = refl_tri; a.refl_t = refl_t;

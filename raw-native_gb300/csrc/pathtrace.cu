@@ -222,6 +222,7 @@ struct PtParams {
     const Node4* nodes;
     const LeafTri* ltris;
     int has_geometry;
+    float short_dir;
     const float* tris;        // 9 a triangle, input order
     const float* nrm;
     const float* uv;
@@ -505,7 +506,7 @@ __device__ __noinline__ void surface_of(const PtParams& P, v3 o, v3 d, int tri, 
 __device__ __noinline__ bool hit(const PtParams& P, v3 o, v3 d, float tmax, Surf& x) {
     if (!P.has_geometry) return false;
     float t;
-    const int tri = walk_closest(P.nodes, P.ltris, o, d, tmax, t, P.err);
+    const int tri = walk_closest(P.nodes, P.ltris, P.short_dir, o, d, tmax, t, P.err);
     if (tri < 0) return false;
     surface_of(P, o, d, tri, t, x);
     return true;
@@ -513,7 +514,7 @@ __device__ __noinline__ bool hit(const PtParams& P, v3 o, v3 d, float tmax, Surf
 __device__ __noinline__ bool visible(const PtParams& P, v3 p, v3 dir, float tmax) {
     if (!P.has_geometry) return true;
     Counts cn;
-    return walk<false, kStack, true, false>(P.nodes, P.ltris, p, dir, tmax, tmax, P.err, cn) == 0;
+    return walk<false, kStack, true, false>(P.nodes, P.ltris, P.short_dir, p, dir, tmax, tmax, P.err, cn) == 0;
 }
 __device__ __forceinline__ v3 offset_of(const Surf& x, v3 dir) {
     const float e = fmul(2e-4f, fadd(1.0f, smax(fabsf(x.p.x), smax(fabsf(x.p.y), fabsf(x.p.z)))));
@@ -1075,7 +1076,7 @@ __global__ void __launch_bounds__(128) pt_wave_shadow(const PtParams P, const Wa
         bool vis = true;
         if (P.has_geometry) {
             Counts cn;
-            vis = walk<false, kStack, true, false>(P.nodes, P.ltris, o, d, tmax, tmax, P.err, cn) == 0;
+            vis = walk<false, kStack, true, false>(P.nodes, P.ltris, P.short_dir, o, d, tmax, tmax, P.err, cn) == 0;
         }
         W.vis[(size_t)(s & 1u) * W.Q + (s >> 1)] = vis ? 1 : 0;
     }
@@ -1083,14 +1084,14 @@ __global__ void __launch_bounds__(128) pt_wave_shadow(const PtParams P, const Wa
 
 // The closest hits of the slots' rays (rt::closest); also restarts the queue and live counts
 // for the next shade pass.
-__global__ void __launch_bounds__(128) pt_wave_extend(const PtParams P, const WaveBufs W) {
+__global__ void __launch_bounds__(128, 8) pt_wave_extend(const PtParams P, const WaveBufs W) {
     using namespace wave;
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i == 0) { W.ctr[0] = 0; W.ctr[1] = 0; }
     if (i >= W.Q || (wu(W, UFL, i) & 3u) != M_TRACE) return;
     float t = 0.0f;
     int tri = -1;
-    if (P.has_geometry) tri = walk_closest(P.nodes, P.ltris, wld3(W, RO, i), wld3(W, RD, i), 1e30f, t, P.err);
+    if (P.has_geometry) tri = walk_closest(P.nodes, P.ltris, P.short_dir, wld3(W, RO, i), wld3(W, RD, i), 1e30f, t, P.err);
     wu(W, UTRI, i) = (uint32_t)tri;
     wf(W, HT, i) = t;
 }
@@ -1324,6 +1325,7 @@ int rn_pathtrace(const rn_ptscene* s, const rn_pt_desc* d, int flags, rn_pt_out*
     const uint32_t npix = (uint32_t)d->width * (uint32_t)d->height;
     PtParams P{};
     P.nodes = s->accel->d_nodes; P.ltris = s->accel->d_tris; P.has_geometry = s->ntri > 0;
+    P.short_dir = short_dir(*s->accel);
     P.tris = s->tris; P.nrm = s->nrm; P.uv = s->uv; P.idx = s->idx; P.tritex = s->tritex; P.texent = s->texent;
     P.texels = s->texels; P.mat = s->mat; P.emit = s->emit; P.cdf = s->cdf; P.nemit = s->nemit; P.area = s->area;
     P.table = table; P.corr = c.trig_corr;

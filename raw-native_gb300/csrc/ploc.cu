@@ -1142,7 +1142,8 @@ struct CollapseCtr {
     uint32_t tasks;              // of the current level
     uint32_t base;               // nodes when it began
     unsigned long long made;     // nodes (low half) and leaf triangles (high half) so far
-    uint32_t err, depth, done, pad;
+    uint32_t err, depth, done;
+    uint32_t far;                // a coordinate beyond kFarCoord
 };
 static_assert(sizeof(CollapseCtr) == 32, "CollapseCtr layout");
 
@@ -1242,6 +1243,9 @@ __device__ __forceinline__ void collapse_tasks(const Task* in, uint32_t m, uint3
             padded(C[k].b, lo, hi);
             nd.lox[k] = lo[0]; nd.loy[k] = lo[1]; nd.loz[k] = lo[2];
             nd.hix[k] = hi[0]; nd.hiy[k] = hi[1]; nd.hiz[k] = hi[2];
+            if (task.wnode == 0)
+                for (int a = 0; a < 3; ++a)
+                    if (!(fmaxf(fabsf(lo[a]), fabsf(hi[a])) <= kFarCoord)) ctr->far = 1;
             if (C[k].cnt <= leaf_max) {
                 const uint32_t first = tri_next;
                 tri_next += C[k].cnt;
@@ -1576,6 +1580,7 @@ static int judge_collapse(const CollapseCtr& hc, rn_accel* acc, rn_status* st) {
     if (placed != acc->ntri) return fail(st, RN_ERR_STATE, "collapse placed %u of %u triangles", placed, acc->ntri);
     acc->nodes = (uint32_t)hc.made;
     acc->depth = hc.depth;
+    acc->far = hc.far != 0;
     return ok(st);
 }
 

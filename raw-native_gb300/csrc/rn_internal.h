@@ -210,11 +210,17 @@ struct rn_accel {
     uint32_t nodes = 0;        // wide nodes
     uint32_t rounds = 0;       // PLOC rounds
     uint32_t depth = 0;        // wide-tree depth (levels)
+    bool far = false;          // a coordinate beyond rn::kFarCoord
     rn::Node4* d_nodes = nullptr;
     rn::LeafTri* d_tris = nullptr;
 };
 
 namespace rn {
+// A direction is short when no component reaches kShortDir. Node tests form its reciprocals with
+// more care (make_inv, trace_device.cuh), and every ray's on a tree with coordinates beyond
+// kFarCoord: `short_dir` is the length below which a walk on this tree does so.
+constexpr float kShortDir = 1e-3f, kFarCoord = 3e11f;
+inline float short_dir(const rn_accel& a) { return a.far ? __builtin_inff() : kShortDir; }
 // PLOC: build the binary tree on the device. Outputs (device): nodes9 (2n-1 x 9 int32 in
 // the reference's layout) when non-null; the binary tree in SoA form for the collapse.
 struct PlocTree {
@@ -243,6 +249,8 @@ int collapse_bvh4(const PlocTree& t, const float* d_tris, rn_accel* acc, int lea
 int collapse_finish(const PlocTree& t, rn_accel* acc, rn_status* st);
 
 // ---------------------------------------------------------------- traversal
+// The batch holds 256 of these in shared memory (its blocks' three shares just fit 132 KB of an SM's
+// L1: 8 bytes more each cost it 2 %).
 struct TraceParams {
     int w, h;
     const float* pos;
@@ -261,9 +269,10 @@ struct TraceParams {
     float* sun;
     uint32_t* err_word;
     int frontier;         // AO-only walks start from a per-warp frontier (0: from the root)
-    int packet_log2;      // log2 of the packet width (pixels per warp row): 2, 3 or 4
     int frontier_tail;    // greedy single-entry steps after the breadth-first frontier build
-    int stack_need;       // entries the walk can push on this tree (rn::stack_need)
+    int16_t packet_log2;  // log2 of the packet width (pixels per warp row): 2, 3 or 4
+    int16_t stack_need;   // entries the walk can push on this tree (rn::stack_need)
+    float short_dir;      // rn::short_dir of the tree
     // copy-through of a G-buffer read from host memory (null: none): every pixel's position,
     // normal, AO and mask are also written to a device buffer laid out as
     // [position w*h*12 B][normal w*h*12 B][ao w*h*4 B][mask w*h B] (mirror_* below)
@@ -291,8 +300,8 @@ int launch_trace(const TraceParams& p, int sm_count, cudaStream_t s, unsigned lo
 
 // ---------------------------------------------------------------- closest hit, hybrid (hybrid.cu)
 // Nearest hits (triangle index, t; -1 / -1 for none) of n rays (6 floats each) below tmax.
-int launch_closest(const Node4* nodes, const LeafTri* tris, int has_geometry, const float* rays, const float* tmax,
-                   uint32_t n, int32_t* tri, float* t, uint32_t* err, cudaStream_t s);
+int launch_closest(const rn_accel& accel, const float* rays, const float* tmax, uint32_t n,
+                   int32_t* tri, float* t, uint32_t* err, cudaStream_t s);
 // The hybrid pass over a G-buffer: sun shadows and mirror reflections per covered pixel.
 int launch_hybrid(int w, int h, const float* pos, const float* nrm, const float* geo_nrm, const uint8_t* mask,
                   const rn_accel* accel,
@@ -325,7 +334,7 @@ int launch_raster(const float* tris, const float* nrm, uint32_t ntri, const floa
                   char* scratch, size_t scratch_bytes, float* depth, float* pos, float* nrm_out, uint8_t* mask,
                   cudaStream_t s, size_t* pairs_needed, const float* albedo_tri = nullptr, float* albedo = nullptr);
 int scan_exclusive_u32(const uint32_t* in, uint32_t* out, uint32_t n, uint32_t* bsum, uint32_t* total, cudaStream_t s);
-int launch_occluded(const Node4* nodes, const LeafTri* tris, int has_geometry, const float* rays,
-                    const float* tmax, uint32_t n, uint8_t* hit, uint32_t* err_word, cudaStream_t s);
+int launch_occluded(const rn_accel& accel, const float* rays, const float* tmax, uint32_t n,
+                    uint8_t* hit, uint32_t* err_word, cudaStream_t s);
 
 }  // namespace rn

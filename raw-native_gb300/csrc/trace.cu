@@ -54,7 +54,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) trace_kernel(const __grid_con
         const int y = (int)(tile / tiles_x) * th + (int)(px >> pl);
         // no lane leaves the loop body early: the next tile fetch is a full-warp shuffle
         if (kCount && tile % stride != 0) continue;
-        trace_packet<kCount, kStackN, kLeafPass, kP, kFew>(p, x, y, x < p.w && y < p.h, toLight, cn, skip, F, (int)(lane >> (5 - kP)));
+        trace_packet<kCount, kStackN, kLeafPass, kP, kFew>(p, p.short_dir, x, y, x < p.w && y < p.h, toLight, cn, skip, F, (int)(lane >> (5 - kP)));
         __syncwarp();                              // the frontier is rebuilt for the next tile
     }
     if (kCount) {
@@ -213,7 +213,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) trace_ao_pool_kernel(const __
                     q = src;
                     o = po;
                     d = sample_direction(pt, pb, pn, (uint32_t)qx, (uint32_t)qy, wi / (uint32_t)nc, p.corr);
-                    iv = make_inv(o, d);
+                    iv = make_inv(o, d, p.short_dir);
                     wr_ready = false;
                     sp = 0;
                     guard = 0;
@@ -313,6 +313,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) trace_ao_pool_kernel(const __
 }
 
 __global__ void occluded_kernel(const Node4* __restrict__ nodes, const LeafTri* __restrict__ tris, int has_geometry,
+                                float short_dir,
                                 const float* __restrict__ rays, const float* __restrict__ tmax, uint32_t n,
                                 uint8_t* __restrict__ hit, uint32_t* err) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -320,7 +321,7 @@ __global__ void occluded_kernel(const Node4* __restrict__ nodes, const LeafTri* 
     const v3 o = load3(rays + (size_t)i * 6), d = load3(rays + (size_t)i * 6 + 3);
     Counts cn;
     const float tm = tmax[i];
-    hit[i] = (has_geometry && walk<false>(nodes, tris, o, d, tm, tm, err, cn) != 0) ? 1 : 0;
+    hit[i] = (has_geometry && walk<false>(nodes, tris, short_dir, o, d, tm, tm, err, cn) != 0) ? 1 : 0;
 }
 
 // AO of listed pixels with one thread per (pixel, sample): the same rays and hit rule as
@@ -350,7 +351,7 @@ __global__ void __launch_bounds__(256) ao_samples_kernel(const __grid_constant__
             const v3 t = normalize(cross(a, n)), b = cross(n, t);
             const v3 origin = add(P, scale(n, 1e-3f));
             const v3 dir = sample_direction(t, b, n, x, y, s, p.corr);
-            const int h = p.has_geometry ? walk<false>(p.nodes, p.tris, origin, dir, p.radius, p.radius, p.err_word, cn) : 0;
+            const int h = p.has_geometry ? walk<false>(p.nodes, p.tris, p.short_dir, origin, dir, p.radius, p.radius, p.err_word, cn) : 0;
             o = (h & HIT_NEAR) ? 0 : 1;
         }
         const unsigned peers = __match_any_sync(0xffffffffu, px);
@@ -433,10 +434,11 @@ int launch_trace(const TraceParams& p, int sm_count, cudaStream_t s, unsigned lo
     return cudaGetLastError() == cudaSuccess ? RN_OK : RN_ERR_CUDA;
 }
 
-int launch_occluded(const Node4* nodes, const LeafTri* tris, int has_geometry, const float* rays, const float* tmax,
-                    uint32_t n, uint8_t* hit, uint32_t* err_word, cudaStream_t s) {
+int launch_occluded(const rn_accel& accel, const float* rays, const float* tmax, uint32_t n,
+                    uint8_t* hit, uint32_t* err_word, cudaStream_t s) {
     if (n == 0) return RN_OK;
-    occluded_kernel<<<(n + 255) / 256, 256, 0, s>>>(nodes, tris, has_geometry, rays, tmax, n, hit, err_word);
+    occluded_kernel<<<(n + 255) / 256, 256, 0, s>>>(accel.d_nodes, accel.d_tris, accel.ntri > 0, short_dir(accel), rays, tmax, n, hit,
+                                                       err_word);
     return cudaGetLastError() == cudaSuccess ? RN_OK : RN_ERR_CUDA;
 }
 

@@ -28,10 +28,12 @@ __device__ __forceinline__ float rcp_approx(float x) {
 // ray straight along an axis visits every node (a sample whose u is exactly zero is the normal
 // itself, one in 2^24: 12 ms of one warp over 146k triangles, 800 x 600 x 64 samples 14.9 -> 4.2 ms,
 // 1280 x 720 x 64 16.8 -> 7.3). At 1e27 a plane's distance says on which side of it the origin
-// lies, its rounding 2^-24 |o| of position, inside the boxes' padding, as long as o * inv is finite
-// (|o| up to kFarOrigin; refine_axis beyond); a component below 1e-27 moves the ray by less than
-// that over any distance the others leave in the scene.
-constexpr float kInvMax = 1e27f, kFarOrigin = 3e11f;
+// lies, its rounding 2^-24 |o| of position, inside the boxes' padding; a component below 1e-27 moves
+// the ray by less than that over any distance the others leave in the scene. From |o| = 3.4e11 on
+// o * inv is infinite, and such a ray stays beyond that coordinate: its boxes are culled, rightly
+// where the scene lies within kFarCoord (else see make_inv).
+constexpr float kInvMax = 1e27f;
+static_assert(kFarCoord * kInvMax < 3.4e38f, "o * inv is finite within kFarCoord");
 __device__ __forceinline__ float inv_clamped(float x) { return fminf(fmaxf(rcp_approx(x), -kInvMax), kInvMax); }
 // For any direction: a component below 1e-28 that is not zero gives NaN, so that its axis
 // constrains nothing: with its reciprocal one of plane * inv and o * inv could overflow alone
@@ -58,22 +60,25 @@ __device__ __forceinline__ float min3(float a, float b, float c) {
 // the hi plane 16 bytes further; the far plane sits at the other of the two), formed once
 // per walk.
 struct Inv { float x, y, z, ox, oy, oz; uint32_t nx, ny, nz; };
-// One axis of a ray with a short direction or a far origin. An infinite o * inv of finite
+// One axis of a ray with a short direction or in a far scene. An infinite o * inv of finite
 // factors would put both planes of every box at the same infinity and cull the boxes that
 // the ray enters: NaN instead, and the axis constrains nothing.
 __device__ __forceinline__ void refine_axis(float o, float d, bool is_short, float& inv, float& oi) {
     if (is_short) { inv = safe_inv(d); oi = o * inv; }
     if (isinf(oi) && !isinf(o) && !isinf(inv)) inv = oi = __int_as_float(0x7fffffff);
 }
-// kUnit: the direction is about of unit length and the origin not far.
+// short_dir: the tree's (rn::short_dir), so a scene with far coordinates costs the others nothing
+// (a test of each origin's size: 0.5 to 1 % of every frame). kUnit: the direction is about of unit
+// length and the origin within kFarCoord.
 template <bool kUnit = false>
-__device__ __forceinline__ Inv make_inv(const v3& o, const v3& d) {
+__device__ __forceinline__ Inv make_inv(const v3& o, const v3& d, float short_dir) {
     Inv r;
     r.x = inv_clamped(d.x); r.y = inv_clamped(d.y); r.z = inv_clamped(d.z);
     r.ox = o.x * r.x; r.oy = o.y * r.y; r.oz = o.z * r.z;
     if (!kUnit) {
-        const bool is_short = !(max3(fabsf(d.x), fabsf(d.y), fabsf(d.z)) >= 1e-3f);
-        if (is_short || max3(fabsf(o.x), fabsf(o.y), fabsf(o.z)) > kFarOrigin) {
+        const float longest = max3(fabsf(d.x), fabsf(d.y), fabsf(d.z));
+        if (!(longest >= short_dir)) {
+            const bool is_short = !(longest >= kShortDir);
             refine_axis(o.x, d.x, is_short, r.x, r.ox);
             refine_axis(o.y, d.y, is_short, r.y, r.oy);
             refine_axis(o.z, d.z, is_short, r.z, r.oz);
@@ -333,9 +338,9 @@ __device__ inline int build_frontier(const Node4* __restrict__ nodes, const floa
 // rays meet an occluder sooner in the nearest child, the path tracer's shadow rays do not gain
 // what the comparisons cost (1080p room, 4 samples: 24.8 ms with them, 24.1 without).
 template <bool kCount, int kStackN = kStack, bool kLeafPass = true, bool kNearest = true>
-__device__ int walk(const Node4* __restrict__ nodes, const LeafTri* __restrict__ tris, const v3& o, const v3& d,
-                    float tnear, float tfar, uint32_t* err, Counts& cn, const Node4* F = nullptr, int fn = 0) {
-    const Inv iv = make_inv(o, d);
+__device__ int walk(const Node4* __restrict__ nodes, const LeafTri* __restrict__ tris, float short_dir, const v3& o,
+                    const v3& d, float tnear, float tfar, uint32_t* err, Counts& cn, const Node4* F = nullptr, int fn = 0) {
+    const Inv iv = make_inv(o, d, short_dir);
     LeafRay wr;                          // the watertight set-up: formed at the first leaf
     bool wr_ready = false;
     float tmax = tfar;
@@ -428,9 +433,9 @@ __device__ int walk(const Node4* __restrict__ nodes, const LeafTri* __restrict__
 // watertight test with 1e-4 < t < tmax, ties to the lowest triangle index (leaf triangles carry
 // their input index). Children are visited nearest entry first; a box is culled only when its
 // (padded, exit-widened) slab entry passes the best t so far, so the answer is the scan's.
-__device__ inline int walk_closest(const Node4* __restrict__ nodes, const LeafTri* __restrict__ tris, const v3& o,
-                            const v3& d, float tmax, float& t_hit, uint32_t* err) {
-    const Inv iv = make_inv(o, d);
+__device__ inline int walk_closest(const Node4* __restrict__ nodes, const LeafTri* __restrict__ tris, float short_dir,
+                            const v3& o, const v3& d, float tmax, float& t_hit, uint32_t* err) {
+    const Inv iv = make_inv(o, d, short_dir);
     const LeafRay wr = make_leaf_ray(o, d);
     float best = tmax;
     int best_tri = -1;
@@ -592,7 +597,7 @@ __device__ __forceinline__ v3 rough_direction(const v3& t, const v3& b, const v3
 // Whether a walk along the rough direction d has anything to descend into: any of the fn grown
 // entries of F is entered before tmax.
 __device__ __forceinline__ bool walk_starts(const v3& o, const v3& d, float tmax, const Node4* F, int fn) {
-    const Inv iv = make_inv<true>(o, d);
+    const Inv iv = make_inv<true>(o, d, kShortDir);
     bool any;
     int g = 0;
     do {
@@ -629,8 +634,8 @@ __device__ __forceinline__ bool walk_starts(const v3& o, const v3& d, float tmax
 // added up at the end; integers, so the split changes no bit.
 constexpr int kChunk = 64, kSieveNum = 7, kSieveDen = 8, kSieveSkip = 15, kFewSpp = 2;
 template <bool kCount, int kStackN = kStack, bool kLeafPass = true, int kP = 0, bool kFew = false>
-__device__ __forceinline__ void trace_packet(const TraceParams& p, int x, int y, bool valid, const v3& toLight,
-                                             Counts& cn, int& skip, Node4* F, int part = 0) {
+__device__ __forceinline__ void trace_packet(const TraceParams& p, float short_dir, int x, int y, bool valid,
+                                             const v3& toLight, Counts& cn, int& skip, Node4* F, int part = 0) {
     const bool lead = kP == 0 || part == 0;        // writes the pixel
     const int span = kP == 0 ? p.spp : (p.spp + (1 << kP) - 1) >> kP;      // a part's samples: first .. first + mine
     const int sbase = kP == 0 ? 0 : part * span, mine = kP == 0 ? p.spp : max(0, min(span, p.spp - sbase));
@@ -670,9 +675,10 @@ __device__ __forceinline__ void trace_packet(const TraceParams& p, int x, int y,
         const TileBox tb = tile_box(origin, m != 0);
         fn = !kFew && p.want_sky ? root_frontier(p.nodes, pl, F) : tile_frontier(p, tb, pl, F);
         // the sieve needs normals of about unit length (its rough rays are not normalized) and
-        // no far origin
+        // origins whose products with a reciprocal stay finite (a rough ray off by 1e-5 that stays
+        // beyond kFarCoord says nothing of the exact one)
         const float n2 = n.x * n.x + n.y * n.y + n.z * n.z;
-        sieve = !kCount && !kFew && fn > 0 && skip == 0 && tb.mag <= kFarOrigin && __all_sync(0xffffffffu, !m || (n2 > 0.9f && n2 < 1.1f));
+        sieve = !kCount && !kFew && fn > 0 && skip == 0 && tb.mag <= kFarCoord && __all_sync(0xffffffffu, !m || (n2 > 0.9f && n2 < 1.1f));
         if (!kCount && fn > 0 && skip > 0) --skip;
         if (sieve) grow_entries(F, fn, tb);
     }
@@ -721,7 +727,7 @@ __device__ __forceinline__ void trace_packet(const TraceParams& p, int x, int y,
         // AO-only walks may start from the warp's frontier; the sky and the sun need the root
         const bool local = s < span && tf == p.radius;
         const int h = p.has_geometry
-                          ? walk<kCount, kStackN, kLeafPass>(p.nodes, p.tris, origin, dir, tn, tf, p.err_word, cn,
+                          ? walk<kCount, kStackN, kLeafPass>(p.nodes, p.tris, short_dir, origin, dir, tn, tf, p.err_word, cn,
                                                              local ? F : nullptr, local ? fn : 0)
                           : 0;
         if (s < span) {
