@@ -264,3 +264,27 @@ def test_small_scene_leaf_keeps_every_bit(rn, restore_tune):
         if ref is None:
             ref = out
         assert all(bool((a == b).all()) for a, b in zip(out, ref)), leaf
+
+
+@pytest.mark.parametrize("w,h", [(1283, 1001), (1632, 1169)])
+def test_ssao_of_a_large_frame(rn, oracle, restore_tune, w, h):
+    """Frames of eight 16-row tiles an SM and more, the size from which that height runs, ragged at
+    the right and lower edge: every height gives the oracle's SSAO bit for bit, and the fused
+    reconcile the separate one's error map and, in the order of its own blocks, its sums."""
+    import os
+    import numpy as np
+    assert ((w + 31) // 32) * ((h + 15) // 16) >= 8 * rn.device_info()["sm_count"]
+    g, acc, _ = _scene(rn, w, h)
+    want = oracle.ssao(g.position.cpu().numpy(), g.normal.cpu().numpy(), g.mask.cpu().numpy(), 24, 1.0,
+                       threads=os.cpu_count() or 1)
+    truth = rn.compute_rtao(g, acc, 4, 1.0)
+    for v in rn.TUNE_KEYS["ssao_tile_h"]:
+        rn.tune_set("ssao_tile_h", v)
+        ss = rn.compute_ssao(g, 24, 1.0)
+        assert np.array_equal(ss.cpu().numpy(), want), (v, int((ss.cpu().numpy() != want).sum()))
+        rec = rn.reconcile(ss, truth, g.mask)
+        out = rn.ao_frame(g, acc, 4, 1.0, 24, 0.12)
+        assert bool((out["ao"] == truth).all()) and bool((out["ss"] == ss).all()), v
+        assert bool((out["err"] == rec.error_map).all()), v
+        assert out["rec"].pixels == rec.pixels and out["rec"].max_error == rec.max_error
+        assert abs(out["rec"].sum_sq - rec.sum_sq) <= 1e-10 * rec.sum_sq
