@@ -288,3 +288,55 @@ def test_ssao_of_a_large_frame(rn, oracle, restore_tune, w, h):
         assert bool((out["err"] == rec.error_map).all()), v
         assert out["rec"].pixels == rec.pixels and out["rec"].max_error == rec.max_error
         assert abs(out["rec"].sum_sq - rec.sum_sq) <= 1e-10 * rec.sum_sq
+
+
+@pytest.mark.parametrize("spp", [7, 15])
+def test_trace_keys_of_the_one_lane_form(rn, oracle, restore_tune, spp):
+    """Below 16 samples every pixel keeps one lane, whatever the frame's size: the oracle's planes
+    bit for bit under every value of every traversal key."""
+    import os
+    import numpy as np
+    import scene as scenes
+    g, acc, tl = _scene(rn, 211, 101)
+    sc = scenes.build_synthetic_scene(11, 300, 60)
+    want = oracle.trace(g.position.cpu().numpy(), g.normal.cpu().numpy(), g.mask.cpu().numpy(), sc.tris, spp, 1.0,
+                        to_light=tl, threads=os.cpu_count() or 1)
+    defaults = {"trace_min_blocks": 3, "trace_packet": 8, "trace_stack": 96, "trace_frontier": 1,
+                "trace_frontier_min_spp": 1, "trace_frontier_tail": 0, "trace_pool": 0, "trace_leaf_pass": 1}
+    for k, v in defaults.items():
+        rn.tune_set(k, v)
+    for k in defaults:
+        for v in rn.TUNE_KEYS[k]:
+            rn.tune_set(k, v)
+            assert np.array_equal(rn.compute_rtao(g, acc, spp, 1.0).cpu().numpy(), want[0]), (k, v)
+            for a, b in zip(rn.compute_rt_visibility(g, acc, spp, 1.0, tl), want):
+                assert np.array_equal(a.cpu().numpy(), b), (k, v)
+        rn.tune_set(k, defaults[k])
+
+
+@pytest.mark.parametrize("boxes,spheres", [(0, 0), (300, 60)])
+def test_large_frame_keeps_one_lane_a_pixel(rn, oracle, restore_tune, boxes, spheres):
+    """More than nine packets a warp: one lane a pixel at any sample count, so the sieve's chunks of
+    64 samples in the form that large frames run; every 97th row against the oracle, for every
+    residency and packet width."""
+    import os
+    import numpy as np
+    import torch
+    import scene as scenes
+    w, h, spp, step = 1921, 1081, 65, 97
+    sc = scenes.build_synthetic_scene(11, boxes, spheres) if boxes else scenes.build_test_scene()
+    cam = scenes.orbit_views(11, 8)[3][3] if boxes else sc.camera
+    tris, nrms = torch.from_numpy(sc.tris).cuda(), torch.from_numpy(sc.normals).cuda()
+    g, acc = rn.rasterize(tris, nrms, cam, w, h), rn.LinearAccel(tris)
+    rows = slice(5, h, step)
+    want = oracle.trace(g.position.cpu().numpy(), g.normal.cpu().numpy(), g.mask.cpu().numpy(), sc.tris, spp, 1.0,
+                        to_light=sc.to_light, threads=os.cpu_count() or 1, row0=5, row_stride=step)
+    for key in ("trace_min_blocks", "trace_packet"):
+        saved = rn.tune_get(key)
+        for v in rn.TUNE_KEYS[key]:
+            rn.tune_set(key, v)
+            got = rn.compute_rt_visibility(g, acc, spp, 1.0, sc.to_light)
+            for a, b in zip(got, want):
+                assert np.array_equal(a[rows].cpu().numpy(), b[rows]), (key, v)
+            assert np.array_equal(rn.compute_rtao(g, acc, spp, 1.0)[rows].cpu().numpy(), want[0][rows]), (key, v)
+        rn.tune_set(key, saved)
