@@ -208,3 +208,62 @@ def test_implicit_gradients_match_torch_over_box_shapes(rn, B, H, W):
     rows and 2-pixel columns, and with both paddings of the input's channels: the same
     comparison and bounds as above."""
     test_unet_gradients_match_torch(rn, B, H, W, False)
+
+
+@pytest.mark.parametrize("B,H,W", [(16, 128, 128), (40, 64, 64)])
+def test_bias_gradients_are_the_sums_of_dz(rn, B, H, W):
+    """The bias gradients, summed from the weight gradient's own boxes of dZ as these pass through a
+    ring of shared memory, against 64-bit sums of the same dZ, ten times over. Every layer passes
+    its first 32 channels on through the centre tap and adds a bias of 1, so that all outputs are
+    positive and every layer's dZ follows from the head's by BF16 roundings, 2 x 2 sums and
+    quarters, formed here. Neighbouring boxes have opposite signs: the sums stay small (an FP32
+    addition of a few thousand terms of z is off by 2e-4 z; some thousand atomics: below 0.1 of
+    the largest z), while a box read before or after its time is off by whole terms."""
+    import torch
+    import rn_ao
+    net = rn.UNet(B, H, W, seed=1)
+    skip = {8: 128, 10: 64, 12: 32}                       # a concatenated layer takes the upsampled half
+    rng = np.random.default_rng(5)
+    parts = []
+    for l, (cin, cout) in enumerate(rn_ao.UNET_CONVS):
+        w = np.zeros((cout, 9, cin), np.float32)
+        if l:
+            for c in range(32):
+                w[c, 4, skip.get(l, 0) + c] = 1.0
+        parts += [w.ravel(), np.ones(cout, np.float32)]
+    wh = (rng.integers(4, 33, 32) * rng.choice([-1, 1], 32) / 256).astype(np.float32)
+    parts += [wh, np.zeros(1, np.float32)]
+    net.set_params(np.concatenate(parts))
+    x = torch.zeros(B, H, W, 5, device="cuda")
+    s = net.forward(x)
+    assert bool((s == s[0, 0, 0]).all()) and 0.01 < float(s[0, 0, 0]) < 0.99
+    g = torch.Generator(device="cuda").manual_seed(2)
+    sign = 1.0 - 2.0 * ((torch.arange(H, device="cuda") // 8 % 2)[:, None] ^ (torch.arange(W, device="cuda") // 32 % 2)[None])
+    y = s - sign * (0.5 + 0.5 * torch.rand(B, H, W, device="cuda", generator=g))
+    diff = s - y
+    dz = 2.0 * diff * s * (1.0 - s) * torch.tensor(1.0 / (B * H * W), device="cuda")
+    z = (dz[..., None] * torch.from_numpy(wh).cuda()).bfloat16()
+
+    def down(t):                                          # the 2 x 2 sums of an upsampled source
+        f = t.float()
+        return (((f[:, ::2, ::2] + f[:, ::2, 1::2]) + f[:, 1::2, ::2]) + f[:, 1::2, 1::2]).bfloat16()
+
+    def spread(t):                                        # a pooled source
+        return (0.25 * t.float()).repeat_interleave(2, 1).repeat_interleave(2, 2).bfloat16()
+    of = {13: z, 12: z}
+    for l in (11, 9, 7):
+        of[l] = of[l - 1] = down(of[l + 1])
+    for l in (5, 3, 1):
+        of[l] = of[l - 1] = spread(of[l + 1])
+    for _ in range(10):
+        net.backward(x, y)
+        grads, o = net.get_grads(), 0
+        for l, (cin, cout) in enumerate(rn_ao.UNET_CONVS):
+            o += cout * 9 * cin
+            got = grads[o:o + cout].astype(np.float64)
+            o += cout
+            want = of[l].double().sum((0, 1, 2)).cpu().numpy()
+            tol = 0.1 * float(of[l].abs().max())
+            assert np.abs(got[:32] - want).max() <= tol, (l, np.abs(got[:32] - want).max() / tol)
+            assert not got[32:].any(), l
+    net.close()
