@@ -638,6 +638,8 @@ int rn_accel_build(const float* tris, uint32_t ntri, int flags, rn_accel** out, 
     if (rc == RN_OK) {
         cudaError_t e = cudaStreamSynchronize(c.stream);
         if (e != cudaSuccess) rc = cuda_fail(st, e, "rn_accel_build");
+    } else if (tree.state) {
+        cudaStreamSynchronize(c.stream);        // still queued: it must not write under a later call
     }
     if (rc == RN_OK) rc = finish_accel(acc, &tree, st);
     if (rc != RN_OK) { rn_accel_free(acc); return rc; }
