@@ -6,12 +6,12 @@
 //   - warp 0, lane 0: TMA producer. Each 64-wide K step loads a 128 x 64 tile of P and a
 //     BN x 64 tile of Q (cp.async.bulk.tensor, 128-byte swizzle) into one of 4 shared-memory
 //     stages and signals the stage's "full" mbarrier with the byte count;
-//   - warp 1: MMA issuer (an elected lane). Per stage, four tcgen05.mma.kind::f16 (M 128, N BN, K 16)
+//   - warp 1: MMA issuer (convergent, an elected lane executing). Per stage, four tcgen05.mma.kind::f16 (M 128, N BN, K 16)
 //     accumulate into a BN-column TMEM accumulator; tcgen05.commit releases the stage
 //     ("empty" mbarrier) when its MMAs have read it, and a final commit signals "done";
 //   - all four warps: epilogue. Each thread owns one row (its warp's TMEM lane quarter),
-//     reads it with tcgen05.ld 16 columns at a time, adds the bias, applies ReLU or the
-//     ReLU-backward gate, and stores BF16 or FP32 (or adds FP32 atomically for split K).
+//     reads it with tcgen05.ld 16 columns at a time, adds the bias, applies ReLU, and stores
+//     BF16 or FP32 (or adds FP32 atomically for split K).
 // Every mbarrier wait is bounded; on a timeout the kernel sets the error word, waits
 // (bounded) for its own copies in flight, frees its TMEM and returns.
 #include "gemm_tc.h"
@@ -117,15 +117,6 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
-// 64 consecutive TMEM columns of this warp's 32 lanes in one load and one wait.
-__device__ __forceinline__ void tmem_ld64(uint32_t taddr, uint32_t (&v)[64]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x64.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32, %33, %34, %35, %36, %37, %38, %39, %40, %41, %42, %43, %44, %45, %46, %47, %48, %49, %50, %51, %52, %53, %54, %55, %56, %57, %58, %59, %60, %61, %62, %63}, [%64];\n"
-        "tcgen05.wait::ld.sync.aligned;"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31]), "=r"(v[32]), "=r"(v[33]), "=r"(v[34]), "=r"(v[35]), "=r"(v[36]), "=r"(v[37]), "=r"(v[38]), "=r"(v[39]), "=r"(v[40]), "=r"(v[41]), "=r"(v[42]), "=r"(v[43]), "=r"(v[44]), "=r"(v[45]), "=r"(v[46]), "=r"(v[47]), "=r"(v[48]), "=r"(v[49]), "=r"(v[50]), "=r"(v[51]), "=r"(v[52]), "=r"(v[53]), "=r"(v[54]), "=r"(v[55]), "=r"(v[56]), "=r"(v[57]), "=r"(v[58]), "=r"(v[59]), "=r"(v[60]), "=r"(v[61]), "=r"(v[62]), "=r"(v[63])
-        : "r"(taddr)
-        : "memory");
-}
 // Zeros into 32 consecutive TMEM columns of this warp's 32 lanes (its wait is separate:
 // tcgen05.wait::st before the columns are handed to the MMAs).
 __device__ __forceinline__ void tmem_zero32(uint32_t taddr) {
@@ -246,17 +237,6 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const __grid_const
                 f[j] = x;
             }
             const size_t o = (size_t)row * e.ldc + col;
-            if (e.gate) {
-                const uint4* g4 = reinterpret_cast<const uint4*>(e.gate + o);
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    const uint4 gv = g4[h];
-                    const __nv_bfloat16* gb = reinterpret_cast<const __nv_bfloat16*>(&gv);
-#pragma unroll
-                    for (int j = 0; j < 8; ++j)
-                        if (!(__bfloat162float(gb[j]) > 0.0f)) f[h * 8 + j] = 0.0f;
-                }
-            }
             if (e.c16) {
                 uint4 out[2];
                 __nv_bfloat16* ob = reinterpret_cast<__nv_bfloat16*>(out);
@@ -1267,9 +1247,10 @@ __global__ void __launch_bounds__(kFan ? kFanThreads : kConvThreads, kFan && !kW
 // read once per group, and every x element nine times, from L2. At the end it adds its tiles
 // to gw with FP32 atomics. The bias gradient, dz's column sums, comes from the same boxes: in the
 // first group's CTAs the epilogue warps, idle until the end, add up each dz box in shared memory
-// before its slot is released (a pass of its own read dz again: 14 passes, 250 us). Roles: warp 0 loads (its lanes issue a tile's atoms together), one
-// lane of warp 1 issues the MMAs, warps 2..5 read the accumulators. Waits are bounded and give
-// up when another role has aborted.
+// before its slot is released (a pass of its own read dz again: 14 passes, 250 us). Roles: warp 0
+// loads (its lanes issue a tile's atoms together), warp 1 issues the MMAs (convergent, an elected
+// lane executing), warps 2..5 read the accumulators. Waits are bounded and give up when another
+// role has aborted.
 struct WgradArgs {
     int nb0, nb1;               // CA-channel chunks of the sources
     int tiles_x, tiles_y;       // 64-pixel boxes per image row / column
@@ -1674,6 +1655,7 @@ int tc_gemm(const __nv_bfloat16* P, int ldp, const __nv_bfloat16* Q, int ldq, in
         return fail(st, RN_ERR_INVALID, "tc_gemm shape M %d N %d K %d splits %d", M, N, K, splits);
     if ((ldp % 8) || (ldq % 8) || ((uintptr_t)P % 16) || ((uintptr_t)Q % 16))
         return fail(st, RN_ERR_INVALID, "tc_gemm operands must be 16-byte aligned rows");
+    if (epi.gate) return fail(st, RN_ERR_INVALID, "tc_gemm: no gated epilogue");
     if (splits > 1 && !(epi.c32 && epi.atomic)) return fail(st, RN_ERR_INVALID, "split K needs an atomic FP32 output");
     int bn = (N == 32 || N == 64 || N == 128 || N == 256) ? N : 128;
     if (N % bn) return fail(st, RN_ERR_INVALID, "tc_gemm N %d", N);

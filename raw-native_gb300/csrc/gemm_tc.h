@@ -14,8 +14,8 @@ struct Epilogue {
     float* c32;                      // FP32 output (split K: accumulated with atomics)
     __nv_bfloat16* c16;              // BF16 output
     const float* bias;               // [N] or null
-    const __nv_bfloat16* gate;       // [M][ldc]: output zeroed where gate is not > 0 (ReLU backward), or null
-                                     // (convolutions: with a BF16 output alone)
+    const __nv_bfloat16* gate;       // convolutions, with a BF16 output alone: [pixels][ldc], the output
+                                     // zeroed where gate is not > 0 (ReLU backward); or null
     int relu;
     int atomic;
     int k_per_split;                 // K range of one grid.z slice (a multiple of 64)
@@ -30,7 +30,7 @@ struct Epilogue {
 };
 
 // One input of an implicit-GEMM 3x3 convolution: an NHWC BF16 tensor at the output's
-// resolution with C channels (C a multiple of 32).
+// resolution with C channels (C a multiple of 32, or of 16 where row tiles take the layer).
 struct ConvSrc {
     const __nv_bfloat16* ptr;
     int C;

@@ -11,8 +11,8 @@
 //      the lower position), merge mutual pairs into nodes numbered by a prefix sum in position
 //      order, compact the survivors. The round count lives on the device: the host launches
 //      rounds in batches and reads the survivor count once per batch, not once per round.
-//   6. collapse: subtree sizes bottom-up, then level by level each 4-wide node takes the
-//      binary node's children and opens the largest-area interior child until it has 4;
+//   6. collapse: level by level (the merges have counted each subtree's triangles) a 4-wide node
+//      takes the binary node's children and opens the largest-area interior child until it has 4;
 //      subtrees of at most leaf_max (<= 8) triangles become leaves with their triangles copied
 //      contiguously (48-byte records).
 #include "rn_internal.h"

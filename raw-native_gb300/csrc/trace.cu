@@ -3,8 +3,9 @@
 //
 // Work: the frame is cut into packets of 32 pixels (8 x 4 by default; 4 x 8 and 16 x 2 are
 // the autotuner's alternatives); each warp takes the next packet from a global counter, one
-// pixel per lane, and walks its `spp` hemisphere rays, then the sun ray,
-// through the 4-wide BVH. Neighbouring lanes trace neighbouring pixels, so the warp's rays
+// pixel per lane, and walks its `spp` hemisphere rays, then the sun ray, through the 4-wide BVH.
+// Small frames are cut into packets of 16 or 8 pixels, two or four lanes sharing each pixel's
+// samples (lanes_log2). Neighbouring lanes trace neighbouring pixels, so the warp's rays
 // start close together and visit similar nodes.
 //
 // One walk per hemisphere ray answers both of the reference's questions about it: a hit
