@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) trace_ao_pool_kernel(const __
                     q = src;
                     o = po;
                     d = sample_direction(pt, pb, pn, (uint32_t)qx, (uint32_t)qy, wi / (uint32_t)nc, p.corr);
-                    iv = make_inv(o, d, p.short_dir);
+                    iv = make_inv<true>(o, d, kShortDir);
                     wr_ready = false;
                     sp = 0;
                     guard = 0;
@@ -402,7 +402,7 @@ void launch_variant(const TraceParams& p, int sm_count, cudaStream_t s, uint32_t
     const int pool = ctx().tune.trace_pool;
     if (counts)
         trace_kernel<true, kMB, kStack, false, 0><<<blocks, 256, 0, s>>>(p, tile_ctr, counts, stride < 1 ? 1 : stride);
-    else if (pool > 0 && !p.want_sky)
+    else if (pool > 0 && !p.want_sky && p.short_dir == kShortDir)      // no far scene (its make_inv)
         trace_ao_pool_kernel<kMB, kStackN><<<blocks, 256, 0, s>>>(p, tile_ctr, pool, ctx().tune.trace_pool_sort);
     else if (p.spp <= kFewSpp)
         trace_kernel<false, kMB, kStackN, true, 0, true><<<blocks, 256, 0, s>>>(p, tile_ctr, nullptr, 1);
