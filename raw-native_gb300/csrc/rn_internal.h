@@ -249,6 +249,10 @@ int collapse_bvh4(const PlocTree& t, const float* d_tris, rn_accel* acc, int lea
 int collapse_finish(const PlocTree& t, rn_accel* acc, rn_status* st);
 
 // ---------------------------------------------------------------- traversal
+// Where AO-only walks start: at the root; from the entries within the radius of the packet's
+// origins; or from the root's live children, which costs little and lets the sieve run.
+enum Frontier : int { FRONTIER_OFF = 0, FRONTIER_NEAR = 1, FRONTIER_ROOT = 2 };
+
 // The batch holds 256 of these in shared memory (its blocks' three shares just fit 132 KB of an SM's
 // L1: 8 bytes more each cost it 2 %).
 struct TraceParams {
@@ -268,7 +272,7 @@ struct TraceParams {
     float* sky;
     float* sun;
     uint32_t* err_word;
-    int frontier;         // AO-only walks start from a per-warp frontier (0: from the root)
+    int frontier;         // Frontier: where AO-only walks start
     int frontier_tail;    // greedy single-entry steps after the breadth-first frontier build
     int16_t packet_log2;  // log2 of the packet width (pixels per warp row): 2, 3 or 4
     int16_t stack_need;   // entries the walk can push on this tree (rn::stack_need)

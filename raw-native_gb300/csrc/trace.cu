@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) trace_ao_pool_kernel(const __
             O = add(P, scale(n, 1e-3f));
         }
         // no plane: an empty frontier is left to the walk's own test
-        const int fn = (p.has_geometry && p.frontier)
+        const int fn = (p.has_geometry && p.frontier == FRONTIER_NEAR)
                            ? max(0, tile_frontier(p, tile_box(O, covered), TilePlane{0.0f, 0.0f, 0.0f, 0.0f, 0.0f}, F)) : 0;
         const unsigned cov = __ballot_sync(0xffffffffu, covered);
         const int nc = __popc(cov);

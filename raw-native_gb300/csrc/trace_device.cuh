@@ -665,15 +665,16 @@ __device__ __forceinline__ void trace_packet(const TraceParams& p, float short_d
     const float tfar_h = p.want_sky ? kFar : p.radius;
     const bool sun = p.want_sky && !p.sun_forced;
     const int slots = span + (sun ? 1 : 0);
-    // what the packet's rays can reach: AO-only walks start from the entries within the radius,
-    // the sky's at the root, whose live children serve the sieve (the frontier is rebuilt for
-    // every packet)
+    // what the packet's rays can reach: AO-only walks start from the entries within the radius, or
+    // from the root's live children; the sky's start at the root, whose live children serve the
+    // sieve (rebuilt for every packet)
     int fn = 0;
     bool sieve = false;
-    if (p.has_geometry && (kFew ? p.frontier && !p.want_sky : p.want_sky || p.frontier)) {
+    const bool near = p.frontier == FRONTIER_NEAR && !p.want_sky;
+    if (p.has_geometry && (near || (!kFew && (p.want_sky || (p.frontier && !kCount))))) {
         const TilePlane pl = tile_plane(n, origin, m != 0, covered);
         const TileBox tb = tile_box(origin, m != 0);
-        fn = !kFew && p.want_sky ? root_frontier(p.nodes, pl, F) : tile_frontier(p, tb, pl, F);
+        fn = near ? tile_frontier(p, tb, pl, F) : root_frontier(p.nodes, pl, F);
         // the sieve needs normals of about unit length (its rough rays are not normalized) and
         // origins whose products with a reciprocal stay finite (a rough ray off by 1e-5 that stays
         // beyond kFarCoord says nothing of the exact one)
