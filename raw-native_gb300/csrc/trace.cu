@@ -379,12 +379,17 @@ int launch_ao_samples(const TraceParams& p, const uint32_t* list, const uint32_t
 // and 2581 / 1461 / 862; 1024 x 768 x 32 (6.7) 212 / 248 / 306, without sky 105 / 100 / 137, 146k
 // 3539 / 3379 / 3360 and 1095 / 937 / 1022; 1283 x 723 x 16 (8) 135 / 169, without 71 / 78, 146k
 // 2046 / 1942 and 633 / 652; 1920 x 1080 x 16 (18) 275 / 355, 146k 4060 / 4068 and 1087 / 1179.
+// The small tree with the sky, one / two lanes by packets a warp: 16 samples 70.0 / 68.1 at 2.8, 73.2 /
+// 75.5 at 3.2, 83.0 / 93.8 at 4.2; 32 samples 128 / 126 at 3.8, 134 / 138 at 4.2; 64 samples 236 / 220 at
+// 4.2, 253 / 249 at 4.8. Up to nine packets two lanes are the faster on deeper trees and from 32
+// samples without the sky (8.8 packets: 106 / 105, 146k triangles 1038 / 923 and with sky 4241 / 4100).
 int lanes_log2(const TraceParams& p, long warps) {
     const long tw = 1L << p.packet_log2, th = 32 >> p.packet_log2;
     const double r = (double)(((p.w + tw - 1) / tw) * ((p.h + th - 1) / th)) / (double)warps;
     const bool deep = p.stack_need >= stack_need(6);           // a tree of six levels and more
     if (p.spp >= 32 && r < (p.want_sky && !deep ? 1.5 : 3.0)) return 2;
-    return p.spp >= 16 && r < (p.want_sky ? (deep ? 9.0 : 4.5) : (p.spp >= 32 ? 9.0 : 4.0)) ? 1 : 0;
+    const double sky = deep ? 9.0 : p.spp >= 64 ? 4.5 : p.spp >= 32 ? 4.0 : 3.0;
+    return p.spp >= 16 && r < (p.want_sky ? sky : p.spp >= 32 ? 9.0 : 4.0) ? 1 : 0;
 }
 
 // Residency variants: the register budget decides how many 256-thread blocks share an SM

@@ -184,7 +184,16 @@ def test_frame_far_from_the_origin(rn, oracle, log2):
         got = rn.compute_rt_visibility(g, acc, 65, 2.0 * scale, to_light=sun)
         for a, b in zip(got, want):
             assert np.array_equal(a, b), int((a != b).sum())
-    assert np.array_equal(rn.compute_rtao(g, acc, 65, 2.0 * scale), want[0])
+    saved = {k: rn.tune_get(k) for k in ("trace_pool", "trace_frontier")}
+    try:
+        for pool in (0, 24):
+            for frontier in (0, 1):
+                rn.tune_set("trace_pool", pool)
+                rn.tune_set("trace_frontier", frontier)
+                assert np.array_equal(rn.compute_rtao(g, acc, 65, 2.0 * scale), want[0]), (pool, frontier)
+    finally:
+        for k, v in saved.items():
+            rn.tune_set(k, v)
 
 
 def _chain(n):
