@@ -20,7 +20,7 @@ namespace {
 
 using namespace trace_dev;
 
-__global__ void __launch_bounds__(128, 8) closest_kernel(const Node4* __restrict__ nodes, const LeafTri* __restrict__ tris, int has_geometry,
+__global__ void __launch_bounds__(128) closest_kernel(const Node4* __restrict__ nodes, const LeafTri* __restrict__ tris, int has_geometry,
                                float short_dir,
                                const float* __restrict__ rays, const float* __restrict__ tmax, uint32_t n,
                                int32_t* __restrict__ tri, float* __restrict__ t_out, uint32_t* err) {

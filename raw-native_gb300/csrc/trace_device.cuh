@@ -31,7 +31,7 @@ __device__ __forceinline__ float rcp_approx(float x) {
 // lies, its rounding 2^-24 |o| of position, inside the boxes' padding; a component below 1e-27 moves
 // the ray by less than that over any distance the others leave in the scene. From |o| = 3.4e11 on
 // o * inv is infinite, and such a ray stays beyond that coordinate: its boxes are culled, rightly
-// where the scene lies within kFarCoord (else see make_inv).
+// where the scene lies within kFarCoord (else see careful_inv).
 constexpr float kInvMax = 1e27f;
 static_assert(kFarCoord * kInvMax < 3.4e38f, "o * inv is finite within kFarCoord");
 __device__ __forceinline__ float inv_clamped(float x) { return fminf(fmaxf(rcp_approx(x), -kInvMax), kInvMax); }
@@ -60,12 +60,14 @@ __device__ __forceinline__ float min3(float a, float b, float c) {
 // the hi plane 16 bytes further; the far plane sits at the other of the two), formed once
 // per walk.
 struct Inv { float x, y, z, ox, oy, oz; uint32_t nx, ny, nz; };
-// One axis of a ray with a short direction or in a far scene. An infinite o * inv of finite
-// factors would put both planes of every box at the same infinity and cull the boxes that
-// the ray enters: NaN instead, and the axis constrains nothing.
-__device__ __forceinline__ void refine_axis(float o, float d, bool is_short, float& inv, float& oi) {
-    if (is_short) { inv = safe_inv(d); oi = o * inv; }
-    if (isinf(oi) && !isinf(o) && !isinf(inv)) inv = oi = __int_as_float(0x7fffffff);
+// One axis of a ray with a short direction or in a far scene: the reciprocal, a finite one kept
+// where its product with the origin is finite too (else both planes of every box lie at the same
+// infinity and the boxes that the ray enters are culled). At that limit a plane of a box around the
+// origin is still more than 5e32 away: its padding, 2^-19 of the coordinate, times the reciprocal.
+__device__ __forceinline__ float careful_inv(float o, float d, float inv, bool is_short) {
+    if (is_short) inv = safe_inv(d);
+    const float lim = 3e38f * rcp_approx(fabsf(o));
+    return fabsf(inv) > lim && !isinf(inv) ? copysignf(lim, inv) : inv;
 }
 // short_dir: the tree's (rn::short_dir), so a scene with far coordinates costs the others nothing
 // (a test of each origin's size: 0.5 to 1 % of every frame). kUnit: the direction is about of unit
@@ -74,16 +76,16 @@ template <bool kUnit = false>
 __device__ __forceinline__ Inv make_inv(const v3& o, const v3& d, float short_dir) {
     Inv r;
     r.x = inv_clamped(d.x); r.y = inv_clamped(d.y); r.z = inv_clamped(d.z);
-    r.ox = o.x * r.x; r.oy = o.y * r.y; r.oz = o.z * r.z;
     if (!kUnit) {
         const float longest = max3(fabsf(d.x), fabsf(d.y), fabsf(d.z));
         if (!(longest >= short_dir)) {
             const bool is_short = !(longest >= kShortDir);
-            refine_axis(o.x, d.x, is_short, r.x, r.ox);
-            refine_axis(o.y, d.y, is_short, r.y, r.oy);
-            refine_axis(o.z, d.z, is_short, r.z, r.oz);
+            r.x = careful_inv(o.x, d.x, r.x, is_short);
+            r.y = careful_inv(o.y, d.y, r.y, is_short);
+            r.z = careful_inv(o.z, d.z, r.z, is_short);
         }
     }
+    r.ox = o.x * r.x; r.oy = o.y * r.y; r.oz = o.z * r.z;
     r.nx = (__float_as_uint(r.x) >> 31) * 16u;
     r.ny = 32u + (__float_as_uint(r.y) >> 31) * 16u;
     r.nz = 64u + (__float_as_uint(r.z) >> 31) * 16u;
