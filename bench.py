@@ -13,9 +13,9 @@ rasterized on the GPU by this library); no dataset is involved.
            G-buffer crosses from host memory and ao, sky, sun, ss and the error map cross
            back (the library's passes read and write mapped host memory themselves, the
            traversal mirroring the G-buffer into HBM for the SSAO; no copy-engine copy)
-  roofline the traversal kernel (trace_kernel): algorithmic bytes per launch = 4-wide node
-           fetches x 128 B + leaf-triangle fetches x 48 B, from the library's traversal
-           counters over the whole frame, divided by the kernel's CUDA-event time
+  roofline the traversal kernel (trace_kernel), bound by instruction issue: the fraction of cycles
+           that issue (committed ncu capture), beside its launch time and DRAM share; node and
+           triangle fetches are the counting build's, which walks every ray
   cpu_baseline  the oracle (a C restatement of the reference's CPU path) on this host's
            cores, on every 4th row of the same frame
   surrogate_4k  (one GPU) the surrogate-versus-plain-RT head-to-head on the 7.88M-triangle
@@ -302,7 +302,6 @@ def run_ours(args):
     torch.cuda.synchronize()
     trace_ms = e4.elapsed_time(e5) / nvis
     peak, peak_kind = measured_peak()
-    achieved = alg_bytes / (trace_ms * 1e-3) / 1e9
     prof = committed_profile()
     traffic = prof.get("dram_bytes_per_launch")
 
@@ -326,23 +325,21 @@ def run_ours(args):
         "e2e": {"value": world * rays / (e2e_ms * 1e-3) / 1e9, "unit": "Grays/s", "ms_per_step": e2e_ms,
                 "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h, "matches_resident": bool(same)},
         "gpu_launches": 2 * args.steps,
-        "roofline": {"bound": "hbm", "kernel": "trace_kernel", "achieved": achieved, "peak": peak,
-                     "unit": "GB/s", "frac": achieved / peak, "peak_source": peak_kind,
-                     "limit": "instruction issue: the algorithmic node/triangle bytes are those of one walk a ray; "
-                              "most are never fetched (a ray that misses the boxes its packet shares in shared "
-                              "memory takes no walk) and L1/L2 serve the rest (the BVH is cache-resident), so frac "
-                              "can pass 1; dram_frac is the HBM share actually used, issue_active the binding "
-                              "limit's fraction",
-                     "binding_limit": "instruction issue (ncu smsp__issue_active of the same kernel)",
-                     "binding_frac": prof.get("issue_active"),
+        # bound by instruction issue: its fraction comes from the committed ncu capture of the kernel.
+        # The counting build's figures (one walk for every ray, no sieve) stand apart: they are
+        # not this kernel's traffic
+        "roofline": {"bound": "instruction issue", "kernel": "trace_kernel", "achieved": prof.get("issue_active"),
+                     "peak": 1.0, "unit": "of the cycles with an instruction issued", "frac": prof.get("issue_active"),
+                     "peak_source": prof.get("source"), "simt_efficiency": prof.get("simt_efficiency"),
+                     "launch_ms": trace_ms, "traffic": traffic,
+                     "dram_gbs": (traffic / (trace_ms * 1e-3) / 1e9) if traffic else None,
                      "dram_frac": (traffic / (trace_ms * 1e-3) / 1e9 / peak) if traffic else None,
-                     "issue_active": prof.get("issue_active"), "simt_efficiency": prof.get("simt_efficiency"),
-                     "profile_source": prof.get("source"),
-                     "traffic": traffic, "algorithmic_bytes_per_launch": alg_bytes, "launch_ms": trace_ms,
+                     "hbm_peak_gbs": peak, "hbm_peak_source": peak_kind,
                      "rays_per_launch": stats["rays"], "sky_rays_per_launch": stats["sky_rays"],
-                     "walks_per_launch": stats["rays"] + covered,
-                     "node_fetches_per_walk": stats["nodes"] / max(1, stats["rays"] + covered),
-                     "tri_fetches_per_walk": stats["tris"] / max(1, stats["rays"] + covered)},
+                     "one_walk_a_ray": {"walks": stats["rays"] + covered,
+                                        "node_fetches_per_walk": stats["nodes"] / max(1, stats["rays"] + covered),
+                                        "tri_fetches_per_walk": stats["tris"] / max(1, stats["rays"] + covered),
+                                        "node_and_triangle_bytes": alg_bytes}},
         "clocks": clocks,
     }
     if cpu:
