@@ -21,6 +21,8 @@
 // - the horizon integral's cosines come from the horizons' cosines by the addition theorem: of
 //   nine trigonometric calls a slice the three arc cosines are left;
 // - no FP64 (two projections with four divisions and a hypot a slice).
+// Over 44 shapes and 88 G-buffers the mean error against 64 bits is 0.947 to 1.008 times, 0.979 on
+// average, what it was with FP64 projections and IEEE roots and quotients.
 // 2561 x 1441, 16 slices of 16 steps: 12.0 -> 6.2 ms (issue 87 % of cycles, 293.8 M -> 174.9 M warp
 // instructions at 1281 x 721).
 #include "rn_internal.h"
