@@ -229,6 +229,47 @@ __device__ __forceinline__ bool below(const TilePlane& t, float lx, float ly, fl
     return (t.nx != 0.0f || t.ny != 0.0f || t.nz != 0.0f) && t.nx * cx + t.ny * cy + t.nz * cz < t.low - m;
 }
 
+// A node's children in registers, a load for each plane: seven in flight.
+struct NodeChildren {
+    float4 lx, hx, ly, hy, lz, hz;
+    int4 word;
+    __device__ __forceinline__ explicit NodeChildren(const Node4* N) {
+        const float4* q = reinterpret_cast<const float4*>(N);
+        lx = __ldg(q); hx = __ldg(q + 1); ly = __ldg(q + 2); hy = __ldg(q + 3); lz = __ldg(q + 4); hz = __ldg(q + 5);
+        word = __ldg(reinterpret_cast<const int4*>(q + 6));
+    }
+    static __device__ __forceinline__ float at(const float4& v, int k) { return k == 0 ? v.x : k == 1 ? v.y : k == 2 ? v.z : v.w; }
+    __device__ __forceinline__ FrontierBox box(int k) const {
+        return FrontierBox{{at(lx, k), at(ly, k), at(lz, k)}, {at(hx, k), at(hy, k), at(hz, k)},
+                           k == 0 ? word.x : k == 1 ? word.y : k == 2 ? word.z : word.w};
+    }
+};
+// The children of N (a bit each) that overlap Q and are not below the packet's plane. kWide: its
+// planes are fetched together, and an unused slot tells by its word; else each value is fetched
+// when it is needed, in fewer registers. The kernels for few samples are bound by these fetches, a
+// dependent chain for each round, and take the wide form (AO of radius 0.02 at 1920 x 1080, 1
+// sample, 744k triangles 233 -> 202 us, 7.88M 275 -> 240); in the others it cost registers that the
+// walks miss (14 triangles, 3840 x 2160, 256 samples with sky 12.9 -> 13.2 ms).
+template <bool kWide>
+__device__ __forceinline__ unsigned frontier_hits(const Node4* N, const float* qlo, const float* qhi, const TilePlane& pl) {
+    unsigned hit = 0;
+    if (kWide) {
+        const NodeChildren ch(N);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const FrontierBox b = ch.box(k);
+            if (b.word != kNoChild && box_overlaps(b.lo[0], b.lo[1], b.lo[2], b.hi[0], b.hi[1], b.hi[2], qlo, qhi) &&
+                !below(pl, b.lo[0], b.lo[1], b.lo[2], b.hi[0], b.hi[1], b.hi[2]))
+                hit |= 1u << k;
+        }
+    } else {
+        for (int k = 0; k < N->meta[0]; ++k)
+            if (box_overlaps(N->lox[k], N->loy[k], N->loz[k], N->hix[k], N->hiy[k], N->hiz[k], qlo, qhi) &&
+                !below(pl, N->lox[k], N->loy[k], N->loz[k], N->hix[k], N->hiy[k], N->hiz[k]))
+                hit |= 1u << k;
+    }
+    return hit;
+}
 // The warp builds the frontier of box [qlo, qhi] into F (all 32 lanes call it); returns its
 // size (0: start at the root; -1: nothing within reach). Breadth first: each round every entry
 // that is an interior node is replaced by its children that overlap Q and are not below the
@@ -237,6 +278,7 @@ __device__ __forceinline__ bool below(const TilePlane& t, float lx, float ly, fl
 // while the result stays within `cap` entries (kFrontier at most). A round costs one dependent node fetch,
 // so the build takes about the tree's depth in fetch latencies. Up to `tail` greedy steps
 // follow, each replacing the largest interior entry by its children while the frontier fits.
+template <bool kWide>
 __device__ inline int build_frontier(const Node4* __restrict__ nodes, const float* qlo, const float* qhi,
                                      const TilePlane& pl, Node4* F, int cap, int tail) {
     const int lane = (int)(threadIdx.x & 31u);
@@ -247,12 +289,7 @@ __device__ inline int build_frontier(const Node4* __restrict__ nodes, const floa
         const bool mine = lane < n;
         const bool inner = mine && word >= 0;
         const Node4* N = nodes + (inner ? word : 0);
-        unsigned hit = 0;
-        if (inner)
-            for (int k = 0; k < N->meta[0]; ++k)
-                if (box_overlaps(N->lox[k], N->loy[k], N->loz[k], N->hix[k], N->hiy[k], N->hiz[k], qlo, qhi) &&
-                    !below(pl, N->lox[k], N->loy[k], N->loz[k], N->hix[k], N->hiy[k], N->hiz[k]))
-                    hit |= 1u << k;
+        const unsigned hit = inner ? frontier_hits<kWide>(N, qlo, qhi, pl) : 0u;
         const int c = inner ? __popc(hit) : (mine ? 1 : 0);
         int incl = c;
         for (int off = 1; off < 32; off <<= 1) {
@@ -264,8 +301,15 @@ __device__ inline int build_frontier(const Node4* __restrict__ nodes, const floa
         __syncwarp();                       // every lane has read its entry of the last round
         int pos = incl - c;
         if (inner) {
-            for (int k = 0; k < 4; ++k)
-                if (hit & (1u << k)) frontier_put(F, pos++, frontier_child(N, k));
+            if constexpr (kWide) {
+                const NodeChildren ch(N);
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    if (hit & (1u << k)) frontier_put(F, pos++, ch.box(k));
+            } else {
+                for (int k = 0; k < 4; ++k)
+                    if (hit & (1u << k)) frontier_put(F, pos++, frontier_child(N, k));
+            }
         } else if (mine) {
             frontier_put(F, pos, FrontierBox{{lo[0], lo[1], lo[2]}, {hi[0], hi[1], hi[2]}, word});
         }
@@ -290,13 +334,8 @@ __device__ inline int build_frontier(const Node4* __restrict__ nodes, const floa
             if (ob > best || (ob == best && ol < bl)) { best = ob; bl = ol; }
         }
         if (best < 0.0f) break;
-        unsigned hit = 0;
         const Node4* N = nodes + (lane == bl ? word : 0);
-        if (lane == bl)
-            for (int k = 0; k < N->meta[0]; ++k)
-                if (box_overlaps(N->lox[k], N->loy[k], N->loz[k], N->hix[k], N->hiy[k], N->hiz[k], qlo, qhi) &&
-                    !below(pl, N->lox[k], N->loy[k], N->loz[k], N->hix[k], N->hiy[k], N->hiz[k]))
-                    hit |= 1u << k;
+        const unsigned hit = lane == bl ? frontier_hits<kWide>(N, qlo, qhi, pl) : 0u;
         const int c = __popc(__shfl_sync(0xffffffffu, hit, bl));
         if (n - 1 + c > cap) break;
         __syncwarp();
@@ -519,15 +558,17 @@ __device__ __forceinline__ TileBox tile_box(const v3& o, bool covered) {
 // The frontier of the warp's packet for AO walks of `radius` (all 32 lanes call it and build
 // it together). Returns its size, 0: the walks start at the root, -1: no triangle is within
 // reach. Below four samples, four entries for each: a round more costs a dependent fetch whatever
-// the samples that start from it (213k triangles, 1920 x 1080, 1 and 3 samples: 284 -> 218 us with
-// the form for few samples below, 449 -> 430 us; 744k, 4 samples: 16 entries 0.5 % slower than 24).
+// the samples that start from it (213k triangles, 1920 x 1080, radius 3: 1 sample 271 us with 8
+// entries, 264 with 4, 3 samples 562 with 24 and 546 with 12; 7.88M triangles, radius 1, 3 samples
+// the other way, 821 and 852; 4 samples 1040 with 24, 1085 with 12).
+template <bool kWide = false>
 __device__ __forceinline__ int tile_frontier(const TraceParams& p, const TileBox& t, const TilePlane& pl, Node4* F) {
     float lo[3] = {t.lo[0], t.lo[1], t.lo[2]}, hi[3] = {t.hi[0], t.hi[1], t.hi[2]};
     if (lo[0] > hi[0]) return 0;
     // grow by the radius with margin for the rounding of t, |d| and the hit point
     const float g = p.radius * 1.0001f + 1e-5f * (t.mag + 1.0f);
     for (int a = 0; a < 3; ++a) { lo[a] -= g; hi[a] += g; }
-    const int n = build_frontier(p.nodes, lo, hi, pl, F, p.spp < 4 ? 4 * p.spp : kFrontier, p.frontier_tail);
+    const int n = build_frontier<kWide>(p.nodes, lo, hi, pl, F, p.spp < 4 ? 4 * p.spp : kFrontier, p.frontier_tail);
     __syncwarp();
     return n;
 }
@@ -676,7 +717,7 @@ __device__ __forceinline__ void trace_packet(const TraceParams& p, float short_d
     if (p.has_geometry && (near || (!kFew && (p.want_sky || (p.frontier && !kCount))))) {
         const TilePlane pl = tile_plane(n, origin, m != 0, covered);
         const TileBox tb = tile_box(origin, m != 0);
-        fn = near ? tile_frontier(p, tb, pl, F) : root_frontier(p.nodes, pl, F);
+        fn = near ? tile_frontier<kFew>(p, tb, pl, F) : root_frontier(p.nodes, pl, F);
         // the sieve needs normals of about unit length (its rough rays are not normalized) and
         // origins whose products with a reciprocal stay finite (a rough ray off by 1e-5 that stays
         // beyond kFarCoord says nothing of the exact one)
