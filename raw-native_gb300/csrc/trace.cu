@@ -392,6 +392,16 @@ int lanes_log2(const TraceParams& p, long warps) {
     return p.spp >= 16 && r < (p.want_sky ? sky : p.spp >= 32 ? 9.0 : 4.0) ? 1 : 0;
 }
 
+// The samples up to which a packet runs in the form for few (trace_packet). AO from the frontier
+// gains by it for longer than frames with the sky, and most in deep trees, whose rays mostly go on
+// past the sieve (radius 1 at 1920 x 1080, 4 and 8 samples: 744k triangles 773 -> 692 and 1306 ->
+// 1219 us, 7.88M 1135 -> 1039 and 1995 -> 1890; 14 triangles, radius 3, 4 samples 125 -> 120, but 6
+// and 8: 141 -> 149, 156 -> 176).
+int few_spp(const TraceParams& p) {
+    if (p.frontier != FRONTIER_NEAR || p.want_sky) return 2;
+    return p.stack_need >= stack_need(6) ? 8 : 4;              // a tree of six levels and more
+}
+
 // Residency variants: the register budget decides how many 256-thread blocks share an SM
 // (2: up to 128 registers, 3: 80, 4: 64, with spills to L1). The launch uses enough
 // blocks to fill every SM at that residency; ctx().tune.trace_min_blocks picks the variant.
@@ -409,7 +419,7 @@ void launch_variant(const TraceParams& p, int sm_count, cudaStream_t s, uint32_t
         trace_kernel<true, kMB, kStack, false, 0><<<blocks, 256, 0, s>>>(p, tile_ctr, counts, stride < 1 ? 1 : stride);
     else if (pool > 0 && !p.want_sky && p.short_dir == kShortDir)      // no far scene (its make_inv)
         trace_ao_pool_kernel<kMB, kStackN><<<blocks, 256, 0, s>>>(p, tile_ctr, pool, ctx().tune.trace_pool_sort);
-    else if (p.spp <= kFewSpp)
+    else if (p.spp <= few_spp(p))
         trace_kernel<false, kMB, kStackN, true, 0, true><<<blocks, 256, 0, s>>>(p, tile_ctr, nullptr, 1);
     else
         switch (lanes_log2(p, 8L * blocks)) {

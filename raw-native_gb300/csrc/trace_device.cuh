@@ -669,13 +669,13 @@ __device__ __forceinline__ bool walk_starts(const v3& o, const v3& d, float tmax
 // built-in scene at 3840 x 2160, 256 spp with sky 25.4 -> 18.9 ms with exact rays in the sieve,
 // 18.0 -> 13.2 with rough ones; views of 744k triangles within 1 % either way (thresholds of
 // 3/8, 5/8, 8/8: 22.0, 19.2 ms, and views 33.6 ms against 33.1).
-// Few samples (kFew: kFewSpp at most) take none of this: what the packet's rays share then costs
+// Few samples (kFew) take none of this: what the packet's rays share then costs
 // more than it saves (built-in scene with sky, 2561 x 1441, 1 sample 155 -> 136 us; from 3 samples
 // on the sieve is the faster one there). AO walks still start from the frontier.
 // With kP > 0 a packet is 32 >> kP pixels and 1 << kP lanes share each (`part`, the lane's high
 // bits): a part takes a run of the pixel's samples, part 0 the sun as well, and the counts are
 // added up at the end; integers, so the split changes no bit.
-constexpr int kChunk = 64, kSieveNum = 7, kSieveDen = 8, kSieveSkip = 15, kFewSpp = 2;
+constexpr int kChunk = 64, kSieveNum = 7, kSieveDen = 8, kSieveSkip = 15;
 template <bool kCount, int kStackN = kStack, bool kLeafPass = true, int kP = 0, bool kFew = false>
 __device__ __forceinline__ void trace_packet(const TraceParams& p, float short_dir, int x, int y, bool valid,
                                              const v3& toLight, Counts& cn, int& skip, Node4* F, int part = 0) {

@@ -284,3 +284,33 @@ def test_few_samples_against_the_scan(rn, oracle, small, spp):
     finally:
         for k, v in saved.items():
             rn.tune_set(k, v)
+
+
+@pytest.mark.parametrize("spp", [1, 4, 5, 7, 8, 9])
+@pytest.mark.parametrize("boxes", [0, 8, 60, 900])
+def test_few_samples_within_a_short_reach(rn, oracle, boxes, spp):
+    """AO from the frontier at the largest numbers of samples that run without the sieve (4, and 8 in
+    trees of six levels and more) and the smallest beyond, for radii from nothing within reach to
+    the whole scene, nodes of fewer than four children among those fetched: the oracle's AO bit for
+    bit."""
+    import scene as scenes
+    if boxes == 0:
+        sc = scenes.build_test_scene()
+        cam = sc.camera
+    else:
+        sc = scenes.build_synthetic_scene(5, boxes, boxes // 6, grid=20, half=8.0, subdiv=2)
+        cam = (6.0, 4.0, 5.0, 0.0, 0.5, 0.0, 0.0, 1.0, 0.0, 0.9)
+    acc = rn.LinearAccel(sc.tris)
+    _, pos, nrm, mask = oracle.rasterize(sc.tris, sc.normals, cam, 61, 43)
+    g = rn.GBuffer(pos, nrm, mask)
+    keys = ("trace_frontier", "trace_frontier_min_spp")
+    saved = {k: rn.tune_get(k) for k in keys}
+    try:
+        rn.tune_set("trace_frontier", 1)
+        rn.tune_set("trace_frontier_min_spp", 1)
+        for radius in (0.005, 0.05, 0.4, 40.0):
+            want = oracle.trace(pos, nrm, mask, sc.tris, spp, radius, threads=THREADS)
+            assert np.array_equal(rn.compute_rtao(g, acc, spp, radius), want), radius
+    finally:
+        for k, v in saved.items():
+            rn.tune_set(k, v)
