@@ -73,7 +73,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) trace_batch_kernel(const Batc
         const int x = (int)(local % tiles_x) * kTileW + (int)(lane % kTileW);
         const int y = (int)(local / tiles_x) * kTileH + (int)(lane / kTileW);
         const v3 toLight = normalize(mk(p.lx, p.ly, p.lz));
-        trace_dev::trace_packet<false>(p, short_dir, x, y, x < p.w && y < p.h, toLight, cn, skip, F);
+        trace_dev::trace_packet<false, trace_dev::kStack, true, 0, false, true>(p, short_dir, x, y, x < p.w && y < p.h, toLight, cn, skip, F);
         __syncwarp();
     }
 }

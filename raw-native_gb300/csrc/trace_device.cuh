@@ -246,10 +246,11 @@ struct NodeChildren {
 };
 // The children of N (a bit each) that overlap Q and are not below the packet's plane. kWide: its
 // planes are fetched together, and an unused slot tells by its word; else each value is fetched
-// when it is needed, in fewer registers. The kernels for few samples are bound by these fetches, a
-// dependent chain for each round, and take the wide form (AO of radius 0.02 at 1920 x 1080, 1
-// sample, 744k triangles 233 -> 202 us, 7.88M 275 -> 240); in the others it cost registers that the
-// walks miss (14 triangles, 3840 x 2160, 256 samples with sky 12.9 -> 13.2 ms).
+// when it is needed, in fewer registers. Few samples are bound by these fetches, a dependent chain
+// for each round: their kernel takes the wide form (AO of radius 0.02 at 1920 x 1080, 1 sample, 744k
+// triangles 233 -> 202 us, 7.88M 275 -> 240), and so do batches (2560 x 1440 and 1281 x 723, 4
+// samples, 744k triangles 2162 -> 2042 us). In the others it cost registers that the walks miss (14
+// triangles, 3840 x 2160, 256 samples with sky 12.9 -> 13.2 ms).
 template <bool kWide>
 __device__ __forceinline__ unsigned frontier_hits(const Node4* N, const float* qlo, const float* qhi, const TilePlane& pl) {
     unsigned hit = 0;
@@ -676,7 +677,7 @@ __device__ __forceinline__ bool walk_starts(const v3& o, const v3& d, float tmax
 // bits): a part takes a run of the pixel's samples, part 0 the sun as well, and the counts are
 // added up at the end; integers, so the split changes no bit.
 constexpr int kChunk = 64, kSieveNum = 7, kSieveDen = 8, kSieveSkip = 15;
-template <bool kCount, int kStackN = kStack, bool kLeafPass = true, int kP = 0, bool kFew = false>
+template <bool kCount, int kStackN = kStack, bool kLeafPass = true, int kP = 0, bool kFew = false, bool kWide = kFew>
 __device__ __forceinline__ void trace_packet(const TraceParams& p, float short_dir, int x, int y, bool valid,
                                              const v3& toLight, Counts& cn, int& skip, Node4* F, int part = 0) {
     const bool lead = kP == 0 || part == 0;        // writes the pixel
@@ -717,7 +718,7 @@ __device__ __forceinline__ void trace_packet(const TraceParams& p, float short_d
     if (p.has_geometry && (near || (!kFew && (p.want_sky || (p.frontier && !kCount))))) {
         const TilePlane pl = tile_plane(n, origin, m != 0, covered);
         const TileBox tb = tile_box(origin, m != 0);
-        fn = near ? tile_frontier<kFew>(p, tb, pl, F) : root_frontier(p.nodes, pl, F);
+        fn = near ? tile_frontier<kWide>(p, tb, pl, F) : root_frontier(p.nodes, pl, F);
         // the sieve needs normals of about unit length (its rough rays are not normalized) and
         // origins whose products with a reciprocal stay finite (a rough ray off by 1e-5 that stays
         // beyond kFarCoord says nothing of the exact one)
